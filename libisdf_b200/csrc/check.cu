@@ -328,8 +328,9 @@ int check_run(const CheckArgs& args, Arena& arena, cudaStream_t s, double* fit_e
   ISDF_CHECK_LAUNCH();
 
   // (ij|V|kl) = Y Y^T; A = Yz Yz^T; T^T = C^T A; ISDF form = C^T T
-  ISDF_TRY(dgemm_store(npair, npair, (int)(2 * nh), b.Y, npair, b.Y, npair, b.ijkl, npair, s));
-  ISDF_TRY(dgemm_store(rk, rk, (int)(2 * nh), b.Yz, rk, b.Yz, rk, b.aux, rk, s));
+  const size_t nscratch = (size_t)ng * kBatch;  // the transforms are done with rho
+  ISDF_TRY(dsyrk_store(npair, (int)(2 * nh), b.Y, npair, b.ijkl, npair, b.rho, nscratch, s));
+  ISDF_TRY(dsyrk_store(rk, (int)(2 * nh), b.Yz, rk, b.aux, rk, b.rho, nscratch, s));
   ISDF_TRY(dgemm_store(npair, rk, rk, b.C, npair, b.aux, rk, b.Tt, npair, s));
   ISDF_TRY(dgemm_store(npair, npair, rk, b.C, npair, b.Tt, npair, b.cac, npair, s));
   k_diff_norms<<<kDiffBlocks, 256, 0, s>>>(b.ijkl, b.cac, (long long)npair * npair, b.part);
@@ -453,8 +454,9 @@ int check_sampled_run(const CheckArgs& args, const int* pairs, int ns, Arena& ar
     ISDF_CHECK_LAUNCH();
   }
   *fit_err = std::sqrt(fe2) / std::sqrt(fr2);
-  ISDF_TRY(dgemm_store(ns, ns, (int)(2 * nh), b.Y, ns, b.Y, ns, b.E, ns, s));
-  ISDF_TRY(dgemm_store(ns, ns, (int)(2 * nh), b.Yf, ns, b.Yf, ns, b.Ef, ns, s));
+  const size_t nscratch = (size_t)ng * kBatch;  // the transforms are done with rho
+  ISDF_TRY(dsyrk_store(ns, (int)(2 * nh), b.Y, ns, b.E, ns, b.rho, nscratch, s));
+  ISDF_TRY(dsyrk_store(ns, (int)(2 * nh), b.Yf, ns, b.Ef, ns, b.rho, nscratch, s));
   double ce2 = 0, cx2 = 0;
   ISDF_TRY(diff_norms(b.E, b.Ef, (long long)ns * ns, b.part, s, &ce2, &cx2));
   *coul_err = std::sqrt(ce2) / std::sqrt(cx2);
@@ -476,7 +478,7 @@ size_t coulomb_matrix_workspace_bytes(const int* num_grid, int rk) {
   a.take<double>((size_t)ng * kBatch);
   a.take<cufftDoubleComplex>((size_t)nh * kBatch);
   a.take<double>((size_t)nh);
-  a.take<double>((size_t)rk * 2 * nh);
+  a.take<double>((size_t)(rk + (rk & 1)) * 2 * nh);
   return a.off;
 }
 
@@ -488,7 +490,8 @@ int coulomb_matrix_run(const int* num_grid, const double* length, const double* 
   double* buf = arena.take<double>((size_t)ng * kBatch);
   cufftDoubleComplex* spec = arena.take<cufftDoubleComplex>((size_t)nh * kBatch);
   double* sw = arena.take<double>((size_t)nh);
-  double* Yz = arena.take<double>((size_t)rk * 2 * nh);
+  const int ldy = rk + (rk & 1);  // 16-byte aligned rows
+  double* Yz = arena.take<double>((size_t)ldy * 2 * nh);
   if (arena.overflowed()) return record_error(ISDF_ERR_NOMEM, "Coulomb matrix: workspace too small");
   const double vol = length[0] * length[1] * length[2];
   k_weights<<<grid_for(nh, 256), 256, 0, s>>>(nx, ny, nz, length[0], length[1], length[2],
@@ -511,12 +514,12 @@ int coulomb_matrix_run(const int* num_grid, const double* length, const double* 
                                 sizeof(double) * (size_t)(kBatch - bc) * ng, s));
     if (cufftExecD2Z(plan.h, buf, spec) != CUFFT_SUCCESS)
       return record_error(ISDF_ERR_CUDA, "Coulomb matrix: cufftExecD2Z failed");
-    k_spectra_to_rows<<<grid_for(nh * bc, 256), 256, 0, s>>>(spec, nh, bc, sw, c0, rk, Yz);
+    k_spectra_to_rows<<<grid_for(nh * bc, 256), 256, 0, s>>>(spec, nh, bc, sw, c0, ldy, Yz);
   }
   ISDF_CHECK_LAUNCH();
   const long long K = 2 * nh;  // the GEMM's depth is an int
   if (K > (1LL << 30)) return record_error(ISDF_ERR_UNSUPPORTED, "Coulomb matrix: grid too large");
-  return dgemm_store(rk, rk, (int)K, Yz, rk, Yz, rk, d_A, rk, s);
+  return dsyrk_store(rk, (int)K, Yz, ldy, d_A, rk, buf, (size_t)ng * kBatch, s);
 }
 
 }  // namespace isdf_b200

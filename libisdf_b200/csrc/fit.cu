@@ -29,6 +29,7 @@
 // diagonal blocks are inverted explicitly; every other block takes part by
 // substitution, as in a blocked dtrsm.
 // theta is column-major Ng x rk (ld = Ng), overwritten in place.
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -107,6 +108,66 @@ __global__ void __launch_bounds__(WsN::THREADS, 3)
       else *p = *p * v;
     }
   });
+}
+
+// ----------------------------------------------------------- Y Y^T
+// C = Y Y^T (n x n, depth K = columns of Y, K >> n: the spectra of the Coulomb
+// products) on the warp-specialised tile. Bound by the FP64 tensor pipe, so
+// the work is cut to the tiles on and below the diagonal, and since those
+// alone leave most SMs idle (15 tiles at n = 320), each tile's depth is split
+// over gridDim.y CTAs. A split keeps its partial tile in `part` and
+// k_syrk_reduce adds the splits in order (the same bits every run) and
+// mirrors the result. n = 320, K = 67 200: 10.9 ms on 9 full-depth 128 x 128
+// tiles, 0.28 ms here; n = 1024, K = 214 272: 34.3 ms and 7.2 ms (31 TFLOP/s).
+__device__ __forceinline__ void syrk_tile(int t, int* bi, int* bj) {
+  int i = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
+  while ((i + 1) * (i + 2) / 2 <= t) ++i;
+  while (i * (i + 1) / 2 > t) --i;
+  *bi = i;
+  *bj = t - i * (i + 1) / 2;
+}
+
+__global__ void __launch_bounds__(WsN::THREADS, 3)
+    k_syrk_ws(int n, int K, int kper, const double* __restrict__ Y, long long ldy,
+              double* __restrict__ part, int* err) {
+  extern __shared__ __align__(128) double smem[];
+  int bi, bj;
+  syrk_tile(blockIdx.x, &bi, &bj);
+  const int m0 = bi * WsN::BM, n0 = bj * WsN::BN;
+  const int k0 = blockIdx.y * kper, kn = min(kper, K - k0);
+  const int m_rem = min(WsN::BM, n - m0), n_rem = min(WsN::BN, n - n0);
+  WsN tile;
+  // an odd edge copies Y's padding row with it (whatever it holds: it only
+  // reaches the outputs past n, which are not stored)
+  if (!tile.run(smem, Y + m0 + k0 * ldy, ldy, (m_rem + 1) & ~1, Y + n0 + k0 * ldy, ldy,
+                (n_rem + 1) & ~1, kn, err))
+    return;
+  if (WsN::producer()) return;
+  double* out = part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (WsN::BM * WsN::BN);
+  tile.for_each([&](int r, int c, double v) { out[c * WsN::BM + r] = v; });
+}
+
+__global__ void __launch_bounds__(256) k_syrk_reduce(int n, int splits,
+                                                     const double* __restrict__ part,
+                                                     double* __restrict__ C, long long ldc,
+                                                     const int* __restrict__ err) {
+  // a pipeline wait ran out: the result says so itself (nothing is read back)
+  const bool bad = *err != 0;
+  constexpr int kTileN = WsN::BM * WsN::BN;
+  int bi, bj;
+  syrk_tile(blockIdx.x, &bi, &bj);
+  for (int e = threadIdx.x + blockIdx.y * 256; e < kTileN; e += 256 * gridDim.y) {
+    const double* p = part + (size_t)blockIdx.x * kTileN + e;
+    double v = 0.0;
+#pragma unroll 8
+    for (int s = 0; s < splits; ++s) v += p[(size_t)s * gridDim.x * kTileN];
+    const int r = bi * WsN::BM + e % WsN::BM, c = bj * WsN::BN + e / WsN::BM;
+    if (bad) v = __longlong_as_double(0x7ff8000000000000LL);
+    if (r < n && c < n && r >= c) {
+      C[r + c * ldc] = v;
+      C[c + r * ldc] = v;
+    }
+  }
 }
 
 // ----------------------------------------------------------- gathers
@@ -407,6 +468,7 @@ int set_smem_attrs() {
   ISDF_TRY(set_attr(k_chol_panel<2>, CoreN::SMEM_BYTES));
   ISDF_TRY(set_attr(k_trsm_gemm<1>, CoreN::SMEM_BYTES));
   ISDF_TRY(set_attr(k_trsm_ws, WsN::SMEM_BYTES));
+  ISDF_TRY(set_attr(k_syrk_ws, WsN::SMEM_BYTES));
   ISDF_TRY(set_attr(k_gemm_zws<0>, WsN::SMEM_BYTES));
   ISDF_TRY(set_attr(k_gemm_zws<1>, WsN::SMEM_BYTES));
   ISDF_TRY(set_attr(k_gemm_zws<2>, WsN::SMEM_BYTES));
@@ -455,6 +517,52 @@ int dgemm_store(int M, int N, int K, const double* A, long long lda, const doubl
     k_gemm_z<1, 2><<<g, 256, CoreZ::SMEM_BYTES, s>>>(M, N, K, A, lda, B, ldb, C, ldc);
   else
     k_gemm_z<1, 1><<<g, 256, CoreZ::SMEM_BYTES, s>>>(M, N, K, A, lda, B, ldb, C, ldc);
+  ISDF_CHECK_LAUNCH();
+  return ISDF_OK;
+}
+
+// Splits of the depth of Y Y^T. All CTAs take the same time, so what counts is
+// how full the last wave of three CTAs per SM is: the fewest waves from three
+// to six that leave at most 3 % of the slots idle (a single wave has no slack
+// for CTAs that run at different speeds: n = 320 took 309 us in one wave, 264
+// in four), a CTA walking at least 256 columns,
+// within what `cap` doubles of scratch hold.
+static int syrk_splits(int tiles, int K, size_t cap) {
+  const int slots = 3 * kNumSMs;
+  const long long most = std::min<long long>(
+      std::min<long long>((K + 255) / 256, 65535),
+      (long long)(cap / ((size_t)tiles * WsN::BM * WsN::BN)));
+  long long best = 1;
+  double best_fill = 0.0;
+  for (int waves = 3; waves <= 6 && best_fill < 0.97; ++waves) {
+    const long long s = std::max<long long>(1, (long long)waves * slots / tiles);
+    const long long w = (s * tiles + slots - 1) / slots;
+    const double fill = (double)(s * tiles) / (double)(w * slots);
+    if (fill > best_fill) {
+      best_fill = fill;
+      best = s;
+    }
+  }
+  return (int)std::min(best, most);
+}
+
+int dsyrk_store(int n, int K, const double* Y, long long ldy, double* C, long long ldc,
+                double* scratch, size_t scratch_doubles, cudaStream_t s) {
+  const int nb = (n + WsN::BM - 1) / WsN::BM, tiles = nb * (nb + 1) / 2;
+  // one double of the scratch holds the pipeline's error flag
+  const size_t cap = scratch_doubles > 0 ? scratch_doubles - 1 : 0;
+  int splits = syrk_splits(tiles, K, cap);
+  if (!vec2_ok(Y, ldy, Y, ldy) || ldy < n + (n & 1) || splits < 1)
+    return dgemm_store(n, n, K, Y, ldy, Y, ldy, C, ldc, s);
+  ISDF_TRY(set_smem_attrs());
+  // whole pipeline stages per split
+  const int kper = ((K + splits - 1) / splits + WsN::BK - 1) / WsN::BK * WsN::BK;
+  splits = (K + kper - 1) / kper;
+  int* err = reinterpret_cast<int*>(scratch + cap);
+  ISDF_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+  k_syrk_ws<<<dim3(tiles, splits), WsN::THREADS, WsN::SMEM_BYTES, s>>>(n, K, kper, Y, ldy, scratch,
+                                                                       err);
+  k_syrk_reduce<<<dim3(tiles, 16), 256, 0, s>>>(n, splits, scratch, C, ldc, err);
   ISDF_CHECK_LAUNCH();
   return ISDF_OK;
 }

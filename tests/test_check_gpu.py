@@ -137,3 +137,23 @@ def test_coulomb_matrix_matches_oracle(torch_cuda, name):
     record_parity(f"Coulomb matrix {name}", "relative difference vs oracle", err, 1e-10)
     assert err <= 1e-10
     assert np.allclose(A, A.T, rtol=0, atol=1e-12 * np.abs(A).max())
+
+
+@pytest.mark.parametrize("rk", [1, 2, 63, 64, 65, 130, 321])
+@pytest.mark.parametrize("ng", [(14, 12, 10), (9, 15, 25)])
+def test_coulomb_matrix_tile_edges(torch_cuda, rk, ng):
+    """Around the 64-wide tiles of the symmetric product, odd and even sizes,
+    depths that split unevenly. The product sums 2 nh terms: its rounding is at
+    most that many half ulps of the norms."""
+    torch = torch_cuda
+    ln = (7.0, 8.0, 9.0)
+    n = ng[0] * ng[1] * ng[2]
+    th = np.asfortranarray(np.random.default_rng(rk).standard_normal((n, rk)))
+    d_th = torch.from_numpy(np.ascontiguousarray(th.T)).cuda()
+    d_A = torch.full((rk, rk), float("nan"), dtype=torch.float64, device="cuda")
+    isdf.coulomb_matrix(isdf.Domain(length=ln, num_grid=ng), d_th, rk, d_A)
+    torch.cuda.synchronize()
+    A, A_o = d_A.cpu().numpy().T, ocheck.coulomb_matrix(th, ng, ln, rk)
+    tol = 2 * (ng[0] // 2 + 1) * ng[1] * ng[2] * 2.0 ** -53
+    assert np.linalg.norm(A - A_o) <= tol * np.linalg.norm(A_o)
+    assert np.array_equal(A, A.T)
