@@ -818,24 +818,34 @@ __global__ void __launch_bounds__(128) k_scatter(const int* __restrict__ label, 
   }
 }
 
+// 2^e for a normal power of two.
+__device__ __forceinline__ double pow2_bits(int e) {
+  return __longlong_as_double((long long)(e + 1023) << 52);
+}
+
 // m successive round-to-nearest additions acc <- fl(acc + c), acc >= 0,
 // c >= 0, with the exact result of the sequential loop. While acc stays in
 // one binade [2^e, 2^(e+1)) every addition adds the same number of ulps
 // (c rounded to the ulp grid), unless c's remainder is exactly half an ulp
 // (a tie, which depends on acc's parity): those steps, binade crossings and
-// subnormal accumulators are taken one at a time; the rest are jumped.
+// accumulators outside [2^-900, 2^900] (where the scaling by the ulp would
+// not be exact) are taken one at a time; the rest are jumped. One thread runs
+// it on the critical path of its cluster, so the scaling is by powers of two
+// built from the exponent bits: the library's ilogb and ldexp and two
+// divisions per binade took most of the 52 us of a fold with a 5551-point
+// zero tail.
 __device__ double repeat_add(double acc, double c, long long m) {
   const double two53 = 9007199254740992.0;
   while (m > 0) {
     if (c == 0.0) return radd(acc, 0.0);
-    if (!(acc >= 2.2250738585072014e-308) || c >= ldexp(1.0, ilogb(acc))) {
+    const int e = (int)((__double_as_longlong(acc) >> 52) & 0x7ff) - 1023;
+    if (e < -900 || e > 900 || c >= pow2_bits(e)) {
       acc = radd(acc, c);
       --m;
       continue;
     }
-    const int e = ilogb(acc);
-    const double u = ldexp(1.0, e - 52);  // ulp of acc
-    const double cu = c / u;              // exact: u is a power of two
+    const double inv = pow2_bits(52 - e);  // 1 / ulp of acc
+    const double cu = c * inv;             // exact: a power of two
     const double q = floor(cu);
     const double r = cu - q;
     if (r == 0.5) {
@@ -845,7 +855,7 @@ __device__ double repeat_add(double acc, double c, long long m) {
     }
     const double qp = q + (r > 0.5 ? 1.0 : 0.0);  // ulps added per step
     if (qp == 0.0) return acc;  // c rounds away now and at every larger exponent
-    const double a = acc / u;   // integer in [2^52, 2^53)
+    const double a = acc * inv;  // integer in [2^52, 2^53)
     const double room = two53 - q - 2.0 - a;
     if (room < 0.0) {
       acc = radd(acc, c);
@@ -854,95 +864,146 @@ __device__ double repeat_add(double acc, double c, long long m) {
     }
     long long k = (long long)floor(room / qp) + 1;
     if (k > m) k = m;
-    acc = __dmul_rn(__dadd_rn(a, __dmul_rn((double)k, qp)), u);  // all exact
+    acc = __dmul_rn(__dadd_rn(a, __dmul_rn((double)k, qp)), pow2_bits(e - 52));  // all exact
     m -= k;
   }
   return acc;
 }
 
-// One warp per cluster: sequential fold over the members (in index order).
-// The zero-tail points p >= npt are identical copies of grid point 0 (weight
-// w[0], coordinates (0, 0, 0)) and come last in their cluster's member list,
-// so their part of the fold is a repeated addition of one value. The members'
-// (w x, w y, w z, w) are read contiguously, kSegBatches batches of 32 ahead
-// of the fold, so that the load latency hides behind the dependent additions.
-constexpr int kSegBatches = 4;
+// The fold of a cluster: acc <- fl(acc + v) over its members in index order
+// (utility.cpp:816-822), one addition after the other, so the largest
+// cluster's chain of dependent additions (8.5 cycles each) bounds the kernel.
+// Once the sum is large against its members the chain is cut where its result
+// is known without it: while acc stays in one binade [2^e, 2^(e+1)), an
+// addition of v >= 0 adds RN(v), v rounded to the multiple of acc's ulp u,
+// whatever acc is (unless v lies exactly half way between two multiples, where
+// acc's parity decides), and sums of such multiples below 2^53 u are exact in
+// any order. A warp then takes kFoldBatch members at once: each lane rounds
+// its own, and one addition of their exact total finishes the lot if acc
+// stays in its binade. A batch with a crossing, a tie, or a member too large
+// (or negative by more than the rounding error of a coordinate) is added one
+// by one. About one member in n ties and every doubling of n crosses, so below
+// kFoldSerial members most batches would fail: those are always added one by
+// one. (A prefix sum up to the first such member instead of the one-by-one
+// batch took 6000 to 8000 cycles a batch, against 2200.)
+constexpr int kFoldRows = 8;
+constexpr int kFoldBatch = 32 * kFoldRows;  // members per step
+constexpr int kFoldSerial = 1024;           // members always added one by one
 
-__device__ __forceinline__ void seg_load(const double4* __restrict__ v, int q, int m, int lane,
-                                         double4 (&out)[kSegBatches]) {
+// acc + the batch held by the warp (v[j] of lane l is member j * 32 + l, zero
+// past the end) where the exact total settles it; false and acc unchanged
+// otherwise.
+__device__ __forceinline__ bool fold_batch(const double (&v)[kFoldRows], double* acc) {
+  const int e = (int)((__double_as_longlong(*acc) >> 52) & 0xfff) - 1023;  // sign in: e > 1023
+  if (e < -900 || e > 900) return false;
+  const double top = pow2_bits(e - 1);   // larger members would change magic's ulp
+  const double neg = -pow2_bits(e - 54);  // a quarter ulp off leaves even the binade's start
+  const double half_u = pow2_bits(e - 53), magic = 1.5 * pow2_bits(e);
+  double sum = 0.0;
+  bool bad = false;
 #pragma unroll
-  for (int j = 0; j < kSegBatches; ++j) {
-    const int i = q + j * 32 + lane;
-    out[j] = i < m ? v[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+  for (int j = 0; j < kFoldRows; ++j) {
+    const double q = __dsub_rn(__dadd_rn(magic, v[j]), magic);  // RN(v) to a multiple of u
+    bad |= !(v[j] > neg && v[j] < top) || fabs(__dsub_rn(v[j], q)) == half_u;
+    sum = __dadd_rn(sum, q);
   }
+  if (__any_sync(0xffffffffu, bad)) return false;
+  for (int o = 16; o > 0; o >>= 1) sum = __dadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, o));
+  const double next = __dadd_rn(*acc, sum);
+  if (!(next < pow2_bits(e + 1))) return false;
+  *acc = next;
+  return true;
 }
 
+// acc + the first cnt members of the batch one by one, from the warp's copy in
+// shared memory (a broadcast load per member; by shuffles the chain took 40 %
+// longer), the next 16 loaded while 16 are added.
+__device__ __forceinline__ double fold_serial(const double* comp, int cnt, double acc) {
+  double x[16], y[16];
+  int e = 0;
+  if (cnt >= 16) {
+#pragma unroll
+    for (int u = 0; u < 16; ++u) x[u] = comp[u];
+    for (; e + 32 <= cnt; e += 16) {
+#pragma unroll
+      for (int u = 0; u < 16; ++u) y[u] = comp[e + 16 + u];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) acc = radd(acc, x[u]);
+#pragma unroll
+      for (int u = 0; u < 16; ++u) x[u] = y[u];
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) acc = radd(acc, x[u]);
+    e += 16;
+  }
+  for (; e < cnt; ++e) acc = radd(acc, comp[e]);
+  return acc;
+}
+
+// One block per cluster, one warp per component (w x, w y, w z, w), each by
+// itself: the components reach their crossings and ties at different members,
+// and a block that stages the members for all four would wait for the slowest
+// in every batch. The next batch is loaded while one is folded. The zero-tail
+// points p >= npt are identical copies of grid point 0 (weight w[0],
+// coordinates (0, 0, 0)) and come last in their cluster's member list, so
+// their part of the fold is a repeated addition of one value (repeat_add).
 // n, npt: the points folded and how many of them are kept points (the rest
 // is zero tail); flag_empty: record an empty cluster in st (off when the sums
 // are one rank's partial sums).
-__global__ void __launch_bounds__(256) k_segsum(const double4* __restrict__ sorted,
-                                                const int* __restrict__ start,
-                                                const int* __restrict__ members,
-                                                const double* __restrict__ px,
-                                                const double* __restrict__ py,
-                                                const double* __restrict__ pz,
-                                                const double* __restrict__ pw,
-                                                const int* __restrict__ label, int n, int npt,
-                                                int flag_empty, KmState* st,
-                                                double4* __restrict__ sums) {
+constexpr int kFoldThreads = 128;
+
+__global__ void __launch_bounds__(kFoldThreads) k_segsum(
+    const double4* __restrict__ sorted, const int* __restrict__ start,
+    const int* __restrict__ members, const double* __restrict__ px, const double* __restrict__ py,
+    const double* __restrict__ pz, const double* __restrict__ pw, const int* __restrict__ label,
+    int n, int npt, int flag_empty, KmState* st, double4* __restrict__ sums) {
   if (st->done) return;
-  const int rk = st->rk;
-  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (c >= rk) return;
-  const double4* v = sorted + start[c];
+  // the clusters that started as the last points of the list reach over the
+  // rest of the box and stay the largest: first come, so that their folds do
+  // not start in a second wave of blocks
+  const int c = gridDim.x - 1 - blockIdx.x;
+  if (c >= st->rk) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double* v = reinterpret_cast<const double*>(sorted + start[c]) + warp;
   int m = members[c];
   long long tail = 0;
   if (npt < n && label[npt] == c) {
     tail = n - npt;
     m -= (int)tail;
   }
-  // lanes 0..3 each fold one component (w x, w y, w z, w) from the warp's
-  // shared-memory copy of the batch: one load and one dependent addition per
-  // member instead of four broadcasts and four additions
-  __shared__ double4 stage[8][32 * kSegBatches];
-  double4* st_w = stage[threadIdx.x >> 5];
-  double acc = 0.0;
-  double4 cur[kSegBatches], nxt[kSegBatches];
-  seg_load(v, 0, m, lane, cur);
-  for (int q = 0; q < m; q += 32 * kSegBatches) {
+  double cur[kFoldRows], nxt[kFoldRows];
+  auto load = [&](int q, double (&out)[kFoldRows]) {
 #pragma unroll
-    for (int j = 0; j < kSegBatches; ++j) st_w[j * 32 + lane] = cur[j];
-    __syncwarp();
-    if (q + 32 * kSegBatches < m) seg_load(v, q + 32 * kSegBatches, m, lane, nxt);
-    const int cnt = min(32 * kSegBatches, m - q);
-    if (lane < 4) {
-      const double* comp = reinterpret_cast<const double*>(st_w) + lane;
-      int e = 0;
-      for (; e + 8 <= cnt; e += 8) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) acc = radd(acc, comp[(e + u) * 4]);
-      }
-      for (; e < cnt; ++e) acc = radd(acc, comp[e * 4]);
+    for (int j = 0; j < kFoldRows; ++j) {
+      const int e = q + j * 32 + lane;
+      out[j] = e < m ? v[(size_t)e * 4] : 0.0;
     }
-    __syncwarp();
+  };
+  __shared__ double stage[kFoldThreads / 32][kFoldBatch];
+  double* comp = stage[warp];
+  double acc = 0.0;
+  load(0, nxt);
+  for (int q = 0; q < m; q += kFoldBatch) {
 #pragma unroll
-    for (int j = 0; j < kSegBatches; ++j) cur[j] = nxt[j];
+    for (int j = 0; j < kFoldRows; ++j) cur[j] = nxt[j];
+    if (q + kFoldBatch < m) load(q + kFoldBatch, nxt);
+    if (q < kFoldSerial || !fold_batch(cur, &acc)) {
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < kFoldRows; ++j) comp[j * 32 + lane] = cur[j];
+      __syncwarp();
+      acc = fold_serial(comp, min(kFoldBatch, m - q), acc);
+    }
   }
-  double ax = __shfl_sync(0xffffffffu, acc, 0);
-  double ay = __shfl_sync(0xffffffffu, acc, 1);
-  double az = __shfl_sync(0xffffffffu, acc, 2);
-  double aw = __shfl_sync(0xffffffffu, acc, 3);
   if (lane == 0) {
     if (tail) {
       const double w0 = pw[npt];
-      aw = repeat_add(aw, w0, tail);
-      ax = repeat_add(ax, rmul(w0, px[npt]), tail);
-      ay = repeat_add(ay, rmul(w0, py[npt]), tail);
-      az = repeat_add(az, rmul(w0, pz[npt]), tail);
+      const double one = warp == 3 ? w0
+                                   : rmul(w0, warp == 0 ? px[npt] : warp == 1 ? py[npt] : pz[npt]);
+      acc = repeat_add(acc, one, tail);
     }
-    sums[c] = make_double4(ax, ay, az, aw);
-    if (flag_empty && aw == 0.0) st->any_empty = 1;
+    reinterpret_cast<double*>(sums + c)[warp] = acc;
+    if (flag_empty && warp == 3 && acc == 0.0) st->any_empty = 1;
   }
 }
 
@@ -1552,7 +1613,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
       k_label_start<<<1, 1024, 0, stream>>>(b.members, b.st, b.start);
       k_scatter<<<ntiles, 128, scatter_smem, stream>>>(b.label, n, b.st, b.hist, b.start, b.px,
                                                        b.py, b.pz, b.pw, b.sorted);
-      k_segsum<<<grid_for(mu, 8), 256, 0, stream>>>(b.sorted, b.start, b.members, b.px, b.py,
+      k_segsum<<<mu, kFoldThreads, 0, stream>>>(b.sorted, b.start, b.members, b.px, b.py,
                                                     b.pz, b.pw, b.label, n, npt, 1, b.st, b.sums);
       k_centroids<<<1, 1024, cmax_smem, stream>>>(b.sums, b.st, b.cen, b.shift, b.cell_of, cg,
                                                   b.nbshift);
@@ -1584,7 +1645,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
       k_scatter<<<ntl, 128, scatter_smem, stream>>>(b.label + lo, cnt, b.st, b.hist, b.start,
                                                     b.px + lo, b.py + lo, b.pz + lo, b.pw + lo,
                                                     b.sorted);
-      k_segsum<<<grid_for(mu, 8), 256, 0, stream>>>(b.sorted, b.start, b.members, b.px + lo,
+      k_segsum<<<mu, kFoldThreads, 0, stream>>>(b.sorted, b.start, b.members, b.px + lo,
                                                     b.py + lo, b.pz + lo, b.pw + lo, b.label + lo,
                                                     cnt, npt_loc, 0, b.st, sb.send + 1);
       k_shard_header<<<1, 1, 0, stream>>>(b.st, sb.send);

@@ -226,3 +226,30 @@ def test_batched_selection_matches_reference(torch_cuda):
     for k, ((piv, rk, it, _), (wp, wr_, wi)) in enumerate(zip(got, want)):
         assert (rk, it) == (wr_, wi), k
         assert np.array_equal(piv, wp), k
+
+
+@pytest.mark.parametrize("kind", ["ties", "binades", "flat", "plane"])
+@pytest.mark.parametrize("length", [(20.0, 20.0, 20.0), (10.26, 9.7, 11.3)])
+def test_select_long_folds_match_oracle(torch_cuda, kind, length):
+    """Clusters of up to thousands of points, whose weighted sums must round as
+    the one-by-one fold does: weights that tie with the sums' last place, that
+    span the kept range, that are all equal, and points in one plane (sums of
+    zeros); exact integer coordinates and rounded ones."""
+    torch = torch_cuda
+    ng = (20, 21, 1 if kind == "plane" else 20)
+    n = ng[0] * ng[1] * ng[2]
+    rng = np.random.default_rng(7)
+    if kind == "ties":
+        w = rng.integers(1, 1 << 12, n) * 2.0 ** rng.integers(-20, 0, n) + 2.0 ** -31
+    elif kind == "binades":
+        w = np.exp(rng.uniform(np.log(2e-8), 0.0, n))
+    else:
+        w = np.full(n, 0.7)
+    w[rng.integers(0, n, n // 9)] = 0.0  # dropped by the filter: a zero tail
+    w[0] = 0.3
+    for mu in (3, 24):
+        piv_o, rk_o, it_o = port.kmeans(w, ng, length, mu, 40)
+        piv, rk, it, _ = isdf.kmeans_select(isdf.Domain(length=length, num_grid=ng),
+                                            torch.from_numpy(w).cuda(), mu, 40, rand_seed=1)
+        assert (rk, it) == (rk_o, it_o)
+        assert np.array_equal(piv, piv_o)
