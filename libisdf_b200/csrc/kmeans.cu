@@ -233,18 +233,18 @@ __global__ void k_warm_centroids(const int* __restrict__ cinit, int rk, int nx, 
 // d = ((dx*dx + dy*dy) + dz*dz) with dx = point - centroid (pdist2,
 // utility.cpp:598-615); label = first centroid reaching the minimum
 // (findMin Dim=1, utility.cpp:579-595).
-constexpr int kAssignThreads = 256;
+constexpr int kAssignThreads = 128;
 
 // ---------------------------------------------------------------- pruned assign
 // Exact spatial pruning: centroids are binned into a uniform nc^3 cell grid
-// over the box; a point visits cells in Chebyshev rings around its own cell
-// and skips a cell only when the squared distance from the point to the
-// cell's box, shrunk by a relative 2e-14 safety factor (well above the
-// rounding of both the box bound and the distance formula), is strictly
-// greater than the best distance found. Every skipped centroid would have
-// computed a strictly larger distance, so the result - the first centroid in
-// index order reaching the minimum computed distance, compared as (d, index)
-// pairs - is the brute-force result bit for bit.
+// over the box, and a search leaves out a cell only when the squared distance
+// from the points to the cell's box (widened by tol), shrunk by a relative
+// 2e-14 safety factor (well above the rounding of both the box bound and the
+// distance formula), is strictly greater than a distance already found. Every
+// centroid left out would have computed a strictly larger distance, so the
+// result - the first centroid in index order reaching the minimum computed
+// distance, compared as (d, index) pairs - is the brute-force result bit for
+// bit.
 struct CellGrid {
   int nc;
   double h[3];
@@ -381,84 +381,11 @@ __device__ __forceinline__ double ref_dist2(double x, double y, double z, const 
 // margin far above the relative error of the rounded squared distances
 // (~1e-15), so the reference's argmin (first minimum of the rounded
 // distances) is the assigned label and the search is skipped. Otherwise the
-// exact ring search runs and the bounds are rebuilt from it: u from the
-// best distance, l from the second best seen, the box bounds of skipped
-// cells and the ring at which the search stopped.
+// search runs and the bounds are rebuilt from it: u from the best distance, l
+// from the second best seen and the radius searched.
 constexpr double kBoundMargin = 1.0 + 1e-12;
 constexpr double kRoundUp = 1.0 + 1e-13;
 constexpr double kRoundDown = 1.0 - 1e-13;
-
-// Exact ring search for the nearest centroid of (x, y, z) (first minimum of
-// the reference's rounded distances), seeded with centroid `old` when it is
-// valid; writes the point's distance bounds and returns the label.
-__device__ __forceinline__ int ring_search(double x, double y, double z, int old, int rk,
-                                           const double4* __restrict__ cen,
-                                           const int* __restrict__ cell_start,
-                                           const double4* __restrict__ cell_cen,
-                                           const CellGrid& g, double2* bnd_p) {
-  const double inf = __longlong_as_double(0x7ff0000000000000LL);
-  double best = inf;
-  int bj = 0x7fffffff;
-  if (old >= 0 && old < rk) {  // any centroid is a valid start
-    best = ref_dist2(x, y, z, cen[old]);
-    bj = old;
-  }
-  const int pi = min(g.nc - 1, max(0, (int)floor(x / g.h[0])));
-  const int pj = min(g.nc - 1, max(0, (int)floor(y / g.h[1])));
-  const int pk = min(g.nc - 1, max(0, (int)floor(z / g.h[2])));
-  double second = inf;  // second-best squared distance seen
-  double floor2 = inf;  // lower bound (squared) on every centroid not seen
-  const double hmin = fmin(g.h[0], fmin(g.h[1], g.h[2]));
-  const double shrink = 1.0 - 2e-14;
-  for (int r = 0; r <= g.nc; ++r) {
-    if (r >= 2) {
-      const double lb = (r - 1) * hmin - g.tol;
-      if (lb > 0.0 && lb * lb * shrink > best) {
-        floor2 = fmin(floor2, lb * lb * shrink);
-        break;
-      }
-    }
-    for (int dk = -r; dk <= r; ++dk) {
-      const int ck = pk + dk;
-      if (ck < 0 || ck >= g.nc) continue;
-      for (int dj = -r; dj <= r; ++dj) {
-        const int cj = pj + dj;
-        if (cj < 0 || cj >= g.nc) continue;
-        for (int di = -r; di <= r; ++di) {
-          if (max(abs(di), max(abs(dj), abs(dk))) != r) continue;
-          const int ci = pi + di;
-          if (ci < 0 || ci >= g.nc) continue;
-          // box lower bound (box widened by tol)
-          const double bx = fmax(0.0, fmax(ci * g.h[0] - g.tol - x, x - (ci + 1) * g.h[0] - g.tol));
-          const double by = fmax(0.0, fmax(cj * g.h[1] - g.tol - y, y - (cj + 1) * g.h[1] - g.tol));
-          const double bz = fmax(0.0, fmax(ck * g.h[2] - g.tol - z, z - (ck + 1) * g.h[2] - g.tol));
-          const double lb = bx * bx + by * by + bz * bz;
-          if (lb * shrink > best) {
-            floor2 = fmin(floor2, lb * shrink);
-            continue;
-          }
-          const int id = ci + g.nc * (cj + g.nc * ck);
-          const int e = cell_start[id + 1];
-          for (int q = cell_start[id]; q < e; ++q) {
-            const double4 c = cell_cen[q];
-            const double d = ref_dist2(x, y, z, c);
-            const int j = (int)c.w;
-            if (d < best || (d == best && j < bj)) {
-              if (j != bj) second = best;
-              best = d;
-              bj = j;
-            } else if (j != bj) {
-              second = fmin(second, d);
-            }
-          }
-        }
-      }
-    }
-  }
-  *bnd_p = make_double2(__dmul_ru(__dsqrt_ru(best), kRoundUp),
-                        __dmul_rd(__dsqrt_rd(fmin(second, floor2)), kRoundDown));
-  return bj;
-}
 
 // Per point, once per selection (the points do not move): its cell and the
 // distances from it to the outside of the 3^3 and 5^3 cell blocks around it
@@ -496,16 +423,30 @@ __global__ void k_point_cells(const double* __restrict__ px, const double* __res
 // (or 32 consecutive points), so the points of a warp that fail the bound
 // test share their candidates: with U the largest of their seed distances
 // (squared distance to the old label, which bounds each one's nearest), every
-// centroid that can be nearest to one of them lies in a cell whose box is
-// within sqrt(U) of the points' bounding box. The warp stages those cells'
-// centroids in shared memory once and every searching lane runs the same loop
-// over them, comparing (d, index) pairs as the ring search does: the label is
-// the ring search's bit for bit. Centroids not staged are more than sqrt(U)
-// from every point of the box, which gives the lower bound. Lanes without a
-// seed (the first assignment), more than 216 cells or more than 160 candidates take the
-// ring search instead.
-constexpr int kWarpCand = 160;   // centroids staged per warp
-constexpr int kWarpCells = 216;  // cells a warp may scan
+// centroid that can be nearest to one of them lies within sqrt(U) of the
+// points' bounding box. The cells of one (y, z) row are contiguous in cell
+// order, so the lanes take a row each, then the rows' centroids 32 at a time:
+// those within sqrt(U) of the box go to shared memory as single-precision
+// offsets from the box's centre, kWarpCand at most before they are scanned
+// (any number of cells and candidates is taken in such portions).
+// The scan keeps the two smallest single-precision distances per point. Their
+// error against the exact distance is below err = 2^-19 (sqrt(U) + h)^2, h the
+// box's half diagonal (three offsets rounded to 24 bits on either side, their
+// difference, and the sum of squares: 2^-20 with the worst signs), so when the
+// second is more than 2 err above the first, the first is the only candidate
+// that can be the portion's nearest, and its distance alone is computed in the
+// reference's rounding; otherwise every candidate within 2 err of the smallest
+// is. Distances so computed are compared as (d, index) pairs: the label is
+// brute force's bit for bit. All other candidates are farther than the second
+// smallest less err, and centroids not staged farther than sqrt(U): the lower
+// bound.
+// What this replaced: FP64 distances to every candidate, and a per-point search
+// in rings of cells where a warp had more than 216 cells or 160 candidates (a
+// few warps in the sparse regions, which the launch then waited for) or, in the
+// first assignment, no seed. A launch late in a selection: 64 000 points and
+// 309 centroids 47 -> 10 us, 151 875 and 505 68 -> 19 us, 884 736 and 2979
+// 140 -> 72 us; the first assignment of the last 9200 -> 510 us.
+constexpr int kWarpCand = 128;   // candidates staged per warp
 
 __device__ __forceinline__ double warp_max(double v) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -516,15 +457,36 @@ __device__ __forceinline__ double warp_min(double v) {
   return v;
 }
 
+// A seed for the first assignment. The centroids start at the first rk points
+// of the list, which fill the lowest planes and rows of the box: the nearest
+// is above, below or beside the point itself. (Any centroid is a valid seed.)
+__device__ __forceinline__ int first_seed(int p, int rk, const int* __restrict__ pidx,
+                                          const AssignMap& am) {
+  if (p < rk) return p;
+  if (!am.brick) return rk - 1;
+  const int t = pidx[p], last = pidx[rk - 1], plane = am.nx * am.ny;
+  int g = t % plane;                  // the point's column in the lowest plane
+  const int top = last / plane;       // the plane the centroids end in
+  if (top > 0) {
+    g += (g + top * plane <= last ? top : top - 1) * plane;
+  } else if (g > last) {              // beyond the rows they cover
+    const int row = last / am.nx;
+    g = g % am.nx + am.nx * (row > 0 ? row - 1 : 0);
+    if (g > last) g = last;
+  }
+  const int j = am.g2p ? am.g2p[g] : g;
+  return j >= 0 && j < rk ? j : rk - 1;
+}
+
 __global__ void __launch_bounds__(kAssignThreads) k_assign_warp(
     const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
-    int n, const double4* __restrict__ cen, const int* __restrict__ cell_start,
-    const double4* __restrict__ cell_cen, CellGrid g, AssignMap am, KmState* st,
-    int* __restrict__ label, int count, double2* __restrict__ bnd,
+    const int* __restrict__ pidx, int n, const double4* __restrict__ cen,
+    const int* __restrict__ cell_start, const double4* __restrict__ cell_cen, CellGrid g,
+    AssignMap am, KmState* st, int* __restrict__ label, int count, double2* __restrict__ bnd,
     const double* __restrict__ shift, const float* __restrict__ nbshift,
     const int* __restrict__ pcell, const double2* __restrict__ pd12) {
   if (st->done) return;
-  __shared__ double4 cand[kAssignThreads / 32][kWarpCand];
+  __shared__ float4 cand[kAssignThreads / 32][kWarpCand];  // offsets; w: place in cell_cen (bits)
   const int rk = st->rk;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int p = assign_point((long long)blockIdx.x * blockDim.x + threadIdx.x, am);
@@ -560,94 +522,146 @@ __global__ void __launch_bounds__(kAssignThreads) k_assign_warp(
   const unsigned mask = __ballot_sync(0xffffffffu, need);
   if (!mask) return;
   const double inf = __longlong_as_double(0x7ff0000000000000LL);
-  double x = 0.0, y = 0.0, z = 0.0, best = inf;
-  int bj = 0x7fffffff;
+  double x = 0.0, y = 0.0, z = 0.0, best = 0.0;
+  int bj = 0;
   if (need) {
     x = px[p];
     y = py[p];
     z = pz[p];
-    if (old >= 0 && old < rk) {
-      best = ref_dist2(x, y, z, cen[old]);
-      bj = old;
-    }
+    bj = old >= 0 && old < rk ? old : first_seed(p, rk, pidx, am);
+    best = ref_dist2(x, y, z, cen[bj]);
   }
   const double shrink = 1.0 - 2e-14;
-  bool ok = __all_sync(0xffffffffu, !need || bj != 0x7fffffff);
-  const double U = warp_max(need ? best : 0.0);
+  const double U = warp_max(best);  // 0 on the lanes that do not search
   const double x0 = warp_min(need ? x : inf), x1 = warp_max(need ? x : -inf);
   const double y0 = warp_min(need ? y : inf), y1 = warp_max(need ? y : -inf);
   const double z0 = warp_min(need ? z : inf), z1 = warp_max(need ? z : -inf);
+  const double xc = 0.5 * (x0 + x1), yc = 0.5 * (y0 + y1), zc = 0.5 * (z0 + z1);
+  const double R = __dmul_ru(__dsqrt_ru(U), kRoundUp) + g.tol;
+  const float fx = (float)(x - xc), fy = (float)(y - yc), fz = (float)(z - zc);
+  const float hx = (float)(x1 - xc), hy = (float)(y1 - yc), hz = (float)(z1 - zc);
+  const double reach = R + (x1 - xc) + (y1 - yc) + (z1 - zc);  // >= sqrt(U) + h
+  // (the last term covers products below the normal range)
+  const float err = __double2float_ru(1.9073486328125e-6 * reach * reach) + 1e-37f;
+  const float far = __double2float_ru(U) + 2.0f * err;  // beyond: more than sqrt(U) from the box
+  const int nc = g.nc;
+  const int i0 = min(nc - 1, max(0, (int)floor((x0 - R) / g.h[0])));
+  const int i1 = min(nc - 1, max(0, (int)floor((x1 + R) / g.h[0])));
+  const int j0 = min(nc - 1, max(0, (int)floor((y0 - R) / g.h[1])));
+  const int j1 = min(nc - 1, max(0, (int)floor((y1 + R) / g.h[1])));
+  const int k0 = min(nc - 1, max(0, (int)floor((z0 - R) / g.h[2])));
+  const int k1 = min(nc - 1, max(0, (int)floor((z1 + R) / g.h[2])));
+  const int nj = j1 - j0 + 1, nrow = nj * (k1 - k0 + 1);
+  float4* cw = cand[wid];
+  double second = inf;
+  // the nearest of the candidates staged, into (best, bj) and second
+  auto scan = [&](int total) {
+    if (!need) return;
+    const float finf = __int_as_float(0x7f800000);
+    float m1 = finf, m2 = finf;
+    int q1 = 0;
+#pragma unroll 4
+    for (int q = 0; q < total; ++q) {
+      const float4 c = cw[q];
+      const float dx = fx - c.x, dy = fy - c.y, dz = fz - c.z;
+      const float d = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      m2 = fminf(m2, fmaxf(m1, d));
+      q1 = d < m1 ? q : q1;
+      m1 = fminf(m1, d);
+    }
+    auto consider = [&](int q) {
+      const double4 c = cell_cen[__float_as_int(cw[q].w)];
+      const double d = ref_dist2(x, y, z, c);
+      const int j = (int)c.w;
+      if (d < best || (d == best && j < bj)) {
+        if (j != bj) second = fmin(second, best);
+        best = d;
+        bj = j;
+      } else if (j != bj) {
+        second = fmin(second, d);
+      }
+    };
+    const float thr = m1 + 2.0f * err;
+    if (m2 > thr) {
+      consider(q1);
+      second = fmin(second, fmax(0.0, (double)m2 - (double)err));
+    } else {
+      float next = finf;  // the smallest distance left out
+      for (int q = 0; q < total; ++q) {
+        const float4 c = cw[q];
+        const float dx = fx - c.x, dy = fy - c.y, dz = fz - c.z;
+        const float d = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        if (!(d > thr)) consider(q);
+        else next = fminf(next, d);
+      }
+      second = fmin(second, fmax(0.0, (double)next - (double)err));
+    }
+  };
   int total = 0;
-  if (ok) {
-    const double R = __dmul_ru(__dsqrt_ru(U), kRoundUp) + g.tol;
-    const int nc = g.nc;
-    const int i0 = min(nc - 1, max(0, (int)floor((x0 - R) / g.h[0])));
-    const int i1 = min(nc - 1, max(0, (int)floor((x1 + R) / g.h[0])));
-    const int j0 = min(nc - 1, max(0, (int)floor((y0 - R) / g.h[1])));
-    const int j1 = min(nc - 1, max(0, (int)floor((y1 + R) / g.h[1])));
-    const int k0 = min(nc - 1, max(0, (int)floor((z0 - R) / g.h[2])));
-    const int k1 = min(nc - 1, max(0, (int)floor((z1 + R) / g.h[2])));
-    const int ni = i1 - i0 + 1, nj = j1 - j0 + 1;
-    const int ncell = ni * nj * (k1 - k0 + 1);
-    if (ncell > kWarpCells) ok = false;
-    for (int base = 0; ok && base < ncell; base += 32) {
-      const int c = base + lane;
-      int cnt = 0, first = 0;
-      if (c < ncell) {
-        const int ci = i0 + c % ni, cj = j0 + (c / ni) % nj, ck = k0 + c / (ni * nj);
-        // distance from the points' box to the cell's box (widened by tol)
-        const double bx = fmax(0.0, fmax(ci * g.h[0] - g.tol - x1, x0 - (ci + 1) * g.h[0] - g.tol));
-        const double by = fmax(0.0, fmax(cj * g.h[1] - g.tol - y1, y0 - (cj + 1) * g.h[1] - g.tol));
-        const double bz = fmax(0.0, fmax(ck * g.h[2] - g.tol - z1, z0 - (ck + 1) * g.h[2] - g.tol));
-        const double lb = bx * bx + by * by + bz * bz;
-        if (!(lb * shrink > U)) {
-          const int id = ci + nc * (cj + nc * ck);
-          first = cell_start[id];
-          cnt = cell_start[id + 1] - first;
-        }
+  for (int base = 0; base < nrow; base += 32) {
+    // one (y, z) row of cells per lane: its centroids are contiguous
+    int cnt = 0, first = 0;
+    if (base + lane < nrow) {
+      const int cj = j0 + (base + lane) % nj, ck = k0 + (base + lane) / nj;
+      // distance from the points' box to the row's (widened by tol)
+      const double by = fmax(0.0, fmax(cj * g.h[1] - g.tol - y1, y0 - (cj + 1) * g.h[1] - g.tol));
+      const double bz = fmax(0.0, fmax(ck * g.h[2] - g.tol - z1, z0 - (ck + 1) * g.h[2] - g.tol));
+      if (!((by * by + bz * bz) * shrink > U)) {
+        const int id = nc * (cj + nc * ck);
+        first = cell_start[id + i0];
+        cnt = cell_start[id + i1 + 1] - first;
       }
-      int off = cnt;  // inclusive scan over the warp
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, off, o);
-        if (lane >= o) off += v;
+    }
+    int off = cnt;  // inclusive scan over the warp
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, off, o);
+      if (lane >= o) off += v;
+    }
+    const int here = __shfl_sync(0xffffffffu, off, 31);
+    for (int e0 = 0; e0 < here; e0 += 32) {
+      const int e = e0 + lane;
+      // the row of ordinal e: the first lane whose inclusive count exceeds it
+      int lo = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const int v = __shfl_sync(0xffffffffu, off, lo + step - 1);
+        if (v <= e) lo += step;
       }
-      const int here = __shfl_sync(0xffffffffu, off, 31);
-      if (total + here > kWarpCand) {
-        ok = false;
-        break;
+      const int at = __shfl_sync(0xffffffffu, first, lo & 31) + e -
+                     (__shfl_sync(0xffffffffu, off, lo & 31) - __shfl_sync(0xffffffffu, cnt, lo & 31));
+      bool in = false;
+      float cx = 0.f, cy = 0.f, cz = 0.f;
+      if (e < here) {
+        const double4 c = cell_cen[at];
+        cx = (float)(c.x - xc);
+        cy = (float)(c.y - yc);
+        cz = (float)(c.z - zc);
+        const float bx = fmaxf(0.f, fabsf(cx) - hx), by = fmaxf(0.f, fabsf(cy) - hy),
+                    bz = fmaxf(0.f, fabsf(cz) - hz);
+        in = !(fmaf(bx, bx, fmaf(by, by, bz * bz)) > far);
       }
-      for (int q = 0; q < cnt; ++q) cand[wid][total + off - cnt + q] = cell_cen[first + q];
-      total += here;
+      const unsigned got = __ballot_sync(0xffffffffu, in);
+      if (in)
+        cw[total + __popc(got & ((1u << lane) - 1u))] = make_float4(cx, cy, cz, __int_as_float(at));
+      total += __popc(got);
+      if (total > kWarpCand - 32) {
+        __syncwarp();
+        scan(total);
+        __syncwarp();
+        total = 0;
+      }
     }
   }
   __syncwarp();
+  if (total > 0) scan(total);
   int changed = 0;
   if (need) {
-    int lab;
-    if (ok) {
-      double second = inf;
-      for (int q = 0; q < total; ++q) {
-        const double4 c = cand[wid][q];
-        const double d = ref_dist2(x, y, z, c);
-        const int j = (int)c.w;
-        if (d < best || (d == best && j < bj)) {
-          if (j != bj) second = best;
-          best = d;
-          bj = j;
-        } else if (j != bj) {
-          second = fmin(second, d);
-        }
-      }
-      // every centroid not staged is more than sqrt(U) from the point
-      const double floor2 = U * shrink;
-      bnd[p] = make_double2(__dmul_ru(__dsqrt_ru(best), kRoundUp),
-                            __dmul_rd(__dsqrt_rd(fmin(second, floor2)), kRoundDown));
-      lab = bj;
-    } else {
-      lab = ring_search(x, y, z, old, rk, cen, cell_start, cell_cen, g, &bnd[p]);
-    }
-    if (count && old != lab) ++changed;
-    label[p] = lab;
+    // every centroid not staged is more than sqrt(U) from the point
+    const double floor2 = U * shrink;
+    bnd[p] = make_double2(__dmul_ru(__dsqrt_ru(best), kRoundUp),
+                          __dmul_rd(__dsqrt_rd(fmin(second, floor2)), kRoundDown));
+    if (count && old != bj) ++changed;
+    label[p] = bj;
   }
   for (int o = 16; o > 0; o >>= 1) changed += __shfl_xor_sync(0xffffffffu, changed, o);
   if (lane == 0) {
@@ -1587,9 +1601,9 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   k_point_cells<<<grid_for(n, 256), 256, 0, stream>>>(b.px, b.py, b.pz, n, cg, b.pcell, b.pd12);
   k_build_cells<<<1, 1024, cell_smem, stream>>>(b.cen, b.st, cg, b.cell_start, b.cell_cen,
                                                 b.cell_of);
-  k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(b.px, b.py, b.pz, n, b.cen, b.cell_start,
-                                                      b.cell_cen, cg, am, b.st, b.label, 0,
-                                                      b.bnd, b.shift, b.nbshift, b.pcell,
+  k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(b.px, b.py, b.pz, b.pidx, n, b.cen,
+                                                      b.cell_start, b.cell_cen, cg, am, b.st,
+                                                      b.label, 0, b.bnd, b.shift, b.nbshift, b.pcell,
                                                       b.pd12);
   ISDF_CHECK_LAUNCH();
 
@@ -1619,7 +1633,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
                                                   b.nbshift);
       k_build_cells<<<1, 1024, cell_smem, stream>>>(b.cen, b.st, cg, b.cell_start, b.cell_cen,
                                                     b.cell_of);
-      k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(b.px, b.py, b.pz, n, b.cen,
+      k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(b.px, b.py, b.pz, b.pidx, n, b.cen,
                                                           b.cell_start, b.cell_cen, cg, am, b.st,
                                                           b.label, 1, b.bnd, b.shift, b.nbshift,
                                                           b.pcell, b.pd12);
@@ -1658,7 +1672,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
                                                   b.nbshift);
       k_build_cells<<<1, 1024, cell_smem, stream>>>(b.cen, b.st, cg, b.cell_start, b.cell_cen,
                                                     b.cell_of);
-      k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(b.px, b.py, b.pz, n, b.cen,
+      k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(b.px, b.py, b.pz, b.pidx, n, b.cen,
                                                           b.cell_start, b.cell_cen, cg, am, b.st,
                                                           b.label, 1, b.bnd, b.shift, b.nbshift,
                                                           b.pcell, b.pd12);

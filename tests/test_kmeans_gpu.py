@@ -253,3 +253,23 @@ def test_select_long_folds_match_oracle(torch_cuda, kind, length):
                                             torch.from_numpy(w).cuda(), mu, 40, rand_seed=1)
         assert (rk, it) == (rk_o, it_o)
         assert np.array_equal(piv, piv_o)
+
+
+@pytest.mark.parametrize("ng,scale", [((24, 24, 24), 1.0), ((5, 7, 90), 1.0), ((31, 30, 2), 1.0),
+                                      ((16, 15, 17), 1e-25), ((16, 15, 17), 1e22)])
+def test_select_search_extremes_match_oracle(torch_cuda, ng, scale):
+    """The shared candidate search where its portions, its single-precision
+    distances and its seeds are at their limits: as many centroids as a few
+    bricks hold, one, boxes thin and long, lengths whose squares leave single
+    precision on either side, weights with dropped points."""
+    torch = torch_cuda
+    n = ng[0] * ng[1] * ng[2]
+    length = tuple(scale * 0.37 * x for x in ng)
+    w = np.random.default_rng(3).uniform(0.1, 1.0, n)
+    w[n // 3:n // 3 + n // 7] = 0.0
+    for mu in (1, 5, n // 3):
+        piv_o, rk_o, it_o = port.kmeans(w, ng, length, mu, 12)
+        piv, rk, it, _ = isdf.kmeans_select(isdf.Domain(length=length, num_grid=ng),
+                                            torch.from_numpy(w).cuda(), mu, 12, rand_seed=1)
+        assert (rk, it) == (rk_o, it_o)
+        assert np.array_equal(piv, piv_o)
