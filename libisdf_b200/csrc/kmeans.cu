@@ -36,14 +36,15 @@ namespace {
 
 constexpr int kTile = 2048;      // points per counting-sort tile (one walking warp each)
 constexpr int kFinalChunk = 4096;  // points per partial argmin chunk
-constexpr int kIterChunk = 8;    // Lloyd iterations launched between host checks
+constexpr int kIterChunk = 8;    // Lloyd iterations launched between host checks (no graph)
+constexpr int kBodyIters = 2;    // Lloyd iterations per body of the loop's graph
 constexpr int kMaxCellsPerDim = 20;  // centroid cell grid of the pruned assignment
 constexpr int kMaxCells = kMaxCellsPerDim * kMaxCellsPerDim * kMaxCellsPerDim;
 
 struct KmState {
-  int s;        // Lloyd iterations completed
-  int flag;     // labels changed in the last assignment
-  int changed;  // accumulator for the running assignment
+  int s;        // Lloyd iterations begun (all of them completed when done)
+  int flag;     // sharded: labels changed in the last assignment, over the ranks
+  int changed;  // labels changed in the last assignment (n before the first iteration)
   int done;
   int rk;       // current number of centroids
   int npt;      // kept points
@@ -52,6 +53,8 @@ struct KmState {
   unsigned long long maxw_bits;
   unsigned long long maxshift_bits;  // largest centroid move of this iteration (bit pattern)
   unsigned long long searches;       // assignments that ran the cell search (all iterations)
+  unsigned ticket;  // blocks of k_hist_scan that have finished
+  int rounds;       // loop bodies run
 };
 
 // ---------------------------------------------------------------- weight
@@ -272,6 +275,37 @@ struct AssignMap {
   const int* g2p;  // grid index -> kept-point index (or -1); nullptr: identity
 };
 
+// One selection as the kernels of a Lloyd iteration see it. They take the job
+// by value and loop over nothing: every buffer is the selection's own.
+struct KmJob {
+  const int* pidx;
+  const double *px, *py, *pz;
+  int* label;
+  int n;
+  double4 *sorted, *cen, *sums;
+  int *hist, *members, *start;
+  double2* bnd;
+  double* shift;
+  float* nbshift;
+  KmState* st;
+  int* cell_start;
+  double4* cell_cen;
+  int* cell_of;
+  const int* pcell;
+  const double2* pd12;
+  CellGrid cg;
+  AssignMap am;
+  // the points folded into the sums: all of them, or a rank's own in a sharded
+  // selection, whose partial sums go elsewhere and decide nothing by themselves
+  const int* f_label;
+  const double *fx, *fy, *fz, *fw;
+  int f_n, f_npt;  // how many, and how many of them are kept points
+  double4* f_sums;
+  int sharded;
+  double max_f;  // the loop goes on while more labels than this change
+  int max_iter;
+};
+
 __device__ __forceinline__ int assign_point(long long t, const AssignMap& am) {
   if (!am.brick) {
     const long long p = am.p_lo + t;
@@ -300,7 +334,6 @@ __global__ void k_grid_to_point(const int* __restrict__ pidx, int npt, int* __re
     g2p[pidx[p]] = p;
 }
 
-// One block: cell of each centroid, counting sort into cell order.
 // In-place inclusive scan of a[0..n) by a block of 1024 threads: every
 // thread sums a contiguous chunk, the chunk totals are scanned across the
 // warp and the block, and each thread rewrites its chunk.
@@ -332,40 +365,6 @@ __device__ void block_inclusive_scan(int* a, int n, int* warp_tot) {
     a[i] = run;
   }
   __syncthreads();
-}
-
-// Centroids into the cell grid (cell_start, cell_cen).
-__global__ void __launch_bounds__(1024) k_build_cells(const double4* __restrict__ cen,
-                                                      const KmState* st, CellGrid g,
-                                                      int* __restrict__ cell_start,
-                                                      double4* __restrict__ cell_cen,
-                                                      int* __restrict__ cell_of) {
-  if (st->done) return;
-  extern __shared__ int sc[];  // ncells + 1 counters
-  __shared__ int warp_tot[32];
-  const int rk = st->rk;
-  const int nc = g.nc, ncells = nc * nc * nc;
-  for (int c = threadIdx.x; c <= ncells; c += blockDim.x) sc[c] = 0;
-  __syncthreads();
-  for (int j = threadIdx.x; j < rk; j += blockDim.x) {
-    const double4 c = cen[j];
-    const int ci = min(nc - 1, max(0, (int)floor(c.x / g.h[0])));
-    const int cj = min(nc - 1, max(0, (int)floor(c.y / g.h[1])));
-    const int ck = min(nc - 1, max(0, (int)floor(c.z / g.h[2])));
-    const int id = ci + nc * (cj + nc * ck);
-    cell_of[j] = id;
-    atomicAdd(&sc[id + 1], 1);
-  }
-  __syncthreads();
-  block_inclusive_scan(sc + 1, ncells, warp_tot);
-  for (int c = threadIdx.x; c <= ncells; c += blockDim.x) cell_start[c] = sc[c];
-  __syncthreads();
-  // placement inside a cell is arbitrary: the search compares (d, index) pairs
-  for (int j = threadIdx.x; j < rk; j += blockDim.x) {
-    const int slot = atomicAdd(&sc[cell_of[j]], 1);
-    const double4 c = cen[j];
-    cell_cen[slot] = make_double4(c.x, c.y, c.z, (double)j);
-  }
 }
 
 // Squared distance in the reference's rounding (pdist2, utility.cpp:598-615).
@@ -478,21 +477,23 @@ __device__ __forceinline__ int first_seed(int p, int rk, const int* __restrict__
   return j >= 0 && j < rk ? j : rk - 1;
 }
 
-__global__ void __launch_bounds__(kAssignThreads) k_assign_warp(
-    const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
-    const int* __restrict__ pidx, int n, const double4* __restrict__ cen,
-    const int* __restrict__ cell_start, const double4* __restrict__ cell_cen, CellGrid g,
-    AssignMap am, KmState* st, int* __restrict__ label, int count, double2* __restrict__ bnd,
-    const double* __restrict__ shift, const float* __restrict__ nbshift,
-    const int* __restrict__ pcell, const double2* __restrict__ pd12) {
+__global__ void __launch_bounds__(kAssignThreads)
+    k_assign_warp(const __grid_constant__ KmJob J, int count) {
+  KmState* st = J.st;
   if (st->done) return;
+  const double *px = J.px, *py = J.py, *pz = J.pz;
+  const double4 *cen = J.cen, *cell_cen = J.cell_cen;
+  const int* cell_start = J.cell_start;
+  const CellGrid& g = J.cg;
+  int* label = J.label;
+  double2* bnd = J.bnd;
   __shared__ float4 cand[kAssignThreads / 32][kWarpCand];  // offsets; w: place in cell_cen (bits)
   const int rk = st->rk;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int p = assign_point((long long)blockIdx.x * blockDim.x + threadIdx.x, am);
+  const int p = assign_point((long long)blockIdx.x * blockDim.x + threadIdx.x, J.am);
   bool need = false;
   int old = -1;
-  if (p >= 0 && p < n) {
+  if (p >= 0 && p < J.n) {
     old = count ? label[p] : -1;
     need = true;
     if (old >= 0 && old < rk && count && !st->reset_bounds) {
@@ -503,14 +504,14 @@ __global__ void __launch_bounds__(kAssignThreads) k_assign_warp(
       // the global maximum further out (at least D2 = dd.y away); no bound
       // across the domain's faces.
       const double gmax = __longlong_as_double((long long)st->maxshift_bits);
-      const int cell = pcell[p];
-      const double near1 = (double)nbshift[cell], near2 = (double)nbshift[kMaxCells + cell];
-      const double2 dd = pd12[p];
+      const int cell = J.pcell[p];
+      const double near1 = (double)J.nbshift[cell], near2 = (double)J.nbshift[kMaxCells + cell];
+      const double2 dd = J.pd12[p];
       double lo = __dsub_rd(b.y, near1);
       lo = fmin(lo, __dsub_rd(fmax(b.y, dd.x), near2));
       lo = fmin(lo, __dsub_rd(fmax(b.y, dd.y), gmax));
       lo = fmax(0.0, lo);
-      double up = __dadd_ru(b.x, shift[old]);
+      double up = __dadd_ru(b.x, J.shift[old]);
       if (!(up * kBoundMargin < lo))
         up = __dmul_ru(__dsqrt_ru(ref_dist2(px[p], py[p], pz[p], cen[old])), kRoundUp);
       if (up * kBoundMargin < lo) {  // the label stays
@@ -528,7 +529,7 @@ __global__ void __launch_bounds__(kAssignThreads) k_assign_warp(
     x = px[p];
     y = py[p];
     z = pz[p];
-    bj = old >= 0 && old < rk ? old : first_seed(p, rk, pidx, am);
+    bj = old >= 0 && old < rk ? old : first_seed(p, rk, J.pidx, J.am);
     best = ref_dist2(x, y, z, cen[bj]);
   }
   const double shrink = 1.0 - 2e-14;
@@ -671,41 +672,42 @@ __global__ void __launch_bounds__(kAssignThreads) k_assign_warp(
 }
 
 // ---------------------------------------------------------------- control
-__global__ void k_iter_begin(KmState* st, double max_f, int max_iter) {
-  if (st->done) return;
-  if (!((double)st->flag > max_f && st->s < max_iter)) {
-    st->done = 1;
-    return;
-  }
-  st->changed = 0;
-  st->any_empty = 0;
-  st->reset_bounds = 0;
-  st->maxshift_bits = 0;
+// The loop test of utility.cpp:812. Every kernel up to the last block of
+// k_hist_scan, which begins the iteration, finds it by itself.
+__device__ __forceinline__ bool goes_on(const KmJob& J) {
+  return J.sharded || ((double)J.st->changed > J.max_f && J.st->s < J.max_iter);
 }
 
-// set_flag = 0 in a sharded selection, whose flag is the ranks' total (k_shard_begin).
-__global__ void k_iter_end(KmState* st, int set_flag) {
-  if (st->done) return;
-  if (set_flag) st->flag = st->changed;
-  st->s += 1;
+// The iteration's loop in a CUDA graph: a WHILE node's body, ended from the
+// device. No iteration waits for the host.
+struct LoopEnd {
+  cudaGraphConditionalHandle handle;
+  int in_graph;
+  int max_rounds;  // bodies after which the loop ends whatever happens
+};
+
+__device__ __forceinline__ void end_loop(const LoopEnd& le) {
+  if (le.in_graph) cudaGraphSetConditional(le.handle, 0);
 }
 
 // ---------------------------------------------------------------- update
 // Stable counting sort of the points by label (tiles of kTile points), then
-// one warp per cluster folds w, w*x, w*y, w*z over the members in increasing
-// point index: the exact sequence of additions of utility.cpp:816-822.
-__global__ void __launch_bounds__(256) k_hist(const int* __restrict__ label, int n,
-                                              const KmState* st, int* __restrict__ hist) {
-  if (st->done) return;
+// one warp per cluster and component folds w, w*x, w*y, w*z over the members
+// in increasing point index: the exact sequence of additions of
+// utility.cpp:816-822.
+__global__ void __launch_bounds__(256) k_hist(const __grid_constant__ KmJob J, const LoopEnd le) {
+  KmState* st = J.st;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && ++st->rounds > le.max_rounds) end_loop(le);
+  if (st->done || !goes_on(J)) return;
   extern __shared__ int sh[];
   const int rk = st->rk;
   for (int l = threadIdx.x; l < rk; l += blockDim.x) sh[l] = 0;
   __syncthreads();
   const int base = blockIdx.x * kTile;
-  const int end = min(base + kTile, n);
-  for (int p = base + threadIdx.x; p < end; p += blockDim.x) atomicAdd(&sh[label[p]], 1);
+  const int end = min(base + kTile, J.f_n);
+  for (int p = base + threadIdx.x; p < end; p += blockDim.x) atomicAdd(&sh[J.f_label[p]], 1);
   __syncthreads();
-  int* row = hist + (size_t)blockIdx.x * rk;
+  int* row = J.hist + (size_t)blockIdx.x * rk;
   for (int l = threadIdx.x; l < rk; l += blockDim.x) row[l] = sh[l];
 }
 
@@ -714,19 +716,31 @@ __global__ void __launch_bounds__(256) k_hist(const int* __restrict__ label, int
 // contiguous range of tiles: the warps' range sums, their exclusive prefix in
 // shared memory, then each warp rewrites its range from that prefix. One
 // thread per label walking all tiles left the scan bound by the latency of
-// its ~ntiles/16 dependent load batches.
+// its ~ntiles/16 dependent load batches. The last block to finish scans the
+// member counts into each label's first slot and begins the iteration: one
+// launch where three single-block kernels ran.
 constexpr int kScanWarps = 16;
 
-__global__ void __launch_bounds__(32 * kScanWarps) k_hist_scan(int* __restrict__ hist, int ntiles,
-                                                               const KmState* st,
-                                                               int* __restrict__ members) {
+__global__ void __launch_bounds__(32 * kScanWarps)
+    k_hist_scan(const __grid_constant__ KmJob J, const LoopEnd le) {
+  KmState* st = J.st;
   if (st->done) return;
+  if (!goes_on(J)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      st->done = 1;
+      end_loop(le);
+    }
+    return;
+  }
   const int rk = st->rk;
+  const int ntiles = (J.f_n + kTile - 1) / kTile;
+  int* hist = J.hist;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int l = blockIdx.x * 32 + lane;
   const int per = (ntiles + kScanWarps - 1) / kScanWarps;
   const int t0 = w * per, t1 = min(t0 + per, ntiles);
   __shared__ int part[kScanWarps][32];
+  __shared__ bool last;
   constexpr int kB = 8;  // loads batched ahead of the additions and stores
   int sum = 0;
   if (l < rk) {
@@ -740,95 +754,125 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_hist_scan(int* __restrict__
   }
   part[w][lane] = sum;
   __syncthreads();
-  if (l >= rk) return;
-  int run = 0;
-  for (int q = 0; q < w; ++q) run += part[q][lane];
-  for (int t = t0; t < t1; t += kB) {
-    int v[kB];
+  if (l < rk) {
+    int run = 0;
+    for (int q = 0; q < w; ++q) run += part[q][lane];
+    for (int t = t0; t < t1; t += kB) {
+      int v[kB];
 #pragma unroll
-    for (int u = 0; u < kB; ++u) v[u] = t + u < t1 ? hist[(size_t)(t + u) * rk + l] : 0;
+      for (int u = 0; u < kB; ++u) v[u] = t + u < t1 ? hist[(size_t)(t + u) * rk + l] : 0;
 #pragma unroll
-    for (int u = 0; u < kB; ++u) {
-      if (t + u < t1) hist[(size_t)(t + u) * rk + l] = run;
-      run += v[u];
-    }
-  }
-  // the last warp's prefix covers every tile (its own range may be empty)
-  if (w == kScanWarps - 1) members[l] = run;
-}
-
-// Exclusive scan of the member counts (one block): start[l].
-__global__ void __launch_bounds__(1024) k_label_start(const int* __restrict__ members,
-                                                      const KmState* st, int* __restrict__ start) {
-  if (st->done) return;
-  __shared__ int part[1024];
-  const int rk = st->rk;
-  const int per = (rk + 1023) / 1024;
-  const int lo = threadIdx.x * per, hi = min(lo + per, rk);
-  int s = 0;
-  for (int i = lo; i < hi; ++i) s += members[i];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    int v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
-    __syncthreads();
-    part[threadIdx.x] += v;
-    __syncthreads();
-  }
-  int run = threadIdx.x ? part[threadIdx.x - 1] : 0;
-  for (int i = lo; i < hi; ++i) {
-    start[i] = run;
-    run += members[i];
-  }
-}
-
-// One tile per block: 128 threads stage the tile's labels in shared memory,
-// then one warp walks them in order and gives every point its stable position
-// (peers with equal labels share one running offset), written over its label.
-// All 128 threads then move the points there: what lands is the point's
-// (w x, w y, w z, w), so that the per-cluster fold reads its members
-// contiguously. The walk has no global loads in its dependent chain; the
-// point loads of the move are independent of one another.
-__global__ void __launch_bounds__(128) k_scatter(const int* __restrict__ label, int n,
-                                                 const KmState* st, const int* __restrict__ hist,
-                                                 const int* __restrict__ start,
-                                                 const double* __restrict__ px,
-                                                 const double* __restrict__ py,
-                                                 const double* __restrict__ pz,
-                                                 const double* __restrict__ pw,
-                                                 double4* __restrict__ sorted) {
-  if (st->done) return;
-  extern __shared__ int sm_scatter[];
-  const int rk = st->rk;
-  int* run = sm_scatter;
-  int* lab = sm_scatter + rk;  // the tile's labels, then the points' positions
-  const int* row = hist + (size_t)blockIdx.x * rk;
-  for (int l = threadIdx.x; l < rk; l += 128) run[l] = start[l] + row[l];
-  const int base = blockIdx.x * kTile;
-  const int cnt = min(kTile, n - base);
-  for (int k = threadIdx.x; k < cnt; k += 128) lab[k] = label[base + k];
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    for (int c = 0; c < cnt; c += 32) {
-      const int k = c + lane;
-      const bool ok = k < cnt;
-      const int l = ok ? lab[k] : -1;
-      const unsigned peers = __match_any_sync(0xffffffffu, l);
-      const int b = ok ? run[l] : 0;
-      __syncwarp();
-      if (ok) {
-        lab[k] = b + __popc(peers & ((1u << lane) - 1u));
-        if (lane == __ffs(peers) - 1) run[l] = b + __popc(peers);
+      for (int u = 0; u < kB; ++u) {
+        if (t + u < t1) hist[(size_t)(t + u) * rk + l] = run;
+        run += v[u];
       }
-      __syncwarp();
+    }
+    // the last warp's prefix covers every tile (its own range may be empty)
+    if (w == kScanWarps - 1) J.members[l] = run;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  // exclusive scan of the member counts: start[l]
+  __threadfence();
+  const int each = (rk + 32 * kScanWarps - 1) / (32 * kScanWarps);
+  const int lo = min(rk, (int)threadIdx.x * each), hi = min(rk, lo + each);
+  int mine = 0;
+  for (int i = lo; i < hi; ++i) mine += __ldcg(J.members + i);
+  int inc = mine;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  int* tot = part[0];
+  if (lane == 31) tot[w] = inc;
+  __syncthreads();
+  int run = inc - mine;
+  for (int q = 0; q < w; ++q) run += tot[q];
+  for (int i = lo; i < hi; ++i) {
+    J.start[i] = run;
+    run += __ldcg(J.members + i);
+  }
+  if (threadIdx.x == 0) {
+    st->ticket = 0;
+    if (!J.sharded) {
+      st->s += 1;
+      st->changed = 0;
+      st->any_empty = 0;
+      st->reset_bounds = 0;
+      st->maxshift_bits = 0;
     }
   }
+}
+
+// The points' (w x, w y, w z, w) into cluster order, so that the per-cluster
+// fold reads its members contiguously. One tile per block, a stretch of
+// kTile / 8 consecutive points per warp: each warp counts its points per label
+// (peers with equal labels in 32 points make one addition), the counts become
+// each warp's offset within the tile, and each warp then gives its points their
+// stable places and moves them. The walks of eight warps run side by side: one
+// warp walking the whole tile took 15 us of a 98 us iteration at 64 000 points
+// whatever their number, and this takes 5.
+constexpr int kScatterWarps = 8;
+
+__global__ void __launch_bounds__(32 * kScatterWarps)
+    k_scatter(const __grid_constant__ KmJob J) {
+  const KmState* st = J.st;
+  if (st->done) return;
+  extern __shared__ __align__(16) unsigned short cnt[];  // [label][warp]
+  const int rk = st->rk;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  constexpr int kPer = kTile / kScatterWarps, kSteps = kPer / 32;
+  uint4* cnt4 = reinterpret_cast<uint4*>(cnt);
+  for (int l = threadIdx.x; l < rk; l += blockDim.x) cnt4[l] = make_uint4(0, 0, 0, 0);
+  const int base = blockIdx.x * kTile + w * kPer;
+  int lab[kSteps];
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i) {
+    const int p = base + i * 32 + lane;
+    lab[i] = p < J.f_n ? J.f_label[p] : -1;
+  }
   __syncthreads();
-  for (int k = threadIdx.x; k < cnt; k += 128) {
-    const int p = base + k;
-    const double w = pw[p];
-    sorted[lab[k]] = make_double4(rmul(w, px[p]), rmul(w, py[p]), rmul(w, pz[p]), w);
+  unsigned peers[kSteps];
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i) {
+    peers[i] = __match_any_sync(0xffffffffu, lab[i]);
+    if (lab[i] >= 0 && lane == __ffs(peers[i]) - 1)
+      cnt[lab[i] * kScatterWarps + w] += (unsigned short)__popc(peers[i]);
+    __syncwarp();
+  }
+  __syncthreads();
+  for (int l = threadIdx.x; l < rk; l += blockDim.x) {
+    uint4 c = cnt4[l];
+    unsigned run = 0;  // two 16-bit counts per word, in warp order
+    unsigned* v = &c.x;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned a = v[q] & 0xffffu, b = v[q] >> 16;
+      v[q] = run | ((run + a) << 16);
+      run += a + b;
+    }
+    cnt4[l] = c;
+  }
+  __syncthreads();
+  const int* row = J.hist + (size_t)blockIdx.x * rk;
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i) {
+    const int l = lab[i];
+    int in = 0;
+    if (l >= 0) in = cnt[l * kScatterWarps + w];
+    __syncwarp();
+    if (l >= 0 && lane == __ffs(peers[i]) - 1)
+      cnt[l * kScatterWarps + w] = (unsigned short)(in + __popc(peers[i]));
+    __syncwarp();
+    if (l >= 0) {
+      const int p = base + i * 32 + lane;
+      const double wt = J.fw[p];
+      J.sorted[J.start[l] + row[l] + in + __popc(peers[i] & ((1u << lane) - 1u))] =
+          make_double4(rmul(wt, J.fx[p]), rmul(wt, J.fy[p]), rmul(wt, J.fz[p]), wt);
+    }
   }
 }
 
@@ -961,27 +1005,22 @@ __device__ __forceinline__ double fold_serial(const double* comp, int cnt, doubl
 // points p >= npt are identical copies of grid point 0 (weight w[0],
 // coordinates (0, 0, 0)) and come last in their cluster's member list, so
 // their part of the fold is a repeated addition of one value (repeat_add).
-// n, npt: the points folded and how many of them are kept points (the rest
-// is zero tail); flag_empty: record an empty cluster in st (off when the sums
-// are one rank's partial sums).
 constexpr int kFoldThreads = 128;
 
-__global__ void __launch_bounds__(kFoldThreads) k_segsum(
-    const double4* __restrict__ sorted, const int* __restrict__ start,
-    const int* __restrict__ members, const double* __restrict__ px, const double* __restrict__ py,
-    const double* __restrict__ pz, const double* __restrict__ pw, const int* __restrict__ label,
-    int n, int npt, int flag_empty, KmState* st, double4* __restrict__ sums) {
+__global__ void __launch_bounds__(kFoldThreads) k_segsum(const __grid_constant__ KmJob J) {
+  KmState* st = J.st;
   if (st->done) return;
+  const int n = J.f_n, npt = J.f_npt;
   // the clusters that started as the last points of the list reach over the
   // rest of the box and stay the largest: first come, so that their folds do
   // not start in a second wave of blocks
   const int c = gridDim.x - 1 - blockIdx.x;
   if (c >= st->rk) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double* v = reinterpret_cast<const double*>(sorted + start[c]) + warp;
-  int m = members[c];
+  const double* v = reinterpret_cast<const double*>(J.sorted + J.start[c]) + warp;
+  int m = J.members[c];
   long long tail = 0;
-  if (npt < n && label[npt] == c) {
+  if (npt < n && J.f_label[npt] == c) {
     tail = n - npt;
     m -= (int)tail;
   }
@@ -1011,32 +1050,88 @@ __global__ void __launch_bounds__(kFoldThreads) k_segsum(
   }
   if (lane == 0) {
     if (tail) {
-      const double w0 = pw[npt];
-      const double one = warp == 3 ? w0
-                                   : rmul(w0, warp == 0 ? px[npt] : warp == 1 ? py[npt] : pz[npt]);
+      const double w0 = J.fw[npt];
+      const double one =
+          warp == 3 ? w0 : rmul(w0, warp == 0 ? J.fx[npt] : warp == 1 ? J.fy[npt] : J.fz[npt]);
       acc = repeat_add(acc, one, tail);
     }
-    reinterpret_cast<double*>(sums + c)[warp] = acc;
-    if (flag_empty && warp == 3 && acc == 0.0) st->any_empty = 1;
+    reinterpret_cast<double*>(J.f_sums + c)[warp] = acc;
+    if (!J.sharded && warp == 3 && acc == 0.0) st->any_empty = 1;
   }
 }
 
-// New centroids = sums / count; an empty cluster takes the last centroid's
-// sums and rk shrinks (utility.cpp:831-853).
-// The update also records how far every centroid moved (rounded upward), the
-// largest move, and for every cell of the grid the largest move of a centroid
-// that sat in its 3 x 3 x 3 neighbourhood before the update (cell_of still
-// holds the previous positions' cells here).
-__global__ void __launch_bounds__(1024) k_centroids(double4* __restrict__ sums, KmState* st,
-                                                    double4* __restrict__ cen,
-                                                    double* __restrict__ shift,
-                                                    const int* __restrict__ cell_of, CellGrid g,
-                                                    float* __restrict__ nbshift) {
+// The empty-cluster compaction of utility.cpp:831-853: the loop there fills each
+// empty place with the last cluster, again while that one is empty too, and
+// shrinks rk. So the clusters below the final rk stay where they are, and the
+// k-th empty place (ascending) takes the k-th non-empty cluster from the end.
+// One block finds both lists by prefix counts (holes, fillers: scratch of rk
+// entries each); the loop by one thread took 1.8 ms at 3000 centroids.
+__device__ int compact_empty(const double4* __restrict__ sums, int rk, double4* __restrict__ cen,
+                             int* __restrict__ holes, int* __restrict__ fillers, int* warp_tot) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int per = (rk + 1023) / 1024;
+  const int b0 = min(rk, tid * per), b1 = min(rk, b0 + per);
+  int mine = 0;
+  for (int i = b0; i < b1; ++i) mine += !(sums[i].w != 0.0);
+  int inc = mine;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  if (lane == 31) warp_tot[w] = inc;
+  __syncthreads();
+  int before = inc - mine, empty = 0;
+  for (int q = 0; q < 32; ++q) {
+    if (q < w) before += warp_tot[q];
+    empty += warp_tot[q];
+  }
+  const int left = rk - empty;
+  for (int i = b0; i < b1; ++i) {
+    const double4 s = sums[i];
+    if (!(s.w != 0.0)) {
+      if (i < left) holes[before] = i;
+      ++before;
+    } else if (i < left) {
+      cen[i] = make_double4(rdiv(s.x, s.w), rdiv(s.y, s.w), rdiv(s.z, s.w), 0.0);
+    } else {
+      fillers[(rk - 1 - i) - (empty - before)] = i;  // non-empty clusters after i
+    }
+  }
+  __syncthreads();
+  // as many fillers at or past `left` as holes below it
+  int nholes = 0;
+  for (int i = left + tid; i < rk; i += 1024) nholes += sums[i].w != 0.0;
+  for (int o = 16; o > 0; o >>= 1) nholes += __shfl_xor_sync(0xffffffffu, nholes, o);
+  __syncthreads();
+  if (lane == 0) warp_tot[w] = nholes;
+  __syncthreads();
+  nholes = 0;
+  for (int q = 0; q < 32; ++q) nholes += warp_tot[q];
+  for (int k = tid; k < nholes; k += 1024) {
+    const double4 s = sums[fillers[k]];
+    cen[holes[k]] = make_double4(rdiv(s.x, s.w), rdiv(s.y, s.w), rdiv(s.z, s.w), 0.0);
+  }
+  __syncthreads();
+  return left;
+}
+
+// New centroids = sums / count (with the compaction above where a cluster is
+// empty), then the centroids into the cell grid (cell_start, cell_cen): one
+// block. The update also records how far every centroid moved (rounded
+// upward), the largest move, and for every cell of the grid the largest move of
+// a centroid that sat in its 3^3 and 5^3 neighbourhoods before the update
+// (cell_of still holds the previous positions' cells there).
+// update = 0: the cells alone (the first centroids).
+__global__ void __launch_bounds__(1024) k_centroids(const __grid_constant__ KmJob J, int update) {
+  KmState* st = J.st;
   if (st->done) return;
+  extern __shared__ unsigned cmax[];  // 3 x ncells + 1 words
+  __shared__ int warp_tot[32];
+  const CellGrid& g = J.cg;
+  const int nc = g.nc, ncells = nc * nc * nc;
   int rk = st->rk;
-  if (!st->any_empty) {
-    extern __shared__ unsigned cmax[];  // 3 x ncells: the cells' maxima, then two pass buffers
-    const int nc = g.nc, ncells = nc * nc * nc;
+  const bool empty = update && st->any_empty;
+  if (update && !empty) {
     unsigned* tmp = cmax + ncells;
     for (int c = threadIdx.x; c < ncells; c += blockDim.x) cmax[c] = 0u;
     __syncthreads();
@@ -1044,17 +1139,17 @@ __global__ void __launch_bounds__(1024) k_centroids(double4* __restrict__ sums, 
     // patterns order as the values do)
     unsigned long long mx = 0ull;
     for (int i = threadIdx.x; i < rk; i += blockDim.x) {
-      double4 s = sums[i];
-      const double4 o = cen[i];
+      double4 s = J.sums[i];
+      const double4 o = J.cen[i];
       const double4 c = make_double4(rdiv(s.x, s.w), rdiv(s.y, s.w), rdiv(s.z, s.w), 0.0);
-      cen[i] = c;
+      J.cen[i] = c;
       // upper bound on the distance the centroid moved (rounded upward)
       const double dx = fabs(c.x - o.x), dy = fabs(c.y - o.y), dz = fabs(c.z - o.z);
       const double d2 = __dadd_ru(__dadd_ru(__dmul_ru(dx, dx), __dmul_ru(dy, dy)), __dmul_ru(dz, dz));
       const double sh = __dmul_ru(__dsqrt_ru(d2), 1.0 + 1e-13);
-      shift[i] = sh;
+      J.shift[i] = sh;
       mx = max(mx, (unsigned long long)__double_as_longlong(sh));
-      atomicMax(&cmax[cell_of[i]], __float_as_uint(__double2float_ru(sh)));
+      atomicMax(&cmax[J.cell_of[i]], __float_as_uint(__double2float_ru(sh)));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -1077,7 +1172,7 @@ __global__ void __launch_bounds__(1024) k_centroids(double4* __restrict__ sums, 
         t2[c] = m;
       }
       __syncthreads();
-      float* out = rad == 1 ? nbshift : nbshift + kMaxCells;
+      float* out = rad == 1 ? J.nbshift : J.nbshift + kMaxCells;
       for (int c = threadIdx.x; c < ncells; c += blockDim.x) {
         const int ck = c / (nc * nc);
         unsigned m = 0u;
@@ -1087,25 +1182,37 @@ __global__ void __launch_bounds__(1024) k_centroids(double4* __restrict__ sums, 
       }
       __syncthreads();
     }
-    return;
-  }
-  if (threadIdx.x != 0) return;
-  st->reset_bounds = 1;
-  for (int i = 0; i < rk; i++) {
-    double4 s = sums[i];
-    if (s.w != 0.0) {
-      sums[i] = make_double4(rdiv(s.x, s.w), rdiv(s.y, s.w), rdiv(s.z, s.w), s.w);
-    } else {
-      rk--;
-      sums[i] = sums[rk];
-      i--;
+  } else if (empty) {
+    // the members' lists of this iteration are done with: scratch
+    rk = compact_empty(J.sums, rk, J.cen, J.members, J.start, warp_tot);
+    if (threadIdx.x == 0) {
+      st->rk = rk;
+      st->reset_bounds = 1;
     }
   }
-  for (int i = 0; i < rk; i++) {
-    double4 s = sums[i];
-    cen[i] = make_double4(s.x, s.y, s.z, 0.0);
+  // the centroids into the cell grid
+  int* sc = reinterpret_cast<int*>(cmax);  // ncells + 1 counters
+  for (int c = threadIdx.x; c <= ncells; c += blockDim.x) sc[c] = 0;
+  __syncthreads();
+  for (int j = threadIdx.x; j < rk; j += blockDim.x) {
+    const double4 c = J.cen[j];
+    const int ci = min(nc - 1, max(0, (int)floor(c.x / g.h[0])));
+    const int cj = min(nc - 1, max(0, (int)floor(c.y / g.h[1])));
+    const int ck = min(nc - 1, max(0, (int)floor(c.z / g.h[2])));
+    const int id = ci + nc * (cj + nc * ck);
+    J.cell_of[j] = id;
+    atomicAdd(&sc[id + 1], 1);
   }
-  st->rk = rk;
+  __syncthreads();
+  block_inclusive_scan(sc + 1, ncells, warp_tot);
+  for (int c = threadIdx.x; c <= ncells; c += blockDim.x) J.cell_start[c] = sc[c];
+  __syncthreads();
+  // placement inside a cell is arbitrary: the search compares (d, index) pairs
+  for (int j = threadIdx.x; j < rk; j += blockDim.x) {
+    const int slot = atomicAdd(&sc[J.cell_of[j]], 1);
+    const double4 c = J.cen[j];
+    J.cell_cen[slot] = make_double4(c.x, c.y, c.z, (double)j);
+  }
 }
 
 // ---------------------------------------------------------------- final
@@ -1176,6 +1283,81 @@ __global__ void k_final_reduce(const double* __restrict__ part_d, const int* __r
   sel[j] = pidx[bi];
 }
 
+// The same where the grid gives the points' places, one warp per centroid: the
+// kept points of a box of grid points around the centroid, (distance, list
+// index) pairs compared, the box doubled until every point outside it (a grid
+// spacing or more beyond its faces, less tol) is farther than the nearest found
+// or the box is the grid. The zero tail's first point (a copy of grid point 0)
+// is compared once. A few points per centroid instead of all of them: 20 us
+// against 1.6 ms at 884 736 points and 2979 centroids.
+__global__ void __launch_bounds__(128)
+    k_final_near(const __grid_constant__ KmJob J, const double dx, const double dy,
+                 const double dz, int* __restrict__ sel) {
+  const int rk = J.st->rk;
+  const int j = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (j >= rk) return;
+  const double4 c = J.cen[j];
+  const AssignMap& am = J.am;
+  const int n3[3] = {am.nx, am.ny, am.nz};
+  const double cc[3] = {c.x, c.y, c.z}, h3[3] = {dx, dy, dz};
+  const double inf = __longlong_as_double(0x7ff0000000000000LL);
+  double best = inf;
+  int bp = 0;
+  for (int r = 1;; r *= 2) {
+    int lo[3], ext[3];
+    double margin = inf;  // every point outside the box is at least this far
+    bool all = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double at = floor(cc[d] / h3[d]);
+      const int f = (int)fmin(fmax(at, 0.0), (double)(n3[d] - 1));
+      lo[d] = max(0, f - r + 1);
+      const int hi = min(n3[d] - 1, f + r);
+      ext[d] = hi - lo[d] + 1;
+      if (lo[d] > 0) {
+        margin = fmin(margin, cc[d] - (lo[d] - 1) * h3[d] - J.cg.tol);
+        all = false;
+      }
+      if (hi < n3[d] - 1) {
+        margin = fmin(margin, (hi + 1) * h3[d] - cc[d] - J.cg.tol);
+        all = false;
+      }
+    }
+    best = inf;
+    bp = 0;
+    if (am.npt < J.n && lane == 0) {  // the zero tail
+      const double d = ref_dist2(J.px[am.npt], J.py[am.npt], J.pz[am.npt], c);
+      if (d < best) {
+        best = d;
+        bp = am.npt;
+      }
+    }
+    const int count = ext[0] * ext[1] * ext[2];
+    for (int e = lane; e < count; e += 32) {
+      const int ix = lo[0] + e % ext[0], iy = lo[1] + (e / ext[0]) % ext[1],
+                iz = lo[2] + e / (ext[0] * ext[1]);
+      const int gp = ix + am.nx * (iy + am.ny * iz);
+      const int p = am.g2p ? am.g2p[gp] : gp;
+      if (p < 0) continue;
+      const double d = ref_dist2(J.px[p], J.py[p], J.pz[p], c);
+      if (d < best || (d == best && p < bp)) {
+        best = d;
+        bp = p;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double od = __shfl_xor_sync(0xffffffffu, best, o);
+      const int op = __shfl_xor_sync(0xffffffffu, bp, o);
+      if (od < best || (od == best && op < bp)) {
+        best = od;
+        bp = op;
+      }
+    }
+    if (all || (margin > 0.0 && best < margin * margin * (1.0 - 1e-12))) break;
+  }
+  if (lane == 0) sel[j] = J.pidx[bp];
+}
+
 // ---------------------------------------------------------------- sharded
 // A rank's record per Lloyd iteration: entry 0 carries the labels its last
 // assignment changed (.x), entries 1..rk its partial centroid sums.
@@ -1185,11 +1367,11 @@ __global__ void k_shard_header(const KmState* st, double4* __restrict__ send) {
 
 // The loop test of utility.cpp:812 on the ranks' total of changed labels
 // (the reference's MPI_Reduce + MPI_Bcast of flag, utility.cpp:908-917),
-// then the per-iteration resets of k_iter_begin.
+// then the iteration's resets.
 __global__ void k_shard_begin(KmState* st, const double4* __restrict__ recv, int ranks, int stride,
                               double max_f, int max_iter) {
   if (st->done) return;
-  if (st->s > 0) {
+  if (st->s > 0) {  // n before the first iteration
     long long f = 0;
     for (int q = 0; q < ranks; ++q) f += (long long)recv[(size_t)q * stride].x;
     st->flag = (int)f;
@@ -1198,6 +1380,7 @@ __global__ void k_shard_begin(KmState* st, const double4* __restrict__ recv, int
     st->done = 1;
     return;
   }
+  st->s += 1;
   st->changed = 0;
   st->any_empty = 0;
   st->reset_bounds = 0;
@@ -1284,9 +1467,9 @@ int set_kmeans_smem_attrs() {
   ISDF_CUDA(cudaFuncSetAttribute(k_hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(int) * kKmeansMaxMu)));
   ISDF_CUDA(cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(int) * (kKmeansMaxMu + kTile))));
+                                 (int)(sizeof(short) * kScatterWarps * kKmeansMaxMu)));
   ISDF_CUDA(cudaFuncSetAttribute(k_centroids, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(3 * sizeof(unsigned) * kMaxCells)));
+                                 (int)(sizeof(unsigned) * (3 * kMaxCells + 1))));
   if (dev >= 0 && dev < 64) done[dev] = true;
   return ISDF_OK;
 }
@@ -1308,8 +1491,8 @@ struct KmBuffers {
   float* nbshift;  // per cell: largest move of a centroid in its 27-cell neighbourhood
   double* part_d;
   int* part_i;
-  int* sel;
   KmState* st;
+  int* sel;        // behind *st: the two are read back together
   int* cell_start;
   double4* cell_cen;
   int* pcell;        // per point: its cell
@@ -1341,8 +1524,8 @@ KmBuffers carve(Arena& a, int n, int mu) {
   b.nbshift = a.take<float>(2 * (size_t)kMaxCells);  // 3^3 and 5^3 neighbourhoods
   b.part_d = a.take<double>((size_t)nchunks * mu);
   b.part_i = a.take<int>((size_t)nchunks * mu);
-  b.sel = a.take<int>(mu);
-  b.st = a.take<KmState>(1);
+  b.st = a.take<KmState>(1 + (sizeof(int) * (size_t)mu + sizeof(KmState) - 1) / sizeof(KmState));
+  b.sel = reinterpret_cast<int*>(b.st + 1);
   b.cell_start = a.take<int>((size_t)kMaxCells + 1);
   b.cell_cen = a.take<double4>(mu);
   b.cell_of = a.take<int>(mu);
@@ -1429,6 +1612,24 @@ struct SeededRand {
   }
 };
 
+// piv = [distinct selected points ascending | the rest ascending]
+// (unique, utility.cpp:617-629, and utility.cpp:973-983); returns rk_eff. The
+// rest is written gap by gap between the selected points.
+static int piv_from_selection(std::vector<int>& sel, int n, int* piv) {
+  std::sort(sel.begin(), sel.end());
+  sel.erase(std::unique(sel.begin(), sel.end()), sel.end());
+  const int rk_eff = (int)sel.size();
+  std::copy(sel.begin(), sel.end(), piv);
+  int* out = piv + rk_eff;
+  int from = 0;
+  for (int k = 0; k <= rk_eff; ++k) {
+    const int to = k < rk_eff ? sel[k] : n;
+    for (int i = from; i < to; ++i) *out++ = i;
+    from = to + 1;
+  }
+  return rk_eff;
+}
+
 int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, KmeansResult* res,
                   Transport* shard) {
   const int n = (int)args.ng;
@@ -1445,7 +1646,6 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   // this rank's points of the n-long list (utility.cpp:682-689); all of them at one rank
   const int lo = shard ? (int)block_start(n, ranks, shard->rank) : 0;
   const int cnt = shard ? (int)block_count(n, ranks, shard->rank) : n;
-  const int ntiles = (n + kTile - 1) / kTile;
   const int nfilter = (n + 1023) / 1024;
   const int nchunks = (n + kFinalChunk - 1) / kFinalChunk;
   // a rank of a sharded selection draws from its own generator (below)
@@ -1471,10 +1671,10 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   ISDF_TRY(read_back(&hst, b.st, sizeof(KmState), stream));
   const int npt = hst.npt;
   res->npt = npt;
-  std::memset(args.piv, 0, sizeof(int) * (size_t)n);
 
   if (npt < mu) {
     // utility.cpp:667-681: piv from the kept list, then a shuffled tail.
+    std::memset(args.piv, 0, sizeof(int) * (size_t)n);
     std::vector<int> index(n, 0);
     ISDF_TRY(read_back(index.data(), b.pidx, sizeof(int) * (size_t)npt, stream));
     int k0 = 0, k1 = 0;
@@ -1542,6 +1742,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   {
     KmState init{};
     init.flag = n;
+    init.changed = n;
     init.rk = mu;
     init.npt = npt;
     init.maxw_bits = hst.maxw_bits;
@@ -1559,7 +1760,6 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
     }
     cg.tol = 1e-9 * lmax;
   }
-  const size_t cell_smem = sizeof(int) * ((size_t)cg.nc * cg.nc * cg.nc + 1);
   AssignMap am{};
   am.nx = args.num_grid[0];
   am.ny = args.num_grid[1];
@@ -1599,131 +1799,159 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   const unsigned pgrid = am.brick ? grid_for(am.nbt + tail_loc, kAssignThreads)
                                   : grid_for(cnt, kAssignThreads);
   k_point_cells<<<grid_for(n, 256), 256, 0, stream>>>(b.px, b.py, b.pz, n, cg, b.pcell, b.pd12);
-  k_build_cells<<<1, 1024, cell_smem, stream>>>(b.cen, b.st, cg, b.cell_start, b.cell_cen,
-                                                b.cell_of);
-  k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(b.px, b.py, b.pz, b.pidx, n, b.cen,
-                                                      b.cell_start, b.cell_cen, cg, am, b.st,
-                                                      b.label, 0, b.bnd, b.shift, b.nbshift, b.pcell,
-                                                      b.pd12);
+  KmJob job{};
+  job.pidx = b.pidx;
+  job.px = b.px;
+  job.py = b.py;
+  job.pz = b.pz;
+  job.label = b.label;
+  job.n = n;
+  job.sorted = b.sorted;
+  job.cen = b.cen;
+  job.sums = b.sums;
+  job.hist = b.hist;
+  job.members = b.members;
+  job.start = b.start;
+  job.bnd = b.bnd;
+  job.shift = b.shift;
+  job.nbshift = b.nbshift;
+  job.st = b.st;
+  job.cell_start = b.cell_start;
+  job.cell_cen = b.cell_cen;
+  job.cell_of = b.cell_of;
+  job.pcell = b.pcell;
+  job.pd12 = b.pd12;
+  job.cg = cg;
+  job.am = am;
+  job.f_label = b.label + lo;
+  job.fx = b.px + lo;
+  job.fy = b.py + lo;
+  job.fz = b.pz + lo;
+  job.fw = b.pw + lo;
+  job.f_n = cnt;
+  job.f_npt = std::max(0, std::min(npt - lo, cnt));
+  job.f_sums = shard ? sb.send + 1 : b.sums;
+  job.sharded = shard ? 1 : 0;
+  job.max_f = 1e-5 * n;  // KmeansTolerance * n (utility.cpp:812)
+  job.max_iter = args.max_iter;
+
+  const size_t cells_smem = sizeof(unsigned) * (3 * (size_t)cg.nc * cg.nc * cg.nc + 1);
+  const size_t hist_smem = sizeof(int) * (size_t)mu;
+  const size_t scatter_smem = sizeof(short) * kScatterWarps * (size_t)mu;
+  ISDF_TRY(set_kmeans_smem_attrs());
+  k_centroids<<<1, 1024, cells_smem, stream>>>(job, 0);
+  k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(job, 0);
   ISDF_CHECK_LAUNCH();
 
-  const size_t cmax_smem = 3 * sizeof(unsigned) * ((size_t)cg.nc * cg.nc * cg.nc);
-  const double max_f = 1e-5 * n;  // KmeansTolerance * n (utility.cpp:812)
-  const size_t hist_smem = sizeof(int) * (size_t)mu;
-  const size_t scatter_smem = sizeof(int) * ((size_t)mu + kTile);
-  ISDF_TRY(set_kmeans_smem_attrs());
-  int chunks = 0;
-  const int max_chunks = args.max_iter / kIterChunk + 2;
-  // One chunk = kIterChunk Lloyd iterations (10 launches each; every kernel
-  // returns at once when the loop has stopped). The chunk is captured once
-  // into a CUDA graph and replayed, which removes the per-launch host cost
-  // that dominates small solves; direct launches are the fallback when the
-  // stream cannot be captured.
-  auto launch_chunk = [&]() {
-    for (int it = 0; it < kIterChunk; ++it) {
-      k_iter_begin<<<1, 1, 0, stream>>>(b.st, max_f, args.max_iter);
-      k_hist<<<ntiles, 256, hist_smem, stream>>>(b.label, n, b.st, b.hist);
-      k_hist_scan<<<(mu + 31) / 32, 32 * kScanWarps, 0, stream>>>(b.hist, ntiles, b.st, b.members);
-      k_label_start<<<1, 1024, 0, stream>>>(b.members, b.st, b.start);
-      k_scatter<<<ntiles, 128, scatter_smem, stream>>>(b.label, n, b.st, b.hist, b.start, b.px,
-                                                       b.py, b.pz, b.pw, b.sorted);
-      k_segsum<<<mu, kFoldThreads, 0, stream>>>(b.sorted, b.start, b.members, b.px, b.py,
-                                                    b.pz, b.pw, b.label, n, npt, 1, b.st, b.sums);
-      k_centroids<<<1, 1024, cmax_smem, stream>>>(b.sums, b.st, b.cen, b.shift, b.cell_of, cg,
-                                                  b.nbshift);
-      k_build_cells<<<1, 1024, cell_smem, stream>>>(b.cen, b.st, cg, b.cell_start, b.cell_cen,
-                                                    b.cell_of);
-      k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(b.px, b.py, b.pz, b.pidx, n, b.cen,
-                                                          b.cell_start, b.cell_cen, cg, am, b.st,
-                                                          b.label, 1, b.bnd, b.shift, b.nbshift,
-                                                          b.pcell, b.pd12);
-      k_iter_end<<<1, 1, 0, stream>>>(b.st, 1);
-    }
+  // One Lloyd iteration up to the sums: six launches with the two below. Every
+  // kernel returns at once when the loop has stopped.
+  const int ntl = (cnt + kTile - 1) / kTile;
+  auto launch_sums = [&](const LoopEnd& le) {
+    k_hist<<<ntl, 256, hist_smem, stream>>>(job, le);
+    k_hist_scan<<<(mu + 31) / 32, 32 * kScanWarps, 0, stream>>>(job, le);
+    k_scatter<<<ntl, 32 * kScatterWarps, scatter_smem, stream>>>(job);
+    k_segsum<<<mu, kFoldThreads, 0, stream>>>(job);
   };
+  auto launch_assign = [&]() {
+    k_centroids<<<1, 1024, cells_smem, stream>>>(job, 1);
+    k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(job, 1);
+  };
+  // The loop is a CUDA graph: a WHILE node whose body is kBodyIters iterations,
+  // ended from the device, so that no iteration waits for the host (reading the
+  // state back after every 8 iterations left the GPU idle for 75 us each time,
+  // and the graph of 8 took twice as long to build). A stream that cannot be
+  // captured takes chunks of kIterChunk iterations and reads the state back.
+  struct LoopGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    ~LoopGraph() {
+      if (exec) cudaGraphExecDestroy(exec);
+      if (graph) cudaGraphDestroy(graph);
+    }
+  } loop;
+  if (!shard) {
+    LoopEnd le{0, 1, args.max_iter / kBodyIters * kBodyIters + 4 * kBodyIters};
+    cudaGraphNodeParams np = {};
+    cudaGraphNode_t node;
+    cudaGraph_t body = nullptr;
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    bool ok = cudaGraphCreate(&loop.graph, 0) == cudaSuccess &&
+              cudaGraphConditionalHandleCreate(&le.handle, loop.graph, 1,
+                                               cudaGraphCondAssignDefault) == cudaSuccess;
+    if (ok) {
+      np.conditional.handle = le.handle;
+      ok = cudaGraphAddNode(&node, loop.graph, nullptr, 0, &np) == cudaSuccess;
+    }
+    if (ok) {
+      body = np.conditional.phGraph_out[0];
+      ok = cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0,
+                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    }
+    if (ok) {
+      for (int it = 0; it < kBodyIters; ++it) {
+        launch_sums(le);
+        launch_assign();
+      }
+      ok = cudaStreamEndCapture(stream, &body) == cudaSuccess;
+    }
+    if (!ok || cudaGraphInstantiate(&loop.exec, loop.graph, 0ull) != cudaSuccess)
+      loop.exec = nullptr;
+    (void)cudaGetLastError();  // a refused capture leaves an error to clear
+  }
   // Sharded: the rank folds its own points [lo, lo + cnt) (utility.cpp:813-822),
   // the ranks exchange their partial sums and changed-label counts (one
   // all-gather per iteration, utility.cpp:825-826,908-917), and every rank
   // combines them in the same order, so that all ranks hold the same
-  // centroids without a broadcast. Its collectives keep the chunk out of a
+  // centroids without a broadcast. Its collectives keep the loop out of a
   // CUDA graph.
-  const int ntl = (cnt + kTile - 1) / kTile;
-  const int npt_loc = std::max(0, std::min(npt - lo, cnt));
   const size_t rec_bytes = sizeof(double4) * ((size_t)mu + 1);
   std::vector<size_t> rcounts(ranks, rec_bytes), rdispls(ranks);
   for (int q = 0; q < ranks; ++q) rdispls[q] = (size_t)q * rec_bytes;
-  auto launch_chunk_sharded = [&]() -> int {
+  const LoopEnd no_graph{0, 0, 0x7fffffff};
+  auto launch_chunk = [&]() -> int {
     for (int it = 0; it < kIterChunk; ++it) {
-      k_hist<<<ntl, 256, hist_smem, stream>>>(b.label + lo, cnt, b.st, b.hist);
-      k_hist_scan<<<(mu + 31) / 32, 32 * kScanWarps, 0, stream>>>(b.hist, ntl, b.st, b.members);
-      k_label_start<<<1, 1024, 0, stream>>>(b.members, b.st, b.start);
-      k_scatter<<<ntl, 128, scatter_smem, stream>>>(b.label + lo, cnt, b.st, b.hist, b.start,
-                                                    b.px + lo, b.py + lo, b.pz + lo, b.pw + lo,
-                                                    b.sorted);
-      k_segsum<<<mu, kFoldThreads, 0, stream>>>(b.sorted, b.start, b.members, b.px + lo,
-                                                    b.py + lo, b.pz + lo, b.pw + lo, b.label + lo,
-                                                    cnt, npt_loc, 0, b.st, sb.send + 1);
-      k_shard_header<<<1, 1, 0, stream>>>(b.st, sb.send);
-      ISDF_CHECK_LAUNCH();
-      ISDF_TRY(shard->allgatherv(sb.send, rec_bytes, sb.recv, rcounts.data(), rdispls.data(),
-                                 stream));
-      k_shard_begin<<<1, 1, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, max_f, args.max_iter);
-      k_shard_sums<<<grid_for(mu, 128), 128, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, b.sums);
-      k_centroids<<<1, 1024, cmax_smem, stream>>>(b.sums, b.st, b.cen, b.shift, b.cell_of, cg,
-                                                  b.nbshift);
-      k_build_cells<<<1, 1024, cell_smem, stream>>>(b.cen, b.st, cg, b.cell_start, b.cell_cen,
-                                                    b.cell_of);
-      k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(b.px, b.py, b.pz, b.pidx, n, b.cen,
-                                                          b.cell_start, b.cell_cen, cg, am, b.st,
-                                                          b.label, 1, b.bnd, b.shift, b.nbshift,
-                                                          b.pcell, b.pd12);
-      k_iter_end<<<1, 1, 0, stream>>>(b.st, 0);
+      launch_sums(no_graph);
+      if (shard) {
+        k_shard_header<<<1, 1, 0, stream>>>(b.st, sb.send);
+        ISDF_CHECK_LAUNCH();
+        ISDF_TRY(shard->allgatherv(sb.send, rec_bytes, sb.recv, rcounts.data(), rdispls.data(),
+                                   stream));
+        k_shard_begin<<<1, 1, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, job.max_f,
+                                           args.max_iter);
+        k_shard_sums<<<grid_for(mu, 128), 128, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, b.sums);
+      }
+      launch_assign();
       ISDF_CHECK_LAUNCH();
     }
     return ISDF_OK;
   };
-  cudaGraphExec_t exec = nullptr;
-  if (!shard) {
-    cudaGraph_t graph = nullptr;
-    if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-      launch_chunk();
-      if (cudaStreamEndCapture(stream, &graph) == cudaSuccess && graph) {
-        if (cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) exec = nullptr;
-        cudaGraphDestroy(graph);
-      }
+  int chunks = 0;
+  const int max_chunks = args.max_iter / kIterChunk + 2;
+  if (loop.exec) {
+    ISDF_CUDA(cudaGraphLaunch(loop.exec, stream));
+  } else {
+    for (;;) {
+      ISDF_TRY(launch_chunk());
+      ISDF_TRY(read_back(&hst, b.st, sizeof(KmState), stream));
+      if (hst.done) break;
+      if (++chunks > max_chunks) return record_error(ISDF_ERR_CUDA, "kmeans: loop did not stop");
     }
-    (void)cudaGetLastError();  // a refused capture leaves an error to clear
   }
-  struct ExecGuard {
-    cudaGraphExec_t e;
-    ~ExecGuard() {
-      if (e) cudaGraphExecDestroy(e);
-    }
-  } guard{exec};
-  for (;;) {
-    if (shard) ISDF_TRY(launch_chunk_sharded());
-    else if (exec) ISDF_CUDA(cudaGraphLaunch(exec, stream));
-    else launch_chunk();
-    ISDF_CHECK_LAUNCH();
-    ISDF_TRY(read_back(&hst, b.st, sizeof(KmState), stream));
-    if (hst.done) break;
-    if (++chunks > max_chunks) return record_error(ISDF_ERR_CUDA, "kmeans: loop did not stop");
-  }
-  res->iters = hst.s;
-  res->search_frac = (double)hst.searches / ((double)cnt * (hst.s + 1));
-  // + the state, per-chunk and selection reads through the mapped mailbox
-  res->launches =
-      4 + 4 + (am.g2p ? 1 : 0) + (chunks + 1) * kIterChunk * (shard ? 12 : 10) + 2 +
-      (readback_mailbox() ? chunks + 3 : 0);
-  const int rk = hst.rk;
 
-  if (!shard) {
-    dim3 fgrid((unsigned)((rk + 127) / 128), (unsigned)nchunks);
+  // the nearest point to every centroid
+  if (!shard && am.brick) {
+    k_final_near<<<grid_for(mu, 4), 128, 0, stream>>>(job, dx0, dx1, dx2, b.sel);
+  } else if (!shard) {
+    dim3 fgrid((unsigned)((mu + 127) / 128), (unsigned)nchunks);
     k_final_partial<<<fgrid, 128, 0, stream>>>(b.px, b.py, b.pz, n, b.cen, b.st, b.part_d,
                                                b.part_i);
-    k_final_reduce<<<grid_for(rk, 128), 128, 0, stream>>>(b.part_d, b.part_i, nchunks, b.st,
+    k_final_reduce<<<grid_for(mu, 128), 128, 0, stream>>>(b.part_d, b.part_i, nchunks, b.st,
                                                           b.pidx, b.sel);
   } else {
     // each rank's first minimum over its points, then MINLOC over the ranks
+    const int rk = hst.rk;
     const int nch = (cnt + kFinalChunk - 1) / kFinalChunk;
     dim3 fgrid((unsigned)((rk + 127) / 128), (unsigned)nch);
     k_final_partial<<<fgrid, 128, 0, stream>>>(b.px + lo, b.py + lo, b.pz + lo, cnt, b.cen, b.st,
@@ -1738,23 +1966,21 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
     k_minloc<<<grid_for(rk, 128), 128, 0, stream>>>(sb.frecv, ranks, mu, b.st, b.sel);
   }
   ISDF_CHECK_LAUNCH();
-  std::vector<int> sel(rk);
-  ISDF_TRY(read_back(sel.data(), b.sel, sizeof(int) * (size_t)rk, stream));
-  // unique (utility.cpp:617-629) and piv (utility.cpp:973-983)
-  std::sort(sel.begin(), sel.end());
-  sel.erase(std::unique(sel.begin(), sel.end()), sel.end());
-  const int rk_eff = (int)sel.size();
-  int k0 = 0, k1 = 0;
-  for (int i = 0; i < n; i++) {
-    if (i == sel[k0]) {
-      args.piv[k0] = i;
-      k0 = std::min(k0 + 1, rk_eff - 1);
-    } else {
-      args.piv[rk_eff + k1] = i;
-      k1++;
-    }
-  }
-  res->rk_eff = rk_eff;
+  // the caller's piv is paged in while the loop runs
+  std::memset(args.piv, 0, sizeof(int) * (size_t)n);
+  std::vector<char> out(sizeof(KmState) + sizeof(int) * (size_t)mu);
+  ISDF_TRY(read_back(out.data(), b.st, out.size(), stream));
+  std::memcpy(&hst, out.data(), sizeof(KmState));
+  if (!hst.done) return record_error(ISDF_ERR_CUDA, "kmeans: loop did not stop");
+  std::vector<int> sel(hst.rk);
+  std::memcpy(sel.data(), out.data() + sizeof(KmState), sizeof(int) * sel.size());
+  res->rk_eff = piv_from_selection(sel, n, args.piv);
+  res->iters = hst.s;
+  res->search_frac = (double)hst.searches / ((double)cnt * (hst.s + 1));
+  // filter, points, cells, first assignment, the loop's bodies, the final
+  // search, and the reads through the mapped mailbox
+  res->launches = 4 + 4 + (am.g2p ? 1 : 0) + hst.rounds * (shard ? 9 : 6) + (am.brick && !shard ? 1 : 2) +
+                  (readback_mailbox() ? chunks + 2 : 0);
   return ISDF_OK;
 }
 
@@ -2085,25 +2311,6 @@ int batch_group(long long n) {
 }
 
 }  // namespace
-
-// piv = [distinct selected points ascending | the rest ascending]
-// (unique, utility.cpp:617-629, and utility.cpp:973-983); returns rk_eff.
-static int piv_from_selection(std::vector<int>& sel, int n, int* piv) {
-  std::sort(sel.begin(), sel.end());
-  sel.erase(std::unique(sel.begin(), sel.end()), sel.end());
-  const int rk_eff = (int)sel.size();
-  int k0 = 0, k1 = 0;
-  for (int i = 0; i < n; i++) {
-    if (i == sel[k0]) {
-      piv[k0] = i;
-      k0 = std::min(k0 + 1, rk_eff - 1);
-    } else {
-      piv[rk_eff + k1] = i;
-      k1++;
-    }
-  }
-  return rk_eff;
-}
 
 size_t kmeans_batch_workspace_bytes(long long ng, int mu) {
   (void)mu;

@@ -273,3 +273,24 @@ def test_select_search_extremes_match_oracle(torch_cuda, ng, scale):
                                             torch.from_numpy(w).cuda(), mu, 12, rand_seed=1)
         assert (rk, it) == (rk_o, it_o)
         assert np.array_equal(piv, piv_o)
+
+
+@pytest.mark.parametrize("mu", [2, 33, 700])
+@pytest.mark.parametrize("ng", [(16, 16, 8), (40, 52, 1), (2051, 1, 1), (13, 17, 29)])
+def test_select_empty_clusters_match_oracle(torch_cuda, ng, mu):
+    """Empty-cluster compaction, counting-sort tiles with remainders and the
+    nearest-point boxes: points with a few distinct places only (most weights
+    dropped or the centroids' first points far from the rest), so that clusters
+    empty at once; iteration caps of 0, 1, odd and even."""
+    torch = torch_cuda
+    n = ng[0] * ng[1] * ng[2]
+    length = (4.0, 5.0, 6.0)
+    rng = np.random.default_rng(n + mu)
+    w = rng.uniform(0.5, 1.0, n) * np.exp(-rng.uniform(0.0, 17.0, n))
+    w[mu // 2:mu] = 2.0 ** -30  # dropped or nearly so: centroids next to others
+    for iters in (0, 1, 2, 7):
+        piv_o, rk_o, it_o = port.kmeans(w, ng, length, mu, iters)
+        piv, rk, it, _ = isdf.kmeans_select(isdf.Domain(length=length, num_grid=ng),
+                                            torch.from_numpy(w).cuda(), mu, iters, rand_seed=1)
+        assert (rk, it) == (rk_o, it_o)
+        assert np.array_equal(piv, piv_o)
