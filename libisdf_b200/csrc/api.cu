@@ -1,5 +1,6 @@
 // C ABI of libisdf_b200 (include/isdf_c.h): argument checks, the per-device
 // workspace, the stream, and the stage order of one ISDF solve.
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -414,8 +415,9 @@ int isdf_kmeans_select_batch(int count, const isdf_domain_t* doms, const double*
     if (count <= 0 || !doms || !d_w || !mu || !max_iter || !piv)
       return record_error(ISDF_ERR_ARG, "kmeans batch: null argument");
     std::vector<KmeansArgs> args(count);
-    size_t need = 4096;
+    size_t need = 0, group = 4096;  // the largest group's
     for (int r = 0; r < count; ++r) {
+      if (r % kKmeansBatchGroup == 0) group = 4096;
       const isdf_domain_t& d = doms[r];
       const long long ng = (long long)d.num_grid[0] * d.num_grid[1] * d.num_grid[2];
       if (!d_w[r] || !piv[r] || d.num_grid[0] <= 0 || d.num_grid[1] <= 0 || d.num_grid[2] <= 0 ||
@@ -432,7 +434,8 @@ int isdf_kmeans_select_batch(int count, const isdf_domain_t* doms, const double*
       a.max_iter = max_iter[r];
       a.rand_seed = rand_seed;
       a.piv = piv[r];
-      need += kmeans_batch_workspace_bytes(ng, mu[r]);
+      group += kmeans_batch_workspace_bytes(ng, mu[r]);
+      need = std::max(need, group);
     }
     std::lock_guard<std::mutex> lock(workspace_mutex());
     Arena arena;

@@ -275,8 +275,11 @@ struct AssignMap {
   const int* g2p;  // grid index -> kept-point index (or -1); nullptr: identity
 };
 
-// One selection as the kernels of a Lloyd iteration see it. They take the job
-// by value and loop over nothing: every buffer is the selection's own.
+// One selection as the kernels of a Lloyd iteration see it: every buffer is the
+// selection's own. The kernels take a batch of them by value and a job per
+// blockIdx.y, its grid sized for the largest: one selection alone (N = 1), or
+// the small ones of a batch side by side, which leave most of the GPU idle one
+// by one.
 struct KmJob {
   const int* pidx;
   const double *px, *py, *pz;
@@ -302,8 +305,16 @@ struct KmJob {
   int f_n, f_npt;  // how many, and how many of them are kept points
   double4* f_sums;
   int sharded;
+  int* sel;      // grid index of the nearest point to each centroid
+  double dx[3];  // grid spacings
   double max_f;  // the loop goes on while more labels than this change
   int max_iter;
+};
+
+constexpr int kBatchJobs = kKmeansBatchGroup;  // selections per launch (6.5 KB of parameters)
+template <int N>
+struct KmJobs {
+  KmJob j[N];
 };
 
 __device__ __forceinline__ int assign_point(long long t, const AssignMap& am) {
@@ -477,8 +488,10 @@ __device__ __forceinline__ int first_seed(int p, int rk, const int* __restrict__
   return j >= 0 && j < rk ? j : rk - 1;
 }
 
+template <int N>
 __global__ void __launch_bounds__(kAssignThreads)
-    k_assign_warp(const __grid_constant__ KmJob J, int count) {
+    k_assign_warp(const __grid_constant__ KmJobs<N> JS, int count) {
+  const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (st->done) return;
   const double *px = J.px, *py = J.py, *pz = J.pz;
@@ -683,7 +696,8 @@ __device__ __forceinline__ bool goes_on(const KmJob& J) {
 struct LoopEnd {
   cudaGraphConditionalHandle handle;
   int in_graph;
-  int max_rounds;  // bodies after which the loop ends whatever happens
+  int max_rounds;  // iterations after which the loop ends whatever happens
+  int* live;       // selections of a batch still running (nullptr: one)
 };
 
 __device__ __forceinline__ void end_loop(const LoopEnd& le) {
@@ -695,10 +709,12 @@ __device__ __forceinline__ void end_loop(const LoopEnd& le) {
 // one warp per cluster and component folds w, w*x, w*y, w*z over the members
 // in increasing point index: the exact sequence of additions of
 // utility.cpp:816-822.
-__global__ void __launch_bounds__(256) k_hist(const __grid_constant__ KmJob J, const LoopEnd le) {
+template <int N>
+__global__ void __launch_bounds__(256) k_hist(const __grid_constant__ KmJobs<N> JS, const LoopEnd le) {
+  const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (blockIdx.x == 0 && threadIdx.x == 0 && ++st->rounds > le.max_rounds) end_loop(le);
-  if (st->done || !goes_on(J)) return;
+  if (st->done || !goes_on(J) || blockIdx.x * kTile >= J.f_n) return;
   extern __shared__ int sh[];
   const int rk = st->rk;
   for (int l = threadIdx.x; l < rk; l += blockDim.x) sh[l] = 0;
@@ -721,14 +737,16 @@ __global__ void __launch_bounds__(256) k_hist(const __grid_constant__ KmJob J, c
 // launch where three single-block kernels ran.
 constexpr int kScanWarps = 16;
 
+template <int N>
 __global__ void __launch_bounds__(32 * kScanWarps)
-    k_hist_scan(const __grid_constant__ KmJob J, const LoopEnd le) {
+    k_hist_scan(const __grid_constant__ KmJobs<N> JS, const LoopEnd le) {
+  const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (st->done) return;
   if (!goes_on(J)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       st->done = 1;
-      end_loop(le);
+      if (!le.live || atomicSub(le.live, 1) == 1) end_loop(le);
     }
     return;
   }
@@ -817,10 +835,12 @@ __global__ void __launch_bounds__(32 * kScanWarps)
 // whatever their number, and this takes 5.
 constexpr int kScatterWarps = 8;
 
+template <int N>
 __global__ void __launch_bounds__(32 * kScatterWarps)
-    k_scatter(const __grid_constant__ KmJob J) {
+    k_scatter(const __grid_constant__ KmJobs<N> JS) {
+  const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   const KmState* st = J.st;
-  if (st->done) return;
+  if (st->done || blockIdx.x * kTile >= J.f_n) return;
   extern __shared__ __align__(16) unsigned short cnt[];  // [label][warp]
   const int rk = st->rk;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1007,7 +1027,9 @@ __device__ __forceinline__ double fold_serial(const double* comp, int cnt, doubl
 // their part of the fold is a repeated addition of one value (repeat_add).
 constexpr int kFoldThreads = 128;
 
-__global__ void __launch_bounds__(kFoldThreads) k_segsum(const __grid_constant__ KmJob J) {
+template <int N>
+__global__ void __launch_bounds__(kFoldThreads) k_segsum(const __grid_constant__ KmJobs<N> JS) {
+  const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (st->done) return;
   const int n = J.f_n, npt = J.f_npt;
@@ -1122,7 +1144,9 @@ __device__ int compact_empty(const double4* __restrict__ sums, int rk, double4* 
 // a centroid that sat in its 3^3 and 5^3 neighbourhoods before the update
 // (cell_of still holds the previous positions' cells there).
 // update = 0: the cells alone (the first centroids).
-__global__ void __launch_bounds__(1024) k_centroids(const __grid_constant__ KmJob J, int update) {
+template <int N>
+__global__ void __launch_bounds__(1024) k_centroids(const __grid_constant__ KmJobs<N> JS, int update) {
+  const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (st->done) return;
   extern __shared__ unsigned cmax[];  // 3 x ncells + 1 words
@@ -1290,16 +1314,17 @@ __global__ void k_final_reduce(const double* __restrict__ part_d, const int* __r
 // or the box is the grid. The zero tail's first point (a copy of grid point 0)
 // is compared once. A few points per centroid instead of all of them: 20 us
 // against 1.6 ms at 884 736 points and 2979 centroids.
+template <int N>
 __global__ void __launch_bounds__(128)
-    k_final_near(const __grid_constant__ KmJob J, const double dx, const double dy,
-                 const double dz, int* __restrict__ sel) {
+    k_final_near(const __grid_constant__ KmJobs<N> JS) {
+  const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   const int rk = J.st->rk;
   const int j = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (j >= rk) return;
   const double4 c = J.cen[j];
   const AssignMap& am = J.am;
   const int n3[3] = {am.nx, am.ny, am.nz};
-  const double cc[3] = {c.x, c.y, c.z}, h3[3] = {dx, dy, dz};
+  const double cc[3] = {c.x, c.y, c.z}, h3[3] = {J.dx[0], J.dx[1], J.dx[2]};
   const double inf = __longlong_as_double(0x7ff0000000000000LL);
   double best = inf;
   int bp = 0;
@@ -1355,7 +1380,7 @@ __global__ void __launch_bounds__(128)
     }
     if (all || (margin > 0.0 && best < margin * margin * (1.0 - 1e-12))) break;
   }
-  if (lane == 0) sel[j] = J.pidx[bp];
+  if (lane == 0) J.sel[j] = J.pidx[bp];
 }
 
 // ---------------------------------------------------------------- sharded
@@ -1464,12 +1489,16 @@ int set_kmeans_smem_attrs() {
   int dev = 0;
   ISDF_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && done[dev]) return ISDF_OK;
-  ISDF_CUDA(cudaFuncSetAttribute(k_hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  ISDF_CUDA(cudaFuncSetAttribute(k_hist<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(int) * kKmeansMaxMu)));
-  ISDF_CUDA(cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  ISDF_CUDA(cudaFuncSetAttribute(k_scatter<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(short) * kScatterWarps * kKmeansMaxMu)));
-  ISDF_CUDA(cudaFuncSetAttribute(k_centroids, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(unsigned) * (3 * kMaxCells + 1))));
+  // (a batch's histograms, kKmeansBatchMaxMu labels at most, need no opt-in)
+  const int cells = (int)(sizeof(unsigned) * (3 * kMaxCells + 1));
+  ISDF_CUDA(cudaFuncSetAttribute(k_centroids<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 cells));
+  ISDF_CUDA(cudaFuncSetAttribute(k_centroids<kBatchJobs>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, cells));
   if (dev >= 0 && dev < 64) done[dev] = true;
   return ISDF_OK;
 }
@@ -1550,6 +1579,163 @@ ShardBuffers carve_shard(Arena& a, int mu, int ranks) {
   b.frecv = a.take<double2>((size_t)ranks * mu);
   return b;
 }
+
+// The cell grid of the pruned assignment: about 1.5 centroids per cell.
+CellGrid cell_grid(const KmeansArgs& args) {
+  CellGrid cg;
+  const int nc = std::max(1, std::min((int)std::lround(std::cbrt(args.mu / 1.5)), kMaxCellsPerDim));
+  cg.nc = nc;
+  double lmax = 0.0;
+  for (int i = 0; i < 3; ++i) {
+    cg.h[i] = args.length[i] / nc;
+    lmax = std::max(lmax, std::fabs(args.length[i]));
+  }
+  cg.tol = 1e-9 * lmax;
+  return cg;
+}
+
+// The job of a whole selection (a sharded one narrows its fold afterwards);
+// am: its thread -> point map.
+KmJob make_job(const KmeansArgs& args, const KmBuffers& b, const CellGrid& cg,
+               const AssignMap& am, int npt) {
+  const int n = (int)args.ng;
+  KmJob job{};
+  job.pidx = b.pidx;
+  job.px = b.px;
+  job.py = b.py;
+  job.pz = b.pz;
+  job.label = b.label;
+  job.n = n;
+  job.sorted = b.sorted;
+  job.cen = b.cen;
+  job.sums = b.sums;
+  job.hist = b.hist;
+  job.members = b.members;
+  job.start = b.start;
+  job.bnd = b.bnd;
+  job.shift = b.shift;
+  job.nbshift = b.nbshift;
+  job.st = b.st;
+  job.cell_start = b.cell_start;
+  job.cell_cen = b.cell_cen;
+  job.cell_of = b.cell_of;
+  job.pcell = b.pcell;
+  job.pd12 = b.pd12;
+  job.cg = cg;
+  job.am = am;
+  job.f_label = b.label;
+  job.fx = b.px;
+  job.fy = b.py;
+  job.fz = b.pz;
+  job.fw = b.pw;
+  job.f_n = n;
+  job.f_npt = npt;
+  job.f_sums = b.sums;
+  job.sel = b.sel;
+  for (int i = 0; i < 3; ++i) job.dx[i] = args.length[i] / args.num_grid[i];
+  job.max_f = 1e-5 * n;  // KmeansTolerance * n (utility.cpp:812)
+  job.max_iter = args.max_iter;
+  return job;
+}
+
+// The map of a whole selection's points (one rank).
+AssignMap brick_map(const KmeansArgs& args, int npt) {
+  const int n = (int)args.ng;
+  AssignMap am{};
+  am.nx = args.num_grid[0];
+  am.ny = args.num_grid[1];
+  am.nz = args.num_grid[2];
+  am.nbx = (am.nx + 3) / 4;
+  am.nby = (am.ny + 3) / 4;
+  am.nbt = (long long)am.nbx * am.nby * ((am.nz + 1) / 2) * 32;
+  am.t0 = 0;
+  am.npt = npt;
+  am.n = n;
+  am.p_lo = 0;
+  am.p_hi = n;
+  am.brick = ((long long)am.nx * am.ny * am.nz == n && am.nbt + n < 0x7fffffffLL);
+  am.g2p = nullptr;
+  return am;
+}
+
+// Grid sizes of the kernels of an iteration: each for the largest of its jobs.
+struct LoopDims {
+  unsigned jobs = 0, tiles = 0, mu = 0, assign = 0;
+  size_t cells_smem = 0;
+
+  void add(const KmJob& job, int mu_, unsigned assign_blocks) {
+    ++jobs;
+    tiles = std::max(tiles, (unsigned)((job.f_n + kTile - 1) / kTile));
+    mu = std::max(mu, (unsigned)mu_);
+    assign = std::max(assign, assign_blocks);
+    const size_t ncells = (size_t)job.cg.nc * job.cg.nc * job.cg.nc;
+    cells_smem = std::max(cells_smem, sizeof(unsigned) * (3 * ncells + 1));
+  }
+};
+
+// One Lloyd iteration is six launches: the sums, then the centroids and the
+// labels. Every kernel returns at once where the loop has stopped.
+template <int N>
+void launch_sums(const KmJobs<N>& J, const LoopDims& d, const LoopEnd& le, cudaStream_t s) {
+  const size_t hist_smem = sizeof(int) * (size_t)d.mu;
+  const size_t scatter_smem = sizeof(short) * kScatterWarps * (size_t)d.mu;
+  k_hist<N><<<dim3(d.tiles, d.jobs), 256, hist_smem, s>>>(J, le);
+  k_hist_scan<N><<<dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, 0, s>>>(J, le);
+  k_scatter<N><<<dim3(d.tiles, d.jobs), 32 * kScatterWarps, scatter_smem, s>>>(J);
+  k_segsum<N><<<dim3(d.mu, d.jobs), kFoldThreads, 0, s>>>(J);
+}
+
+template <int N>
+void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, cudaStream_t s) {
+  k_centroids<N><<<dim3(1, d.jobs), 1024, d.cells_smem, s>>>(J, update);
+  k_assign_warp<N><<<dim3(d.assign, d.jobs), kAssignThreads, 0, s>>>(J, update);
+}
+
+// The loop as a CUDA graph: a WHILE node whose body is kBodyIters iterations,
+// ended from the device, so that no iteration waits for the host (reading the
+// state back after every 8 iterations left the GPU idle for 75 us each time,
+// and the graph of 8 took twice as long to build). exec stays null on a stream
+// that cannot be captured.
+struct LoopGraph {
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  ~LoopGraph() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+  }
+
+  template <int N>
+  void build(const KmJobs<N>& J, const LoopDims& d, int max_iter, int* live, cudaStream_t s) {
+    LoopEnd le{0, 1, max_iter / kBodyIters * kBodyIters + 4 * kBodyIters, live};
+    cudaGraphNodeParams np = {};
+    cudaGraphNode_t node;
+    cudaGraph_t body = nullptr;
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess &&
+              cudaGraphConditionalHandleCreate(&le.handle, graph, 1,
+                                               cudaGraphCondAssignDefault) == cudaSuccess;
+    if (ok) {
+      np.conditional.handle = le.handle;
+      ok = cudaGraphAddNode(&node, graph, nullptr, 0, &np) == cudaSuccess;
+    }
+    if (ok) {
+      body = np.conditional.phGraph_out[0];
+      ok = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0,
+                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    }
+    if (ok) {
+      for (int it = 0; it < kBodyIters; ++it) {
+        launch_sums(J, d, le, s);
+        launch_assign(J, d, 1, s);
+      }
+      ok = cudaStreamEndCapture(s, &body) == cudaSuccess;
+    }
+    if (!ok || cudaGraphInstantiate(&exec, graph, 0ull) != cudaSuccess) exec = nullptr;
+    (void)cudaGetLastError();  // a refused capture leaves an error to clear
+  }
+};
 
 }  // namespace
 
@@ -1748,32 +1934,10 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
     init.maxw_bits = hst.maxw_bits;
     ISDF_CUDA(cudaMemcpyAsync(b.st, &init, sizeof(KmState), cudaMemcpyHostToDevice, stream));
   }
-  CellGrid cg;
-  {
-    int nc = (int)std::lround(std::cbrt(mu / 1.5));
-    nc = std::max(1, std::min(nc, kMaxCellsPerDim));
-    cg.nc = nc;
-    double lmax = 0.0;
-    for (int i = 0; i < 3; ++i) {
-      cg.h[i] = args.length[i] / nc;
-      lmax = std::max(lmax, std::fabs(args.length[i]));
-    }
-    cg.tol = 1e-9 * lmax;
-  }
-  AssignMap am{};
-  am.nx = args.num_grid[0];
-  am.ny = args.num_grid[1];
-  am.nz = args.num_grid[2];
-  am.nbx = (am.nx + 3) / 4;
-  am.nby = (am.ny + 3) / 4;
-  am.nbt = (long long)am.nbx * am.nby * ((am.nz + 1) / 2) * 32;
-  am.t0 = 0;
-  am.npt = npt;
-  am.n = n;
+  const CellGrid cg = cell_grid(args);
+  AssignMap am = brick_map(args, npt);
   am.p_lo = lo;
   am.p_hi = lo + cnt;
-  am.brick = ((long long)am.nx * am.ny * am.nz == n && am.nbt + n < 0x7fffffffLL);
-  am.g2p = nullptr;
   if (am.brick && npt < n) {
     ISDF_CUDA(cudaMemsetAsync(b.g2p, 0xff, sizeof(int) * (size_t)n, stream));
     k_grid_to_point<<<grid_for(npt, 256), 256, 0, stream>>>(b.pidx, npt, b.g2p);
@@ -1799,107 +1963,27 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   const unsigned pgrid = am.brick ? grid_for(am.nbt + tail_loc, kAssignThreads)
                                   : grid_for(cnt, kAssignThreads);
   k_point_cells<<<grid_for(n, 256), 256, 0, stream>>>(b.px, b.py, b.pz, n, cg, b.pcell, b.pd12);
-  KmJob job{};
-  job.pidx = b.pidx;
-  job.px = b.px;
-  job.py = b.py;
-  job.pz = b.pz;
-  job.label = b.label;
-  job.n = n;
-  job.sorted = b.sorted;
-  job.cen = b.cen;
-  job.sums = b.sums;
-  job.hist = b.hist;
-  job.members = b.members;
-  job.start = b.start;
-  job.bnd = b.bnd;
-  job.shift = b.shift;
-  job.nbshift = b.nbshift;
-  job.st = b.st;
-  job.cell_start = b.cell_start;
-  job.cell_cen = b.cell_cen;
-  job.cell_of = b.cell_of;
-  job.pcell = b.pcell;
-  job.pd12 = b.pd12;
-  job.cg = cg;
-  job.am = am;
-  job.f_label = b.label + lo;
-  job.fx = b.px + lo;
-  job.fy = b.py + lo;
-  job.fz = b.pz + lo;
-  job.fw = b.pw + lo;
-  job.f_n = cnt;
-  job.f_npt = std::max(0, std::min(npt - lo, cnt));
-  job.f_sums = shard ? sb.send + 1 : b.sums;
-  job.sharded = shard ? 1 : 0;
-  job.max_f = 1e-5 * n;  // KmeansTolerance * n (utility.cpp:812)
-  job.max_iter = args.max_iter;
-
-  const size_t cells_smem = sizeof(unsigned) * (3 * (size_t)cg.nc * cg.nc * cg.nc + 1);
-  const size_t hist_smem = sizeof(int) * (size_t)mu;
-  const size_t scatter_smem = sizeof(short) * kScatterWarps * (size_t)mu;
-  ISDF_TRY(set_kmeans_smem_attrs());
-  k_centroids<<<1, 1024, cells_smem, stream>>>(job, 0);
-  k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(job, 0);
-  ISDF_CHECK_LAUNCH();
-
-  // One Lloyd iteration up to the sums: six launches with the two below. Every
-  // kernel returns at once when the loop has stopped.
-  const int ntl = (cnt + kTile - 1) / kTile;
-  auto launch_sums = [&](const LoopEnd& le) {
-    k_hist<<<ntl, 256, hist_smem, stream>>>(job, le);
-    k_hist_scan<<<(mu + 31) / 32, 32 * kScanWarps, 0, stream>>>(job, le);
-    k_scatter<<<ntl, 32 * kScatterWarps, scatter_smem, stream>>>(job);
-    k_segsum<<<mu, kFoldThreads, 0, stream>>>(job);
-  };
-  auto launch_assign = [&]() {
-    k_centroids<<<1, 1024, cells_smem, stream>>>(job, 1);
-    k_assign_warp<<<pgrid, kAssignThreads, 0, stream>>>(job, 1);
-  };
-  // The loop is a CUDA graph: a WHILE node whose body is kBodyIters iterations,
-  // ended from the device, so that no iteration waits for the host (reading the
-  // state back after every 8 iterations left the GPU idle for 75 us each time,
-  // and the graph of 8 took twice as long to build). A stream that cannot be
-  // captured takes chunks of kIterChunk iterations and reads the state back.
-  struct LoopGraph {
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    ~LoopGraph() {
-      if (exec) cudaGraphExecDestroy(exec);
-      if (graph) cudaGraphDestroy(graph);
-    }
-  } loop;
-  if (!shard) {
-    LoopEnd le{0, 1, args.max_iter / kBodyIters * kBodyIters + 4 * kBodyIters};
-    cudaGraphNodeParams np = {};
-    cudaGraphNode_t node;
-    cudaGraph_t body = nullptr;
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    bool ok = cudaGraphCreate(&loop.graph, 0) == cudaSuccess &&
-              cudaGraphConditionalHandleCreate(&le.handle, loop.graph, 1,
-                                               cudaGraphCondAssignDefault) == cudaSuccess;
-    if (ok) {
-      np.conditional.handle = le.handle;
-      ok = cudaGraphAddNode(&node, loop.graph, nullptr, 0, &np) == cudaSuccess;
-    }
-    if (ok) {
-      body = np.conditional.phGraph_out[0];
-      ok = cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0,
-                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-    }
-    if (ok) {
-      for (int it = 0; it < kBodyIters; ++it) {
-        launch_sums(le);
-        launch_assign();
-      }
-      ok = cudaStreamEndCapture(stream, &body) == cudaSuccess;
-    }
-    if (!ok || cudaGraphInstantiate(&loop.exec, loop.graph, 0ull) != cudaSuccess)
-      loop.exec = nullptr;
-    (void)cudaGetLastError();  // a refused capture leaves an error to clear
+  KmJobs<1> jobs;
+  KmJob& job = jobs.j[0];
+  job = make_job(args, b, cg, am, npt);
+  if (shard) {
+    job.f_label += lo;
+    job.fx += lo;
+    job.fy += lo;
+    job.fz += lo;
+    job.fw += lo;
+    job.f_n = cnt;
+    job.f_npt = std::max(0, std::min(npt - lo, cnt));
+    job.f_sums = sb.send + 1;
+    job.sharded = 1;
   }
+  LoopDims dims;
+  dims.add(job, mu, pgrid);
+  ISDF_TRY(set_kmeans_smem_attrs());
+  launch_assign(jobs, dims, 0, stream);
+  ISDF_CHECK_LAUNCH();
+  LoopGraph loop;
+  if (!shard) loop.build(jobs, dims, args.max_iter, nullptr, stream);
   // Sharded: the rank folds its own points [lo, lo + cnt) (utility.cpp:813-822),
   // the ranks exchange their partial sums and changed-label counts (one
   // all-gather per iteration, utility.cpp:825-826,908-917), and every rank
@@ -1909,10 +1993,10 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   const size_t rec_bytes = sizeof(double4) * ((size_t)mu + 1);
   std::vector<size_t> rcounts(ranks, rec_bytes), rdispls(ranks);
   for (int q = 0; q < ranks; ++q) rdispls[q] = (size_t)q * rec_bytes;
-  const LoopEnd no_graph{0, 0, 0x7fffffff};
+  const LoopEnd no_graph{0, 0, 0x7fffffff, nullptr};
   auto launch_chunk = [&]() -> int {
     for (int it = 0; it < kIterChunk; ++it) {
-      launch_sums(no_graph);
+      launch_sums(jobs, dims, no_graph, stream);
       if (shard) {
         k_shard_header<<<1, 1, 0, stream>>>(b.st, sb.send);
         ISDF_CHECK_LAUNCH();
@@ -1922,7 +2006,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
                                            args.max_iter);
         k_shard_sums<<<grid_for(mu, 128), 128, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, b.sums);
       }
-      launch_assign();
+      launch_assign(jobs, dims, 1, stream);
       ISDF_CHECK_LAUNCH();
     }
     return ISDF_OK;
@@ -1942,7 +2026,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
 
   // the nearest point to every centroid
   if (!shard && am.brick) {
-    k_final_near<<<grid_for(mu, 4), 128, 0, stream>>>(job, dx0, dx1, dx2, b.sel);
+    k_final_near<1><<<grid_for(mu, 4), 128, 0, stream>>>(jobs);
   } else if (!shard) {
     dim3 fgrid((unsigned)((mu + 127) / 128), (unsigned)nchunks);
     k_final_partial<<<fgrid, 128, 0, stream>>>(b.px, b.py, b.pz, n, b.cen, b.st, b.part_d,
@@ -1985,365 +2069,37 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
 }
 
 // ===================================================================== batched small selections
-// Several small K-means selections in one cooperative launch (the serving
-// loop's batches of small requests): a group of G CTAs runs one request's
-// whole Lloyd loop - assignment, stable counting sort by label, sequential
-// per-cluster folds, centroid update with the empty-cluster compaction, the
-// change count and the final nearest point per centroid - with software group
-// barriers between the phases, so a batch of B requests costs one launch
-// instead of ~10 launches per iteration per request. The arithmetic and every
-// order of summation are the single-request path's (and the reference's,
-// utility.cpp:813-945): piv is the same bit for bit. The assignment is a
-// brute-force scan over the centroids held in shared memory, which suits the
-// small systems this path serves (mu <= 512).
+// Several small K-means selections at once (the serving loop's batches of small
+// requests): the kernels of kmeans_select with a job per blockIdx.y, up to
+// kBatchJobs of them, in one loop graph that ends when the last job has. A
+// small selection alone is bound by the latency of its launches, so a batch
+// costs little more than one; piv is the single selection's bit for bit, the
+// kernels being the same. Eight 36^3 systems with 256 centroids: 28.0 ms in one
+// cooperative launch of a group of CTAs per system (brute-force assignment,
+// group barriers between the phases), 8.2 ms here.
 namespace {
 
-constexpr int kBatchThreads = 256;
-constexpr int kBatchWarps = kBatchThreads / 32;
+// The states and selections of a batch lie in one block, so that one copy
+// initialises them and one reads them back.
+constexpr size_t kBatchRecord = sizeof(KmState) + sizeof(int) * kKmeansBatchMaxMu;
 
-struct KmBatchJob {
-  const double *px, *py, *pz, *pw;
-  const int* pidx;
-  int* label;
-  double4* sorted;
-  double4* cen;
-  double4* sums;
-  int* hist;   // per sub-block label counts, then each sub-block's first slot per label
-  int* tot;    // members per cluster
-  int* sel;    // grid index of the nearest point per centroid
-  int n, npt, mu, max_iter;
-  double max_f;
-  int rk, iters, err, any_empty;
-  int changed[2];
-  unsigned bar_count, bar_gen;
-};
-
-// All CTAs of one request's group meet here. Bounded: a CTA that waits
-// longer than ~1 s sets err and returns false, and so does every CTA that
-// sees err afterwards, so a failing group ends instead of hanging.
-__device__ bool group_barrier(KmBatchJob* J, int G) {
-  __shared__ int ok_s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    __threadfence();
-    const unsigned gen = *(volatile unsigned*)&J->bar_gen;
-    if (atomicAdd(&J->bar_count, 1u) == (unsigned)G - 1) {
-      J->bar_count = 0;
-      __threadfence();
-      atomicAdd(&J->bar_gen, 1u);
-    } else {
-      long long spins = 0;
-      while (*(volatile unsigned*)&J->bar_gen == gen) {
-        if (++spins > (1LL << 24)) {
-          atomicExch(&J->err, 1);
-          ok = 0;
-          break;
-        }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-    ok_s = ok && *(volatile int*)&J->err == 0;
-  }
-  __syncthreads();
-  return ok_s != 0;
-}
-
-// Loads of data that other CTAs of the launch wrote: through L2 (L1 is not
-// coherent across SMs within a kernel).
-__device__ __forceinline__ double4 ldcg4(const double4* p) {
-  const double* d = reinterpret_cast<const double*>(p);
-  return make_double4(__ldcg(d), __ldcg(d + 1), __ldcg(d + 2), __ldcg(d + 3));
-}
-
-// Exclusive scan of v[0..m) (m <= kKmeansBatchMaxMu) into out, one block.
-__device__ void block_scan(const int* v, int m, int* out) {
-  __shared__ int part[kBatchThreads];
-  const int per = (m + kBatchThreads - 1) / kBatchThreads;
-  const int lo = min(m, (int)threadIdx.x * per), hi = min(m, lo + per);
-  int t = 0;
-  for (int i = lo; i < hi; ++i) t += __ldcg(v + i);
-  part[threadIdx.x] = t;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int i = 0; i < kBatchThreads; ++i) {
-      const int x = part[i];
-      part[i] = run;
-      run += x;
-    }
-  }
-  __syncthreads();
-  int run = part[threadIdx.x];
-  for (int i = lo; i < hi; ++i) {
-    out[i] = run;
-    run += __ldcg(v + i);
-  }
-  __syncthreads();
-}
-
-__global__ void __launch_bounds__(kBatchThreads) k_kmeans_batch(KmBatchJob* jobs, int G) {
-  KmBatchJob* J = jobs + blockIdx.x / G;
-  const int c = blockIdx.x % G;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __shared__ double cx[kKmeansBatchMaxMu], cy[kKmeansBatchMaxMu], cz[kKmeansBatchMaxMu];
-  __shared__ int run[kBatchWarps][kKmeansBatchMaxMu];
-  __shared__ int sstart[kKmeansBatchMaxMu];
-  __shared__ int red[kBatchWarps];
-  const int n = J->n, npt = J->npt;
-  const int nsub = G * kBatchWarps;
-  const int per = (n + nsub - 1) / nsub;
-  const int sb = c * kBatchWarps + warp;
-  const int sb_lo = min(n, sb * per), sb_hi = min(n, sb_lo + per);
-  const int cta_lo = min(n, c * kBatchWarps * per), cta_hi = min(n, cta_lo + kBatchWarps * per);
-  volatile KmBatchJob* VJ = J;
-
-  auto load_cen = [&](int rk) {
-    for (int i = threadIdx.x; i < rk; i += kBatchThreads) {
-      const double4 q = ldcg4(J->cen + i);
-      cx[i] = q.x;
-      cy[i] = q.y;
-      cz[i] = q.z;
-    }
-    __syncthreads();
-  };
-  // labels of this CTA's points (first minimum, pdist2's rounding); returns
-  // the number of labels that changed (valid in thread 0)
-  auto assign = [&](int rk) -> int {
-    int ch = 0;
-    for (int p = cta_lo + threadIdx.x; p < cta_hi; p += kBatchThreads) {
-      const double x = J->px[p], y = J->py[p], z = J->pz[p];
-      double best = ref_dist2(x, y, z, make_double4(cx[0], cy[0], cz[0], 0.0));
-      int bj = 0;
-      for (int j = 1; j < rk; ++j) {
-        const double d = ref_dist2(x, y, z, make_double4(cx[j], cy[j], cz[j], 0.0));
-        if (d < best) {
-          best = d;
-          bj = j;
-        }
-      }
-      if (__ldcg(J->label + p) != bj) ++ch;
-      J->label[p] = bj;
-    }
-    for (int o = 16; o > 0; o >>= 1) ch += __shfl_xor_sync(0xffffffffu, ch, o);
-    if (lane == 0) red[warp] = ch;
-    __syncthreads();
-    int t = 0;
-    if (threadIdx.x == 0)
-      for (int w = 0; w < kBatchWarps; ++w) t += red[w];
-    __syncthreads();
-    return t;
-  };
-
-  int rk = J->mu;
-  load_cen(rk);
-  assign(rk);
-  if (!group_barrier(J, G)) return;
-  int flag = n, s = 0;
-  while ((double)flag > J->max_f && s < J->max_iter) {
-    const int par = s & 1;
-    // 1. label counts per sub-block (one warp each)
-    for (int k = lane; k < rk; k += 32) run[warp][k] = 0;
-    __syncwarp();
-    for (int p = sb_lo + lane; p < sb_hi; p += 32) atomicAdd(&run[warp][__ldcg(J->label + p)], 1);
-    __syncwarp();
-    for (int k = lane; k < rk; k += 32) J->hist[(size_t)sb * kKmeansBatchMaxMu + k] = run[warp][k];
-    if (!group_barrier(J, G)) return;
-    // 2. per cluster, each sub-block's offset within the cluster and the
-    // cluster's size (every CTA has read last iteration's change count)
-    if (c == 0 && threadIdx.x == 0) {
-      VJ->changed[par ^ 1] = 0;
-      VJ->any_empty = 0;
-    }
-    for (int k = c + G * threadIdx.x; k < rk; k += G * kBatchThreads) {
-      int acc = 0;
-      for (int q = 0; q < nsub; ++q) {
-        int* h = J->hist + (size_t)q * kKmeansBatchMaxMu + k;
-        const int v = __ldcg(h);
-        *h = acc;
-        acc += v;
-      }
-      J->tot[k] = acc;
-    }
-    if (!group_barrier(J, G)) return;
-    // 3. stable scatter of (w x, w y, w z, w) into cluster order
-    block_scan(J->tot, rk, sstart);
-    for (int k = lane; k < rk; k += 32)
-      run[warp][k] = sstart[k] + __ldcg(J->hist + (size_t)sb * kKmeansBatchMaxMu + k);
-    __syncwarp();
-    for (int base = sb_lo; base < sb_hi; base += 32) {
-      const int p = base + lane;
-      const bool ok = p < sb_hi;
-      const int l = ok ? __ldcg(J->label + p) : -1;
-      const unsigned peers = __match_any_sync(0xffffffffu, l);
-      const int b = ok ? run[warp][l] : 0;
-      __syncwarp();
-      if (ok) {
-        const double w = J->pw[p];
-        const int r = __popc(peers & ((1u << lane) - 1u));
-        J->sorted[b + r] = make_double4(rmul(w, J->px[p]), rmul(w, J->py[p]), rmul(w, J->pz[p]), w);
-        if (lane == __ffs(peers) - 1) run[warp][l] = b + __popc(peers);
-      }
-      __syncwarp();
-    }
-    if (!group_barrier(J, G)) return;
-    // 4. per cluster and component, the sequential fold in point order; the
-    // zero tail (copies of grid point 0, last in their cluster) by repeat_add
-    const int tail_label = npt < n ? __ldcg(J->label + npt) : -1;
-    for (int kq = c * kBatchThreads + threadIdx.x; kq < 4 * rk; kq += G * kBatchThreads) {
-      const int k = kq >> 2, q = kq & 3;
-      int m = __ldcg(J->tot + k);
-      long long tail = 0;
-      if (k == tail_label) {
-        tail = n - npt;
-        m -= (int)tail;
-      }
-      const double* v = reinterpret_cast<const double*>(J->sorted + sstart[k]) + q;
-      double acc = 0.0;
-      for (int e = 0; e < m; ++e) acc = radd(acc, __ldcg(v + (size_t)e * 4));
-      if (tail) {
-        const double w0 = J->pw[npt];
-        const double val = q == 3 ? w0 : rmul(w0, q == 0 ? J->px[npt] : q == 1 ? J->py[npt] : J->pz[npt]);
-        acc = repeat_add(acc, val, tail);
-      }
-      reinterpret_cast<double*>(J->sums + k)[q] = acc;
-      if (q == 3 && acc == 0.0) VJ->any_empty = 1;
-    }
-    if (!group_barrier(J, G)) return;
-    // 5. new centroids = sums / count; an empty cluster takes the last one's
-    // sums and rk shrinks (utility.cpp:831-853), in order, by one thread
-    if (c == 0) {
-      if (!VJ->any_empty) {
-        for (int i = threadIdx.x; i < rk; i += kBatchThreads) {
-          const double4 q = ldcg4(J->sums + i);
-          J->cen[i] = make_double4(rdiv(q.x, q.w), rdiv(q.y, q.w), rdiv(q.z, q.w), 0.0);
-        }
-      } else if (threadIdx.x == 0) {
-        int r = rk;
-        for (int i = 0; i < r; i++) {
-          const double4 q = ldcg4(J->sums + i);
-          if (q.w != 0.0) {
-            J->sums[i] = make_double4(rdiv(q.x, q.w), rdiv(q.y, q.w), rdiv(q.z, q.w), q.w);
-          } else {
-            r--;
-            J->sums[i] = ldcg4(J->sums + r);
-            i--;
-          }
-        }
-        for (int i = 0; i < r; i++) {
-          const double4 q = ldcg4(J->sums + i);
-          J->cen[i] = make_double4(q.x, q.y, q.z, 0.0);
-        }
-        VJ->rk = r;
-      }
-    }
-    if (!group_barrier(J, G)) return;
-    // 6. reassignment and the change count
-    rk = VJ->rk;
-    load_cen(rk);
-    const int ch = assign(rk);
-    if (threadIdx.x == 0 && ch) atomicAdd(&J->changed[par], ch);
-    if (!group_barrier(J, G)) return;
-    flag = VJ->changed[par];
-    ++s;
-  }
-  // nearest point to every centroid (first minimum over points), one warp each
-  load_cen(rk);
-  for (int j = c * kBatchWarps + warp; j < rk; j += nsub) {
-    const double4 q = make_double4(cx[j], cy[j], cz[j], 0.0);
-    double best = __longlong_as_double(0x7ff0000000000000LL);
-    int bi = 0x7fffffff;
-    for (int p = lane; p < n; p += 32) {
-      const double d = ref_dist2(J->px[p], J->py[p], J->pz[p], q);
-      if (d < best) {
-        best = d;
-        bi = p;
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ob < best || (ob == best && oi < bi)) {
-        best = ob;
-        bi = oi;
-      }
-    }
-    if (lane == 0) J->sel[j] = J->pidx[bi];
-  }
-  if (c == 0 && threadIdx.x == 0) VJ->iters = s;
-}
-
-struct BatchBuffers {
-  int* pidx;
-  double *px, *py, *pz, *pw;
-  int* label;
-  double4 *sorted, *cen, *sums;
-  int *hist, *tot, *sel, *tile_cnt;
-  KmState* st;
-};
-
-BatchBuffers carve_batch(Arena& a, int n, int G) {
-  BatchBuffers b;
-  const int nfilter = (n + 1023) / 1024;
-  b.pidx = a.take<int>(n);
-  b.px = a.take<double>(n);
-  b.py = a.take<double>(n);
-  b.pz = a.take<double>(n);
-  b.pw = a.take<double>(n);
-  b.label = a.take<int>(n);
-  b.sorted = a.take<double4>(n);
-  b.cen = a.take<double4>(kKmeansBatchMaxMu);
-  b.sums = a.take<double4>(kKmeansBatchMaxMu);
-  b.hist = a.take<int>((size_t)G * kBatchWarps * kKmeansBatchMaxMu);
-  b.tot = a.take<int>(kKmeansBatchMaxMu);
-  b.sel = a.take<int>(kKmeansBatchMaxMu);
-  b.tile_cnt = a.take<int>(nfilter);
-  b.st = a.take<KmState>(1);
-  return b;
-}
-
-constexpr int kBatchMaxGroup = 16;  // CTAs per request
-
-int batch_group(long long n) {
-  long long g = (n + 4095) / 4096;
-  return (int)std::max(1LL, std::min((long long)kBatchMaxGroup, g));
-}
-
-}  // namespace
-
-size_t kmeans_batch_workspace_bytes(long long ng, int mu) {
-  (void)mu;
-  Arena a;
-  a.counting = true;
-  // the histogram sized for the largest group: a batch runs every request
-  // with the largest group any of its requests needs
-  carve_batch(a, (int)ng, kBatchMaxGroup);
-  a.take<KmBatchJob>(1);
-  return a.off + 512;
-}
-
-int kmeans_select_batch(const KmeansArgs* args, int count, Arena& arena, cudaStream_t stream,
-                        KmeansResult* res) {
-  if (count <= 0) return ISDF_OK;
-  int G = 1;
+int select_group(const KmeansArgs* args, int count, Arena& arena, cudaStream_t stream,
+                 KmeansResult* res) {
+  std::vector<KmBuffers> bufs(count);
+  char* records = arena.take<char>(kBatchRecord * (size_t)count);
+  int* live = arena.take<int>(1);
   for (int r = 0; r < count; ++r) {
-    const KmeansArgs& a = args[r];
-    if (a.ng <= 1 || a.ng > kKmeansBatchMaxNg || a.mu <= 0 || a.mu > kKmeansBatchMaxMu ||
-        a.mu > a.ng || a.max_iter < 0 || a.warm)
-      return record_error(ISDF_ERR_UNSUPPORTED, "kmeans batch: request outside the batched sizes");
-    G = std::max(G, batch_group(a.ng));
+    bufs[r] = carve(arena, (int)args[r].ng, args[r].mu);
+    bufs[r].st = reinterpret_cast<KmState*>(records + kBatchRecord * (size_t)r);
+    bufs[r].sel = reinterpret_cast<int*>(bufs[r].st + 1);
   }
-  std::vector<BatchBuffers> bufs(count);
-  for (int r = 0; r < count; ++r) bufs[r] = carve_batch(arena, (int)args[r].ng, G);
-  KmBatchJob* d_jobs = arena.take<KmBatchJob>((size_t)count);
   if (arena.overflowed()) return record_error(ISDF_ERR_NOMEM, "kmeans batch: workspace too small");
   // filter: maxW, kept-point compaction, zero tail (per request)
+  ISDF_CUDA(cudaMemsetAsync(records, 0, kBatchRecord * (size_t)count, stream));
   for (int r = 0; r < count; ++r) {
     const int n = (int)args[r].ng;
     const int nfilter = (n + 1023) / 1024;
-    const BatchBuffers& b = bufs[r];
-    ISDF_CUDA(cudaMemsetAsync(b.st, 0, sizeof(KmState), stream));
+    const KmBuffers& b = bufs[r];
     ISDF_CUDA(cudaMemsetAsync(b.pidx, 0, sizeof(int) * (size_t)n, stream));
     k_maxw<<<kNumSMs * 4, 256, 0, stream>>>(args[r].d_w, n, b.st);
     k_filter_count<<<nfilter, 256, 0, stream>>>(args[r].d_w, n, b.st, b.tile_cnt);
@@ -2351,20 +2107,28 @@ int kmeans_select_batch(const KmeansArgs* args, int count, Arena& arena, cudaStr
     k_filter_scatter<<<nfilter, 256, 0, stream>>>(args[r].d_w, n, b.st, b.tile_cnt, b.pidx);
   }
   ISDF_CHECK_LAUNCH();
-  std::vector<KmBatchJob> jobs;
-  std::vector<int> slot;  // request of each batched job
+  std::vector<char> host(kBatchRecord * (size_t)count);
+  ISDF_TRY(read_back(host.data(), records, host.size(), stream));
+  auto state = [&](int r) -> KmState {
+    KmState st;
+    std::memcpy(&st, host.data() + kBatchRecord * (size_t)r, sizeof(st));
+    return st;
+  };
+  KmJobs<kBatchJobs> jobs;
+  LoopDims dims;
+  int max_iter = 0;
+  std::vector<int> slot;  // request of each job
   for (int r = 0; r < count; ++r) {
     const KmeansArgs& a = args[r];
     const int n = (int)a.ng, mu = a.mu;
-    const BatchBuffers& b = bufs[r];
-    KmState hst;
-    ISDF_TRY(read_back(&hst, b.st, sizeof(KmState), stream));
+    const KmBuffers& b = bufs[r];
+    const KmState hst = state(r);
     res[r] = KmeansResult();
     res[r].npt = hst.npt;
     if (a.rand_seed >= 0) std::srand((unsigned)a.rand_seed);
-    std::memset(a.piv, 0, sizeof(int) * (size_t)n);
     if (hst.npt < mu) {
       // utility.cpp:667-681: piv from the kept list, then a shuffled tail
+      std::memset(a.piv, 0, sizeof(int) * (size_t)n);
       std::vector<int> index(n, 0);
       ISDF_TRY(read_back(index.data(), b.pidx, sizeof(int) * (size_t)hst.npt, stream));
       int k0 = 0, k1 = 0;
@@ -2388,61 +2152,93 @@ int kmeans_select_batch(const KmeansArgs* args, int count, Arena& arena, cudaStr
     k_points<<<grid_for(n, 256), 256, 0, stream>>>(b.pidx, a.d_w, n, a.num_grid[0], a.num_grid[1],
                                                    dx0, dx1, dx2, b.px, b.py, b.pz, b.pw, mu,
                                                    b.cen);
-    ISDF_CUDA(cudaMemsetAsync(b.label, 0xff, sizeof(int) * (size_t)n, stream));
-    KmBatchJob j;
-    std::memset(&j, 0, sizeof(j));
-    j.px = b.px;
-    j.py = b.py;
-    j.pz = b.pz;
-    j.pw = b.pw;
-    j.pidx = b.pidx;
-    j.label = b.label;
-    j.sorted = b.sorted;
-    j.cen = b.cen;
-    j.sums = b.sums;
-    j.hist = b.hist;
-    j.tot = b.tot;
-    j.sel = b.sel;
-    j.n = n;
-    j.npt = hst.npt;
-    j.mu = mu;
-    j.max_iter = a.max_iter;
-    j.max_f = 1e-5 * n;  // KmeansTolerance * n (utility.cpp:812)
-    j.rk = mu;
-    jobs.push_back(j);
+    const CellGrid cg = cell_grid(a);
+    AssignMap am = brick_map(a, hst.npt);
+    if (hst.npt < n) {
+      ISDF_CUDA(cudaMemsetAsync(b.g2p, 0xff, sizeof(int) * (size_t)n, stream));
+      k_grid_to_point<<<grid_for(hst.npt, 256), 256, 0, stream>>>(b.pidx, hst.npt, b.g2p);
+      am.g2p = b.g2p;
+    }
+    k_point_cells<<<grid_for(n, 256), 256, 0, stream>>>(b.px, b.py, b.pz, n, cg, b.pcell, b.pd12);
+    KmState init{};
+    init.flag = n;
+    init.changed = n;
+    init.rk = mu;
+    init.npt = hst.npt;
+    init.maxw_bits = hst.maxw_bits;
+    std::memcpy(host.data() + kBatchRecord * (size_t)r, &init, sizeof(init));
+    KmJob& job = jobs.j[slot.size()];
+    job = make_job(a, b, cg, am, hst.npt);
+    dims.add(job, mu, grid_for(am.nbt + (n - hst.npt), kAssignThreads));
+    max_iter = std::max(max_iter, a.max_iter);
     slot.push_back(r);
   }
   ISDF_CHECK_LAUNCH();
-  if (jobs.empty()) return ISDF_OK;
-  // every CTA of the launch must be resident at once (the group barriers)
-  int dev = 0, per_sm = 0, coop = 0;
-  ISDF_CUDA(cudaGetDevice(&dev));
-  ISDF_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-  if (!coop) return record_error(ISDF_ERR_UNSUPPORTED, "kmeans batch: no cooperative launch");
-  int nsm = 0;
-  ISDF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  ISDF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_kmeans_batch, kBatchThreads, 0));
-  const int max_jobs = std::max(1, per_sm * nsm / G);
-  ISDF_CUDA(cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(KmBatchJob) * jobs.size(),
-                            cudaMemcpyHostToDevice, stream));
-  for (size_t j0 = 0; j0 < jobs.size(); j0 += (size_t)max_jobs) {
-    const int nj = (int)std::min<size_t>((size_t)max_jobs, jobs.size() - j0);
-    KmBatchJob* dj = d_jobs + j0;
-    int g = G;
-    void* kargs[] = {(void*)&dj, (void*)&g};
-    ISDF_CUDA(cudaLaunchCooperativeKernel((const void*)k_kmeans_batch, dim3((unsigned)(nj * G)),
-                                          dim3(kBatchThreads), kargs, 0, stream));
+  if (slot.empty()) return ISDF_OK;
+  const int nj = (int)slot.size();
+  ISDF_CUDA(cudaMemcpyAsync(records, host.data(), host.size(), cudaMemcpyHostToDevice, stream));
+  ISDF_CUDA(cudaMemcpyAsync(live, &nj, sizeof(int), cudaMemcpyHostToDevice, stream));
+  ISDF_TRY(set_kmeans_smem_attrs());
+  launch_assign(jobs, dims, 0, stream);
+  ISDF_CHECK_LAUNCH();
+  LoopGraph loop;
+  loop.build(jobs, dims, max_iter, live, stream);
+  if (loop.exec) {
+    ISDF_CUDA(cudaGraphLaunch(loop.exec, stream));
+  } else {
+    const LoopEnd no_graph{0, 0, 0x7fffffff, live};
+    for (int left = nj, chunks = 0; left > 0; ++chunks) {
+      if (chunks > max_iter / kIterChunk + 2)
+        return record_error(ISDF_ERR_CUDA, "kmeans batch: loop did not stop");
+      for (int it = 0; it < kIterChunk; ++it) {
+        launch_sums(jobs, dims, no_graph, stream);
+        launch_assign(jobs, dims, 1, stream);
+      }
+      ISDF_CHECK_LAUNCH();
+      ISDF_TRY(read_back(&left, live, sizeof(int), stream));
+    }
   }
-  std::vector<KmBatchJob> out(jobs.size());
-  ISDF_TRY(read_back(out.data(), d_jobs, sizeof(KmBatchJob) * jobs.size(), stream));
-  for (size_t j = 0; j < jobs.size(); ++j) {
-    const int r = slot[j];
-    if (out[j].err) return record_error(ISDF_ERR_TIMEOUT, "kmeans batch: a group barrier timed out");
-    std::vector<int> sel(out[j].rk);
-    ISDF_TRY(read_back(sel.data(), bufs[r].sel, sizeof(int) * sel.size(), stream));
-    res[r].iters = out[j].iters;
+  k_final_near<kBatchJobs><<<dim3(grid_for(dims.mu, 4), dims.jobs), 128, 0, stream>>>(jobs);
+  ISDF_CHECK_LAUNCH();
+  ISDF_TRY(read_back(host.data(), records, host.size(), stream));
+  for (int r : slot) {
+    const KmState hst = state(r);
+    if (!hst.done) return record_error(ISDF_ERR_CUDA, "kmeans batch: loop did not stop");
+    std::vector<int> sel(hst.rk);
+    std::memcpy(sel.data(), host.data() + kBatchRecord * (size_t)r + sizeof(KmState),
+                sizeof(int) * sel.size());
+    res[r].iters = hst.s;
+    res[r].search_frac = (double)hst.searches / ((double)args[r].ng * (hst.s + 1));
     res[r].rk_eff = piv_from_selection(sel, (int)args[r].ng, args[r].piv);
-    res[r].launches = 8 + (int)((jobs.size() + max_jobs - 1) / max_jobs);
+    res[r].launches = 8 + hst.rounds * 6 / nj;
+  }
+  return ISDF_OK;
+}
+
+}  // namespace
+
+size_t kmeans_batch_workspace_bytes(long long ng, int mu) {
+  Arena a;
+  a.counting = true;
+  a.take<char>(kBatchRecord);
+  a.take<int>(1);
+  carve(a, (int)ng, mu);
+  return a.off;
+}
+
+int kmeans_select_batch(const KmeansArgs* args, int count, Arena& arena, cudaStream_t stream,
+                        KmeansResult* res) {
+  for (int r = 0; r < count; ++r) {
+    const KmeansArgs& a = args[r];
+    if (a.ng <= 1 || a.ng > kKmeansBatchMaxNg || a.mu <= 0 || a.mu > kKmeansBatchMaxMu ||
+        a.mu > a.ng || a.max_iter < 0 || a.warm)
+      return record_error(ISDF_ERR_UNSUPPORTED, "kmeans batch: request outside the batched sizes");
+  }
+  // a group's buffers are free once its results have been read back
+  const size_t mark = arena.off;
+  for (int r = 0; r < count; r += kBatchJobs) {
+    arena.off = mark;
+    ISDF_TRY(select_group(args + r, std::min(kBatchJobs, count - r), arena, stream, res + r));
   }
   return ISDF_OK;
 }

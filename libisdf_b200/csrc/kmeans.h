@@ -33,9 +33,12 @@ struct KmeansResult {
 
 size_t kmeans_workspace_bytes(long long ng, int mu);
 
-// Batched selection of small systems in one cooperative launch (the serving
-// loop's batches): cold start only, ng <= kKmeansBatchMaxNg, mu <= kKmeansBatchMaxMu.
-// piv and the results equal kmeans_select()'s for each request.
+// Batched selection of small systems, kKmeansBatchGroup of them per launch (the
+// serving loop's batches): cold start only, ng <= kKmeansBatchMaxNg,
+// mu <= kKmeansBatchMaxMu. piv and the results equal kmeans_select()'s for each
+// request. The groups run one after the other in the same workspace, which
+// holds the largest group's requests.
+constexpr int kKmeansBatchGroup = 16;
 constexpr int kKmeansBatchMaxMu = 512;
 constexpr long long kKmeansBatchMaxNg = 1 << 20;
 size_t kmeans_batch_workspace_bytes(long long ng, int mu);

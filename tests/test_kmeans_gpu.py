@@ -294,3 +294,30 @@ def test_select_empty_clusters_match_oracle(torch_cuda, ng, mu):
                                             torch.from_numpy(w).cuda(), mu, iters, rand_seed=1)
         assert (rk, it) == (rk_o, it_o)
         assert np.array_equal(piv, piv_o)
+
+
+def test_select_batch_groups_match_single(torch_cuda):
+    """A batch of more than one launch's systems, of different grids, mu and
+    iteration caps (one stops at once, one has fewer kept points than mu):
+    every result equals the single selection's."""
+    torch = torch_cuda
+    rng = np.random.default_rng(11)
+    doms, ws, mus, its = [], [], [], []
+    for k in range(19):
+        ng = tuple(int(x) for x in rng.integers(6, 25, 3))
+        n = ng[0] * ng[1] * ng[2]
+        w = rng.uniform(0.0, 1.0, n)
+        w[rng.integers(0, n, n // 4)] = 0.0
+        mu = int(rng.integers(1, min(513, n // 3)))
+        if k == 7:
+            w[:] = 0.0
+            w[5:5 + mu // 2] = 1.0  # fewer kept points than mu
+        doms.append(isdf.Domain(length=(5.0, 6.0, 7.0), num_grid=ng))
+        ws.append(torch.from_numpy(w).cuda())
+        mus.append(mu)
+        its.append((0, 1, 30, 100)[k % 4])
+    got = isdf.kmeans_select_batch(doms, ws, mus, its, rand_seed=1)
+    for d, w, mu, it, g in zip(doms, ws, mus, its, got):
+        one = isdf.kmeans_select(d, w, mu, it, rand_seed=1)
+        assert g[1:] == one[1:]
+        assert np.array_equal(g[0], one[0])
