@@ -172,6 +172,35 @@ struct Core {
         f(r + 8, c + 1, acc[i][j][3]);
       }
   }
+
+  // *at(row, col) = op(*at(row, col), value) for every accumulator element at
+  // has a place for (else nullptr). A column of the warp's tiles at a time is
+  // read before any of it is written: element by element, each read would wait
+  // for the write before it (the compiler cannot know that they differ).
+  template <class At, class Op>
+  __device__ void read_modify(At at, Op op) const {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int wm0 = (warp >> 2) * WM, wn0 = (warp & 3) * WN;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      double old[MT][4];
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const double* p = at(wm0 + i * 16 + g + 8 * (h >> 1), wn0 + j * 8 + 2 * t + (h & 1));
+          old[i][h] = p ? *p : 0.0;
+        }
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          double* p = at(wm0 + i * 16 + g + 8 * (h >> 1), wn0 + j * 8 + 2 * t + (h & 1));
+          if (p) *p = op(old[i][h], acc[i][j][h]);
+        }
+    }
+  }
 };
 
 // A row of zeros: the source of the warp-specialised tile's copies for the
@@ -339,6 +368,35 @@ struct WsTile {
         f(r + 8, c, acc[i][j][2]);
         f(r + 8, c + 1, acc[i][j][3]);
       }
+  }
+
+  // *at(row, col) = op(*at(row, col), value) for every accumulator element at
+  // has a place for (else nullptr). A column of the warp's tiles at a time is
+  // read before any of it is written: element by element, each read would wait
+  // for the write before it (the compiler cannot know that they differ).
+  template <class At, class Op>
+  __device__ void read_modify(At at, Op op) const {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int wm0 = (warp / WGN) * WM, wn0 = (warp % WGN) * WN;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      double old[MT][4];
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const double* p = at(wm0 + i * 16 + g + 8 * (h >> 1), wn0 + j * 8 + 2 * t + (h & 1));
+          old[i][h] = p ? *p : 0.0;
+        }
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          double* p = at(wm0 + i * 16 + g + 8 * (h >> 1), wn0 + j * 8 + 2 * t + (h & 1));
+          if (p) *p = op(old[i][h], acc[i][j][h]);
+        }
+    }
   }
 };
 

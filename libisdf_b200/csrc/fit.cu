@@ -49,6 +49,7 @@ constexpr int kNB = 64;  // Cholesky / triangular-solve block size
 
 using CoreZ = dmma::Core<128, 128>;  // Z GEMM, Cholesky trailing update
 using CoreN = dmma::Core<128, 64>;   // panel and triangular-solve steps
+using CoreS = dmma::Core<64, 64>;    // Cholesky trailing update, small
 using WsN = dmma::WsTile<64, 64, 2, 2, 16, 4>;  // triangular-solve steps, 3 CTAs per SM
 
 // 16-byte cp.async needs 16-byte aligned rows: base aligned, even leading dimension.
@@ -73,13 +74,15 @@ __global__ void __launch_bounds__(256) k_gemm_z(int M, int N, int K, const doubl
   core.zero();
   const int m_rem = (int)(M - m0 < CoreZ::BM ? M - m0 : CoreZ::BM);
   core.run<VEC>(smem, A + m0, lda, B + n0, ldb, m_rem, N - n0, 0, K);
+  auto at = [&](int r, int c) -> double* {
+    return r < m_rem && n0 + c < N ? C + (m0 + r) + (long long)(n0 + c) * ldc : nullptr;
+  };
+  if (MODE == 2) {
+    core.read_modify(at, [](double old, double v) { return old * v; });
+    return;
+  }
   core.for_each([&](int r, int c, double v) {
-    if (r < m_rem && n0 + c < N) {
-      double* p = C + (m0 + r) + (long long)(n0 + c) * ldc;
-      if (MODE == 0) *p = v * v;
-      else if (MODE == 1) *p = v;
-      else *p = *p * v;
-    }
+    if (double* p = at(r, c)) *p = MODE == 0 ? v * v : v;
   });
 }
 
@@ -100,13 +103,15 @@ __global__ void __launch_bounds__(WsN::THREADS, 3)
   WsN tile;
   if (!tile.run(smem, A + m0, lda, m_rem, B + n0, ldb, n_rem, K, err)) return;
   if (WsN::producer()) return;
+  auto at = [&](int r, int c) -> double* {
+    return r < m_rem && c < n_rem ? C + (m0 + r) + (long long)(n0 + c) * ldc : nullptr;
+  };
+  if (MODE == 2) {
+    tile.read_modify(at, [](double old, double v) { return old * v; });
+    return;
+  }
   tile.for_each([&](int r, int c, double v) {
-    if (r < m_rem && c < n_rem) {
-      double* p = C + (m0 + r) + (long long)(n0 + c) * ldc;
-      if (MODE == 0) *p = v * v;
-      else if (MODE == 1) *p = v;
-      else *p = *p * v;
-    }
+    if (double* p = at(r, c)) *p = MODE == 0 ? v * v : v;
   });
 }
 
@@ -193,12 +198,24 @@ __global__ void k_gather_cct(const double* __restrict__ Z, long long ng,
   }
 }
 
-// trace in index order, eps = 1e-10 * (trace / rk), diagonal += eps
-__global__ void k_regularise(double* P, int rk, double* eps_out) {
+// trace in index order, eps = 1e-10 * (trace / rk), diagonal += eps. The
+// diagonal is staged in shared memory: one thread reading it from global memory
+// while it adds took 56 us at rk = 1600.
+__global__ void __launch_bounds__(256) k_regularise(double* P, int rk, double* eps_out) {
   __shared__ double eps;
+  __shared__ double diag[1024];
+  double tr = 0.0;
+  for (int base = 0; base < rk; base += 1024) {
+    const int cnt = min(1024, rk - base);
+    for (int i = threadIdx.x; i < cnt; i += 256) diag[i] = P[(long long)(base + i) * (rk + 1)];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 16
+      for (int i = 0; i < cnt; ++i) tr = radd(tr, diag[i]);
+    }
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
-    double tr = 0.0;
-    for (int i = 0; i < rk; ++i) tr = radd(tr, P[(long long)i * rk + i]);
     eps = rmul(1e-10, rdiv(tr, (double)rk));
     *eps_out = eps;
   }
@@ -215,61 +232,113 @@ __global__ void k_regularise(double* P, int rk, double* eps_out) {
 //   dinvT[k*64 + n] = X(n, k)   (right factor of a forward step)
 //   dinv [k*64 + n] = X(k, n)   (right factor of a backward step)
 // info: first failing global column + 1 (kept if already set).
-__global__ void __launch_bounds__(256) k_potf2(double* A, int lda, int k0, int bs,
-                                               double* __restrict__ dinvT,
-                                               double* __restrict__ dinv, int* info) {
+//
+// One block, bound by its chain of bs square roots and divisions (about 110 and
+// 190 cycles each) and the exchanges between them. Warps 0-7 factor,
+// right-looking: four threads per row hold its columns in registers (column c
+// in thread c % 4), so a step is the square root, the division of the column,
+// and at most 16 updates per thread. Warps 8-15 invert one row behind: row i of
+// X needs rows up to i of L only. Four lanes per column of X hold every fourth
+// entry in registers and sum in order of k. 49 us a block, where the
+// factorisation in shared memory followed by the inversion took 70 (25 blocks:
+// 1.8 ms of a 17.7 ms mixed fit with 1600 points). Two-dimensional register
+// tiles for the factor, the inverting warps on mbarriers instead of the block's
+// barriers, and fewer warps took 62 to 72.
+constexpr int kPotf2Threads = 512;
+
+// p ? a : b as a register move: written with ?:, a choice among an array's
+// entries becomes an indexed access, which puts the array in local memory.
+__device__ __forceinline__ double select(bool p, double a, double b) {
+  double r;
+  asm("{\n .reg .pred p;\n setp.ne.s32 p, %3, 0;\n selp.f64 %0, %1, %2, p;\n}\n"
+      : "=d"(r)
+      : "d"(a), "d"(b), "r"((int)p));
+  return r;
+}
+
+__global__ void __launch_bounds__(kPotf2Threads) k_potf2(double* A, int lda, int k0, int bs,
+                                                         double* __restrict__ dinvT,
+                                                         double* __restrict__ dinv, int* info) {
   extern __shared__ double potf2_smem[];
   double(*a)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(potf2_smem);  // a[row][col]
   double(*x)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(potf2_smem + kNB * (kNB + 1));
+  __shared__ double root;
   const int tid = threadIdx.x;
-  for (int e = tid; e < kNB * kNB; e += 256) {
-    int r = e % kNB, c = e / kNB;
+  for (int e = tid; e < kNB * kNB; e += kPotf2Threads) {
+    const int r = e % kNB, c = e / kNB;
     a[r][c] = (r < bs && c < bs && r >= c) ? A[(long long)(k0 + r) + (long long)(k0 + c) * lda]
                                            : 0.0;
     x[r][c] = 0.0;
   }
   __syncthreads();
-  // right-looking: the trailing update on a 16 x 16 thread grid (thread
-  // (ty, tx) takes rows ty, ty + 16, ... and columns tx, tx + 16, ...)
-  const int ty = tid >> 4, tx = tid & 15;
-  for (int j = 0; j < bs; ++j) {
-    if (tid == 0) {
-      double d = a[j][j];
-      if (!(d > 0.0)) atomicCAS(info, 0, k0 + j + 1);
-      a[j][j] = sqrt(d);
+  const bool factor = tid < 256;
+  const int own = (tid & 255) >> 2, q = tid & 3;  // row of L (factor) or column of X (invert)
+  // factor: this row's columns q, q + 4, ...; invert: r[u] is X(own + q + 4 u,
+  // own), zero until it is known
+  double r[kNB / 4];
+#pragma unroll
+  for (int u = 0; u < kNB / 4; ++u) r[u] = factor ? a[own][4 * u + q] : 0.0;
+  double sum = 0.0;  // invert: this lane's share of the next row's sum
+  // step j: the factor warps finish column j; the others invert row j - 1
+  for (int j = 0; j <= bs; ++j) {
+    if (factor && j < bs) {
+      double v = 0.0;  // a(own, j), in the thread that holds column j
+#pragma unroll
+      for (int u = 0; u < kNB / 4; ++u) v = select(u == j >> 2, r[u], v);
+      if (own == j && q == (j & 3)) {
+        if (!(v > 0.0)) atomicCAS(info, 0, k0 + j + 1);
+        v = sqrt(v);
+        root = v;
+        a[j][j] = v;
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (own > j && own < bs && q == (j & 3)) a[own][j] = v / root;
+    } else if (!factor && j > 0) {
+      const int i = j - 1;
+      double s = sum;  // over k = own + q, own + q + 4, ... < i
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      // (a zero numerator takes the division's slow path, for the whole warp:
+      // columns not begun divide 1)
+      const double xi = (own < i ? -s : 1.0) / a[i][i];
+      if (own <= i && ((i - own) & 3) == q) {
+        x[i][own] = xi;
+#pragma unroll
+        for (int u = 0; u < kNB / 4; ++u) r[u] = select(u == (i - own) >> 2, xi, r[u]);
+      }
     }
     __syncthreads();
-    const double djj = a[j][j];
-    for (int i = j + 1 + tid; i < bs; i += 256) a[i][j] = a[i][j] / djj;
-    __syncthreads();
-    for (int i = j + 1 + ty; i < bs; i += 16) {
-      const double lij = a[i][j];
-      for (int c = j + 1 + tx; c <= i; c += 16) a[i][c] -= lij * a[c][j];
+    if (factor && j < bs) {
+      if (own > j && own < bs) {
+        const double lij = a[own][j];
+#pragma unroll
+        for (int u = 0; u < kNB / 4; ++u) {
+          const int c = 4 * u + q;
+          if (c > j && c <= own) r[u] -= lij * a[c][j];
+        }
+      }
+    } else if (!factor && j < bs) {
+      // row j of L is complete (its last entry now): the sums of row j of X;
+      // the entries of X not known yet, and L right of the diagonal, are zero
+      const double* row = a[j] + own + q;
+      sum = 0.0;
+#pragma unroll
+      for (int u = 0; u < kNB / 4; ++u)
+        if (own + q + 4 * u < kNB) sum = fma(row[4 * u], r[u], sum);
     }
-    __syncthreads();
   }
-  // X = L^{-1} row by row, x(i, c) = -(sum_{c <= k < i} L(i, k) x(k, c)) / L(i, i):
-  // four threads per column, each summing every fourth k
-  {
-    const int c = tid >> 2, part = tid & 3;
-    for (int i = 0; i < bs; ++i) {
-      double sum = 0.0;
-      if (c < i)
-        for (int k = c + part; k < i; k += 4) sum = fma(a[i][k], x[k][c], sum);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      if (part == 0 && c <= i) x[i][c] = c == i ? 1.0 / a[i][i] : -sum / a[i][i];
-      __syncthreads();
-    }
-  }
-  for (int e = tid; e < kNB * kNB; e += 256) {
-    int r = e % kNB, c = e / kNB;
-    if (r < bs && c < bs) A[(long long)(k0 + r) + (long long)(k0 + c) * lda] = r >= c ? a[r][c] : 0.0;
-    int k = e / kNB, n = e % kNB;
+  __syncthreads();
+  for (int e = tid; e < kNB * kNB; e += kPotf2Threads) {
+    const int rr = e % kNB, c = e / kNB;
+    if (rr < bs && c < bs)
+      A[(long long)(k0 + rr) + (long long)(k0 + c) * lda] = rr >= c ? a[rr][c] : 0.0;
+    const int k = e / kNB, n = e % kNB;
     dinvT[e] = x[n][k];
     dinv[e] = x[k][n];
   }
 }
+
+constexpr size_t smem_bytes_potf2 = sizeof(double) * 2 * kNB * (kNB + 1);
 
 // Panel: L[k0+bs:, k0:k0+bs] = A[k0+bs:, k0:k0+bs] * X^T, in place (a CTA
 // reads its whole row tile before it writes it back).
@@ -288,22 +357,27 @@ __global__ void __launch_bounds__(256) k_chol_panel(double* A, int lda, int k0, 
 
 // Trailing update of the lower part: A[r, c] -= sum_k L[r, k] L[c, k] for
 // r, c >= k0+bs, k in the panel. Tiles wholly above the diagonal are skipped.
-template <int VEC>
+// Depth 64 only: a short launch whose time is the read and write of A and the
+// latency of one tile, so smaller tiles (T = CoreS) pay until the 128 x 128
+// ones fill the GPU.
+template <class T, int VEC>
 __global__ void __launch_bounds__(256) k_chol_update(double* A, int lda, int k0, int bs, int n) {
   extern __shared__ double smem[];
   const int base = k0 + bs;
-  const int n0 = base + blockIdx.x * CoreZ::BN;
-  const int m0 = base + blockIdx.y * CoreZ::BM;
-  if (m0 + CoreZ::BM <= n0) return;
-  CoreZ core;
+  const int n0 = base + blockIdx.x * T::BN;
+  const int m0 = base + blockIdx.y * T::BM;
+  if (m0 + T::BM <= n0) return;
+  T core;
   core.zero();
   // B(k, c) = L[n0 + c, k0 + k]
-  core.run<VEC>(smem, A + m0 + (long long)k0 * lda, lda, A + n0 + (long long)k0 * lda, lda,
-                n - m0, n - n0, 0, bs);
-  core.for_each([&](int r, int c, double v) {
-    const int gr = m0 + r, gc = n0 + c;
-    if (gr < n && gc < n && gr >= gc) A[gr + (long long)gc * lda] -= v;
-  });
+  core.template run<VEC>(smem, A + m0 + (long long)k0 * lda, lda, A + n0 + (long long)k0 * lda, lda,
+                         n - m0, n - n0, 0, bs);
+  core.read_modify(
+      [&](int r, int c) -> double* {
+        const int gr = m0 + r, gc = n0 + c;
+        return gr < n && gc < n && gr >= gc ? A + gr + (long long)gc * lda : nullptr;
+      },
+      [](double old, double v) { return old - v; });
 }
 
 // Clears the strict upper triangle left over in the factor's storage.
@@ -443,8 +517,6 @@ __global__ void __launch_bounds__(256) k_trinv_x(const double* __restrict__ Tb,
   });
 }
 
-constexpr size_t smem_bytes_potf2 = sizeof(double) * 2 * kNB * (kNB + 1);
-
 template <class K>
 int set_attr(K kernel, size_t bytes) {
   ISDF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
@@ -462,8 +534,10 @@ int set_smem_attrs() {
   ISDF_TRY(set_attr(k_gemm_z<1, 1>, CoreZ::SMEM_BYTES));
   ISDF_TRY(set_attr(k_gemm_z<2, 1>, CoreZ::SMEM_BYTES));
   ISDF_TRY(set_attr(k_gemm_z<1, 2>, CoreZ::SMEM_BYTES));
-  ISDF_TRY(set_attr(k_chol_update<1>, CoreZ::SMEM_BYTES));
-  ISDF_TRY(set_attr(k_chol_update<2>, CoreZ::SMEM_BYTES));
+  ISDF_TRY(set_attr(k_chol_update<CoreZ, 1>, CoreZ::SMEM_BYTES));
+  ISDF_TRY(set_attr(k_chol_update<CoreZ, 2>, CoreZ::SMEM_BYTES));
+  ISDF_TRY(set_attr(k_chol_update<CoreS, 1>, CoreS::SMEM_BYTES));
+  ISDF_TRY(set_attr(k_chol_update<CoreS, 2>, CoreS::SMEM_BYTES));
   ISDF_TRY(set_attr(k_chol_panel<1>, CoreN::SMEM_BYTES));
   ISDF_TRY(set_attr(k_chol_panel<2>, CoreN::SMEM_BYTES));
   ISDF_TRY(set_attr(k_trsm_gemm<1>, CoreN::SMEM_BYTES));
@@ -575,6 +649,9 @@ size_t fit_workspace_bytes(long long ng, int nstate, int rk) {
   return a.off;
 }
 
+// Remaining rows from which the trailing update takes 128 x 128 tiles.
+constexpr int kCholWide = 3072;
+
 // Lower Cholesky of P (rk x rk, column-major) in place, with per-block
 // inverses for the solve. Returns the failing column + 1 in *info (0 = ok).
 static int cholesky(const FitBuffers& b, int rk, cudaStream_t s) {
@@ -583,19 +660,22 @@ static int cholesky(const FitBuffers& b, int rk, cudaStream_t s) {
   for (int kb = 0; kb < nblk; ++kb) {
     const int k0 = kb * kNB;
     const int bs = min(kNB, rk - k0);
-    k_potf2<<<1, 256, smem_bytes_potf2, s>>>(b.P, rk, k0, bs, b.dinvT + (size_t)kb * kNB * kNB,
+    k_potf2<<<1, kPotf2Threads, smem_bytes_potf2, s>>>(b.P, rk, k0, bs, b.dinvT + (size_t)kb * kNB * kNB,
                                              b.dinv + (size_t)kb * kNB * kNB, b.info);
     const int rem = rk - k0 - bs;
     if (rem > 0) {
       const double* dT = b.dinvT + (size_t)kb * kNB * kNB;
       const unsigned pg = (unsigned)((rem + CoreN::BM - 1) / CoreN::BM);
-      dim3 g((rem + CoreZ::BN - 1) / CoreZ::BN, (rem + CoreZ::BM - 1) / CoreZ::BM);
-      if (v2) {
-        k_chol_panel<2><<<pg, 256, CoreN::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk, dT);
-        k_chol_update<2><<<g, 256, CoreZ::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk);
+      if (v2) k_chol_panel<2><<<pg, 256, CoreN::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk, dT);
+      else k_chol_panel<1><<<pg, 256, CoreN::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk, dT);
+      if (rem >= kCholWide) {
+        const dim3 g((rem + CoreZ::BN - 1) / CoreZ::BN, (rem + CoreZ::BM - 1) / CoreZ::BM);
+        auto k = v2 ? k_chol_update<CoreZ, 2> : k_chol_update<CoreZ, 1>;
+        k<<<g, 256, CoreZ::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk);
       } else {
-        k_chol_panel<1><<<pg, 256, CoreN::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk, dT);
-        k_chol_update<1><<<g, 256, CoreZ::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk);
+        const dim3 g((rem + CoreS::BN - 1) / CoreS::BN, (rem + CoreS::BM - 1) / CoreS::BM);
+        auto k = v2 ? k_chol_update<CoreS, 2> : k_chol_update<CoreS, 1>;
+        k<<<g, 256, CoreS::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk);
       }
     }
   }
