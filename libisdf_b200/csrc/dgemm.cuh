@@ -204,8 +204,39 @@ struct Core {
 };
 
 // A row of zeros: the source of the warp-specialised tile's copies for the
-// columns and rows outside the operands.
+// columns and rows past the depth.
 static __device__ __align__(128) double g_zero_row[256];
+
+// The producer's copies of one column of an A tile: `valid` (<= BM) contiguous
+// doubles at src, into a shared-memory row. Bulk copies want 16-byte addresses
+// and sizes. With an even leading dimension every column starts on one; with an
+// odd one every other column starts 8 bytes behind one, so its copy starts at
+// the element before (the column above's last, or the same column's previous
+// row), and the fragments of that column are read one place further on
+// (a_shift): both parities of k lie in fixed lanes, so that the shift is a
+// constant per lane. A copy may take one element past its rows, but never past
+// the operand: the tile that ends the columns of an odd leading dimension has
+// an odd number of rows, whose last one in an aligned column goes by itself.
+struct ColumnCopy {
+  uint32_t aligned, shifted;  // bytes of a copy of an aligned / shifted column
+  bool last;                  // the last row of an aligned column goes by itself
+  bool odd;                   // odd leading dimension
+
+  __device__ ColumnCopy(int valid, long long ld) {
+    odd = (ld & 1) != 0;
+    last = odd && (valid & 1);
+    aligned = (uint32_t)(odd ? valid & ~1 : (valid + 1) & ~1) * 8u;
+    shifted = (uint32_t)((valid + 2) & ~1) * 8u;
+  }
+  __device__ static bool is_shifted(const double* src) {
+    return (reinterpret_cast<size_t>(src) & 8) != 0;
+  }
+  // bytes of n columns from src on
+  __device__ uint32_t bytes(const double* src, int n) const {
+    const int sh = !odd ? 0 : (n + (is_shifted(src) ? 1 : 0)) / 2;
+    return (uint32_t)sh * shifted + (uint32_t)(n - sh) * aligned;
+  }
+};
 
 // Warp-specialised FP64 tensor-core tile. WGM x WGN consumer warps compute
 // the BM x BN tile with mma.sync f64 (warp tile (BM/WGM) x (BN/WGN)); one
@@ -213,16 +244,16 @@ static __device__ __align__(128) double g_zero_row[256];
 // per stage BK columns of A (BM contiguous doubles each) and BK rows of B (BN
 // contiguous doubles each), each into a padded shared-memory row (same
 // fragment layout as Core), all completing on the stage's "full" mbarrier by
-// transaction count. A column or row past K, and the rows / columns past
-// m_rem / n_rem, are copied from a zero row, so every stage carries the same
-// byte count and the fragments never read stale shared memory. Each consumer
-// warp releases a stage through its "empty" mbarrier after a proxy fence (its
-// shared-memory reads are generic-proxy accesses, the refill an async-proxy
-// write: without the fence, served solves running side by side saw stages
-// overwritten under the readers), so nothing in the K loop synchronises the
-// whole CTA.
-// Requirements (host-checked): A and B 16-byte aligned; lda, ldb, m_rem and
-// n_rem even.
+// transaction count. A column or row past K is copied from a zero row; the rows
+// and columns past m_rem / n_rem keep whatever is there, which only reaches
+// accumulators that are not stored. Each consumer warp releases a stage through
+// its "empty" mbarrier after a proxy fence (its shared-memory reads are
+// generic-proxy accesses, the refill an async-proxy write: without the fence,
+// served solves running side by side saw stages overwritten under the readers),
+// so nothing in the K loop synchronises the whole CTA.
+// Requirements (host-checked): the allocations A and B lie in start 16-byte
+// aligned; ldb even, B's rows 16-byte aligned and n_rem rounded up to even
+// within them; m_rem even where lda is even (or the row behind it readable).
 template <int BM_, int BN_, int WGM, int WGN, int BK_, int ST_>
 struct WsTile {
   static constexpr int BM = BM_, BN = BN_, BK = BK_, ST = ST_;
@@ -233,15 +264,15 @@ struct WsTile {
   static constexpr int A_STAGE = BK * LDA_S, B_STAGE = BK * LDB_S;
   static constexpr size_t BAR_OFF = sizeof(double) * ST * (A_STAGE + B_STAGE);
   static constexpr size_t SMEM_BYTES = BAR_OFF + 16 * ST + 16;
-  static constexpr uint32_t STAGE_TX = (uint32_t)(BK * (BM + BN) * sizeof(double));
-  static_assert(BM <= 256 && BN <= 256, "zero row");
+  static constexpr uint32_t ZERO_A = (BM + 2) * 8u, ZERO_B = BN * 8u;
+  static_assert(BM + 2 <= 256 && BN <= 256, "zero row");
   static_assert(WM % 16 == 0 && WN % 8 == 0 && BK % 8 == 0, "tile shape");
 
   double acc[MT][NT][4];
 
   __device__ static bool producer() { return (threadIdx.x >> 5) == NW; }
 
-  // acc = A[0:m_rem, 0:K] * B[0:K, 0:n_rem] (zero outside), with
+  // acc = A[0:m_rem, 0:K] * B[0:K, 0:n_rem] (unspecified outside), with
   // A(m, k) = A[m + k*lda] and B(k, n) = B[k*ldb + n]. Every thread of the
   // CTA calls it. Returns false (and sets *err) when a wait ran out; the
   // producer warp returns with acc unset.
@@ -267,6 +298,8 @@ struct WsTile {
     if (warp == NW) {
       // ------------------------------------------------------------ copies
       int issued = 0;
+      const ColumnCopy cc(min(BM, m_rem), lda);
+      const uint32_t b_bytes = (uint32_t)((min(BN, n_rem) + 1) & ~1) * 8u;
       for (int kt = 0; kt < nk; ++kt) {
         const int s = kt % ST;
         bool w = true;
@@ -275,23 +308,36 @@ struct WsTile {
           ok = false;
           break;
         }
-        if (lane == 0) mbar_expect_tx(fb + 8u * s, STAGE_TX);
+        const int k0 = kt * BK, kv = min(BK, K - k0);
+        const double* ak = A + (long long)k0 * lda;
+        double* as = As + s * A_STAGE;
+        const uint32_t bs = smem_u32(Bs + s * B_STAGE);
+        if (cc.last) {
+          for (int c = lane; c < kv; c += 32) {
+            const double* src = ak + (long long)c * lda;
+            if (!ColumnCopy::is_shifted(src))
+              as[c * LDA_S + min(BM, m_rem) - 1] = src[min(BM, m_rem) - 1];
+          }
+          __syncwarp();
+        }
+        if (lane == 0)
+          mbar_expect_tx(fb + 8u * s, cc.bytes(ak, kv) + (uint32_t)kv * b_bytes +
+                                          (uint32_t)(BK - kv) * (ZERO_A + ZERO_B));
         __syncwarp();
-        const uint32_t as = smem_u32(As + s * A_STAGE), bs = smem_u32(Bs + s * B_STAGE);
-        const int k0 = kt * BK;
         for (int c = lane; c < 2 * BK; c += 32) {
           const bool is_a = c < BK;
-          const int k = k0 + (is_a ? c : c - BK);
-          const int rows = is_a ? BM : BN;
-          const int valid = k < K ? min(rows, is_a ? m_rem : n_rem) : 0;
-          const uint32_t dst = is_a ? as + (uint32_t)(c * LDA_S * 8)
-                                    : bs + (uint32_t)((c - BK) * LDB_S * 8);
-          if (valid > 0)
-            bulk_copy(dst, is_a ? A + (long long)k * lda : B + (long long)k * ldb,
-                      (uint32_t)valid * 8u, fb + 8u * s);
-          if (valid < rows)
-            bulk_copy(dst + (uint32_t)valid * 8u, g_zero_row, (uint32_t)(rows - valid) * 8u,
-                      fb + 8u * s);
+          const int k = is_a ? c : c - BK;
+          const uint32_t dst = is_a ? smem_u32(as + k * LDA_S) : bs + (uint32_t)(k * LDB_S * 8);
+          if (k >= kv) {
+            bulk_copy(dst, g_zero_row, is_a ? ZERO_A : ZERO_B, fb + 8u * s);
+          } else if (is_a) {
+            const double* src = ak + (long long)k * lda;
+            const bool sh = ColumnCopy::is_shifted(src);
+            const uint32_t bytes = sh ? cc.shifted : cc.aligned;
+            if (bytes) bulk_copy(dst, src - (sh ? 1 : 0), bytes, fb + 8u * s);
+          } else {
+            bulk_copy(dst, B + (long long)(k0 + k) * ldb, b_bytes, fb + 8u * s);
+          }
         }
         ++issued;
       }
@@ -312,6 +358,8 @@ struct WsTile {
         for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0;
     const int g = lane >> 2, t = lane & 3;
     const int wm0 = (warp / WGN) * WM, wn0 = (warp % WGN) * WN;
+    // the shifted columns of this lane (k = t mod 4): see ColumnCopy
+    const int a_shift = (lda & 1) ? (ColumnCopy::is_shifted(A) ? t + 1 : t) & 1 : 0;
     for (int kt = 0; kt < nk; ++kt) {
       const int s = kt % ST;
       if (!__all_sync(0xffffffffu, mbar_wait(fb + 8u * s, (uint32_t)(kt / ST) & 1u, abortp))) {
@@ -325,7 +373,7 @@ struct WsTile {
         double a[MT][4], b[NT][2];
 #pragma unroll
         for (int i = 0; i < MT; ++i) {
-          const double* p = as + (kk + t) * LDA_S + wm0 + i * 16 + g;
+          const double* p = as + (kk + t) * LDA_S + wm0 + i * 16 + g + a_shift;
           a[i][0] = p[0];
           a[i][1] = p[8];
           a[i][2] = p[4 * LDA_S];

@@ -59,6 +59,13 @@ __host__ __device__ inline bool vec2_ok(const void* a, long long lda, const void
          (lda % 2) == 0 && (ldb % 2) == 0;
 }
 
+// The warp-specialised tile's operands: the buffer A lies in 16-byte aligned (its
+// leading dimension may be odd, see dmma::ColumnCopy), the rows of B too.
+inline bool ws_ok(const void* a_buffer, const void* b, long long ldb) {
+  return ((reinterpret_cast<size_t>(a_buffer) | reinterpret_cast<size_t>(b)) & 15) == 0 &&
+         ldb % 2 == 0;
+}
+
 // ----------------------------------------------------------- Z C^T GEMM
 // mode 0: C = acc*acc (S1 = S2); mode 1: C = acc (first factor);
 // mode 2: C = C * acc (second factor, S1 != S2).
@@ -86,8 +93,8 @@ __global__ void __launch_bounds__(256) k_gemm_z(int M, int N, int K, const doubl
   });
 }
 
-// The same product on the warp-specialised tile (16-byte aligned operands,
-// even sizes and leading dimensions).
+// The same product on the warp-specialised tile (ws_ok: any Ng, an even leading
+// dimension of B).
 template <int MODE>
 __global__ void __launch_bounds__(WsN::THREADS, 3)
     k_gemm_zws(int M, int N, int K, const double* __restrict__ A, long long lda,
@@ -176,14 +183,15 @@ __global__ void __launch_bounds__(256) k_syrk_reduce(int n, int splits,
 }
 
 // ----------------------------------------------------------- gathers
-// Bm[k*rk + j] = psi[piv_j + (k0 + k)*ng]  (depth-major B operand)
+// Bm[k*ldb + j] = psi[piv_j + (k0 + k)*ng]  (depth-major B operand)
 __global__ void k_gather_psimu(const double* __restrict__ psi, long long ng, int nstate,
-                               const int* __restrict__ piv, int rk, double* __restrict__ Bm) {
+                               const int* __restrict__ piv, int rk, int ldb,
+                               double* __restrict__ Bm) {
   const long long total = (long long)nstate * rk;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
     int k = (int)(e / rk), j = (int)(e % rk);
-    Bm[e] = psi[(long long)piv[j] + (long long)k * ng];
+    Bm[(long long)k * ldb + j] = psi[(long long)piv[j] + (long long)k * ng];
   }
 }
 
@@ -556,7 +564,8 @@ int set_smem_attrs() {
 
 struct FitBuffers {
   int* piv;
-  double* Bm;
+  double* Bm;  // nstate x rk, row length ldb (rk, rounded up to even where padded)
+  int ldb;
   double* P;  // C C^T, then L (column-major rk x rk)
   double* W;  // one triangular-solve block operand, rk x 64
   double* dinvT;
@@ -566,11 +575,14 @@ struct FitBuffers {
   int* err;
 };
 
-FitBuffers carve(Arena& a, int nstate, int rk) {
+// pad = false: the rows of Bm as they come (a scratch array without room for the
+// padding).
+FitBuffers carve(Arena& a, int nstate, int rk, bool pad = true) {
   FitBuffers b;
   const int nblk = (rk + kNB - 1) / kNB;
   b.piv = a.take<int>(rk);
-  b.Bm = a.take<double>((size_t)nstate * rk);
+  b.ldb = pad ? rk + (rk & 1) : rk;
+  b.Bm = a.take<double>((size_t)nstate * b.ldb);
   b.P = a.take<double>((size_t)rk * rk);
   b.W = a.take<double>((size_t)rk * kNB);
   b.dinvT = a.take<double>((size_t)nblk * kNB * kNB);
@@ -641,11 +653,11 @@ int dsyrk_store(int n, int K, const double* Y, long long ldy, double* C, long lo
   return ISDF_OK;
 }
 
-size_t fit_workspace_bytes(long long ng, int nstate, int rk) {
+size_t fit_workspace_bytes(long long ng, int nstate, int rk, bool pad) {
   (void)ng;
   Arena a;
   a.counting = true;
-  carve(a, nstate, rk);
+  carve(a, nstate, rk, pad);
   return a.off;
 }
 
@@ -702,7 +714,12 @@ int fit_fp64(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* res, 
   const int rk = args.rk;
   if (ng <= 0 || rk <= 0 || args.nstate <= 0) return record_error(ISDF_ERR_ARG, "fit: bad sizes");
   ISDF_TRY(set_smem_attrs());
+  const size_t mark0 = arena.off;
   FitBuffers b = carve(arena, args.nstate, rk);
+  if (arena.overflowed()) {
+    arena.off = mark0;
+    b = carve(arena, args.nstate, rk, false);
+  }
   if (arena.overflowed()) return record_error(ISDF_ERR_NOMEM, "fit: workspace too small");
   StageEvents ev;
   if (timed) ISDF_TRY(ev.create());
@@ -715,10 +732,11 @@ int fit_fp64(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* res, 
   ISDF_CUDA(cudaMemsetAsync(b.info, 0, 2 * sizeof(int), s));
   if (args.d_psimu) {
     b.Bm = const_cast<double*>(args.d_psimu);
+    b.ldb = rk;
   } else {
     ISDF_CUDA(cudaMemcpyAsync(b.piv, args.piv, sizeof(int) * rk, cudaMemcpyHostToDevice, s));
     k_gather_psimu<<<grid_for((long long)args.nstate * rk, 256), 256, 0, s>>>(
-        args.d_psi, ng, args.nstate, b.piv, rk, b.Bm);
+        args.d_psi, ng, args.nstate, b.piv, rk, b.ldb, b.Bm);
   }
 
   // Z C^T into theta
@@ -729,24 +747,24 @@ int fit_fp64(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* res, 
   ISDF_CUDA(mark(0));
   const double* A1 = args.d_psi + (long long)lo1 * ng;
   const double* A2 = args.d_psi + (long long)lo2 * ng;
-  const double* B1 = b.Bm + (size_t)lo1 * rk;
-  const double* B2 = b.Bm + (size_t)lo2 * rk;
-  const bool zv2 = vec2_ok(A1, ng, B1, rk) && vec2_ok(A2, ng, B2, rk);
+  const double* B1 = b.Bm + (size_t)lo1 * b.ldb;
+  const double* B2 = b.Bm + (size_t)lo2 * b.ldb;
+  const int ldb = b.ldb;
+  const bool zws = ws_ok(args.d_psi, b.Bm, ldb);
   const size_t zs = CoreZ::SMEM_BYTES;
-  // warp-specialised tile: 16-byte aligned operands, Ng and rk even (vec2_ok)
   const unsigned zw = (unsigned)(((rk + WsN::BN - 1) / WsN::BN) * ((ng + WsN::BM - 1) / WsN::BM));
   const int wt = WsN::THREADS;
   const size_t ws = WsN::SMEM_BYTES;
   double* th = args.d_theta;
   if (same) {
-    if (zv2) k_gemm_zws<0><<<zw, wt, ws, s>>>((int)ng, rk, K1, A1, ng, B1, rk, th, ng, b.err);
-    else k_gemm_z<0, 1><<<zg, 256, zs, s>>>((int)ng, rk, K1, A1, ng, B1, rk, args.d_theta, ng);
-  } else if (zv2) {
-    k_gemm_zws<1><<<zw, wt, ws, s>>>((int)ng, rk, K1, A1, ng, B1, rk, th, ng, b.err);
-    k_gemm_zws<2><<<zw, wt, ws, s>>>((int)ng, rk, K2, A2, ng, B2, rk, th, ng, b.err);
+    if (zws) k_gemm_zws<0><<<zw, wt, ws, s>>>((int)ng, rk, K1, A1, ng, B1, ldb, th, ng, b.err);
+    else k_gemm_z<0, 1><<<zg, 256, zs, s>>>((int)ng, rk, K1, A1, ng, B1, ldb, th, ng);
+  } else if (zws) {
+    k_gemm_zws<1><<<zw, wt, ws, s>>>((int)ng, rk, K1, A1, ng, B1, ldb, th, ng, b.err);
+    k_gemm_zws<2><<<zw, wt, ws, s>>>((int)ng, rk, K2, A2, ng, B2, ldb, th, ng, b.err);
   } else {
-    k_gemm_z<1, 1><<<zg, 256, zs, s>>>((int)ng, rk, K1, A1, ng, B1, rk, args.d_theta, ng);
-    k_gemm_z<2, 1><<<zg, 256, zs, s>>>((int)ng, rk, K2, A2, ng, B2, rk, args.d_theta, ng);
+    k_gemm_z<1, 1><<<zg, 256, zs, s>>>((int)ng, rk, K1, A1, ng, B1, ldb, th, ng);
+    k_gemm_z<2, 1><<<zg, 256, zs, s>>>((int)ng, rk, K2, A2, ng, B2, ldb, th, ng);
   }
   ISDF_CHECK_LAUNCH();
 
@@ -757,10 +775,10 @@ int fit_fp64(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* res, 
     // the product of rows j and nu sums the same terms in the same order)
     dim3 cg((unsigned)((rk + CoreZ::BN - 1) / CoreZ::BN), (unsigned)((rk + CoreZ::BM - 1) / CoreZ::BM));
     if (same) {
-      k_gemm_z<0, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, rk, B1, rk, b.P, rk);
+      k_gemm_z<0, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, rk);
     } else {
-      k_gemm_z<1, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, rk, B1, rk, b.P, rk);
-      k_gemm_z<2, 1><<<cg, 256, zs, s>>>(rk, rk, K2, B2, rk, B2, rk, b.P, rk);
+      k_gemm_z<1, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, rk);
+      k_gemm_z<2, 1><<<cg, 256, zs, s>>>(rk, rk, K2, B2, b.ldb, B2, b.ldb, b.P, rk);
     }
   } else {
     k_gather_cct<<<grid_for((long long)rk * rk, 256), 256, 0, s>>>(args.d_theta, ng, b.piv, rk,
@@ -1035,10 +1053,11 @@ int fit_mixed_s(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* re
   ISDF_CUDA(cudaMemsetAsync(mb.err, 0, sizeof(int), s));
   if (args.d_psimu) {
     b.Bm = const_cast<double*>(args.d_psimu);
+    b.ldb = rk;
   } else {
     ISDF_CUDA(cudaMemcpyAsync(b.piv, args.piv, sizeof(int) * rk, cudaMemcpyHostToDevice, s));
     k_gather_psimu<<<grid_for((long long)args.nstate * rk, 256), 256, 0, s>>>(
-        args.d_psi, ng, args.nstate, b.piv, rk, b.Bm);
+        args.d_psi, ng, args.nstate, b.piv, rk, b.ldb, b.Bm);
   }
   ISDF_CUDA(cudaEventRecord(ev.e[0], s));
 
@@ -1050,7 +1069,7 @@ int fit_mixed_s(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* re
     const int kp = round_up(K, ozaki::BKB);
     ISDF_TRY((slice_operand<SZ, false>(args.d_psi + (long long)lo * ng, 1, ng, (int)ng, K, mp, kp,
                                       mb.ea, mb.PA, s)));
-    ISDF_TRY((slice_operand<SZ, true>(b.Bm + (size_t)lo * rk, 1, rk, rk, K, np, kp, mb.eb, mb.PB,
+    ISDF_TRY((slice_operand<SZ, true>(b.Bm + (size_t)lo * b.ldb, 1, b.ldb, rk, K, np, kp, mb.eb, mb.PB,
                                      s)));
     if (same)
       ISDF_TRY((ozaki_gemm<SZ, 1, 0>(mb, mb.ea, (int)ng, rk, kp, args.d_theta, ng, mb.ez, s)));
@@ -1068,15 +1087,15 @@ int fit_mixed_s(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* re
   {
     const int lo1 = args.nocc - args.nv1, K1 = args.nv1 + args.nc1;
     const int lo2 = args.nocc - args.nv2, K2 = args.nv2 + args.nc2;
-    const double* B1 = b.Bm + (size_t)lo1 * rk;
-    const double* B2 = b.Bm + (size_t)lo2 * rk;
+    const double* B1 = b.Bm + (size_t)lo1 * b.ldb;
+    const double* B2 = b.Bm + (size_t)lo2 * b.ldb;
     dim3 cg((unsigned)((rk + CoreZ::BN - 1) / CoreZ::BN), (unsigned)((rk + CoreZ::BM - 1) / CoreZ::BM));
     const size_t zs = CoreZ::SMEM_BYTES;
     if (same) {
-      k_gemm_z<0, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, rk, B1, rk, b.P, rk);
+      k_gemm_z<0, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, rk);
     } else {
-      k_gemm_z<1, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, rk, B1, rk, b.P, rk);
-      k_gemm_z<2, 1><<<cg, 256, zs, s>>>(rk, rk, K2, B2, rk, B2, rk, b.P, rk);
+      k_gemm_z<1, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, rk);
+      k_gemm_z<2, 1><<<cg, 256, zs, s>>>(rk, rk, K2, B2, b.ldb, B2, b.ldb, b.P, rk);
     }
   }
   k_regularise<<<1, 256, 0, s>>>(b.P, rk, b.eps);

@@ -29,7 +29,8 @@ struct FitResult {
   float t_gemm_ms = 0;  // the triangular stage's GEMM launches alone (0: not timed apart)
 };
 
-size_t fit_workspace_bytes(long long ng, int nstate, int rk);
+// pad = false: the least the FP64 fit runs in (psi(mu) without its padding).
+size_t fit_workspace_bytes(long long ng, int nstate, int rk, bool pad = true);
 
 // Mixed-precision fit: the large products as INT8-sliced (`slices` = 5..7)
 // GEMMs on the tcgen05 tensor cores, FP64 Cholesky and triangular inverse.

@@ -59,7 +59,7 @@ int fit_noalloc(const double* d_psi, long long ng, int nstate, int nocc, int nv1
   for (int j = 0; j < rk; ++j)
     if (piv[j] < 0 || piv[j] >= ng)
       return record_error(ISDF_ERR_ARG, "isdf_fit_noalloc: pivot outside the grid");
-  const size_t need = fit_workspace_bytes(ng, nstate, rk);
+  const size_t need = fit_workspace_bytes(ng, nstate, rk, /*pad=*/false);
   if (need > (size_t)ISDF_NOALLOC_SCRATCH_BYTES) {
     static thread_local char msg[200];
     snprintf(msg, sizeof(msg),

@@ -167,3 +167,23 @@ def test_fit_warp_specialised_tiles_equal_cp_async_tiles(torch_cuda, name):
         outs.append(d_theta.cpu().numpy())
     assert np.isfinite(outs[0]).all()
     assert np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("ng", [(5, 7, 9), (13, 5, 1), (3, 3, 3), (8, 8, 8), (11, 16, 4), (9, 7, 21)])
+@pytest.mark.parametrize("window", [(4, 4, 6, 4, 6), (3, 2, 1, 3, 4), (5, 1, 0, 5, 3)])
+def test_fit_odd_sizes(torch_cuda, ng, window):
+    """Row tiles with odd remainders, odd and even numbers of points and of
+    grid rows, state windows that start at odd columns: theta against the numpy
+    fit. theta is determined to cond(C C^T) 2^-53; the bound allows 1e3 of it."""
+    n = ng[0] * ng[1] * ng[2]
+    rng = np.random.default_rng(n)
+    psi = np.asfortranarray(rng.standard_normal((n, 10)))
+    for rk in sorted({1, 2, 9, min(n, 17), min(n, 26)}):
+        piv = np.sort(rng.choice(n, size=rk, replace=False)).astype(np.int32)
+        th = _run_fit(torch_cuda, psi, *window, rk, piv)
+        th_o = ofit.getbasis(psi, *window, rk, piv)
+        nocc, nv1, nc1, nv2, nc2 = window
+        s1, s2 = psi[piv, nocc - nv1:nocc + nc1], psi[piv, nocc - nv2:nocc + nc2]
+        cct = (s1 @ s1.T) * (s2 @ s2.T)
+        cct += 1e-10 * np.trace(cct) / rk * np.eye(rk)
+        assert ofit.rel(th, th_o) <= 1e3 * np.linalg.cond(cct) * 2.0 ** -53
