@@ -50,7 +50,7 @@ constexpr int kNB = 64;  // Cholesky / triangular-solve block size
 using CoreZ = dmma::Core<128, 128>;  // Z GEMM, Cholesky trailing update
 using CoreN = dmma::Core<128, 64>;   // panel and triangular-solve steps
 using CoreS = dmma::Core<64, 64>;    // Cholesky trailing update, small
-using WsN = dmma::WsTile<64, 64, 2, 2, 16, 4>;  // triangular-solve steps, 3 CTAs per SM
+using WsN = dmma::WsTile<64, 64, 2, 2, 16, 4>;  // Z C^T, Y Y^T: 3 CTAs per SM
 
 // 16-byte cp.async needs 16-byte aligned rows: base aligned, even leading dimension.
 __host__ __device__ inline bool vec2_ok(const void* a, long long lda, const void* b,
@@ -195,27 +195,28 @@ __global__ void k_gather_psimu(const double* __restrict__ psi, long long ng, int
   }
 }
 
-// P(mu, nu) = Z(piv_nu, mu), column-major rk x rk.
+// P(mu, nu) = Z(piv_nu, mu), column-major rk x rk, leading dimension ld.
 __global__ void k_gather_cct(const double* __restrict__ Z, long long ng,
-                             const int* __restrict__ piv, int rk, double* __restrict__ P) {
+                             const int* __restrict__ piv, int rk, int ld,
+                             double* __restrict__ P) {
   const long long total = (long long)rk * rk;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
     int mu = (int)(e % rk), nu = (int)(e / rk);
-    P[e] = Z[(long long)piv[nu] + (long long)mu * ng];
+    P[mu + (long long)nu * ld] = Z[(long long)piv[nu] + (long long)mu * ng];
   }
 }
 
 // trace in index order, eps = 1e-10 * (trace / rk), diagonal += eps. The
 // diagonal is staged in shared memory: one thread reading it from global memory
 // while it adds took 56 us at rk = 1600.
-__global__ void __launch_bounds__(256) k_regularise(double* P, int rk, double* eps_out) {
+__global__ void __launch_bounds__(256) k_regularise(double* P, int rk, int ld, double* eps_out) {
   __shared__ double eps;
   __shared__ double diag[1024];
   double tr = 0.0;
   for (int base = 0; base < rk; base += 1024) {
     const int cnt = min(1024, rk - base);
-    for (int i = threadIdx.x; i < cnt; i += 256) diag[i] = P[(long long)(base + i) * (rk + 1)];
+    for (int i = threadIdx.x; i < cnt; i += 256) diag[i] = P[(long long)(base + i) * (ld + 1)];
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll 16
@@ -229,7 +230,7 @@ __global__ void __launch_bounds__(256) k_regularise(double* P, int rk, double* e
   }
   __syncthreads();
   for (int i = threadIdx.x; i < rk; i += blockDim.x) {
-    double* d = P + (long long)i * rk + i;
+    double* d = P + (long long)i * ld + i;
     *d = radd(*d, eps);
   }
 }
@@ -388,23 +389,13 @@ __global__ void __launch_bounds__(256) k_chol_update(double* A, int lda, int k0,
       [](double old, double v) { return old - v; });
 }
 
-// Clears the strict upper triangle left over in the factor's storage.
-__global__ void k_clear_upper(double* L, int n) {
-  const long long total = (long long)n * n;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(e % n), c = (int)(e / n);
-    if (r < c) L[e] = 0.0;
-  }
-}
-
 // ----------------------------------------------------------- triangular solve
 // W_K (depth-major, 64 columns, W[k*64 + n]) for column block [c0, c0+bs):
 //  forward  (rows k < c0+bs): k < c0: -sum_j L(c0+j, k) D^T(j, n);  else D^T(k-c0, n)
 //  backward (rows k >= c0):   k >= c0+bs: -sum_j L(k, c0+j) D(j, n); else D(k-c0, n)
 // with dT[j*64 + n] = D(n, j) and d[j*64 + n] = D(j, n), D = L_KK^{-1} (zero-padded).
 template <bool FORWARD>
-__global__ void __launch_bounds__(256) k_build_w(const double* __restrict__ L, int rk, int c0,
+__global__ void __launch_bounds__(256) k_build_w(const double* __restrict__ L, int ld, int rk, int c0,
                                                  int bs, const double* __restrict__ dmat,
                                                  double* __restrict__ W) {
   __shared__ double ds[kNB * kNB];
@@ -417,7 +408,7 @@ __global__ void __launch_bounds__(256) k_build_w(const double* __restrict__ L, i
     if (FORWARD ? (k < c0) : (k >= c0 + bs)) {
       double s = 0.0;
       for (int j = 0; j < bs; ++j) {
-        const double l = FORWARD ? L[(c0 + j) + (long long)k * rk] : L[k + (long long)(c0 + j) * rk];
+        const double l = FORWARD ? L[(c0 + j) + (long long)k * ld] : L[k + (long long)(c0 + j) * ld];
         s = fma(l, ds[j * kNB + n], s);
       }
       v = -s;
@@ -443,16 +434,71 @@ __global__ void __launch_bounds__(256) k_trsm_gemm(double* theta, long long ng, 
   });
 }
 
-// The same step on the warp-specialised tile (theta 16-byte aligned, Ng even).
+// ---- the steps on the warp-specialised tile (theta 16-byte aligned, any Ng).
+// The W_K panels of all steps are built beforehand in place of L, in two launches
+// instead of one (10 to 13 us) before every step: the forward panel of block K in
+// the rows of block K left of the diagonal, the backward panel in the mirror image
+// above it, each with W(k, n) at P[c0 + n + k ld], and the diagonal block holds
+// D^T for the forward steps and D for the backward ones.
+//
+// Tried instead of a launch per step: one launch for both sweeps, with the CTAs
+// taking (step, row tile) units from a list (522 us against 585 at 64 000 rows and
+// 309 points, the same at 245 760 and 1201 or 512 000 and 2007), and CTAs that take
+// their own row tiles through all steps (134 ms against 127 at 2007: the three CTAs
+// of an SM do not share its tensor pipe evenly, and units that long leave a tail).
+// A step of depth K runs at 34.2 TFLOP/s for K near 1600 and 31.8 near 430.
+//
+// Panels: W_K(k, n) = -sum_j L(c0 + j, k) D(n, j) for k < c0 (forward, in place)
+//         W_K(k, n) = -sum_j L(k, c0 + j) D(j, n) for k >= c0 + bs (backward, to
+// column k above the diagonal; all of them before the forward ones).
+template <bool FORWARD>
+__global__ void __launch_bounds__(256) k_build_panels(double* P, int ld, int rk,
+                                                      const double* __restrict__ dmat) {
+  __shared__ double ds[kNB * kNB];
+  __shared__ double v[4][kNB];
+  const int c0 = blockIdx.y * kNB, bs = min(kNB, rk - c0);
+  const int klo = FORWARD ? 0 : c0 + bs, khi = FORWARD ? c0 : rk;
+  if (klo + (int)blockIdx.x * 4 >= khi) return;
+  for (int e = threadIdx.x; e < kNB * kNB; e += 256)
+    ds[e] = dmat[(size_t)blockIdx.y * kNB * kNB + e];
+  const int n = threadIdx.x & 63, w = threadIdx.x >> 6;
+  for (int k0 = klo + blockIdx.x * 4; k0 < khi; k0 += gridDim.x * 4) {
+    const int k = k0 + w;
+    __syncthreads();
+    if (k < khi && n < bs)
+      v[w][n] = FORWARD ? P[(c0 + n) + (long long)k * ld] : P[k + (long long)(c0 + n) * ld];
+    __syncthreads();
+    if (k < khi && n < bs) {
+      double s = 0.0;
+#pragma unroll 8
+      for (int j = 0; j < bs; ++j) s = fma(v[w][j], ds[j * kNB + n], s);
+      P[(c0 + n) + (long long)k * ld] = -s;
+    }
+  }
+}
+
+// D^T (forward) or D (backward) into the diagonal blocks of P.
+__global__ void __launch_bounds__(256) k_diag_panels(double* P, int ld, int rk,
+                                                     const double* __restrict__ dmat) {
+  const int c0 = blockIdx.x * kNB, bs = min(kNB, rk - c0);
+  const double* d = dmat + (size_t)blockIdx.x * kNB * kNB;
+  for (int e = threadIdx.x; e < kNB * kNB; e += 256) {
+    const int k = e / kNB, n = e % kNB;
+    if (k < bs && n < bs) P[(c0 + n) + (long long)(c0 + k) * ld] = d[e];
+  }
+}
+
+// theta[rows, c0:c0+bs] = theta[rows, kb:ke] * W[kb:ke, 0:bs], in place per row
+// tile, W(k, n) = P[c0 + n + k ld].
 __global__ void __launch_bounds__(WsN::THREADS, 3)
     k_trsm_ws(double* theta, long long ng, int c0, int bs, int kb, int ke,
-              const double* __restrict__ W, int* err) {
+              const double* __restrict__ P, int ld, int* err) {
   extern __shared__ __align__(128) double smem[];
   const long long m0 = (long long)blockIdx.x * WsN::BM;
   const int m_rem = (int)(ng - m0 < WsN::BM ? ng - m0 : WsN::BM);
   WsN tile;
-  if (!tile.run(smem, theta + m0 + (long long)kb * ng, ng, m_rem, W + (long long)kb * kNB, kNB,
-                kNB, ke - kb, err))
+  if (!tile.run(smem, theta + m0 + (long long)kb * ng, ng, m_rem, P + c0 + (long long)kb * ld, ld,
+                bs, ke - kb, err))
     return;
   if (WsN::producer()) return;
   tile.for_each([&](int r, int c, double v) {
@@ -566,8 +612,9 @@ struct FitBuffers {
   int* piv;
   double* Bm;  // nstate x rk, row length ldb (rk, rounded up to even where padded)
   int ldb;
-  double* P;  // C C^T, then L (column-major rk x rk)
-  double* W;  // one triangular-solve block operand, rk x 64
+  double* P;  // C C^T, then L, then the sweeps' panels (column-major rk x rk)
+  int ldp;    // its leading dimension (rk, rounded up to even where padded)
+  double* W;  // one triangular-solve block operand, rk x 64 (unpadded P, unaligned theta)
   double* dinvT;
   double* dinv;
   double* eps;
@@ -575,15 +622,16 @@ struct FitBuffers {
   int* err;
 };
 
-// pad = false: the rows of Bm as they come (a scratch array without room for the
-// padding).
+// pad = false: the rows of Bm and the columns of P as they come (a scratch array
+// without room for the padding; the mixed form).
 FitBuffers carve(Arena& a, int nstate, int rk, bool pad = true) {
   FitBuffers b;
   const int nblk = (rk + kNB - 1) / kNB;
   b.piv = a.take<int>(rk);
   b.ldb = pad ? rk + (rk & 1) : rk;
   b.Bm = a.take<double>((size_t)nstate * b.ldb);
-  b.P = a.take<double>((size_t)rk * rk);
+  b.ldp = pad ? rk + (rk & 1) : rk;
+  b.P = a.take<double>((size_t)b.ldp * rk);
   b.W = a.take<double>((size_t)rk * kNB);
   b.dinvT = a.take<double>((size_t)nblk * kNB * kNB);
   b.dinv = a.take<double>((size_t)nblk * kNB * kNB);
@@ -668,30 +716,30 @@ constexpr int kCholWide = 3072;
 // inverses for the solve. Returns the failing column + 1 in *info (0 = ok).
 static int cholesky(const FitBuffers& b, int rk, cudaStream_t s) {
   const int nblk = (rk + kNB - 1) / kNB;
-  const bool v2 = (rk % 2) == 0;
+  const int ld = b.ldp;
+  const bool v2 = (ld % 2) == 0;
   for (int kb = 0; kb < nblk; ++kb) {
     const int k0 = kb * kNB;
     const int bs = min(kNB, rk - k0);
-    k_potf2<<<1, kPotf2Threads, smem_bytes_potf2, s>>>(b.P, rk, k0, bs, b.dinvT + (size_t)kb * kNB * kNB,
+    k_potf2<<<1, kPotf2Threads, smem_bytes_potf2, s>>>(b.P, ld, k0, bs, b.dinvT + (size_t)kb * kNB * kNB,
                                              b.dinv + (size_t)kb * kNB * kNB, b.info);
     const int rem = rk - k0 - bs;
     if (rem > 0) {
       const double* dT = b.dinvT + (size_t)kb * kNB * kNB;
       const unsigned pg = (unsigned)((rem + CoreN::BM - 1) / CoreN::BM);
-      if (v2) k_chol_panel<2><<<pg, 256, CoreN::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk, dT);
-      else k_chol_panel<1><<<pg, 256, CoreN::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk, dT);
+      if (v2) k_chol_panel<2><<<pg, 256, CoreN::SMEM_BYTES, s>>>(b.P, ld, k0, bs, rk, dT);
+      else k_chol_panel<1><<<pg, 256, CoreN::SMEM_BYTES, s>>>(b.P, ld, k0, bs, rk, dT);
       if (rem >= kCholWide) {
         const dim3 g((rem + CoreZ::BN - 1) / CoreZ::BN, (rem + CoreZ::BM - 1) / CoreZ::BM);
         auto k = v2 ? k_chol_update<CoreZ, 2> : k_chol_update<CoreZ, 1>;
-        k<<<g, 256, CoreZ::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk);
+        k<<<g, 256, CoreZ::SMEM_BYTES, s>>>(b.P, ld, k0, bs, rk);
       } else {
         const dim3 g((rem + CoreS::BN - 1) / CoreS::BN, (rem + CoreS::BM - 1) / CoreS::BM);
         auto k = v2 ? k_chol_update<CoreS, 2> : k_chol_update<CoreS, 1>;
-        k<<<g, 256, CoreS::SMEM_BYTES, s>>>(b.P, rk, k0, bs, rk);
+        k<<<g, 256, CoreS::SMEM_BYTES, s>>>(b.P, ld, k0, bs, rk);
       }
     }
   }
-  k_clear_upper<<<grid_for((long long)rk * rk, 256), 256, 0, s>>>(b.P, rk);
   ISDF_CHECK_LAUNCH();
   return ISDF_OK;
 }
@@ -726,8 +774,9 @@ int fit_fp64(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* res, 
   auto mark = [&](int i) { return timed ? cudaEventRecord(ev.e[i], s) : cudaSuccess; };
   const int nblk_ = (rk + kNB - 1) / kNB;
   const bool same_ = (args.nv1 == args.nv2 && args.nc1 == args.nc2);
-  res->launches = 1 + (same_ ? 1 : 2) + 2 + (nblk_ + 2 * (nblk_ - 1) + 1) + 4 * nblk_ +
-                  (readback_mailbox() ? 2 : 0);
+  const bool tws = ws_ok(args.d_theta, b.P, b.ldp);
+  res->launches = 1 + (same_ ? 1 : 2) + 2 + (nblk_ + 2 * (nblk_ - 1)) +
+                  (tws ? 2 * nblk_ + 4 : 4 * nblk_) + (readback_mailbox() ? 2 : 0);
 
   ISDF_CUDA(cudaMemsetAsync(b.info, 0, 2 * sizeof(int), s));
   if (args.d_psimu) {
@@ -775,16 +824,16 @@ int fit_fp64(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* res, 
     // the product of rows j and nu sums the same terms in the same order)
     dim3 cg((unsigned)((rk + CoreZ::BN - 1) / CoreZ::BN), (unsigned)((rk + CoreZ::BM - 1) / CoreZ::BM));
     if (same) {
-      k_gemm_z<0, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, rk);
+      k_gemm_z<0, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, b.ldp);
     } else {
-      k_gemm_z<1, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, rk);
-      k_gemm_z<2, 1><<<cg, 256, zs, s>>>(rk, rk, K2, B2, b.ldb, B2, b.ldb, b.P, rk);
+      k_gemm_z<1, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, b.ldp);
+      k_gemm_z<2, 1><<<cg, 256, zs, s>>>(rk, rk, K2, B2, b.ldb, B2, b.ldb, b.P, b.ldp);
     }
   } else {
     k_gather_cct<<<grid_for((long long)rk * rk, 256), 256, 0, s>>>(args.d_theta, ng, b.piv, rk,
-                                                                  b.P);
+                                                                  b.ldp, b.P);
   }
-  k_regularise<<<1, 256, 0, s>>>(b.P, rk, b.eps);
+  k_regularise<<<1, 256, 0, s>>>(b.P, rk, b.ldp, b.eps);
   ISDF_TRY(cholesky(b, rk, s));
   ISDF_CUDA(mark(2));
   int info = 0;
@@ -795,26 +844,36 @@ int fit_fp64(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* res, 
   // theta L^T = Z C^T (forward over column blocks), then theta L = Y (backward)
   const int nblk = (rk + kNB - 1) / kNB;
   const unsigned tg = (unsigned)((ng + CoreN::BM - 1) / CoreN::BM);
-  const unsigned wg = (unsigned)((ng + WsN::BM - 1) / WsN::BM);
-  const bool tv2 = vec2_ok(args.d_theta, ng, b.W, kNB);
-  auto step = [&](int c0, int bs, int kb, int ke) {
-    if (tv2)  // 16-byte aligned columns: bulk copies
-      k_trsm_ws<<<wg, WsN::THREADS, WsN::SMEM_BYTES, s>>>(args.d_theta, ng, c0, bs, kb, ke, b.W,
-                                                           b.err);
-    else
+  if (tws) {
+    const dim3 pg((unsigned)std::min(64, (rk + 3) / 4), (unsigned)nblk);
+    const unsigned wg = (unsigned)((ng + WsN::BM - 1) / WsN::BM);
+    auto step = [&](int c0, int bs, int kb, int ke) {
+      k_trsm_ws<<<wg, WsN::THREADS, WsN::SMEM_BYTES, s>>>(args.d_theta, ng, c0, bs, kb, ke, b.P,
+                                                          b.ldp, b.err);
+    };
+    k_build_panels<false><<<pg, 256, 0, s>>>(b.P, b.ldp, rk, b.dinv);
+    k_build_panels<true><<<pg, 256, 0, s>>>(b.P, b.ldp, rk, b.dinvT);
+    k_diag_panels<<<nblk, 256, 0, s>>>(b.P, b.ldp, rk, b.dinvT);
+    for (int c0 = 0; c0 < rk; c0 += kNB) step(c0, min(kNB, rk - c0), 0, min(c0 + kNB, rk));
+    k_diag_panels<<<nblk, 256, 0, s>>>(b.P, b.ldp, rk, b.dinv);
+    for (int c0 = (nblk - 1) * kNB; c0 >= 0; c0 -= kNB) step(c0, min(kNB, rk - c0), c0, rk);
+  } else {
+    // a theta that does not start 16-byte aligned, or no room for P's padding
+    auto step = [&](int c0, int bs, int kb, int ke) {
       k_trsm_gemm<1><<<tg, 256, CoreN::SMEM_BYTES, s>>>(args.d_theta, ng, c0, bs, kb, ke, b.W);
-  };
-  for (int kb = 0; kb < nblk; ++kb) {
-    const int c0 = kb * kNB, bs = min(kNB, rk - c0);
-    k_build_w<true><<<(c0 + bs + 3) / 4 < 1024 ? (c0 + bs + 3) / 4 : 1024, 256, 0, s>>>(
-        b.P, rk, c0, bs, b.dinvT + (size_t)kb * kNB * kNB, b.W);
-    step(c0, bs, 0, c0 + bs);
-  }
-  for (int kb = nblk - 1; kb >= 0; --kb) {
-    const int c0 = kb * kNB, bs = min(kNB, rk - c0);
-    k_build_w<false><<<(rk - c0 + 3) / 4 < 1024 ? (rk - c0 + 3) / 4 : 1024, 256, 0, s>>>(
-        b.P, rk, c0, bs, b.dinv + (size_t)kb * kNB * kNB, b.W);
-    step(c0, bs, c0, rk);
+    };
+    for (int kb = 0; kb < nblk; ++kb) {
+      const int c0 = kb * kNB, bs = min(kNB, rk - c0);
+      k_build_w<true><<<(c0 + bs + 3) / 4 < 1024 ? (c0 + bs + 3) / 4 : 1024, 256, 0, s>>>(
+          b.P, b.ldp, rk, c0, bs, b.dinvT + (size_t)kb * kNB * kNB, b.W);
+      step(c0, bs, 0, c0 + bs);
+    }
+    for (int kb = nblk - 1; kb >= 0; --kb) {
+      const int c0 = kb * kNB, bs = min(kNB, rk - c0);
+      k_build_w<false><<<(rk - c0 + 3) / 4 < 1024 ? (rk - c0 + 3) / 4 : 1024, 256, 0, s>>>(
+          b.P, b.ldp, rk, c0, bs, b.dinv + (size_t)kb * kNB * kNB, b.W);
+      step(c0, bs, c0, rk);
+    }
   }
   ISDF_CHECK_LAUNCH();
   ISDF_CUDA(mark(3));
@@ -1042,7 +1101,7 @@ int fit_mixed_s(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* re
   constexpr int SZ = S > 5 ? S - 1 : S;
   const long long ng = args.ng;
   const int rk = args.rk;
-  FitBuffers b = carve(arena, args.nstate, rk);
+  FitBuffers b = carve(arena, args.nstate, rk, false);
   MixedBuffers mb = carve_mixed(arena, ng, args.nstate, rk, S);
   if (arena.overflowed()) return record_error(ISDF_ERR_NOMEM, "mixed fit: workspace too small");
   StageEvents ev;
@@ -1092,13 +1151,13 @@ int fit_mixed_s(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* re
     dim3 cg((unsigned)((rk + CoreZ::BN - 1) / CoreZ::BN), (unsigned)((rk + CoreZ::BM - 1) / CoreZ::BM));
     const size_t zs = CoreZ::SMEM_BYTES;
     if (same) {
-      k_gemm_z<0, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, rk);
+      k_gemm_z<0, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, b.ldp);
     } else {
-      k_gemm_z<1, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, rk);
-      k_gemm_z<2, 1><<<cg, 256, zs, s>>>(rk, rk, K2, B2, b.ldb, B2, b.ldb, b.P, rk);
+      k_gemm_z<1, 1><<<cg, 256, zs, s>>>(rk, rk, K1, B1, b.ldb, B1, b.ldb, b.P, b.ldp);
+      k_gemm_z<2, 1><<<cg, 256, zs, s>>>(rk, rk, K2, B2, b.ldb, B2, b.ldb, b.P, b.ldp);
     }
   }
-  k_regularise<<<1, 256, 0, s>>>(b.P, rk, b.eps);
+  k_regularise<<<1, 256, 0, s>>>(b.P, rk, b.ldp, b.eps);
   ISDF_TRY(cholesky(b, rk, s));
   int info = 0;
   ISDF_TRY(read_back(&info, b.info, sizeof(int), s));
@@ -1154,7 +1213,7 @@ int fit_mixed_s(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* re
   const int nblk = (rk + kNB - 1) / kNB;
   int levels = 0;
   for (int lv = kNB; lv < rk; lv *= 2) ++levels;
-  res->launches = 1 + (same ? 3 : 6) * 2 + 2 + (nblk + 2 * (nblk - 1) + 1) + 1 + 2 * levels + 10 +
+  res->launches = 1 + (same ? 3 : 6) * 2 + 2 + (nblk + 2 * (nblk - 1)) + 1 + 2 * levels + 10 +
                   (readback_mailbox() ? 2 : 0);
   return ISDF_OK;
 }
@@ -1164,7 +1223,7 @@ int fit_mixed_s(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* re
 size_t fit_mixed_workspace_bytes(long long ng, int nstate, int rk, int slices) {
   Arena a;
   a.counting = true;
-  carve(a, nstate, rk);
+  carve(a, nstate, rk, false);
   carve_mixed(a, ng, nstate, rk, slices);
   return a.off;
 }
