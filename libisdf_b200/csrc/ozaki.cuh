@@ -31,17 +31,22 @@
 // bulk copies (cp.async.bulk, no tensor map, no multicast) issued by one
 // thread and completing on the stage's mbarrier by transaction count.
 //
-// Warp roles (320 threads, one persistent CTA per SM): warps 0-7 run the
-// epilogue (warp w reads TMEM lanes 32 (w % 4) .. + 31 and half of the tile's
-// columns, so that two warps share each lane quarter and the conversion and
-// stores of a tile take half as long), one thread of warp 8 issues the MMAs
-// and warp 8 owns the TMEM allocation, one thread of warp 9 issues the copies
-// into an NSTAGE-deep ring that runs ahead across tiles. Each ring
+// Warp roles (576 threads, one persistent CTA per SM): warps 0-15 run the
+// epilogue (warp w reads TMEM lanes 32 (w % 4) .. + 31 and a quarter of the
+// tile's columns), one thread of warp 16 issues the MMAs and warp 16 owns the
+// TMEM allocation, one thread of warp 17 issues the copies into an NSTAGE-deep
+// ring that runs ahead across tiles. Each ring
 // slot has a "full" mbarrier (expect-tx arrival plus the copies' bytes) and
 // an "empty" mbarrier (tcgen05.commit after the slot's MMAs); acc_full /
 // acc_empty hand the accumulators between the MMA thread and the epilogue,
 // which releases them as soon as they are in registers and stores while the
-// next tile's MMAs run. Every wait is bounded: a timeout sets a shared abort
+// next tile's MMAs run. The accumulators fill most of the TMEM, so that no MMA
+// runs while they are drained, and the drain bounds the short-K products: the
+// levels are read and converted two at a time, and the accumulators released
+// before the last two are converted. (With eight warps
+// that converted every level by the conversion instruction first, Z C^T of
+// 216 000 x 1600, K = 224 took 2.53 ms against 1.73, and the triangular products
+// of that size 4.69 against 4.26.) Every wait is bounded: a timeout sets a shared abort
 // flag and *err, the other waiters give up on seeing the flag, and before
 // the CTA exits the kernel still waits (bounded) for its issued copies and
 // MMAs, freeing its TMEM last.
@@ -61,7 +66,7 @@ namespace ozaki {
 
 constexpr int BM = 128, BN = 64, BKB = 32;  // tile rows, tile columns, K bytes per stage
 constexpr int kTmemCols = 512;
-constexpr int kEpiWarps = 8;  // two per TMEM lane quarter, each draining half the columns
+constexpr int kEpiWarps = 16;  // four per TMEM lane quarter, each draining a quarter of the columns
 constexpr int kThreads = (kEpiWarps + 2) * 32;
 constexpr int kGroupM = 8;
 constexpr int kSmemLimit = 232448;  // 227 KB per CTA
@@ -138,6 +143,13 @@ __host__ __device__ __forceinline__ long long tiled_offset(long long blk, int kb
 __device__ __forceinline__ double pow2(int e) {
   return (e >= -1022 && e <= 1023) ? __longlong_as_double((long long)(e + 1023) << 52)
                                    : ldexp(1.0, e);
+}
+
+// A signed 32-bit accumulator as a double, exactly: its bits (sign flipped, so
+// unsigned) under the exponent of 2^52, less 2^52 + 2^31. One addition on the
+// FP64 pipe instead of a conversion at a quarter of its rate.
+__device__ __forceinline__ double int_value(uint32_t v) {
+  return __dsub_rn(__hiloint2double(0x43300000, (int)(v ^ 0x80000000u)), 4503601774854144.0);
 }
 
 // Tile id -> (first row, first column), grouped raster: kGroupM row blocks
@@ -308,6 +320,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // warp w reads TMEM lanes 32 (w % 4) .. + 31 (its rows) and columns
     // [ (w / 4) CW, + CW )
     constexpr int CW = BN / (kEpiWarps / 4);
+    static_assert(CW == 16, "one TMEM load per level");
     const int q = warp & 3, c_lo = (warp >> 2) * CW;
     double w[S];  // 254^{-(d+2)}
     w[0] = 1.0 / (kBase * kBase);
@@ -325,32 +338,38 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int row = q * 32 + lane;
       const long long m = m0 + row;
       const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
+      // per column the levels accumulate in order d = 0, 1, ...
+      constexpr int H = S - 2;  // levels converted before the release, two at a time
       double out[CW];
 #pragma unroll
       for (int j = 0; j < CW; ++j) out[j] = 0.0;
+      uint32_t v[2][CW];
       if (nk > 0) {
-        // 16 columns per TMEM round trip, two levels at a time; per column the
-        // levels accumulate in order d = 0, 1, ...
 #pragma unroll
-        for (int c0 = 0; c0 < CW; c0 += 16) {
+        for (int d0 = 0; d0 < H; d0 += 2) {
 #pragma unroll
-          for (int d = 0; d < S; d += 2) {
-            uint32_t va[16], vb[16];
-            ISDF_TMEM_LD16(va, lane_base + (uint32_t)(d * BN + c_lo + c0));
-            if (d + 1 < S) ISDF_TMEM_LD16(vb, lane_base + (uint32_t)((d + 1) * BN + c_lo + c0));
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+          for (int d = d0; d < d0 + 2 && d < H; ++d)
+            ISDF_TMEM_LD16(v[d - d0], lane_base + (uint32_t)(d * BN + c_lo));
+          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              out[c0 + j] = __fma_rn((double)(int)va[j], w[d], out[c0 + j]);
-              if (d + 1 < S)
-                out[c0 + j] = __fma_rn((double)(int)vb[j], w[d + 1], out[c0 + j]);
-            }
-          }
+          for (int d = d0; d < d0 + 2 && d < H; ++d)
+#pragma unroll
+            for (int j = 0; j < CW; ++j) out[j] = __fma_rn(int_value(v[d - d0][j]), w[d], out[j]);
         }
+#pragma unroll
+        for (int d = H; d < S; ++d)
+          ISDF_TMEM_LD16(v[d - H], lane_base + (uint32_t)(d * BN + c_lo));
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
       }
       // accumulators drained: the MMA thread may start the next tile
       asm volatile("tcgen05.fence::before_thread_sync;\n");
       mbar_arrive(acc_empty);
+      if (nk > 0) {
+#pragma unroll
+        for (int d = H; d < S; ++d)
+#pragma unroll
+          for (int j = 0; j < CW; ++j) out[j] = __fma_rn(int_value(v[d - H][j]), w[d], out[j]);
+      }
       if (m < M) {
         const double sa = pow2(ea[m]);
         double amax = 0.0;

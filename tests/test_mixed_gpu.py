@@ -58,3 +58,30 @@ def test_mixed_s1_ne_s2(torch_cuda):
     fd = ofit.fitted_densities(th, g["psi"], *a, rk, g["piv"])
     fd_ref = ofit.fitted_densities(g["theta"], g["psi"], *a, rk, g["piv"])
     assert ofit.rel(fd, fd_ref) <= 1e-6
+
+
+@pytest.mark.parametrize("slices", [5, 6, 7])
+@pytest.mark.parametrize("n,rk", [((5, 5, 5), 1), ((8, 8, 4), 33), ((9, 8, 8), 64), ((11, 9, 7), 130)])
+def test_mixed_tile_edges(torch_cuda, n, rk, slices):
+    """Every digit count around the 128 x 64 tiles: theta of the mixed form against
+    the FP64 form's on a well-conditioned system. A product truncates 254^-digits
+    of its operands' scales per term, which the two triangular inverses amplify by
+    cond(L) <= sqrt(cond(C C^T)) each."""
+    torch = torch_cuda
+    ng = n[0] * n[1] * n[2]
+    rng = np.random.default_rng(ng)
+    psi = np.asfortranarray(rng.standard_normal((ng, 24)))
+    piv = np.zeros(ng, dtype=np.int32)
+    d_psi = torch.from_numpy(np.ascontiguousarray(psi.T)).cuda()
+    dom = isdf.Domain(length=(3.0, 4.0, 5.0), num_grid=n)
+    th = []
+    for prec in (isdf.PRECISION_FP64, isdf.PRECISION_MIXED):
+        d_theta = torch.zeros((rk, ng), dtype=torch.float64, device="cuda")
+        r = isdf.ISDF(d_psi, dom, 12, 24, 12, 12, 12, 12, rk, d_theta, piv, 5,
+                      options=isdf.Options(precision=prec, mixed_slices=slices))
+        th.append(d_theta.cpu().numpy())
+    p = piv[:r.rk_eff]
+    cct = (psi[p] @ psi[p].T) ** 2
+    cond = np.linalg.cond(cct + 1e-10 * np.trace(cct) / len(p) * np.eye(len(p)))
+    err = np.linalg.norm(th[0] - th[1]) / np.linalg.norm(th[0])
+    assert err <= cond * max(rk, 24) * 254.0 ** -min(slices, 5 if slices < 7 else 6) + cond * 1e-14
