@@ -28,6 +28,7 @@
 #include "common.cuh"
 #include "solve.h"
 #include "kmeans.h"
+#include "loop_graph.h"
 #include "readback.h"
 
 namespace isdf_b200 {
@@ -691,19 +692,6 @@ __device__ __forceinline__ bool goes_on(const KmJob& J) {
   return J.sharded || ((double)J.st->changed > J.max_f && J.st->s < J.max_iter);
 }
 
-// The iteration's loop in a CUDA graph: a WHILE node's body, ended from the
-// device. No iteration waits for the host.
-struct LoopEnd {
-  cudaGraphConditionalHandle handle;
-  int in_graph;
-  int max_rounds;  // iterations after which the loop ends whatever happens
-  int* live;       // selections of a batch still running (nullptr: one)
-};
-
-__device__ __forceinline__ void end_loop(const LoopEnd& le) {
-  if (le.in_graph) cudaGraphSetConditional(le.handle, 0);
-}
-
 // ---------------------------------------------------------------- update
 // Stable counting sort of the points by label (tiles of kTile points), then
 // one warp per cluster and component folds w, w*x, w*y, w*z over the members
@@ -734,19 +722,20 @@ __global__ void __launch_bounds__(256) k_hist(const __grid_constant__ KmJobs<N> 
 // thread per label walking all tiles left the scan bound by the latency of
 // its ~ntiles/16 dependent load batches. The last block to finish scans the
 // member counts into each label's first slot and begins the iteration: one
-// launch where three single-block kernels ran.
+// launch where three single-block kernels ran. The last selection of a batch to
+// stop (live: how many still run; nullptr for one alone) ends the loop.
 constexpr int kScanWarps = 16;
 
 template <int N>
 __global__ void __launch_bounds__(32 * kScanWarps)
-    k_hist_scan(const __grid_constant__ KmJobs<N> JS, const LoopEnd le) {
+    k_hist_scan(const __grid_constant__ KmJobs<N> JS, const LoopEnd le, int* live) {
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (st->done) return;
   if (!goes_on(J)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       st->done = 1;
-      if (!le.live || atomicSub(le.live, 1) == 1) end_loop(le);
+      if (!live || atomicSub(live, 1) == 1) end_loop(le);
     }
     return;
   }
@@ -1676,11 +1665,12 @@ struct LoopDims {
 // One Lloyd iteration is six launches: the sums, then the centroids and the
 // labels. Every kernel returns at once where the loop has stopped.
 template <int N>
-void launch_sums(const KmJobs<N>& J, const LoopDims& d, const LoopEnd& le, cudaStream_t s) {
+void launch_sums(const KmJobs<N>& J, const LoopDims& d, const LoopEnd& le, int* live,
+                 cudaStream_t s) {
   const size_t hist_smem = sizeof(int) * (size_t)d.mu;
   const size_t scatter_smem = sizeof(short) * kScatterWarps * (size_t)d.mu;
   k_hist<N><<<dim3(d.tiles, d.jobs), 256, hist_smem, s>>>(J, le);
-  k_hist_scan<N><<<dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, 0, s>>>(J, le);
+  k_hist_scan<N><<<dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, 0, s>>>(J, le, live);
   k_scatter<N><<<dim3(d.tiles, d.jobs), 32 * kScatterWarps, scatter_smem, s>>>(J);
   k_segsum<N><<<dim3(d.mu, d.jobs), kFoldThreads, 0, s>>>(J);
 }
@@ -1691,51 +1681,19 @@ void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, cudaStream
   k_assign_warp<N><<<dim3(d.assign, d.jobs), kAssignThreads, 0, s>>>(J, update);
 }
 
-// The loop as a CUDA graph: a WHILE node whose body is kBodyIters iterations,
-// ended from the device, so that no iteration waits for the host (reading the
-// state back after every 8 iterations left the GPU idle for 75 us each time,
-// and the graph of 8 took twice as long to build). exec stays null on a stream
-// that cannot be captured.
-struct LoopGraph {
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  ~LoopGraph() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-  }
-
-  template <int N>
-  void build(const KmJobs<N>& J, const LoopDims& d, int max_iter, int* live, cudaStream_t s) {
-    LoopEnd le{0, 1, max_iter / kBodyIters * kBodyIters + 4 * kBodyIters, live};
-    cudaGraphNodeParams np = {};
-    cudaGraphNode_t node;
-    cudaGraph_t body = nullptr;
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess &&
-              cudaGraphConditionalHandleCreate(&le.handle, graph, 1,
-                                               cudaGraphCondAssignDefault) == cudaSuccess;
-    if (ok) {
-      np.conditional.handle = le.handle;
-      ok = cudaGraphAddNode(&node, graph, nullptr, 0, &np) == cudaSuccess;
+// The Lloyd loop as a graph with kBodyIters iterations per body: no iteration
+// waits for the host (reading the state back after every 8 iterations left the GPU
+// idle for 75 us each time, and the graph of 8 took twice as long to build).
+template <int N>
+void build_loop(LoopGraph& loop, const KmJobs<N>& J, const LoopDims& d, int max_iter, int* live,
+                cudaStream_t s) {
+  loop.build(s, max_iter / kBodyIters * kBodyIters + 4 * kBodyIters, [&](const LoopEnd& le) {
+    for (int it = 0; it < kBodyIters; ++it) {
+      launch_sums(J, d, le, live, s);
+      launch_assign(J, d, 1, s);
     }
-    if (ok) {
-      body = np.conditional.phGraph_out[0];
-      ok = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0,
-                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-    }
-    if (ok) {
-      for (int it = 0; it < kBodyIters; ++it) {
-        launch_sums(J, d, le, s);
-        launch_assign(J, d, 1, s);
-      }
-      ok = cudaStreamEndCapture(s, &body) == cudaSuccess;
-    }
-    if (!ok || cudaGraphInstantiate(&exec, graph, 0ull) != cudaSuccess) exec = nullptr;
-    (void)cudaGetLastError();  // a refused capture leaves an error to clear
-  }
-};
+  });
+}
 
 }  // namespace
 
@@ -1983,7 +1941,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   launch_assign(jobs, dims, 0, stream);
   ISDF_CHECK_LAUNCH();
   LoopGraph loop;
-  if (!shard) loop.build(jobs, dims, args.max_iter, nullptr, stream);
+  if (!shard) build_loop(loop, jobs, dims, args.max_iter, nullptr, stream);
   // Sharded: the rank folds its own points [lo, lo + cnt) (utility.cpp:813-822),
   // the ranks exchange their partial sums and changed-label counts (one
   // all-gather per iteration, utility.cpp:825-826,908-917), and every rank
@@ -1993,10 +1951,10 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   const size_t rec_bytes = sizeof(double4) * ((size_t)mu + 1);
   std::vector<size_t> rcounts(ranks, rec_bytes), rdispls(ranks);
   for (int q = 0; q < ranks; ++q) rdispls[q] = (size_t)q * rec_bytes;
-  const LoopEnd no_graph{0, 0, 0x7fffffff, nullptr};
+  const LoopEnd no_graph{0, 0, 0x7fffffff};
   auto launch_chunk = [&]() -> int {
     for (int it = 0; it < kIterChunk; ++it) {
-      launch_sums(jobs, dims, no_graph, stream);
+      launch_sums(jobs, dims, no_graph, nullptr, stream);
       if (shard) {
         k_shard_header<<<1, 1, 0, stream>>>(b.st, sb.send);
         ISDF_CHECK_LAUNCH();
@@ -2182,16 +2140,16 @@ int select_group(const KmeansArgs* args, int count, Arena& arena, cudaStream_t s
   launch_assign(jobs, dims, 0, stream);
   ISDF_CHECK_LAUNCH();
   LoopGraph loop;
-  loop.build(jobs, dims, max_iter, live, stream);
+  build_loop(loop, jobs, dims, max_iter, live, stream);
   if (loop.exec) {
     ISDF_CUDA(cudaGraphLaunch(loop.exec, stream));
   } else {
-    const LoopEnd no_graph{0, 0, 0x7fffffff, live};
+    const LoopEnd no_graph{0, 0, 0x7fffffff};
     for (int left = nj, chunks = 0; left > 0; ++chunks) {
       if (chunks > max_iter / kIterChunk + 2)
         return record_error(ISDF_ERR_CUDA, "kmeans batch: loop did not stop");
       for (int it = 0; it < kIterChunk; ++it) {
-        launch_sums(jobs, dims, no_graph, stream);
+        launch_sums(jobs, dims, no_graph, live, stream);
         launch_assign(jobs, dims, 1, stream);
       }
       ISDF_CHECK_LAUNCH();

@@ -1,0 +1,62 @@
+// A device-ended loop as a CUDA graph: a WHILE node whose body is captured from
+// the caller's launches and which a kernel of the body ends, so that no round of
+// the loop waits for the host.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace isdf_b200 {
+
+// What the body's kernels get: with in_graph, end_loop() lets the running body be
+// the last. max_rounds bounds the loop whatever else happens: the kernel that
+// counts the rounds ends the loop beyond it.
+struct LoopEnd {
+  cudaGraphConditionalHandle handle;
+  int in_graph;
+  int max_rounds;
+};
+
+__device__ __forceinline__ void end_loop(const LoopEnd& le) {
+  if (le.in_graph) cudaGraphSetConditional(le.handle, 0);
+}
+
+struct LoopGraph {
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;  // null on a stream that cannot be captured
+  ~LoopGraph() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+  }
+
+  // body(le) launches one body of the loop on s.
+  template <class F>
+  void build(cudaStream_t s, int max_rounds, F body_launches) {
+    LoopEnd le{0, 1, max_rounds};
+    cudaGraphNodeParams np = {};
+    cudaGraphNode_t node;
+    cudaGraph_t body = nullptr;
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess &&
+              cudaGraphConditionalHandleCreate(&le.handle, graph, 1,
+                                               cudaGraphCondAssignDefault) == cudaSuccess;
+    if (ok) {
+      np.conditional.handle = le.handle;
+      ok = cudaGraphAddNode(&node, graph, nullptr, 0, &np) == cudaSuccess;
+    }
+    if (ok) {
+      body = np.conditional.phGraph_out[0];
+      ok = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0,
+                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    }
+    if (ok) {
+      body_launches(le);
+      ok = cudaStreamEndCapture(s, &body) == cudaSuccess;
+    }
+    if (!ok || cudaGraphInstantiate(&exec, graph, 0ull) != cudaSuccess) exec = nullptr;
+    (void)cudaGetLastError();  // a refused capture leaves an error to clear
+  }
+};
+
+}  // namespace isdf_b200

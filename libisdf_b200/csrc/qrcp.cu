@@ -42,6 +42,7 @@
 #include "common.cuh"
 #include "dgemm.cuh"
 #include "fit.h"
+#include "loop_graph.h"
 #include "readback.h"
 #include "qrcp.h"
 #include "solve.h"
@@ -51,16 +52,41 @@ namespace isdf_b200 {
 namespace {
 
 constexpr int kMaxPre = 128;  // numPre limit: one 128-wide tile holds every column of Qm
+constexpr int kRecomputeGrid = 148;
 
 struct QrState {
-  unsigned long long maxbits;  // max residual norm of the active columns (bit pattern)
-  int minpos;                  // first position holding that maximum
+  unsigned long long maxbits;  // max norm of the columns before the filter (bit pattern)
   int done;
   int nrec;                    // columns flagged for a norm recompute in this step
   int ntot;
   int total_rec;               // norms recomputed over the whole selection
+  int k;                       // pivots picked
+  int step;                    // the running step (k - 1), -1 where there is none
+  int rounds;                  // steps begun, with or without a pivot
   int pad;
 };
+
+// The columns whose residual norm is the largest, by block of a pivot step's last
+// kernels: the largest norm and the first position (in the pivoted order) holding
+// it, as LAPACK's idamax over the remaining columns picks it.
+struct Best {
+  double nu;
+  int pos;
+};
+
+__device__ __forceinline__ Best better(const Best& a, const Best& b) {
+  return a.nu > b.nu || (a.nu == b.nu && a.pos < b.pos) ? a : b;
+}
+
+__device__ __forceinline__ Best warp_best(Best v) {
+  for (int o = 16; o > 0; o >>= 1) {
+    Best u;
+    u.nu = __shfl_xor_sync(0xffffffffu, v.nu, o);
+    u.pos = __shfl_xor_sync(0xffffffffu, v.pos, o);
+    v = better(v, u);
+  }
+  return v;
+}
 
 // dgeqpf's recompute threshold sqrt(eps), eps = dlamch('Epsilon') = 2^-53.
 __device__ __forceinline__ double tol3z() { return sqrt(1.1102230246251565e-16); }
@@ -188,7 +214,6 @@ __global__ void k_compact(const double* __restrict__ A, const double* __restrict
   const long long ld = ntot + (ntot & 1);
   if ((ntot & 1) && blockIdx.x == 0 && threadIdx.x == 0)
     for (int j = 0; j < p; ++j) Ac[ntot + j * ld] = Bc[ntot + j * ld] = 0.0;
-  double mx = 0.0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ntot; c += gridDim.x * blockDim.x) {
     const long long r = idx[c];
     for (int j = 0; j < p; ++j) {
@@ -201,59 +226,70 @@ __global__ void k_compact(const double* __restrict__ A, const double* __restrict
     pos[c] = c;
     perm[c] = c;
     active[c] = 1;
-    mx = fmax(mx, v);
   }
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((threadIdx.x & 31) == 0 && mx > 0.0)
-    atomicMax(&st->maxbits, (unsigned long long)__double_as_longlong(mx));
 }
 
-__global__ void k_reset_max(QrState* st) {
-  st->maxbits = 0ull;
-  st->minpos = INT_MAX;
+// The first step's candidates: one per block of 64 columns, none from recomputes.
+__global__ void __launch_bounds__(64) k_first_best(const double* __restrict__ nu, int ntot,
+                                                   int blocks, Best* __restrict__ best) {
+  Best v{0.0, INT_MAX};
+  const int c = blockIdx.x * 64 + threadIdx.x;
+  if ((int)blockIdx.x < blocks && c < ntot) v = Best{nu[c], c};
+  v = warp_best(v);
+  __shared__ Best half;
+  if (threadIdx.x == 32) half = v;
+  __syncthreads();
+  if (threadIdx.x == 0) best[blockIdx.x] = better(v, half);
 }
 
 // ------------------------------------------------------------- one pivot step
-// First position (in the pivoted order) holding the maximal residual norm, as
-// LAPACK's idamax over the remaining columns picks it.
-__global__ void k_argpos(const double* __restrict__ nu, const int* __restrict__ pos,
-                         const unsigned char* __restrict__ active, int ntot, QrState* st) {
-  if (st->done) return;
-  const double mx = __longlong_as_double((long long)st->maxbits);
-  int best = INT_MAX;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ntot; c += gridDim.x * blockDim.x)
-    if (active[c] && nu[c] == mx) best = min(best, pos[c]);
-  for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-  if ((threadIdx.x & 31) == 0 && best != INT_MAX) atomicMin(&st->minpos, best);
-}
-
-// Pivot bookkeeping (one thread) and the pivot's feature vector
-// x[i + j*p] = B(c, i) * A(c, j).
-__global__ void k_pick(int k, int p, int ld, const double* __restrict__ Ac,
-                       const double* __restrict__ Bc, int* __restrict__ pos,
-                       int* __restrict__ perm, unsigned char* __restrict__ active,
-                       int* __restrict__ sel, QrState* st, double* __restrict__ x) {
+// The pivot: the best of the blocks' candidates, its bookkeeping (one thread) and
+// its feature vector x[i + j*p] = B(c, i) * A(c, j). The step number comes from the
+// device, so that every step is the same launches and they loop in a graph; past
+// the last step, or where no norm is left, it ends the loop.
+__global__ void __launch_bounds__(1024) k_pick(int kmax, int p, int ld, int nbest,
+                                               const Best* __restrict__ best,
+                                               const double* __restrict__ Ac,
+                                               const double* __restrict__ Bc,
+                                               int* __restrict__ pos, int* __restrict__ perm,
+                                               unsigned char* __restrict__ active,
+                                               int* __restrict__ sel, QrState* st,
+                                               double* __restrict__ x, const LoopEnd le) {
   __shared__ int col;
-  if (threadIdx.x == 0) {
-    col = -1;
-    const double mx = __longlong_as_double((long long)st->maxbits);
-    if (!st->done && mx > 0.0 && st->minpos != INT_MAX) {
-      const int q = st->minpos;
-      const int c = perm[q];
-      const int ck = perm[k];
-      perm[k] = c;
-      perm[q] = ck;
-      pos[ck] = q;
-      pos[c] = k;
-      active[c] = 0;
-      sel[k] = c;
-      col = c;
-    } else {
-      st->done = 1;
+  __shared__ Best warp_v[32];
+  const int k = st->k;
+  const bool run = !st->done && k < kmax;
+  Best v{0.0, INT_MAX};
+  if (run)
+    for (int i = threadIdx.x; i < nbest; i += 1024) v = better(v, best[i]);
+  v = warp_best(v);
+  if ((threadIdx.x & 31) == 0) warp_v[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    v = warp_best(warp_v[threadIdx.x]);
+    if (threadIdx.x == 0) {
+      col = -1;
+      if (run && v.nu > 0.0 && v.pos != INT_MAX) {
+        const int q = v.pos;
+        const int c = perm[q];
+        const int ck = perm[k];
+        perm[k] = c;
+        perm[q] = ck;
+        pos[ck] = q;
+        pos[c] = k;
+        active[c] = 0;
+        sel[k] = c;
+        col = c;
+        st->k = k + 1;
+        st->step = k;
+      } else {
+        if (run) st->done = 1;
+        st->step = -1;
+        end_loop(le);
+      }
+      st->nrec = 0;
+      if (++st->rounds > le.max_rounds) end_loop(le);
     }
-    st->maxbits = 0ull;
-    st->minpos = INT_MAX;
-    st->nrec = 0;
   }
   __syncthreads();
   if (col < 0) return;
@@ -266,12 +302,11 @@ __global__ void k_pick(int k, int p, int ld, const double* __restrict__ Ac,
 
 // cdot[l] = Q[:, l] . x for l < k: one block per l (a strided partial per
 // thread, then a fixed-order tree), so the sums do not depend on scheduling.
-__global__ void __launch_bounds__(256) k_qt_x(const double* __restrict__ Q, int m, int k,
+__global__ void __launch_bounds__(256) k_qt_x(const double* __restrict__ Q, int m,
                                               const double* __restrict__ x, const QrState* st,
                                               double* __restrict__ cdot) {
-  if (st->done) return;
   const int l = blockIdx.x;
-  if (l >= k) return;
+  if (l >= st->step) return;
   __shared__ double red[8];
   const double* q = Q + (long long)l * m;
   double s = 0.0;
@@ -290,10 +325,11 @@ __global__ void __launch_bounds__(256) k_qt_x(const double* __restrict__ Q, int 
 // x -= Q[:, 0:k] cdot: a block takes 32 consecutive rows (one per lane), its
 // 32 warps the columns l = w (mod 32), and the 32 partials are added in warp
 // order (enough loads in flight per SM to stream Q from L2).
-__global__ void __launch_bounds__(1024) k_x_minus_qc(const double* __restrict__ Q, int m, int k,
+__global__ void __launch_bounds__(1024) k_x_minus_qc(const double* __restrict__ Q, int m,
                                                      const double* __restrict__ cdot,
                                                      const QrState* st, double* __restrict__ x) {
-  if (st->done) return;
+  const int k = st->step;
+  if (k <= 0) return;
   __shared__ double red[32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
@@ -311,11 +347,12 @@ __global__ void __launch_bounds__(1024) k_x_minus_qc(const double* __restrict__ 
   }
 }
 
-// q_k = x / |x| into Q[:, k] and into Qm (depth-major: Qm[i*p + j] = q[i + j*p]).
-__global__ void __launch_bounds__(1024) k_normalise(int k, int p, const double* __restrict__ x,
+// q_k = x / |x| into Q[:, k] and into Qm (depth-major: Qm[i*ldq + j] = q[i + j*p]).
+__global__ void __launch_bounds__(1024) k_normalise(int p, int ldq, const double* __restrict__ x,
                                                     QrState* st, double* __restrict__ Q,
                                                     double* __restrict__ Qm) {
-  if (st->done) return;
+  const int k = st->step;
+  if (k < 0 || st->done) return;
   const int m = p * p;
   __shared__ double red[32];
   double s = 0.0;
@@ -339,75 +376,17 @@ __global__ void __launch_bounds__(1024) k_normalise(int k, int p, const double* 
     const double q = x[e] * inv;
     Q[(long long)k * m + e] = q;
     const int i = e % p, j = e / p;
-    Qm[i * p + j] = q;
+    Qm[i * ldq + j] = q;
   }
 }
 
 // Residual-norm downdate of every active column with t_c = q_k . x_c, and the
-// maximum of the new norms for the next step.
-using CoreU = dmma::Core<128, 128>;
-template <int VEC>
-__global__ void __launch_bounds__(256) k_update(const double* __restrict__ Ac,
-                                                const double* __restrict__ Bc, int ntot, int ld,
-                                                int p,
-                                                const double* __restrict__ Qm,
-                                                const unsigned char* __restrict__ active,
-                                                double* __restrict__ nu,
-                                                double* __restrict__ nu0, QrState* st,
-                                                int* __restrict__ rec_list) {
-  if (st->done) return;
-  extern __shared__ double smem[];
-  const int m0 = blockIdx.x * CoreU::BM;
-  const int m_rem = min(CoreU::BM, ntot - m0);
-  CoreU core;
-  core.zero();
-  core.run<VEC>(smem, Bc + m0, ld, Qm, p, m_rem, p, 0, p);
-  // row dot with A, reduced over the 4 lanes of a quad and the 4 column warps
-  double* red = smem;  // [4][128], the pipeline buffers are free again
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int wm0 = (warp >> 2) * CoreU::WM, wn0 = (warp & 3) * CoreU::WN;
-#pragma unroll
-  for (int i = 0; i < CoreU::MT; ++i) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = wm0 + i * 16 + g + 8 * h;
-      double s = 0.0;
-      if (r < m_rem) {
-#pragma unroll
-        for (int j = 0; j < CoreU::NT; ++j) {
-          const int c = wn0 + j * 8 + 2 * t;
-          if (c < p) s = fma(Ac[(m0 + r) + (long long)c * ld], core.acc[i][j][2 * h], s);
-          if (c + 1 < p) s = fma(Ac[(m0 + r) + (long long)(c + 1) * ld], core.acc[i][j][2 * h + 1], s);
-        }
-      }
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      if (t == 0) red[(warp & 3) * CoreU::BM + r] = s;
-    }
-  }
-  __syncthreads();
-  double mx = 0.0;
-  if (threadIdx.x < CoreU::BM && (int)threadIdx.x < m_rem) {
-    const int c = m0 + threadIdx.x;
-    if (active[c]) {
-      const double tdot = red[threadIdx.x] + red[CoreU::BM + threadIdx.x] +
-                          red[2 * CoreU::BM + threadIdx.x] + red[3 * CoreU::BM + threadIdx.x];
-      if (downdate_norm(c, tdot, nu, nu0, st, rec_list)) mx = nu[c];
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((threadIdx.x & 31) == 0 && mx > 0.0)
-    atomicMax(&st->maxbits, (unsigned long long)__double_as_longlong(mx));
-}
-
-// The same downdate on the warp-specialised tile (16-byte aligned Bc and Qm,
-// p even; the even leading dimension lets the last odd row copy its zero
-// padding partner): 64 rows x BN columns, BN = p rounded up to a multiple of
-// 8 (the columns past p copied as zeros), four DMMA warps of 16 full rows
-// each, so the row dot with A closes inside a quad of lanes. BN tracks p
-// instead of a fixed 128-wide tile: at most 7 padding columns take
-// tensor-core work.
+// block's candidate for the next pivot, on the warp-specialised tile: 64 rows x
+// BN columns, BN = p rounded up to a multiple of 8, four DMMA warps of 16 full rows
+// each, so the row dot with A closes inside a quad of lanes. Qm's rows are
+// ldq = p rounded up to even long (16-byte aligned for an odd p as well: on a 48^3
+// grid with p = 31 the 128-column tile that odd p took until then ran 44 us a step,
+// this one 17). An odd last row copies its zero padding partner.
 template <int BN>
 using UpdTile = dmma::WsTile<64, BN, 4, 1, 16, 3>;
 // three CTAs per SM while the accumulators leave room (136 registers)
@@ -419,21 +398,21 @@ struct UpdMinBlocks {
 template <int BN, int MINB>
 __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
     k_update_ws(const double* __restrict__ Ac, const double* __restrict__ Bc, int ntot, int ld,
-                int p,
+                int p, int ldq,
                 const double* __restrict__ Qm, const unsigned char* __restrict__ active,
-                double* __restrict__ nu, double* __restrict__ nu0, QrState* st,
-                int* __restrict__ rec_list, int* err) {
+                const int* __restrict__ pos, double* __restrict__ nu, double* __restrict__ nu0,
+                QrState* st, int* __restrict__ rec_list, Best* __restrict__ best, int* err) {
   using T = UpdTile<BN>;
-  if (st->done) return;
+  if (st->step < 0 || st->done) return;
   extern __shared__ __align__(128) double smem[];
   const int m0 = blockIdx.x * T::BM;
   const int m_rem = min(T::BM, ntot - m0);
   T tile;
-  if (!tile.run(smem, Bc + m0, ld, (m_rem + 1) & ~1, Qm, p, p, p, err)) return;
+  if (!tile.run(smem, Bc + m0, ld, (m_rem + 1) & ~1, Qm, ldq, p, p, err)) return;
   if (T::producer()) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  double mx = 0.0;
+  Best v{0.0, INT_MAX};
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int r = warp * 16 + g + 8 * h;
@@ -450,12 +429,14 @@ __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     if (t == 0 && r < m_rem) {
       const int c = m0 + r;
-      if (active[c] && downdate_norm(c, s, nu, nu0, st, rec_list)) mx = fmax(mx, nu[c]);
+      if (active[c] && downdate_norm(c, s, nu, nu0, st, rec_list))
+        v = better(v, Best{nu[c], pos[c]});
     }
   }
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if (lane == 0 && mx > 0.0)
-    atomicMax(&st->maxbits, (unsigned long long)__double_as_longlong(mx));
+  v = warp_best(v);
+  // one candidate per warp: the producer warp has left, so the block's four warps
+  // share no barrier
+  if (lane == 0) best[blockIdx.x * T::NW + warp] = v;
 }
 
 // Exact residual norms of the columns the downdate flagged in this step
@@ -464,21 +445,25 @@ __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
 // on q_0..q_k twice (classical Gram-Schmidt: all k+1 dots, one warp per q_l
 // with a fixed lane order, then the update, one thread per feature summing
 // over l in order), and the residual's norm becomes nu[c] and the new
-// reference nu0[c]. cbuf: gridDim.x x k1 doubles of scratch for the dots.
-constexpr int kRecomputeGrid = 148;
+// reference nu0[c]. cbuf: gridDim.x x kmax doubles of scratch for the dots. Every
+// block leaves its candidate for the next pivot.
 __global__ void __launch_bounds__(256) k_recompute(const double* __restrict__ Ac,
                                                    const double* __restrict__ Bc, int ld, int p,
-                                                   const double* __restrict__ Q, int m, int k1,
+                                                   const double* __restrict__ Q, int m, int kmax,
                                                    const int* __restrict__ rec_list,
+                                                   const int* __restrict__ pos,
                                                    double* __restrict__ nu,
                                                    double* __restrict__ nu0, QrState* st,
-                                                   double* __restrict__ cbuf) {
+                                                   double* __restrict__ cbuf,
+                                                   Best* __restrict__ best) {
   extern __shared__ double x[];  // m features
   __shared__ double red[8];
-  if (st->done) return;
+  const int k1 = st->step + 1;
+  if (k1 <= 0 || st->done) return;
   const int nrec = st->nrec;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* c = cbuf + (size_t)blockIdx.x * k1;
+  double* c = cbuf + (size_t)blockIdx.x * kmax;
+  Best found{0.0, INT_MAX};  // thread 0: the block's candidate
   for (int f = blockIdx.x; f < nrec; f += gridDim.x) {
     const int col = rec_list[f];
     for (int e = threadIdx.x; e < m; e += 256) {
@@ -513,11 +498,12 @@ __global__ void __launch_bounds__(256) k_recompute(const double* __restrict__ Ac
       const double v = sqrt(t);
       nu[col] = v;
       nu0[col] = v;
-      if (v > 0.0) atomicMax(&st->maxbits, (unsigned long long)__double_as_longlong(v));
+      found = better(found, Best{v, pos[col]});
       atomicAdd(&st->total_rec, 1);
     }
     __syncthreads();
   }
+  if (threadIdx.x == 0) best[blockIdx.x] = found;
 }
 
 // Householder QR of the K x p draws (host, FP64): returns p orthonormal columns
@@ -576,6 +562,7 @@ std::vector<double> gaussian_draws(int m, int n) {
 struct QrBuffers {
   double *A, *B, *norm2, *Ac, *Bc, *nu, *nu0, *Q, *Qm, *x, *cdot, *G1, *G2, *rec_dots;
   int *idx, *pos, *perm, *sel, *tile_cnt, *rec_list;
+  Best* best;  // candidates: four per 64 columns, then one per recompute block
   unsigned char* active;
   QrState* st;
   int* err;  // a bounded pipeline wait of the update ran out
@@ -593,7 +580,7 @@ QrBuffers carve(Arena& a, long long n, int p, int k1, int k2, int kmax) {
   b.nu = a.take<double>((size_t)n);
   b.nu0 = a.take<double>((size_t)n);
   b.Q = a.take<double>((size_t)m * kmax);
-  b.Qm = a.take<double>((size_t)m);
+  b.Qm = a.take<double>((size_t)p * (p + (p & 1)));
   b.x = a.take<double>((size_t)m);
   b.cdot = a.take<double>((size_t)kmax);
   b.G1 = a.take<double>((size_t)k1 * p);
@@ -606,6 +593,7 @@ QrBuffers carve(Arena& a, long long n, int p, int k1, int k2, int kmax) {
   b.rec_list = a.take<int>((size_t)n);
   b.rec_dots = a.take<double>((size_t)kRecomputeGrid * kmax);
   b.active = a.take<unsigned char>((size_t)n);
+  b.best = a.take<Best>((size_t)(4 * ((n + 63) / 64) + kRecomputeGrid));
   b.st = a.take<QrState>(1);
   b.err = a.take<int>(1);
   return b;
@@ -617,8 +605,6 @@ int set_update_attrs() {
   int dev = 0;
   ISDF_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && done[dev]) return ISDF_OK;
-  ISDF_CUDA(cudaFuncSetAttribute(k_update<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)CoreU::SMEM_BYTES));
   ISDF_CUDA(cudaFuncSetAttribute(k_recompute, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(double) * kMaxPre * kMaxPre)));
 #define ISDF_UPD_ATTR(BN)                                                                  \
@@ -650,7 +636,8 @@ void launch_update_bn(const QrBuffers& b, int ntot, int ld, int p, cudaStream_t 
   using T = UpdTile<BN>;
   const unsigned grid = (unsigned)((ntot + T::BM - 1) / T::BM);
   k_update_ws<BN, UpdMinBlocks<BN>::value><<<grid, T::THREADS, T::SMEM_BYTES, s>>>(
-      b.Ac, b.Bc, ntot, ld, p, b.Qm, b.active, b.nu, b.nu0, b.st, b.rec_list, b.err);
+      b.Ac, b.Bc, ntot, ld, p, p + (p & 1), b.Qm, b.active, b.pos, b.nu, b.nu0, b.st, b.rec_list,
+      b.best, b.err);
 }
 
 // The downdate on the narrowest warp-specialised tile that holds p columns
@@ -731,10 +718,9 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
   k_keep_count<<<ntiles, 256, 0, s>>>(b.norm2, n, b.st, b.tile_cnt);
   k_scan_tiles<<<1, 1024, 0, s>>>(b.tile_cnt, ntiles, &b.st->ntot);
   k_keep_scatter<<<ntiles, 256, 0, s>>>(b.norm2, n, b.st, b.tile_cnt, b.idx);
-  k_reset_max<<<1, 1, 0, s>>>(b.st);
   k_compact<<<kNumSMs * 4, 256, 0, s>>>(b.A, b.B, n, p, b.idx, b.norm2, b.st, b.Ac, b.Bc, b.nu,
                                         b.nu0, b.pos, b.perm, b.active);
-  launches += 6;
+  launches += 5;
   ISDF_CHECK_LAUNCH();
   QrState hst;
   ISDF_TRY(read_back(&hst, b.st, sizeof(QrState), s));
@@ -744,32 +730,45 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
 
   // pivoted Gram-Schmidt over the kept columns
   const int ld = ntot + (ntot & 1);  // Ac / Bc leading dimension (k_compact)
-  const unsigned ugrid = (unsigned)((ntot + CoreU::BM - 1) / CoreU::BM);
-  const bool uv2 = ((reinterpret_cast<size_t>(b.Bc) | reinterpret_cast<size_t>(b.Qm)) & 15) == 0 &&
-                   p % 2 == 0;
-  const unsigned agrid = (unsigned)std::min(kNumSMs * 8, (ntot + 255) / 256);
-  for (int k = 0; k < kmax; ++k) {
-    k_argpos<<<agrid, 256, 0, s>>>(b.nu, b.pos, b.active, ntot, b.st);
-    k_pick<<<1, 1024, 0, s>>>(k, p, ld, b.Ac, b.Bc, b.pos, b.perm, b.active, b.sel, b.st, b.x);
-    launches += 2;
-    if (k > 0) {
-      for (int pass = 0; pass < 2; ++pass) {
-        k_qt_x<<<k, 256, 0, s>>>(b.Q, m, k, b.x, b.st, b.cdot);
-        k_x_minus_qc<<<(m + 31) / 32, 1024, 0, s>>>(b.Q, m, k, b.cdot, b.st, b.x);
-        launches += 2;
+  const int ldq = p + (p & 1);
+  const int ublocks = (ntot + 63) / 64, nbest = 4 * ublocks + kRecomputeGrid;
+  // the first candidates: one per 64 columns, the other places empty
+  ISDF_CUDA(cudaMemsetAsync(b.best, 0, sizeof(Best) * (size_t)nbest, s));
+  if (ublocks > 0) k_first_best<<<ublocks, 64, 0, s>>>(b.nu, ntot, ublocks, b.best);
+  // One pivot step; the step number lives on the device.
+  auto step = [&](const LoopEnd& le) {
+    k_pick<<<1, 1024, 0, s>>>(kmax, p, ld, nbest, b.best, b.Ac, b.Bc, b.pos, b.perm, b.active,
+                              b.sel, b.st, b.x, le);
+    for (int pass = 0; pass < 2; ++pass) {
+      k_qt_x<<<kmax, 256, 0, s>>>(b.Q, m, b.x, b.st, b.cdot);
+      k_x_minus_qc<<<(m + 31) / 32, 1024, 0, s>>>(b.Q, m, b.cdot, b.st, b.x);
+    }
+    k_normalise<<<1, 1024, 0, s>>>(p, ldq, b.x, b.st, b.Q, b.Qm);
+    launch_update_ws(b, ntot, ld, p, s);
+    k_recompute<<<kRecomputeGrid, 256, sizeof(double) * m, s>>>(
+        b.Ac, b.Bc, ld, p, b.Q, m, kmax_cap, b.rec_list, b.pos, b.nu, b.nu0, b.st, b.rec_dots,
+        b.best + 4 * (size_t)ublocks);
+  };
+  if (kmax > 0) {
+    // a graph that loops on the device: launched step by step, the nine launches
+    // of a step took the host longer than the GPU at numPre = 31
+    constexpr int kBodySteps = 4;
+    LoopGraph loop;
+    loop.build(s, kmax + 2 * kBodySteps, [&](const LoopEnd& le) {
+      for (int i = 0; i < kBodySteps; ++i) step(le);
+    });
+    if (loop.exec) {
+      ISDF_CUDA(cudaGraphLaunch(loop.exec, s));
+      // (the graph must outlive its launch)
+      ISDF_TRY(read_back(&hst, b.st, sizeof(QrState), s));
+    } else {
+      const LoopEnd no_graph{0, 0, 0x7fffffff};
+      for (int k = 0; k < kmax; ++k) {
+        step(no_graph);
+        if ((k & 255) == 255) ISDF_CHECK_LAUNCH();
       }
     }
-    k_normalise<<<1, 1024, 0, s>>>(k, p, b.x, b.st, b.Q, b.Qm);
-    if (uv2)  // 16-byte aligned rows: the warp-specialised tile
-      launch_update_ws(b, ntot, ld, p, s);
-    else
-      k_update<1><<<ugrid, 256, CoreU::SMEM_BYTES, s>>>(b.Ac, b.Bc, ntot, ld, p, b.Qm, b.active, b.nu,
-                                                        b.nu0, b.st, b.rec_list);
-    k_recompute<<<kRecomputeGrid, 256, sizeof(double) * m, s>>>(b.Ac, b.Bc, ld, p, b.Q, m, k + 1,
-                                                                b.rec_list, b.nu, b.nu0, b.st,
-                                                                b.rec_dots);
-    launches += 3;
-    if ((k & 255) == 255) ISDF_CHECK_LAUNCH();
+    launches += 8 * kmax + 1;
   }
   ISDF_CHECK_LAUNCH();
 

@@ -96,3 +96,17 @@ def test_qrcp_si8_synthetic(torch_cuda):
     err = ofit.rel(fd, fd_o)
     record_parity("qrcp Si8-like", "fitted densities vs oracle", err, 1e-10)
     assert err <= 1e-10
+
+
+@pytest.mark.parametrize("mu,factor", [(1, 1.0), (2, 2.0), (9, 1.0), (64, 4.0), (72, 4.0), (97, 6.2)])
+def test_qrcp_num_pre_edges(torch_cuda, mu, factor):
+    """numPre 1, 2, 3, 16, 17 and 25 (the downdate tile's narrowest and the widths
+    around its multiples of 8), pivot counts around the loop graph's body of four
+    steps."""
+    ng = (11, 10, 9)
+    psi = np.asfortranarray(np.random.default_rng(5).standard_normal((990, 30)))
+    a = (15, 15, 15, 15, 13)
+    piv, th, rep = _gpu_qrcp(torch_cuda, psi, ng, (3.0, 3.0, 3.0), a, mu, factor, 3)
+    k = check_all_pivots(f"qrcp numPre {qrcp.num_pre(mu, factor)}", psi, a, mu, factor, 3, piv,
+                         rep.qrcp_steps)
+    assert k == min(mu, rep.npt, qrcp.num_pre(mu, factor) ** 2)
