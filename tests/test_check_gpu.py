@@ -157,3 +157,23 @@ def test_coulomb_matrix_tile_edges(torch_cuda, rk, ng):
     tol = 2 * (ng[0] // 2 + 1) * ng[1] * ng[2] * 2.0 ** -53
     assert np.linalg.norm(A - A_o) <= tol * np.linalg.norm(A_o)
     assert np.array_equal(A, A.T)
+
+
+@pytest.mark.parametrize("ng", [(16, 12, 10), (9, 15, 25), (7, 7, 13)])
+def test_coulomb_matrix_leaves_theta(torch_cuda, ng):
+    """theta is the caller's: whole batches are transformed from it in place of a
+    copy, the rest through one, aligned columns or not; it must come back as it
+    was, and the result agree with the oracle's."""
+    torch = torch_cuda
+    rk, n = 300, ng[0] * ng[1] * ng[2]
+    th = np.asfortranarray(np.random.default_rng(1).standard_normal((n, rk)))
+    d_th = torch.from_numpy(np.ascontiguousarray(th.T)).cuda()
+    before = d_th.clone()
+    d_A = torch.empty((rk, rk), dtype=torch.float64, device="cuda")
+    ln = (7.0, 8.0, 9.0)
+    isdf.coulomb_matrix(isdf.Domain(length=ln, num_grid=ng), d_th, rk, d_A)
+    torch.cuda.synchronize()
+    assert torch.equal(d_th, before)
+    A_o = ocheck.coulomb_matrix(th, ng, ln, rk)
+    tol = 2 * (ng[0] // 2 + 1) * ng[1] * ng[2] * 2.0 ** -53
+    assert np.linalg.norm(d_A.cpu().numpy().T - A_o) <= tol * np.linalg.norm(A_o)
