@@ -594,8 +594,9 @@ int isdf_coulomb_matrix(const isdf_domain_t* dom, const double* d_theta, int rk,
     if (dom->num_grid[0] <= 0 || dom->num_grid[1] <= 0 || dom->num_grid[2] <= 0 || rk <= 0 ||
         rk > ng)
       return record_error(ISDF_ERR_ARG, "sizes");
-    const size_t need = coulomb_matrix_workspace_bytes(dom->num_grid, rk);
     std::lock_guard<std::mutex> lock(workspace_mutex());
+    size_t need = 0;
+    ISDF_TRY(coulomb_matrix_workspace_bytes(dom->num_grid, rk, &need));
     Arena arena;
     cudaStream_t ls;
     ISDF_TRY(acquire_workspace(need + 4096, &arena, &ls));
@@ -649,6 +650,7 @@ void isdf_release_workspace(void) {
     cudaDeviceSynchronize();
     cudaFree(g_cache[dev].buf);
   }
+  release_coulomb_plans(dev);
   g_cache[dev].buf = nullptr;
   g_cache[dev].cap = 0;
 }

@@ -490,16 +490,83 @@ int check_sampled_run(const CheckArgs& args, const int* pairs, int ns, Arena& ar
 // code applies to interpolation-point quantities, the first consumer of theta.
 // Here: batched cuFFT D2Z half spectra weighted by sqrt(w V) into one real
 // matrix Yz (rk x 2 nh), then A = Yz Yz^T on the FP64 tensor cores.
-size_t coulomb_matrix_workspace_bytes(const int* num_grid, int rk) {
+//
+// Making a cuFFT plan took longer than the rest of the call for one cell (1.4 of
+// 2.2 ms at 40^3 and 320 columns), so the plans of the last kPlans grids are kept
+// per device. Their work areas are not: each call gives the plan one from its own
+// workspace, so that a kept plan holds no device buffer and two calls share no more
+// than they share of the workspace. Callers hold the device's workspace mutex;
+// isdf_release_workspace() gives the plans back.
+namespace {
+constexpr int kPlans = 4;
+struct KeptPlan {
+  int dims[3] = {0, 0, 0};
+  cufftHandle h = 0;
+  size_t work = 0;
+  unsigned long long used = 0;  // 0: empty
+};
+KeptPlan g_plans[64][kPlans];
+unsigned long long g_plan_uses[64];
+
+int kept_plan(const int* num_grid, KeptPlan** out) {
+  int dev = 0;
+  ISDF_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return record_error(ISDF_ERR_UNSUPPORTED, "device index");
+  KeptPlan* oldest = &g_plans[dev][0];
+  for (KeptPlan& p : g_plans[dev]) {
+    if (p.used && p.dims[0] == num_grid[0] && p.dims[1] == num_grid[1] && p.dims[2] == num_grid[2]) {
+      p.used = ++g_plan_uses[dev];
+      *out = &p;
+      return ISDF_OK;
+    }
+    if (p.used < oldest->used) oldest = &p;
+  }
+  KeptPlan& p = *oldest;
+  if (p.used) {
+    p.used = 0;
+    (void)cudaDeviceSynchronize();  // a transform may still be running
+    cufftDestroy(p.h);
+  }
+  int dims[3] = {num_grid[2], num_grid[1], num_grid[0]};
+  if (cufftCreate(&p.h) != CUFFT_SUCCESS)
+    return record_error(ISDF_ERR_CUDA, "Coulomb matrix: cufftCreate failed");
+  if (cufftSetAutoAllocation(p.h, 0) != CUFFT_SUCCESS ||
+      cufftMakePlanMany(p.h, 3, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_D2Z, kBatch, &p.work) !=
+          CUFFT_SUCCESS) {
+    cufftDestroy(p.h);
+    return record_error(ISDF_ERR_CUDA, "Coulomb matrix: cufftMakePlanMany failed");
+  }
+  for (int i = 0; i < 3; ++i) p.dims[i] = num_grid[i];
+  p.used = ++g_plan_uses[dev];
+  *out = &p;
+  return ISDF_OK;
+}
+}  // namespace
+
+void release_coulomb_plans(int dev) {
+  if (dev < 0 || dev >= 64) return;
+  (void)cudaDeviceSynchronize();
+  for (KeptPlan& p : g_plans[dev])
+    if (p.used) {
+      p.used = 0;
+      cufftDestroy(p.h);
+    }
+}
+
+int coulomb_matrix_workspace_bytes(const int* num_grid, int rk, size_t* bytes) {
   const long long ng = (long long)num_grid[0] * num_grid[1] * num_grid[2];
   const long long nh = (long long)(num_grid[0] / 2 + 1) * num_grid[1] * num_grid[2];
+  KeptPlan* plan = nullptr;
+  ISDF_TRY(kept_plan(num_grid, &plan));
   Arena a;
   a.counting = true;
   a.take<double>((size_t)ng * kBatch);
   a.take<cufftDoubleComplex>((size_t)nh * kBatch);
   a.take<double>((size_t)nh);
   a.take<double>((size_t)(rk + (rk & 1)) * 2 * nh);
-  return a.off;
+  a.take<char>(plan->work);
+  *bytes = a.off;
+  return ISDF_OK;
 }
 
 int coulomb_matrix_run(const int* num_grid, const double* length, const double* d_theta, int rk,
@@ -512,17 +579,15 @@ int coulomb_matrix_run(const int* num_grid, const double* length, const double* 
   double* sw = arena.take<double>((size_t)nh);
   const int ldy = rk + (rk & 1);  // 16-byte aligned rows
   double* Yz = arena.take<double>((size_t)ldy * 2 * nh);
+  KeptPlan* plan = nullptr;
+  ISDF_TRY(kept_plan(num_grid, &plan));
+  char* work = arena.take<char>(plan->work);
   if (arena.overflowed()) return record_error(ISDF_ERR_NOMEM, "Coulomb matrix: workspace too small");
   const double vol = length[0] * length[1] * length[2];
   k_weights<<<grid_for(nh, 256), 256, 0, s>>>(nx, ny, nz, length[0], length[1], length[2],
                                              vol / (double)ng, sw);
-  Plan plan;
-  int dims[3] = {nz, ny, nx};
-  if (cufftPlanMany(&plan.h, 3, dims, nullptr, 1, 0, nullptr, 1, 0, CUFFT_D2Z, kBatch) !=
-      CUFFT_SUCCESS)
-    return record_error(ISDF_ERR_CUDA, "Coulomb matrix: cufftPlanMany failed");
-  plan.ok = true;
-  if (cufftSetStream(plan.h, s) != CUFFT_SUCCESS)
+  if ((plan->work && cufftSetWorkArea(plan->h, work) != CUFFT_SUCCESS) ||
+      cufftSetStream(plan->h, s) != CUFFT_SUCCESS)
     return record_error(ISDF_ERR_CUDA, "Coulomb matrix: cufftSetStream failed");
   for (int c0 = 0; c0 < rk; c0 += kBatch) {
     const int bc = std::min(kBatch, rk - c0);
@@ -537,7 +602,7 @@ int coulomb_matrix_run(const int* num_grid, const double* length, const double* 
         ISDF_CUDA(cudaMemsetAsync(buf + (long long)bc * ng, 0,
                                   sizeof(double) * (size_t)(kBatch - bc) * ng, s));
     }
-    if (cufftExecD2Z(plan.h, copy ? buf : const_cast<double*>(cols), spec) != CUFFT_SUCCESS)
+    if (cufftExecD2Z(plan->h, copy ? buf : const_cast<double*>(cols), spec) != CUFFT_SUCCESS)
       return record_error(ISDF_ERR_CUDA, "Coulomb matrix: cufftExecD2Z failed");
     k_spectra_to_rows<<<trans_grid(nh, bc), 256, 0, s>>>(spec, nh, bc, sw, c0, ldy, Yz);
   }

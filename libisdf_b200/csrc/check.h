@@ -23,7 +23,9 @@ int check_run(const CheckArgs& args, Arena& arena, cudaStream_t s, double* fit_e
               double* coul_err);
 
 // A = Re(zeta^H V zeta) (rk x rk, column-major, device), zeta = FFT(theta columns).
-size_t coulomb_matrix_workspace_bytes(const int* num_grid, int rk);
+// (under the device's workspace mutex, as coulomb_matrix_run)
+int coulomb_matrix_workspace_bytes(const int* num_grid, int rk, size_t* bytes);
+void release_coulomb_plans(int dev);
 int coulomb_matrix_run(const int* num_grid, const double* length, const double* d_theta, int rk,
                        double* d_A, Arena& arena, cudaStream_t s);
 

@@ -177,3 +177,46 @@ def test_coulomb_matrix_leaves_theta(torch_cuda, ng):
     A_o = ocheck.coulomb_matrix(th, ng, ln, rk)
     tol = 2 * (ng[0] // 2 + 1) * ng[1] * ng[2] * 2.0 ** -53
     assert np.linalg.norm(d_A.cpu().numpy().T - A_o) <= tol * np.linalg.norm(A_o)
+
+
+def test_coulomb_matrix_kept_plans(torch_cuda):
+    """More grids in turn than plans are kept, twice over, with the workspace
+    released in between and from two threads: the same results each time."""
+    import threading
+
+    torch = torch_cuda
+    rk, ln = 5, (7.0, 8.0, 9.0)
+    grids = [(8, 6, 4), (9, 6, 4), (8, 7, 4), (8, 6, 5), (10, 6, 4), (4, 6, 8)]
+    ths = [np.asfortranarray(np.random.default_rng(k).standard_normal((g[0] * g[1] * g[2], rk)))
+           for k, g in enumerate(grids)]
+    want = [ocheck.coulomb_matrix(t, g, ln, rk) for t, g in zip(ths, grids)]
+    lib = isdf.lib()
+
+    def run(fail):
+        try:
+            st = torch.cuda.Stream()
+            for rep in range(2):
+                for t, g, w in zip(ths, grids, want):
+                    d_th = torch.from_numpy(np.ascontiguousarray(t.T)).cuda()
+                    d_A = torch.empty((rk, rk), dtype=torch.float64, device="cuda")
+                    torch.cuda.synchronize()
+                    with lock:  # one workspace: calls on different streams in turn
+                        isdf.coulomb_matrix(isdf.Domain(length=ln, num_grid=g), d_th, rk, d_A,
+                                            stream=st.cuda_stream)
+                        torch.cuda.synchronize()
+                    a = d_A.cpu().numpy().T
+                    if not np.linalg.norm(a - w) <= 1e-12 * np.linalg.norm(w):
+                        fail.append((rep, g))
+        except Exception as e:  # noqa: BLE001 - reported by the assertion below
+            fail.append(repr(e))
+
+    lock = threading.Lock()
+    fail = []
+    run(fail)
+    lib.isdf_release_workspace()
+    threads = [threading.Thread(target=run, args=(fail,)) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not fail
