@@ -912,13 +912,42 @@ constexpr int kSliceK = 32;     // K bytes per slicing tile
 // Ozaki GEMM (ozaki::tiled_offset: blocks of R rows, 32-byte K blocks; the A
 // side unstacked with R = 128, the B side stacked with R = 64), rows padded to
 // mp and K to kp with zeros, and exponents e[m] (|x| 2^-e < 1/2).
-__global__ void k_row_exponent(const double* __restrict__ X, long long rs, long long ks, int M,
-                               int K, int* __restrict__ e) {
+__device__ __forceinline__ int exponent_of(double mx) { return mx > 0.0 ? ilogb(mx) + 2 : 0; }
+
+// Contiguous rows (rs = 1, the A side's ng of them): a thread per row.
+__global__ void k_row_exponent(const double* __restrict__ X, long long ks, int M, int K,
+                               int* __restrict__ e) {
   for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
     double mx = 0.0;
-    for (int k = 0; k < K; ++k) mx = fmax(mx, fabs(X[m * rs + k * ks]));
-    e[m] = mx > 0.0 ? ilogb(mx) + 2 : 0;
+#pragma unroll 8
+    for (int k = 0; k < K; ++k) mx = fmax(mx, fabs(X[m + k * ks]));
+    e[m] = exponent_of(mx);
   }
+}
+
+// The B side's few rows: a block for 32 of them, 32 warps over the columns (rs = 1)
+// or a warp per row and 128 bytes of it at a time (ks = 1). A thread per row left
+// most SMs idle: 253 us for 1600 x 1600, 13 here.
+__global__ void __launch_bounds__(1024)
+    k_row_exponent_b(const double* __restrict__ X, long long rs, long long ks, int M, int K,
+                     int* __restrict__ e) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m0 = blockIdx.x * 32;
+  double mx = 0.0;
+  if (rs == 1) {
+    __shared__ double part[32][33];
+    if (m0 + lane < M) {
+#pragma unroll 4
+      for (int k = w; k < K; k += 32) mx = fmax(mx, fabs(X[m0 + lane + k * ks]));
+    }
+    part[w][lane] = mx;
+    __syncthreads();
+    mx = part[lane][w];  // row m0 + w, the warps' shares over the lanes
+  } else if (m0 + w < M) {
+#pragma unroll 4
+    for (int k = lane; k < K; k += 32) mx = fmax(mx, fabs(X[(m0 + w) * rs + k * ks]));
+  }
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0 && m0 + w < M) e[m0 + w] = exponent_of(mx);
 }
 
 // Row exponents from the binade maxima the GEMM epilogue gathered: the same
@@ -1047,7 +1076,8 @@ template <int S, bool B_SIDE>
 int slice_operand(const double* X, long long rs, long long ks, int M, int K, int mp, int kp,
                   int* e, int8_t* P, cudaStream_t s, bool gathered = false) {
   if (gathered) k_exp_from_max<<<grid_for(M, 256), 256, 0, s>>>(e, M);
-  else k_row_exponent<<<grid_for(M, 256), 256, 0, s>>>(X, rs, ks, M, K, e);
+  else if (!B_SIDE && rs == 1) k_row_exponent<<<grid_for(M, 256), 256, 0, s>>>(X, ks, M, K, e);
+  else k_row_exponent_b<<<(M + 31) / 32, 1024, 0, s>>>(X, rs, ks, M, K, e);
   dim3 g((unsigned)(kp / kSliceK), (unsigned)((mp + kSliceTile - 1) / kSliceTile));
   if (B_SIDE) {
     k_slice<S, ozaki::BN, true><<<g, 256, 0, s>>>(X, rs, ks, M, K, mp, kp, e, P);
