@@ -252,6 +252,7 @@ constexpr int kAssignThreads = 128;
 struct CellGrid {
   int nc;
   double h[3];
+  double inv_h[3];  // (a cell found with it is off by rounding only, far inside tol)
   double tol;
 };
 
@@ -490,7 +491,7 @@ __device__ __forceinline__ int first_seed(int p, int rk, const int* __restrict__
 }
 
 template <int N>
-__global__ void __launch_bounds__(kAssignThreads)
+__global__ void __launch_bounds__(kAssignThreads, 8)
     k_assign_warp(const __grid_constant__ KmJobs<N> JS, int count) {
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
@@ -560,12 +561,12 @@ __global__ void __launch_bounds__(kAssignThreads)
   const float err = __double2float_ru(1.9073486328125e-6 * reach * reach) + 1e-37f;
   const float far = __double2float_ru(U) + 2.0f * err;  // beyond: more than sqrt(U) from the box
   const int nc = g.nc;
-  const int i0 = min(nc - 1, max(0, (int)floor((x0 - R) / g.h[0])));
-  const int i1 = min(nc - 1, max(0, (int)floor((x1 + R) / g.h[0])));
-  const int j0 = min(nc - 1, max(0, (int)floor((y0 - R) / g.h[1])));
-  const int j1 = min(nc - 1, max(0, (int)floor((y1 + R) / g.h[1])));
-  const int k0 = min(nc - 1, max(0, (int)floor((z0 - R) / g.h[2])));
-  const int k1 = min(nc - 1, max(0, (int)floor((z1 + R) / g.h[2])));
+  const int i0 = min(nc - 1, max(0, (int)floor((x0 - R) * g.inv_h[0])));
+  const int i1 = min(nc - 1, max(0, (int)floor((x1 + R) * g.inv_h[0])));
+  const int j0 = min(nc - 1, max(0, (int)floor((y0 - R) * g.inv_h[1])));
+  const int j1 = min(nc - 1, max(0, (int)floor((y1 + R) * g.inv_h[1])));
+  const int k0 = min(nc - 1, max(0, (int)floor((z0 - R) * g.inv_h[2])));
+  const int k1 = min(nc - 1, max(0, (int)floor((z1 + R) * g.inv_h[2])));
   const int nj = j1 - j0 + 1, nrow = nj * (k1 - k0 + 1);
   float4* cw = cand[wid];
   double second = inf;
@@ -782,12 +783,16 @@ __global__ void __launch_bounds__(32 * kScanWarps)
   if (threadIdx.x == 0) last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
   __syncthreads();
   if (!last) return;
-  // exclusive scan of the member counts: start[l]
+  // exclusive scan of the member counts: start[l] (staged in shared memory: a
+  // thread walking its labels in global memory waits for each)
   __threadfence();
+  extern __shared__ int mem[];  // rk counts
+  for (int i = threadIdx.x; i < rk; i += 32 * kScanWarps) mem[i] = __ldcg(J.members + i);
+  __syncthreads();
   const int each = (rk + 32 * kScanWarps - 1) / (32 * kScanWarps);
   const int lo = min(rk, (int)threadIdx.x * each), hi = min(rk, lo + each);
   int mine = 0;
-  for (int i = lo; i < hi; ++i) mine += __ldcg(J.members + i);
+  for (int i = lo; i < hi; ++i) mine += mem[i];
   int inc = mine;
   for (int o = 1; o < 32; o <<= 1) {
     const int v = __shfl_up_sync(0xffffffffu, inc, o);
@@ -799,9 +804,12 @@ __global__ void __launch_bounds__(32 * kScanWarps)
   int run = inc - mine;
   for (int q = 0; q < w; ++q) run += tot[q];
   for (int i = lo; i < hi; ++i) {
-    J.start[i] = run;
-    run += __ldcg(J.members + i);
+    const int v = mem[i];
+    mem[i] = run;
+    run += v;
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < rk; i += 32 * kScanWarps) J.start[i] = mem[i];
   if (threadIdx.x == 0) {
     st->ticket = 0;
     if (!J.sharded) {
@@ -1007,6 +1015,26 @@ __device__ __forceinline__ double fold_serial(const double* comp, int cnt, doubl
   return acc;
 }
 
+// Cluster c's centroid (sums / count, utility.cpp:831-841) beside its count, and
+// an upper bound on the distance it moved (rounded upward); an empty cluster is
+// recorded, and the update compacts (its own entry is not used then).
+__device__ __forceinline__ void store_centroid(const double4& s, int c,
+                                               const double4* __restrict__ cen,
+                                               double4* __restrict__ sums,
+                                               double* __restrict__ shift, KmState* st) {
+  if (!(s.w != 0.0)) {
+    sums[c] = s;
+    st->any_empty = 1;
+    return;
+  }
+  const double4 o = cen[c];
+  const double4 n = make_double4(rdiv(s.x, s.w), rdiv(s.y, s.w), rdiv(s.z, s.w), s.w);
+  const double dx = fabs(n.x - o.x), dy = fabs(n.y - o.y), dz = fabs(n.z - o.z);
+  const double d2 = __dadd_ru(__dadd_ru(__dmul_ru(dx, dx), __dmul_ru(dy, dy)), __dmul_ru(dz, dz));
+  sums[c] = n;
+  shift[c] = __dmul_ru(__dsqrt_ru(d2), 1.0 + 1e-13);
+}
+
 // One block per cluster, one warp per component (w x, w y, w z, w), each by
 // itself: the components reach their crossings and ties at different members,
 // and a block that stages the members for all four would wait for the slowest
@@ -1044,6 +1072,7 @@ __global__ void __launch_bounds__(kFoldThreads) k_segsum(const __grid_constant__
     }
   };
   __shared__ double stage[kFoldThreads / 32][kFoldBatch];
+  __shared__ double total[4];
   double* comp = stage[warp];
   double acc = 0.0;
   load(0, nxt);
@@ -1066,8 +1095,13 @@ __global__ void __launch_bounds__(kFoldThreads) k_segsum(const __grid_constant__
           warp == 3 ? w0 : rmul(w0, warp == 0 ? J.fx[npt] : warp == 1 ? J.fy[npt] : J.fz[npt]);
       acc = repeat_add(acc, one, tail);
     }
-    reinterpret_cast<double*>(J.f_sums + c)[warp] = acc;
-    if (!J.sharded && warp == 3 && acc == 0.0) st->any_empty = 1;
+    total[warp] = acc;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double4 s = make_double4(total[0], total[1], total[2], total[3]);
+    if (J.sharded) J.f_sums[c] = s;  // a rank's partial sums
+    else store_centroid(s, c, J.cen, J.sums, J.shift, st);
   }
 }
 
@@ -1076,7 +1110,7 @@ __global__ void __launch_bounds__(kFoldThreads) k_segsum(const __grid_constant__
 // shrinks rk. So the clusters below the final rk stay where they are, and the
 // k-th empty place (ascending) takes the k-th non-empty cluster from the end.
 // One block finds both lists by prefix counts (holes, fillers: scratch of rk
-// entries each); the loop by one thread took 1.8 ms at 3000 centroids.
+// entries each; sums: the centroids beside their counts); the loop by one thread took 1.8 ms at 3000 centroids.
 __device__ int compact_empty(const double4* __restrict__ sums, int rk, double4* __restrict__ cen,
                              int* __restrict__ holes, int* __restrict__ fillers, int* warp_tot) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -1103,7 +1137,7 @@ __device__ int compact_empty(const double4* __restrict__ sums, int rk, double4* 
       if (i < left) holes[before] = i;
       ++before;
     } else if (i < left) {
-      cen[i] = make_double4(rdiv(s.x, s.w), rdiv(s.y, s.w), rdiv(s.z, s.w), 0.0);
+      cen[i] = make_double4(s.x, s.y, s.z, 0.0);
     } else {
       fillers[(rk - 1 - i) - (empty - before)] = i;  // non-empty clusters after i
     }
@@ -1120,47 +1154,40 @@ __device__ int compact_empty(const double4* __restrict__ sums, int rk, double4* 
   for (int q = 0; q < 32; ++q) nholes += warp_tot[q];
   for (int k = tid; k < nholes; k += 1024) {
     const double4 s = sums[fillers[k]];
-    cen[holes[k]] = make_double4(rdiv(s.x, s.w), rdiv(s.y, s.w), rdiv(s.z, s.w), 0.0);
+    cen[holes[k]] = make_double4(s.x, s.y, s.z, 0.0);
   }
   __syncthreads();
   return left;
 }
 
-// New centroids = sums / count (with the compaction above where a cluster is
-// empty), then the centroids into the cell grid (cell_start, cell_cen): one
-// block. The update also records how far every centroid moved (rounded
-// upward), the largest move, and for every cell of the grid the largest move of
-// a centroid that sat in its 3^3 and 5^3 neighbourhoods before the update
-// (cell_of still holds the previous positions' cells there).
+// The new centroids (with the compaction above where a cluster is empty) into
+// place, then into the cell grid (cell_start, cell_cen): one block, so whatever
+// the folds' blocks can do (the divisions, the moves) they have done. The update
+// also takes the largest move, and for every cell of the grid the largest move of
+// a centroid that sat in its 3^3 and 5^3 neighbourhoods before the update (cell_of
+// still holds the previous positions' cells there).
 // update = 0: the cells alone (the first centroids).
 template <int N>
 __global__ void __launch_bounds__(1024) k_centroids(const __grid_constant__ KmJobs<N> JS, int update) {
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (st->done) return;
-  extern __shared__ unsigned cmax[];  // 3 x ncells + 1 words
+  extern __shared__ unsigned cmax[];  // 4 x ncells + 1 words
   __shared__ int warp_tot[32];
   const CellGrid& g = J.cg;
   const int nc = g.nc, ncells = nc * nc * nc;
   int rk = st->rk;
   const bool empty = update && st->any_empty;
   if (update && !empty) {
-    unsigned* tmp = cmax + ncells;
     for (int c = threadIdx.x; c < ncells; c += blockDim.x) cmax[c] = 0u;
     __syncthreads();
     // the largest move: one atomic per warp (the moves are >= 0, so their bit
     // patterns order as the values do)
     unsigned long long mx = 0ull;
     for (int i = threadIdx.x; i < rk; i += blockDim.x) {
-      double4 s = J.sums[i];
-      const double4 o = J.cen[i];
-      const double4 c = make_double4(rdiv(s.x, s.w), rdiv(s.y, s.w), rdiv(s.z, s.w), 0.0);
-      J.cen[i] = c;
-      // upper bound on the distance the centroid moved (rounded upward)
-      const double dx = fabs(c.x - o.x), dy = fabs(c.y - o.y), dz = fabs(c.z - o.z);
-      const double d2 = __dadd_ru(__dadd_ru(__dmul_ru(dx, dx), __dmul_ru(dy, dy)), __dmul_ru(dz, dz));
-      const double sh = __dmul_ru(__dsqrt_ru(d2), 1.0 + 1e-13);
-      J.shift[i] = sh;
+      const double4 c = J.sums[i];
+      const double sh = J.shift[i];
+      J.cen[i] = make_double4(c.x, c.y, c.z, 0.0);
       mx = max(mx, (unsigned long long)__double_as_longlong(sh));
       atomicMax(&cmax[J.cell_of[i]], __float_as_uint(__double2float_ru(sh)));
     }
@@ -1168,33 +1195,34 @@ __global__ void __launch_bounds__(1024) k_centroids(const __grid_constant__ KmJo
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if ((threadIdx.x & 31) == 0 && mx) atomicMax(&st->maxshift_bits, mx);
     __syncthreads();
-    // 3^3 and 5^3 neighbourhood maxima as separable passes (x, y, z)
-    unsigned* t2 = tmp + ncells;
-    for (int rad = 1; rad <= 2; ++rad) {
+    // 3^3 and 5^3 neighbourhood maxima together, as separable passes (x, y, z):
+    // from one array of cells (or a pair, by radius) into the next pair
+    unsigned *a1 = cmax + ncells, *a2 = a1 + ncells, *b2 = a2 + ncells;
+    auto pass = [&](int axis, const unsigned* in1, const unsigned* in2, unsigned* out1,
+                    unsigned* out2) {
+      const int step = axis == 0 ? 1 : axis == 1 ? nc : nc * nc;
       for (int c = threadIdx.x; c < ncells; c += blockDim.x) {
-        const int ci = c % nc;
-        unsigned m = 0u;
-        for (int d = max(-rad, -ci); d <= min(rad, nc - 1 - ci); ++d) m = max(m, cmax[c + d]);
-        tmp[c] = m;
+        const int at = (c / step) % nc;
+        unsigned m1 = in1[c], m2 = in2[c];
+        if (at > 0) {
+          m1 = max(m1, in1[c - step]);
+          m2 = max(m2, in2[c - step]);
+        }
+        if (at > 1) m2 = max(m2, in2[c - 2 * step]);
+        if (at < nc - 1) {
+          m1 = max(m1, in1[c + step]);
+          m2 = max(m2, in2[c + step]);
+        }
+        if (at < nc - 2) m2 = max(m2, in2[c + 2 * step]);
+        out1[c] = m1;
+        out2[c] = m2;
       }
       __syncthreads();
-      for (int c = threadIdx.x; c < ncells; c += blockDim.x) {
-        const int cj = (c / nc) % nc;
-        unsigned m = 0u;
-        for (int d = max(-rad, -cj); d <= min(rad, nc - 1 - cj); ++d) m = max(m, tmp[c + d * nc]);
-        t2[c] = m;
-      }
-      __syncthreads();
-      float* out = rad == 1 ? J.nbshift : J.nbshift + kMaxCells;
-      for (int c = threadIdx.x; c < ncells; c += blockDim.x) {
-        const int ck = c / (nc * nc);
-        unsigned m = 0u;
-        for (int d = max(-rad, -ck); d <= min(rad, nc - 1 - ck); ++d)
-          m = max(m, t2[c + d * nc * nc]);
-        out[c] = __uint_as_float(m);
-      }
-      __syncthreads();
-    }
+    };
+    pass(0, cmax, cmax, a1, a2);
+    pass(1, a1, a2, cmax, b2);
+    pass(2, cmax, b2, reinterpret_cast<unsigned*>(J.nbshift),
+         reinterpret_cast<unsigned*>(J.nbshift) + kMaxCells);
   } else if (empty) {
     // the members' lists of this iteration are done with: scratch
     rk = compact_empty(J.sums, rk, J.cen, J.members, J.start, warp_tot);
@@ -1209,9 +1237,9 @@ __global__ void __launch_bounds__(1024) k_centroids(const __grid_constant__ KmJo
   __syncthreads();
   for (int j = threadIdx.x; j < rk; j += blockDim.x) {
     const double4 c = J.cen[j];
-    const int ci = min(nc - 1, max(0, (int)floor(c.x / g.h[0])));
-    const int cj = min(nc - 1, max(0, (int)floor(c.y / g.h[1])));
-    const int ck = min(nc - 1, max(0, (int)floor(c.z / g.h[2])));
+    const int ci = min(nc - 1, max(0, (int)floor(c.x * g.inv_h[0])));
+    const int cj = min(nc - 1, max(0, (int)floor(c.y * g.inv_h[1])));
+    const int ck = min(nc - 1, max(0, (int)floor(c.z * g.inv_h[2])));
     const int id = ci + nc * (cj + nc * ck);
     J.cell_of[j] = id;
     atomicAdd(&sc[id + 1], 1);
@@ -1410,7 +1438,8 @@ __device__ __forceinline__ double4 add4(const double4& a, const double4& b) {
 // MPICH's binomial algorithm runs it), evaluated rank by rank with a stack of
 // completed subtrees: (r0 + r1) + (r2 + r3) for 4 ranks, (r0 + r1) + r2 for 3.
 __global__ void k_shard_sums(KmState* st, const double4* __restrict__ recv, int ranks, int stride,
-                             double4* __restrict__ sums) {
+                             const double4* __restrict__ cen, double4* __restrict__ sums,
+                             double* __restrict__ shift) {
   if (st->done) return;
   const int rk = st->rk;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1432,8 +1461,7 @@ __global__ void k_shard_sums(KmState* st, const double4* __restrict__ recv, int 
   }
   double4 acc = val[top - 1];
   for (int i = top - 2; i >= 0; --i) acc = add4(val[i], acc);
-  sums[c] = acc;
-  if (acc.w == 0.0) st->any_empty = 1;
+  store_centroid(acc, c, cen, sums, shift, st);
 }
 
 // One rank's nearest point per centroid: the first minimum over its points
@@ -1482,8 +1510,10 @@ int set_kmeans_smem_attrs() {
                                  (int)(sizeof(int) * kKmeansMaxMu)));
   ISDF_CUDA(cudaFuncSetAttribute(k_scatter<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(short) * kScatterWarps * kKmeansMaxMu)));
+  ISDF_CUDA(cudaFuncSetAttribute(k_hist_scan<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(int) * kKmeansMaxMu)));
   // (a batch's histograms, kKmeansBatchMaxMu labels at most, need no opt-in)
-  const int cells = (int)(sizeof(unsigned) * (3 * kMaxCells + 1));
+  const int cells = (int)(sizeof(unsigned) * (4 * kMaxCells + 1));
   ISDF_CUDA(cudaFuncSetAttribute(k_centroids<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  cells));
   ISDF_CUDA(cudaFuncSetAttribute(k_centroids<kBatchJobs>,
@@ -1577,6 +1607,7 @@ CellGrid cell_grid(const KmeansArgs& args) {
   double lmax = 0.0;
   for (int i = 0; i < 3; ++i) {
     cg.h[i] = args.length[i] / nc;
+    cg.inv_h[i] = 1.0 / cg.h[i];
     lmax = std::max(lmax, std::fabs(args.length[i]));
   }
   cg.tol = 1e-9 * lmax;
@@ -1658,7 +1689,7 @@ struct LoopDims {
     mu = std::max(mu, (unsigned)mu_);
     assign = std::max(assign, assign_blocks);
     const size_t ncells = (size_t)job.cg.nc * job.cg.nc * job.cg.nc;
-    cells_smem = std::max(cells_smem, sizeof(unsigned) * (3 * ncells + 1));
+    cells_smem = std::max(cells_smem, sizeof(unsigned) * (4 * ncells + 1));
   }
 };
 
@@ -1670,7 +1701,8 @@ void launch_sums(const KmJobs<N>& J, const LoopDims& d, const LoopEnd& le, int* 
   const size_t hist_smem = sizeof(int) * (size_t)d.mu;
   const size_t scatter_smem = sizeof(short) * kScatterWarps * (size_t)d.mu;
   k_hist<N><<<dim3(d.tiles, d.jobs), 256, hist_smem, s>>>(J, le);
-  k_hist_scan<N><<<dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, 0, s>>>(J, le, live);
+  k_hist_scan<N><<<dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, hist_smem, s>>>(J, le,
+                                                                                             live);
   k_scatter<N><<<dim3(d.tiles, d.jobs), 32 * kScatterWarps, scatter_smem, s>>>(J);
   k_segsum<N><<<dim3(d.mu, d.jobs), kFoldThreads, 0, s>>>(J);
 }
@@ -1962,7 +1994,8 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
                                    stream));
         k_shard_begin<<<1, 1, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, job.max_f,
                                            args.max_iter);
-        k_shard_sums<<<grid_for(mu, 128), 128, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, b.sums);
+        k_shard_sums<<<grid_for(mu, 128), 128, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, b.cen,
+                                                            b.sums, b.shift);
       }
       launch_assign(jobs, dims, 1, stream);
       ISDF_CHECK_LAUNCH();
