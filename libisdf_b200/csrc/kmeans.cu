@@ -21,6 +21,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "arena.h"
@@ -439,13 +440,14 @@ __global__ void k_point_cells(const double* __restrict__ px, const double* __res
 // points' bounding box. The cells of one (y, z) row are contiguous in cell
 // order, so the lanes take a row each, then the rows' centroids 32 at a time:
 // those within sqrt(U) of the box go to shared memory as single-precision
-// offsets from the box's centre, kWarpCand at most before they are scanned
-// (any number of cells and candidates is taken in such portions).
-// The scan keeps the two smallest single-precision distances per point. Their
-// error against the exact distance is below err = 2^-19 (sqrt(U) + h)^2, h the
-// box's half diagonal (three offsets rounded to 24 bits on either side, their
-// difference, and the sum of squares: 2^-20 with the worst signs), so when the
-// second is more than 2 err above the first, the first is the only candidate
+// offsets c from the box's centre, (-2 c, |c|^2), kWarpCand at most before they
+// are scanned (any number of cells and candidates is taken in such portions).
+// The scan keeps the two smallest |c|^2 - 2 p.c per point, the squared distance
+// less |p|^2 in three multiply-adds. Their error against the exact distance is
+// below err = 2^-18 r^2, r = sqrt(U) + h and h the box's half diagonal (all
+// offsets are at most r long; rounding both, |c|^2, |p|^2 and the three sums
+// comes to 22 2^-24 r^2 with the worst signs), so when the second is more than
+// 2 err above the first, the first is the only candidate
 // that can be the portion's nearest, and its distance alone is computed in the
 // reference's rounding; otherwise every candidate within 2 err of the smallest
 // is. Distances so computed are compared as (d, index) pairs: the label is
@@ -456,17 +458,27 @@ __global__ void k_point_cells(const double* __restrict__ px, const double* __res
 // in rings of cells where a warp had more than 216 cells or 160 candidates (a
 // few warps in the sparse regions, which the launch then waited for) or, in the
 // first assignment, no seed. A launch late in a selection: 64 000 points and
-// 309 centroids 47 -> 10 us, 151 875 and 505 68 -> 19 us, 884 736 and 2979
-// 140 -> 72 us; the first assignment of the last 9200 -> 510 us.
+// 309 centroids 47 -> 10 us, 151 875 and 505 68 -> 18 us, 884 736 and 2979
+// 140 -> 52 us; the first assignment of the last 9200 -> 510 us.
 constexpr int kWarpCand = 128;   // candidates staged per warp
 
-__device__ __forceinline__ double warp_max(double v) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+// The warp's least float / largest float / largest non-negative float, by the
+// integer reductions (a float's bits, the negative ones' magnitude flipped, order as
+// the values do).
+__device__ __forceinline__ int float_order(float v) {
+  const int i = __float_as_int(v);
+  return i ^ ((i >> 31) & 0x7fffffff);
 }
-__device__ __forceinline__ double warp_min(double v) {
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+__device__ __forceinline__ float order_float(int i) {
+  return __int_as_float(i ^ ((i >> 31) & 0x7fffffff));
+}
+__device__ __forceinline__ double warp_least(bool in, double v) {
+  const int i = in ? float_order(__double2float_rd(v)) : 0x7fffffff;
+  return (double)order_float(__reduce_min_sync(0xffffffffu, i));
+}
+__device__ __forceinline__ double warp_most(bool in, double v) {
+  const int i = in ? float_order(__double2float_ru(v)) : (int)0x80000000;
+  return (double)order_float(__reduce_max_sync(0xffffffffu, i));
 }
 
 // A seed for the first assignment. The centroids start at the first rk points
@@ -502,7 +514,8 @@ __global__ void __launch_bounds__(kAssignThreads, 8)
   const CellGrid& g = J.cg;
   int* label = J.label;
   double2* bnd = J.bnd;
-  __shared__ float4 cand[kAssignThreads / 32][kWarpCand];  // offsets; w: place in cell_cen (bits)
+  __shared__ float4 cand[kAssignThreads / 32][kWarpCand];  // -2 c, |c|^2
+  __shared__ int cand_at[kAssignThreads / 32][kWarpCand];  // place in cell_cen
   const int rk = st->rk;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int p = assign_point((long long)blockIdx.x * blockDim.x + threadIdx.x, J.am);
@@ -548,17 +561,20 @@ __global__ void __launch_bounds__(kAssignThreads, 8)
     best = ref_dist2(x, y, z, cen[bj]);
   }
   const double shrink = 1.0 - 2e-14;
-  const double U = warp_max(best);  // 0 on the lanes that do not search
-  const double x0 = warp_min(need ? x : inf), x1 = warp_max(need ? x : -inf);
-  const double y0 = warp_min(need ? y : inf), y1 = warp_max(need ? y : -inf);
-  const double z0 = warp_min(need ? z : inf), z1 = warp_max(need ? z : -inf);
+  // (all rounded outward to single precision: what they bound stays bounded)
+  const double U = warp_most(true, best);  // 0 on the lanes that do not search
+  const double x0 = warp_least(need, x), x1 = warp_most(need, x);
+  const double y0 = warp_least(need, y), y1 = warp_most(need, y);
+  const double z0 = warp_least(need, z), z1 = warp_most(need, z);
   const double xc = 0.5 * (x0 + x1), yc = 0.5 * (y0 + y1), zc = 0.5 * (z0 + z1);
   const double R = __dmul_ru(__dsqrt_ru(U), kRoundUp) + g.tol;
   const float fx = (float)(x - xc), fy = (float)(y - yc), fz = (float)(z - zc);
-  const float hx = (float)(x1 - xc), hy = (float)(y1 - yc), hz = (float)(z1 - zc);
+  const float pp = fmaf(fx, fx, fmaf(fy, fy, fz * fz));
+  const float hx = __double2float_ru(x1 - xc), hy = __double2float_ru(y1 - yc),
+              hz = __double2float_ru(z1 - zc);
   const double reach = R + (x1 - xc) + (y1 - yc) + (z1 - zc);  // >= sqrt(U) + h
   // (the last term covers products below the normal range)
-  const float err = __double2float_ru(1.9073486328125e-6 * reach * reach) + 1e-37f;
+  const float err = __double2float_ru(3.814697265625e-6 * reach * reach) + 1e-37f;
   const float far = __double2float_ru(U) + 2.0f * err;  // beyond: more than sqrt(U) from the box
   const int nc = g.nc;
   const int i0 = min(nc - 1, max(0, (int)floor((x0 - R) * g.inv_h[0])));
@@ -569,6 +585,7 @@ __global__ void __launch_bounds__(kAssignThreads, 8)
   const int k1 = min(nc - 1, max(0, (int)floor((z1 + R) * g.inv_h[2])));
   const int nj = j1 - j0 + 1, nrow = nj * (k1 - k0 + 1);
   float4* cw = cand[wid];
+  int* cat = cand_at[wid];
   double second = inf;
   // the nearest of the candidates staged, into (best, bj) and second
   auto scan = [&](int total) {
@@ -579,14 +596,13 @@ __global__ void __launch_bounds__(kAssignThreads, 8)
 #pragma unroll 4
     for (int q = 0; q < total; ++q) {
       const float4 c = cw[q];
-      const float dx = fx - c.x, dy = fy - c.y, dz = fz - c.z;
-      const float d = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      const float d = fmaf(fx, c.x, fmaf(fy, c.y, fmaf(fz, c.z, c.w)));
       m2 = fminf(m2, fmaxf(m1, d));
       q1 = d < m1 ? q : q1;
       m1 = fminf(m1, d);
     }
     auto consider = [&](int q) {
-      const double4 c = cell_cen[__float_as_int(cw[q].w)];
+      const double4 c = cell_cen[cat[q]];
       const double d = ref_dist2(x, y, z, c);
       const int j = (int)c.w;
       if (d < best || (d == best && j < bj)) {
@@ -600,17 +616,16 @@ __global__ void __launch_bounds__(kAssignThreads, 8)
     const float thr = m1 + 2.0f * err;
     if (m2 > thr) {
       consider(q1);
-      second = fmin(second, fmax(0.0, (double)m2 - (double)err));
+      second = fmin(second, fmax(0.0, (double)m2 + (double)pp - (double)err));
     } else {
       float next = finf;  // the smallest distance left out
       for (int q = 0; q < total; ++q) {
         const float4 c = cw[q];
-        const float dx = fx - c.x, dy = fy - c.y, dz = fz - c.z;
-        const float d = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        const float d = fmaf(fx, c.x, fmaf(fy, c.y, fmaf(fz, c.z, c.w)));
         if (!(d > thr)) consider(q);
         else next = fminf(next, d);
       }
-      second = fmin(second, fmax(0.0, (double)next - (double)err));
+      second = fmin(second, fmax(0.0, (double)next + (double)pp - (double)err));
     }
   };
   int total = 0;
@@ -657,8 +672,11 @@ __global__ void __launch_bounds__(kAssignThreads, 8)
         in = !(fmaf(bx, bx, fmaf(by, by, bz * bz)) > far);
       }
       const unsigned got = __ballot_sync(0xffffffffu, in);
-      if (in)
-        cw[total + __popc(got & ((1u << lane) - 1u))] = make_float4(cx, cy, cz, __int_as_float(at));
+      if (in) {
+        const int to = total + __popc(got & ((1u << lane) - 1u));
+        cw[to] = make_float4(-2.f * cx, -2.f * cy, -2.f * cz, fmaf(cx, cx, fmaf(cy, cy, cz * cz)));
+        cat[to] = at;
+      }
       total += __popc(got);
       if (total > kWarpCand - 32) {
         __syncwarp();
@@ -749,35 +767,41 @@ __global__ void __launch_bounds__(32 * kScanWarps)
   const int t0 = w * per, t1 = min(t0 + per, ntiles);
   __shared__ int part[kScanWarps][32];
   __shared__ bool last;
-  constexpr int kB = 8;  // loads batched ahead of the additions and stores
-  int sum = 0;
-  if (l < rk) {
-    for (int t = t0; t < t1; t += kB) {
-      int v[kB];
+  // kB tiles of a warp's range are held at once, their loads all ahead of the sums
+  auto scan = [&](auto held) {
+    constexpr int kB = decltype(held)::value;
+    int v[kB];
+    auto load = [&](int t) {
 #pragma unroll
       for (int u = 0; u < kB; ++u) v[u] = t + u < t1 ? hist[(size_t)(t + u) * rk + l] : 0;
+    };
+    int sum = 0;
+    if (l < rk) {
+      for (int t = t0; t < t1; t += kB) {
+        load(t);
 #pragma unroll
-      for (int u = 0; u < kB; ++u) sum += v[u];
-    }
-  }
-  part[w][lane] = sum;
-  __syncthreads();
-  if (l < rk) {
-    int run = 0;
-    for (int q = 0; q < w; ++q) run += part[q][lane];
-    for (int t = t0; t < t1; t += kB) {
-      int v[kB];
-#pragma unroll
-      for (int u = 0; u < kB; ++u) v[u] = t + u < t1 ? hist[(size_t)(t + u) * rk + l] : 0;
-#pragma unroll
-      for (int u = 0; u < kB; ++u) {
-        if (t + u < t1) hist[(size_t)(t + u) * rk + l] = run;
-        run += v[u];
+        for (int u = 0; u < kB; ++u) sum += v[u];
       }
     }
-    // the last warp's prefix covers every tile (its own range may be empty)
-    if (w == kScanWarps - 1) J.members[l] = run;
-  }
+    part[w][lane] = sum;
+    __syncthreads();
+    if (l < rk) {
+      int run = 0;
+      for (int q = 0; q < w; ++q) run += part[q][lane];
+      for (int t = t0; t < t1; t += kB) {
+        if (per > kB) load(t);  // else still there
+#pragma unroll
+        for (int u = 0; u < kB; ++u) {
+          if (t + u < t1) hist[(size_t)(t + u) * rk + l] = run;
+          run += v[u];
+        }
+      }
+      // the last warp's prefix covers every tile (its own range may be empty)
+      if (w == kScanWarps - 1) J.members[l] = run;
+    }
+  };
+  if (per <= 4) scan(std::integral_constant<int, 4>());
+  else scan(std::integral_constant<int, 16>());
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
