@@ -40,6 +40,7 @@ constexpr int kTile = 2048;      // points per counting-sort tile (one walking w
 constexpr int kFinalChunk = 4096;  // points per partial argmin chunk
 constexpr int kIterChunk = 8;    // Lloyd iterations launched between host checks (no graph)
 constexpr int kBodyIters = 2;    // Lloyd iterations per body of the loop's graph
+constexpr int kAheadIters = 4;   // Lloyd iterations launched before the graph is built
 constexpr int kMaxCellsPerDim = 20;  // centroid cell grid of the pruned assignment
 constexpr int kMaxCells = kMaxCellsPerDim * kMaxCellsPerDim * kMaxCellsPerDim;
 
@@ -1739,11 +1740,18 @@ void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, cudaStream
 
 // The Lloyd loop as a graph with kBodyIters iterations per body: no iteration
 // waits for the host (reading the state back after every 8 iterations left the GPU
-// idle for 75 us each time, and the graph of 8 took twice as long to build).
+// idle for 75 us each time, and the graph of 8 took twice as long to build). The
+// first kAheadIters iterations are launched directly: they run while the host
+// builds the graph (150 us, in which a small selection's GPU was idle).
 template <int N>
 void build_loop(LoopGraph& loop, const KmJobs<N>& J, const LoopDims& d, int max_iter, int* live,
                 cudaStream_t s) {
-  loop.build(s, max_iter / kBodyIters * kBodyIters + 4 * kBodyIters, [&](const LoopEnd& le) {
+  const LoopEnd no_graph{0, 0, 0x7fffffff};
+  for (int it = 0; it < kAheadIters; ++it) {
+    launch_sums(J, d, no_graph, live, s);
+    launch_assign(J, d, 1, s);
+  }
+  loop.build(s, kAheadIters + max_iter + 4 * kBodyIters, [&](const LoopEnd& le) {
     for (int it = 0; it < kBodyIters; ++it) {
       launch_sums(J, d, le, live, s);
       launch_assign(J, d, 1, s);
