@@ -389,11 +389,14 @@ __global__ void __launch_bounds__(1024) k_normalise(int p, int ldq, const double
 // this one 17). An odd last row copies its zero padding partner.
 template <int BN>
 using UpdTile = dmma::WsTile<64, BN, 4, 1, 16, 3>;
-// three CTAs per SM while the accumulators leave room (136 registers)
+// CTAs per SM while the accumulators (and, for the narrow tiles, the columns of A
+// read ahead of the dot) leave registers: a narrow tile's CTA is short, and its
+// loads' latency is what it waits for
 template <int BN>
 struct UpdMinBlocks {
-  static constexpr int value = BN <= 96 ? 3 : 2;
+  static constexpr int value = BN <= 40 ? 4 : BN <= 96 ? 3 : 2;
 };
+constexpr int kUpdAhead = 40;  // widest tile whose columns of A are read ahead
 
 template <int BN, int MINB>
 __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
@@ -408,10 +411,24 @@ __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
   const int m0 = blockIdx.x * T::BM;
   const int m_rem = min(T::BM, ntot - m0);
   T tile;
-  if (!tile.run(smem, Bc + m0, ld, (m_rem + 1) & ~1, Qm, ldq, p, p, err)) return;
-  if (T::producer()) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
+  constexpr bool kAhead = BN <= kUpdAhead;
+  double av[2][kAhead ? T::NT : 1][2];
+  auto load_a = [&](int h, int j, int e) -> double {
+    const int r = warp * 16 + g + 8 * h, c = j * 8 + 2 * t + e;
+    return r < m_rem && c < p ? Ac[(m0 + r) + (long long)c * ld] : 0.0;
+  };
+  if (kAhead && !T::producer()) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int j = 0; j < (kAhead ? T::NT : 1); ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) av[h][j][e] = load_a(h, j, e);
+  }
+  if (!tile.run(smem, Bc + m0, ld, (m_rem + 1) & ~1, Qm, ldq, p, p, err)) return;
+  if (T::producer()) return;
   Best v{0.0, INT_MAX};
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -419,11 +436,11 @@ __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
     double s = 0.0;
     if (r < m_rem) {
 #pragma unroll
-      for (int j = 0; j < T::NT; ++j) {
-        const int c = j * 8 + 2 * t;
-        if (c < p) s = fma(Ac[(m0 + r) + (long long)c * ld], tile.acc[0][j][2 * h], s);
-        if (c + 1 < p) s = fma(Ac[(m0 + r) + (long long)(c + 1) * ld], tile.acc[0][j][2 * h + 1], s);
-      }
+      for (int j = 0; j < T::NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (j * 8 + 2 * t + e < p)
+            s = fma(kAhead ? av[h][kAhead ? j : 0][e] : load_a(h, j, e), tile.acc[0][j][2 * h + e], s);
     }
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
@@ -434,9 +451,14 @@ __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
     }
   }
   v = warp_best(v);
-  // one candidate per warp: the producer warp has left, so the block's four warps
-  // share no barrier
-  if (lane == 0) best[blockIdx.x * T::NW + warp] = v;
+  __shared__ Best warp_v[T::NW];
+  if (lane == 0) warp_v[warp] = v;
+  asm volatile("bar.sync 1, %0;" ::"n"(T::NW * 32) : "memory");  // the DMMA warps
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < T::NW; ++w) v = better(v, warp_v[w]);
+    best[blockIdx.x] = v;
+  }
 }
 
 // Exact residual norms of the columns the downdate flagged in this step
@@ -562,7 +584,7 @@ std::vector<double> gaussian_draws(int m, int n) {
 struct QrBuffers {
   double *A, *B, *norm2, *Ac, *Bc, *nu, *nu0, *Q, *Qm, *x, *cdot, *G1, *G2, *rec_dots;
   int *idx, *pos, *perm, *sel, *tile_cnt, *rec_list;
-  Best* best;  // candidates: four per 64 columns, then one per recompute block
+  Best* best;  // candidates: one per 64 columns, then one per recompute block
   unsigned char* active;
   QrState* st;
   int* err;  // a bounded pipeline wait of the update ran out
@@ -593,7 +615,7 @@ QrBuffers carve(Arena& a, long long n, int p, int k1, int k2, int kmax) {
   b.rec_list = a.take<int>((size_t)n);
   b.rec_dots = a.take<double>((size_t)kRecomputeGrid * kmax);
   b.active = a.take<unsigned char>((size_t)n);
-  b.best = a.take<Best>((size_t)(4 * ((n + 63) / 64) + kRecomputeGrid));
+  b.best = a.take<Best>((size_t)((n + 63) / 64 + kRecomputeGrid));
   b.st = a.take<QrState>(1);
   b.err = a.take<int>(1);
   return b;
@@ -731,8 +753,8 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
   // pivoted Gram-Schmidt over the kept columns
   const int ld = ntot + (ntot & 1);  // Ac / Bc leading dimension (k_compact)
   const int ldq = p + (p & 1);
-  const int ublocks = (ntot + 63) / 64, nbest = 4 * ublocks + kRecomputeGrid;
-  // the first candidates: one per 64 columns, the other places empty
+  const int ublocks = (ntot + 63) / 64, nbest = ublocks + kRecomputeGrid;
+  // the first candidates: one per 64 columns, none from recomputes
   ISDF_CUDA(cudaMemsetAsync(b.best, 0, sizeof(Best) * (size_t)nbest, s));
   if (ublocks > 0) k_first_best<<<ublocks, 64, 0, s>>>(b.nu, ntot, ublocks, b.best);
   // One pivot step; the step number lives on the device.
@@ -747,14 +769,16 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
     launch_update_ws(b, ntot, ld, p, s);
     k_recompute<<<kRecomputeGrid, 256, sizeof(double) * m, s>>>(
         b.Ac, b.Bc, ld, p, b.Q, m, kmax_cap, b.rec_list, b.pos, b.nu, b.nu0, b.st, b.rec_dots,
-        b.best + 4 * (size_t)ublocks);
+        b.best + ublocks);
   };
   if (kmax > 0) {
     // a graph that loops on the device: launched step by step, the nine launches
     // of a step took the host longer than the GPU at numPre = 31
-    constexpr int kBodySteps = 4;
+    constexpr int kBodySteps = 4, kAheadSteps = 8;
+    const LoopEnd ahead{0, 0, 0x7fffffff};
+    for (int i = 0; i < std::min(kmax, kAheadSteps); ++i) step(ahead);  // while it is built
     LoopGraph loop;
-    loop.build(s, kmax + 2 * kBodySteps, [&](const LoopEnd& le) {
+    loop.build(s, kAheadSteps + kmax + 2 * kBodySteps, [&](const LoopEnd& le) {
       for (int i = 0; i < kBodySteps; ++i) step(le);
     });
     if (loop.exec) {
@@ -762,9 +786,8 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
       // (the graph must outlive its launch)
       ISDF_TRY(read_back(&hst, b.st, sizeof(QrState), s));
     } else {
-      const LoopEnd no_graph{0, 0, 0x7fffffff};
-      for (int k = 0; k < kmax; ++k) {
-        step(no_graph);
+      for (int k = kAheadSteps; k < kmax; ++k) {
+        step(ahead);
         if ((k & 255) == 255) ISDF_CHECK_LAUNCH();
       }
     }
