@@ -322,27 +322,32 @@ __global__ void __launch_bounds__(256) k_qt_x(const double* __restrict__ Q, int 
   }
 }
 
-// x -= Q[:, 0:k] cdot: a block takes 32 consecutive rows (one per lane), its
-// 32 warps the columns l = w (mod 32), and the 32 partials are added in warp
-// order (enough loads in flight per SM to stream Q from L2).
-__global__ void __launch_bounds__(1024) k_x_minus_qc(const double* __restrict__ Q, int m,
-                                                     const double* __restrict__ cdot,
-                                                     const QrState* st, double* __restrict__ x) {
+// x -= Q[:, 0:k] cdot: a block takes kMinusRows consecutive rows, its 32 groups of
+// as many lanes the columns l = w (mod 32), and the 32 partials are added in group
+// order. Q streams from L2 (4.9 MB at 961 features and 640 pivots); eight rows a
+// block spread it over 121 SMs (32 rows left 31 SMs to do it: 5.3 us a pass).
+constexpr int kMinusRows = 8;
+__global__ void __launch_bounds__(32 * kMinusRows) k_x_minus_qc(const double* __restrict__ Q,
+                                                                int m,
+                                                                const double* __restrict__ cdot,
+                                                                const QrState* st,
+                                                                double* __restrict__ x) {
   const int k = st->step;
   if (k <= 0) return;
-  __shared__ double red[32][33];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int i = blockIdx.x * 32 + lane;
+  __shared__ double red[32][kMinusRows + 1];
+  const int r = threadIdx.x % kMinusRows, w = threadIdx.x / kMinusRows;
+  const int i = blockIdx.x * kMinusRows + r;
   double s = 0.0;
   if (i < m) {
-#pragma unroll 4
+#pragma unroll 10
     for (int l = w; l < k; l += 32) s = fma(Q[i + (long long)l * m], cdot[l], s);
   }
-  red[w][lane] = s;
+  red[w][r] = s;
   __syncthreads();
   if (w == 0 && i < m) {
-    double v = red[0][lane];
-    for (int u = 1; u < 32; ++u) v += red[u][lane];
+    double v = red[0][r];
+#pragma unroll
+    for (int u = 1; u < 32; ++u) v += red[u][r];
     x[i] -= v;
   }
 }
@@ -763,7 +768,8 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
                               b.sel, b.st, b.x, le);
     for (int pass = 0; pass < 2; ++pass) {
       k_qt_x<<<kmax, 256, 0, s>>>(b.Q, m, b.x, b.st, b.cdot);
-      k_x_minus_qc<<<(m + 31) / 32, 1024, 0, s>>>(b.Q, m, b.cdot, b.st, b.x);
+      k_x_minus_qc<<<(m + kMinusRows - 1) / kMinusRows, 32 * kMinusRows, 0, s>>>(
+          b.Q, m, b.cdot, b.st, b.x);
     }
     k_normalise<<<1, 1024, 0, s>>>(p, ldq, b.x, b.st, b.Q, b.Qm);
     launch_update_ws(b, ntot, ld, p, s);
