@@ -506,6 +506,7 @@ __device__ __forceinline__ int first_seed(int p, int rk, const int* __restrict__
 template <int N>
 __global__ void __launch_bounds__(kAssignThreads, 8)
     k_assign_warp(const __grid_constant__ KmJobs<N> JS, int count) {
+  after_previous();
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (st->done) return;
@@ -719,6 +720,7 @@ __device__ __forceinline__ bool goes_on(const KmJob& J) {
 // utility.cpp:816-822.
 template <int N>
 __global__ void __launch_bounds__(256) k_hist(const __grid_constant__ KmJobs<N> JS, const LoopEnd le) {
+  after_previous();
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (blockIdx.x == 0 && threadIdx.x == 0 && ++st->rounds > le.max_rounds) end_loop(le);
@@ -749,6 +751,7 @@ constexpr int kScanWarps = 16;
 template <int N>
 __global__ void __launch_bounds__(32 * kScanWarps)
     k_hist_scan(const __grid_constant__ KmJobs<N> JS, const LoopEnd le, int* live) {
+  after_previous();
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (st->done) return;
@@ -860,6 +863,7 @@ constexpr int kScatterWarps = 8;
 template <int N>
 __global__ void __launch_bounds__(32 * kScatterWarps)
     k_scatter(const __grid_constant__ KmJobs<N> JS) {
+  after_previous();
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   const KmState* st = J.st;
   if (st->done || blockIdx.x * kTile >= J.f_n) return;
@@ -1071,6 +1075,7 @@ constexpr int kFoldThreads = 128;
 
 template <int N>
 __global__ void __launch_bounds__(kFoldThreads) k_segsum(const __grid_constant__ KmJobs<N> JS) {
+  after_previous();
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (st->done) return;
@@ -1194,6 +1199,7 @@ __device__ int compact_empty(const double4* __restrict__ sums, int rk, double4* 
 // update = 0: the cells alone (the first centroids).
 template <int N>
 __global__ void __launch_bounds__(1024) k_centroids(const __grid_constant__ KmJobs<N> JS, int update) {
+  after_previous();
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
   if (st->done) return;
@@ -1725,17 +1731,17 @@ void launch_sums(const KmJobs<N>& J, const LoopDims& d, const LoopEnd& le, int* 
                  cudaStream_t s) {
   const size_t hist_smem = sizeof(int) * (size_t)d.mu;
   const size_t scatter_smem = sizeof(short) * kScatterWarps * (size_t)d.mu;
-  k_hist<N><<<dim3(d.tiles, d.jobs), 256, hist_smem, s>>>(J, le);
-  k_hist_scan<N><<<dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, hist_smem, s>>>(J, le,
-                                                                                             live);
-  k_scatter<N><<<dim3(d.tiles, d.jobs), 32 * kScatterWarps, scatter_smem, s>>>(J);
-  k_segsum<N><<<dim3(d.mu, d.jobs), kFoldThreads, 0, s>>>(J);
+  launch_early(k_hist<N>, dim3(d.tiles, d.jobs), 256, hist_smem, s, J, le);
+  launch_early(k_hist_scan<N>, dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, hist_smem, s, J, le,
+               live);
+  launch_early(k_scatter<N>, dim3(d.tiles, d.jobs), 32 * kScatterWarps, scatter_smem, s, J);
+  launch_early(k_segsum<N>, dim3(d.mu, d.jobs), kFoldThreads, 0, s, J);
 }
 
 template <int N>
 void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, cudaStream_t s) {
-  k_centroids<N><<<dim3(1, d.jobs), 1024, d.cells_smem, s>>>(J, update);
-  k_assign_warp<N><<<dim3(d.assign, d.jobs), kAssignThreads, 0, s>>>(J, update);
+  launch_early(k_centroids<N>, dim3(1, d.jobs), 1024, d.cells_smem, s, J, update);
+  launch_early(k_assign_warp<N>, dim3(d.assign, d.jobs), kAssignThreads, 0, s, J, update);
 }
 
 // The Lloyd loop as a graph with kBodyIters iterations per body: no iteration

@@ -1,6 +1,7 @@
 // A device-ended loop as a CUDA graph: a WHILE node whose body is captured from
 // the caller's launches and which a kernel of the body ends, so that no round of
-// the loop waits for the host.
+// the loop waits for the host; and launches whose start overlaps the kernel before
+// them, for loops of many short kernels.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -18,6 +19,38 @@ struct LoopEnd {
 
 __device__ __forceinline__ void end_loop(const LoopEnd& le) {
   if (le.in_graph) cudaGraphSetConditional(le.handle, 0);
+}
+
+// Begins a kernel launched by launch_early (what no kernel of the loop writes may
+// be read before): waits for the whole of
+// the kernel before it and its writes, then lets the next kernel's blocks become
+// resident (they wait here in turn). Every block passes here before it reads,
+// writes or returns: a kernel that completed without waiting would let the next one
+// run ahead of the one before it. What follows reads its state through plain
+// pointers first, so that no read-only load moves above the wait.
+__device__ __forceinline__ void after_previous() {
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+}
+
+// Launches k, a kernel that begins with after_previous(), so that its blocks are
+// set up while the kernel before it on the stream drains (also as an edge of a
+// captured graph). An ordinary launch starts them only when that kernel has
+// finished: about a microsecond on each kernel of a loop.
+template <class... P, class... A>
+void launch_early(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                  const A&... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
 }
 
 struct LoopGraph {

@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(1024) k_pick(int kmax, int p, int ld, int nbes
                                                unsigned char* __restrict__ active,
                                                int* __restrict__ sel, QrState* st,
                                                double* __restrict__ x, const LoopEnd le) {
+  after_previous();
   __shared__ int col;
   __shared__ Best warp_v[32];
   const int k = st->k;
@@ -305,6 +306,7 @@ __global__ void __launch_bounds__(1024) k_pick(int kmax, int p, int ld, int nbes
 __global__ void __launch_bounds__(256) k_qt_x(const double* __restrict__ Q, int m,
                                               const double* __restrict__ x, const QrState* st,
                                               double* __restrict__ cdot) {
+  after_previous();
   const int l = blockIdx.x;
   if (l >= st->step) return;
   __shared__ double red[8];
@@ -332,6 +334,7 @@ __global__ void __launch_bounds__(32 * kMinusRows) k_x_minus_qc(const double* __
                                                                 const double* __restrict__ cdot,
                                                                 const QrState* st,
                                                                 double* __restrict__ x) {
+  after_previous();
   const int k = st->step;
   if (k <= 0) return;
   __shared__ double red[32][kMinusRows + 1];
@@ -356,6 +359,7 @@ __global__ void __launch_bounds__(32 * kMinusRows) k_x_minus_qc(const double* __
 __global__ void __launch_bounds__(1024) k_normalise(int p, int ldq, const double* __restrict__ x,
                                                     QrState* st, double* __restrict__ Q,
                                                     double* __restrict__ Qm) {
+  after_previous();
   const int k = st->step;
   if (k < 0 || st->done) return;
   const int m = p * p;
@@ -411,7 +415,6 @@ __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
                 const int* __restrict__ pos, double* __restrict__ nu, double* __restrict__ nu0,
                 QrState* st, int* __restrict__ rec_list, Best* __restrict__ best, int* err) {
   using T = UpdTile<BN>;
-  if (st->step < 0 || st->done) return;
   extern __shared__ __align__(128) double smem[];
   const int m0 = blockIdx.x * T::BM;
   const int m_rem = min(T::BM, ntot - m0);
@@ -432,6 +435,8 @@ __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
 #pragma unroll
         for (int e = 0; e < 2; ++e) av[h][j][e] = load_a(h, j, e);
   }
+  after_previous();  // (A does not change from step to step)
+  if (st->step < 0 || st->done) return;
   if (!tile.run(smem, Bc + m0, ld, (m_rem + 1) & ~1, Qm, ldq, p, p, err)) return;
   if (T::producer()) return;
   Best v{0.0, INT_MAX};
@@ -483,6 +488,7 @@ __global__ void __launch_bounds__(256) k_recompute(const double* __restrict__ Ac
                                                    double* __restrict__ nu0, QrState* st,
                                                    double* __restrict__ cbuf,
                                                    Best* __restrict__ best) {
+  after_previous();
   extern __shared__ double x[];  // m features
   __shared__ double red[8];
   const int k1 = st->step + 1;
@@ -662,9 +668,9 @@ template <int BN>
 void launch_update_bn(const QrBuffers& b, int ntot, int ld, int p, cudaStream_t s) {
   using T = UpdTile<BN>;
   const unsigned grid = (unsigned)((ntot + T::BM - 1) / T::BM);
-  k_update_ws<BN, UpdMinBlocks<BN>::value><<<grid, T::THREADS, T::SMEM_BYTES, s>>>(
-      b.Ac, b.Bc, ntot, ld, p, p + (p & 1), b.Qm, b.active, b.pos, b.nu, b.nu0, b.st, b.rec_list,
-      b.best, b.err);
+  launch_early(k_update_ws<BN, UpdMinBlocks<BN>::value>, grid, T::THREADS, T::SMEM_BYTES, s, b.Ac,
+               b.Bc, ntot, ld, p, p + (p & 1), b.Qm, b.active, b.pos, b.nu, b.nu0, b.st,
+               b.rec_list, b.best, b.err);
 }
 
 // The downdate on the narrowest warp-specialised tile that holds p columns
@@ -764,18 +770,17 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
   if (ublocks > 0) k_first_best<<<ublocks, 64, 0, s>>>(b.nu, ntot, ublocks, b.best);
   // One pivot step; the step number lives on the device.
   auto step = [&](const LoopEnd& le) {
-    k_pick<<<1, 1024, 0, s>>>(kmax, p, ld, nbest, b.best, b.Ac, b.Bc, b.pos, b.perm, b.active,
-                              b.sel, b.st, b.x, le);
+    launch_early(k_pick, 1, 1024, 0, s, kmax, p, ld, nbest, b.best, b.Ac, b.Bc, b.pos, b.perm,
+                 b.active, b.sel, b.st, b.x, le);
     for (int pass = 0; pass < 2; ++pass) {
-      k_qt_x<<<kmax, 256, 0, s>>>(b.Q, m, b.x, b.st, b.cdot);
-      k_x_minus_qc<<<(m + kMinusRows - 1) / kMinusRows, 32 * kMinusRows, 0, s>>>(
-          b.Q, m, b.cdot, b.st, b.x);
+      launch_early(k_qt_x, kmax, 256, 0, s, b.Q, m, b.x, b.st, b.cdot);
+      launch_early(k_x_minus_qc, (m + kMinusRows - 1) / kMinusRows, 32 * kMinusRows, 0, s, b.Q, m,
+                   b.cdot, b.st, b.x);
     }
-    k_normalise<<<1, 1024, 0, s>>>(p, ldq, b.x, b.st, b.Q, b.Qm);
+    launch_early(k_normalise, 1, 1024, 0, s, p, ldq, b.x, b.st, b.Q, b.Qm);
     launch_update_ws(b, ntot, ld, p, s);
-    k_recompute<<<kRecomputeGrid, 256, sizeof(double) * m, s>>>(
-        b.Ac, b.Bc, ld, p, b.Q, m, kmax_cap, b.rec_list, b.pos, b.nu, b.nu0, b.st, b.rec_dots,
-        b.best + ublocks);
+    launch_early(k_recompute, kRecomputeGrid, 256, sizeof(double) * m, s, b.Ac, b.Bc, ld, p, b.Q,
+                 m, kmax_cap, b.rec_list, b.pos, b.nu, b.nu0, b.st, b.rec_dots, b.best + ublocks);
   };
   if (kmax > 0) {
     // a graph that loops on the device: launched step by step, the nine launches
