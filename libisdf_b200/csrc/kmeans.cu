@@ -1190,13 +1190,26 @@ __device__ int compact_empty(const double4* __restrict__ sums, int rk, double4* 
   return left;
 }
 
-// The new centroids (with the compaction above where a cluster is empty) into
-// place, then into the cell grid (cell_start, cell_cen): one block, so whatever
-// the folds' blocks can do (the divisions, the moves) they have done. The update
-// also takes the largest move, and for every cell of the grid the largest move of
-// a centroid that sat in its 3^3 and 5^3 neighbourhoods before the update (cell_of
-// still holds the previous positions' cells there).
+__device__ __forceinline__ int cell_index(const CellGrid& g, double x, double y, double z) {
+  const int nc = g.nc;
+  const int ci = min(nc - 1, max(0, (int)floor(x * g.inv_h[0])));
+  const int cj = min(nc - 1, max(0, (int)floor(y * g.inv_h[1])));
+  const int ck = min(nc - 1, max(0, (int)floor(z * g.inv_h[2])));
+  return ci + nc * (cj + nc * ck);
+}
+
+// After the folds (whose blocks have done the divisions and the moves), two blocks,
+// bound by the latency of their phases, which do not need each other:
+//  - block 0 sorts the new centroids (compacted as above where a cluster is empty)
+//    into the cell grid (cell_start, cell_cen), the first kCenHeld per thread read
+//    once;
+//  - block 1 puts them into place and takes the largest move, and for every cell
+//    the largest move of a centroid that sat in its 3^3 and 5^3 neighbourhoods
+//    before the update (cell_of still holds the previous positions' cells there).
+// One block for both took 14.9 us at 2979 centroids, 5.2 at 309.
 // update = 0: the cells alone (the first centroids).
+constexpr int kCenHeld = 3;
+
 template <int N>
 __global__ void __launch_bounds__(1024) k_centroids(const __grid_constant__ KmJobs<N> JS, int update) {
   after_previous();
@@ -1207,20 +1220,24 @@ __global__ void __launch_bounds__(1024) k_centroids(const __grid_constant__ KmJo
   __shared__ int warp_tot[32];
   const CellGrid& g = J.cg;
   const int nc = g.nc, ncells = nc * nc * nc;
-  int rk = st->rk;
   const bool empty = update && st->any_empty;
-  if (update && !empty) {
+  if (blockIdx.x == 1) {
+    if (!update || empty) return;
+    const int rk = st->rk;
     for (int c = threadIdx.x; c < ncells; c += blockDim.x) cmax[c] = 0u;
     __syncthreads();
     // the largest move: one atomic per warp (the moves are >= 0, so their bit
     // patterns order as the values do)
     unsigned long long mx = 0ull;
+#pragma unroll kCenHeld
     for (int i = threadIdx.x; i < rk; i += blockDim.x) {
       const double4 c = J.sums[i];
       const double sh = J.shift[i];
+      const int was = J.cell_of[i];
       J.cen[i] = make_double4(c.x, c.y, c.z, 0.0);
+      J.cell_of[i] = cell_index(g, c.x, c.y, c.z);
       mx = max(mx, (unsigned long long)__double_as_longlong(sh));
-      atomicMax(&cmax[J.cell_of[i]], __float_as_uint(__double2float_ru(sh)));
+      atomicMax(&cmax[was], __float_as_uint(__double2float_ru(sh)));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -1254,36 +1271,65 @@ __global__ void __launch_bounds__(1024) k_centroids(const __grid_constant__ KmJo
     pass(1, a1, a2, cmax, b2);
     pass(2, cmax, b2, reinterpret_cast<unsigned*>(J.nbshift),
          reinterpret_cast<unsigned*>(J.nbshift) + kMaxCells);
-  } else if (empty) {
+    return;
+  }
+  int rk = st->rk;
+  const double4* from = J.cen;
+  if (empty) {
     // the members' lists of this iteration are done with: scratch
     rk = compact_empty(J.sums, rk, J.cen, J.members, J.start, warp_tot);
     if (threadIdx.x == 0) {
       st->rk = rk;
       st->reset_bounds = 1;
     }
+  } else if (update) {
+    from = J.sums;
   }
-  // the centroids into the cell grid
+  const bool own_cells = !update || empty;  // else block 1 writes them
   int* sc = reinterpret_cast<int*>(cmax);  // ncells + 1 counters
   for (int c = threadIdx.x; c <= ncells; c += blockDim.x) sc[c] = 0;
+  double3 held[kCenHeld];
+  int cell[kCenHeld];
+#pragma unroll
+  for (int q = 0; q < kCenHeld; ++q) {
+    const int j = threadIdx.x + q * 1024;
+    if (j < rk) {
+      const double4 c = from[j];
+      held[q] = make_double3(c.x, c.y, c.z);
+    }
+  }
   __syncthreads();
-  for (int j = threadIdx.x; j < rk; j += blockDim.x) {
-    const double4 c = J.cen[j];
-    const int ci = min(nc - 1, max(0, (int)floor(c.x * g.inv_h[0])));
-    const int cj = min(nc - 1, max(0, (int)floor(c.y * g.inv_h[1])));
-    const int ck = min(nc - 1, max(0, (int)floor(c.z * g.inv_h[2])));
-    const int id = ci + nc * (cj + nc * ck);
-    J.cell_of[j] = id;
+  auto count = [&](int j, double x, double y, double z) {
+    const int id = cell_index(g, x, y, z);
+    if (own_cells) J.cell_of[j] = id;
     atomicAdd(&sc[id + 1], 1);
+    return id;
+  };
+#pragma unroll
+  for (int q = 0; q < kCenHeld; ++q) {
+    const int j = threadIdx.x + q * 1024;
+    if (j < rk) cell[q] = count(j, held[q].x, held[q].y, held[q].z);
+  }
+  for (int j = threadIdx.x + kCenHeld * 1024; j < rk; j += 1024) {
+    const double4 c = from[j];
+    count(j, c.x, c.y, c.z);
   }
   __syncthreads();
   block_inclusive_scan(sc + 1, ncells, warp_tot);
   for (int c = threadIdx.x; c <= ncells; c += blockDim.x) J.cell_start[c] = sc[c];
   __syncthreads();
   // placement inside a cell is arbitrary: the search compares (d, index) pairs
-  for (int j = threadIdx.x; j < rk; j += blockDim.x) {
-    const int slot = atomicAdd(&sc[J.cell_of[j]], 1);
-    const double4 c = J.cen[j];
-    J.cell_cen[slot] = make_double4(c.x, c.y, c.z, (double)j);
+#pragma unroll
+  for (int q = 0; q < kCenHeld; ++q) {
+    const int j = threadIdx.x + q * 1024;
+    if (j < rk)
+      J.cell_cen[atomicAdd(&sc[cell[q]], 1)] =
+          make_double4(held[q].x, held[q].y, held[q].z, (double)j);
+  }
+  for (int j = threadIdx.x + kCenHeld * 1024; j < rk; j += 1024) {
+    const double4 c = from[j];
+    J.cell_cen[atomicAdd(&sc[cell_index(g, c.x, c.y, c.z)], 1)] =
+        make_double4(c.x, c.y, c.z, (double)j);
   }
 }
 
@@ -1740,7 +1786,7 @@ void launch_sums(const KmJobs<N>& J, const LoopDims& d, const LoopEnd& le, int* 
 
 template <int N>
 void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, cudaStream_t s) {
-  launch_early(k_centroids<N>, dim3(1, d.jobs), 1024, d.cells_smem, s, J, update);
+  launch_early(k_centroids<N>, dim3(2, d.jobs), 1024, d.cells_smem, s, J, update);
   launch_early(k_assign_warp<N>, dim3(d.assign, d.jobs), kAssignThreads, 0, s, J, update);
 }
 
