@@ -137,7 +137,7 @@ int isdf_kmeans_select(const isdf_domain_t* dom, const double* d_w, int mu, int 
 
 /* No counterpart in the reference (one system per call): the K-means
  * selections of `count` small systems (Ng <= 2^20, mu <= 512, cold start) in
- * one cooperative launch, a group of CTAs per system; each result equals
+ * the same launches, a row of blocks per system; each result equals
  * isdf_kmeans_select()'s on the same input, bit for bit. Arrays of `count`:
  * doms, d_w (device weights), mu, max_iter, piv (host int[Ng] each, fully
  * written), rk_eff / iters / npt (outputs). rand_seed as in

@@ -308,7 +308,7 @@ def kmeans_select(domain: Domain, d_w, mu: int, max_iter: int, rand_seed: int = 
 
 
 def kmeans_select_batch(domains, d_ws, mus, max_iters, rand_seed: int = -1, stream: int = 0):
-    """The K-means selections of several small systems in one launch; returns
+    """The K-means selections of several small systems in shared launches; returns
     a list of (piv int32[Ng], rk_eff, iterations, npt), one per system."""
     n = len(domains)
     doms = (_Domain * n)(*[d._c() for d in domains])

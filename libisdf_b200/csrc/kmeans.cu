@@ -460,7 +460,7 @@ __global__ void k_point_cells(const double* __restrict__ px, const double* __res
 // few warps in the sparse regions, which the launch then waited for) or, in the
 // first assignment, no seed. A launch late in a selection: 64 000 points and
 // 309 centroids 47 -> 10 us, 151 875 and 505 68 -> 18 us, 884 736 and 2979
-// 140 -> 52 us; the first assignment of the last 9200 -> 510 us.
+// 140 -> 55 us; the first assignment of the last 9200 -> 510 us.
 constexpr int kWarpCand = 128;   // candidates staged per warp
 
 // The warp's least float / largest float / largest non-negative float, by the
@@ -2151,7 +2151,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
 // costs little more than one; piv is the single selection's bit for bit, the
 // kernels being the same. Eight 36^3 systems with 256 centroids: 28.0 ms in one
 // cooperative launch of a group of CTAs per system (brute-force assignment,
-// group barriers between the phases), 8.2 ms here.
+// group barriers between the phases), 7.1 ms here.
 namespace {
 
 // The states and selections of a batch lie in one block, so that one copy
