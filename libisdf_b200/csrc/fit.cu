@@ -1013,7 +1013,7 @@ MixedBuffers carve_mixed(Arena& a, long long ng, int nstate, int rk, int slices)
   MixedBuffers b;
   const int kmax = round_up(nstate > rk ? nstate : rk, ozaki::BKB);
   const long long mp = round_up(ng, ozaki::BM);
-  const int np = round_up(rk, 128);
+  const int np = round_up(rk, 128) + 128;  // whole tiles of any width (at most 96 columns)
   b.PA = a.take<int8_t>((size_t)slices * mp * kmax);
   b.PB = a.take<int8_t>((size_t)slices * np * kmax);
   b.ea = a.take<int>((size_t)mp);
@@ -1069,7 +1069,7 @@ __global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ X
   }
 }
 
-// A side: R = 128 row blocks; B side: the stacked 64-column blocks.
+// A side: R = 128 row blocks; B side: the stacked tile_columns(S)-column blocks.
 // gathered = true: e holds the binade maxima from the producing GEMM's
 // epilogue, and the pass over X that k_row_exponent makes is saved.
 template <int S, bool B_SIDE>
@@ -1080,7 +1080,7 @@ int slice_operand(const double* X, long long rs, long long ks, int M, int K, int
   else k_row_exponent_b<<<(M + 31) / 32, 1024, 0, s>>>(X, rs, ks, M, K, e);
   dim3 g((unsigned)(kp / kSliceK), (unsigned)((mp + kSliceTile - 1) / kSliceTile));
   if (B_SIDE) {
-    k_slice<S, ozaki::BN, true><<<g, 256, 0, s>>>(X, rs, ks, M, K, mp, kp, e, P);
+    k_slice<S, ozaki::tile_columns(S), true><<<g, 256, 0, s>>>(X, rs, ks, M, K, mp, kp, e, P);
   } else if (rs == 1) {
     dim3 gr((unsigned)((mp + 255) / 256), (unsigned)(kp / 16));
     k_slice_rows<S><<<gr, 256, 0, s>>>(X, ks, M, K, mp, kp, e, P);
@@ -1107,7 +1107,8 @@ int ozaki_gemm(const MixedBuffers& b, const int* ea, int M, int N, int kp, doubl
   if (kp > ozaki::kMaxK)
     return record_error(ISDF_ERR_UNSUPPORTED, "mixed fit: K beyond the INT32-exact limit (16384)");
   const long long tiles =
-      (long long)((N + ozaki::BN - 1) / ozaki::BN) * ((M + ozaki::BM - 1) / ozaki::BM);
+      (long long)((N + ozaki::tile_columns(S) - 1) / ozaki::tile_columns(S)) *
+      ((M + ozaki::BM - 1) / ozaki::BM);
   if (tiles > 0x7fffffffLL) return record_error(ISDF_ERR_UNSUPPORTED, "mixed fit: too many tiles");
   static int sms[64] = {};
   if (dev >= 0 && dev < 64 && !sms[dev])
@@ -1137,7 +1138,7 @@ int fit_mixed_s(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* re
   StageEvents ev;
   ISDF_TRY(ev.create());
   const int mp = round_up(ng, ozaki::BM);
-  const int np = round_up(rk, 128);
+  const int np = round_up(rk, ozaki::tile_columns(S)), npz = round_up(rk, ozaki::tile_columns(SZ));
   ISDF_CUDA(cudaMemsetAsync(b.info, 0, 2 * sizeof(int), s));
   ISDF_CUDA(cudaMemsetAsync(mb.err, 0, sizeof(int), s));
   if (args.d_psimu) {
@@ -1158,7 +1159,7 @@ int fit_mixed_s(const FitArgs& args, Arena& arena, cudaStream_t s, FitResult* re
     const int kp = round_up(K, ozaki::BKB);
     ISDF_TRY((slice_operand<SZ, false>(args.d_psi + (long long)lo * ng, 1, ng, (int)ng, K, mp, kp,
                                       mb.ea, mb.PA, s)));
-    ISDF_TRY((slice_operand<SZ, true>(b.Bm + (size_t)lo * b.ldb, 1, b.ldb, rk, K, np, kp, mb.eb, mb.PB,
+    ISDF_TRY((slice_operand<SZ, true>(b.Bm + (size_t)lo * b.ldb, 1, b.ldb, rk, K, npz, kp, mb.eb, mb.PB,
                                      s)));
     if (same)
       ISDF_TRY((ozaki_gemm<SZ, 1, 0>(mb, mb.ea, (int)ng, rk, kp, args.d_theta, ng, mb.ez, s)));

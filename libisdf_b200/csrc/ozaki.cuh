@@ -14,20 +14,25 @@
 // Pairs with t + u >= S are dropped (the usual truncation of the scheme); the
 // dropped part is below (S+1)/4 * 254^{-S} of 2^{ea+eb} K, 2^-47 at S = 6.
 //
-// CTA tile: 128 rows x 64 output columns, S accumulators of 64 TMEM columns
+// CTA tile: 128 rows x BN output columns, S accumulators of BN TMEM columns
 // (column block d holds S_d). The B tile of a stage stacks the S slices along
-// N (row u*64 + j = slice u, column j), so that one A slice t meets all the B
-// slices it pairs with in a single MMA of N = (S - t) * 64 columns (split at
+// N (row u*BN + j = slice u, column j), so that one A slice t meets all the B
+// slices it pairs with in a single MMA of N = (S - t) * BN columns (split at
 // 256) whose accumulator starts at column block t: pair (t, u) lands in block
-// t + u. That is 2S - 1 or fewer MMAs per K step instead of S(S+1)/2 narrow
+// t + u. BN is 80 at six digits and 96 at five (480 TMEM columns), 64 otherwise:
+// a tile reads (128 + BN) S bytes per K from L2, about 10 TB/s in the triangular
+// products, and the operand reads fill 0.9 of the shared memory's pipe. With 64
+// columns everywhere (13 % and 22 % more reads per product, and a tenth more
+// reads of A by the MMAs) a fit of 373 248 rows, 4314 points and 864 states took
+// 155.5 ms against 150.0, its triangular products 47.8 + 54.4 against 44.1 + 51.2. That is 2S - 1 or fewer MMAs per K step instead of S(S+1)/2 narrow
 // ones, and the shared-memory reads per MMA fall accordingly.
 //
 // Operands arrive pre-tiled (the slicing kernel writes them so): for each
 // 128-row block of A and each 32-byte K block, the S slice tiles are one
 // contiguous S x 4 KB run in the canonical K-major no-swizzle UMMA layout
-// ([slice][16-byte K chunk][row][16 B]); for each 64-column block of B and K
-// block, the stacked tile is one contiguous S x 2 KB run
-// ([chunk][slice * 64 + column][16 B]). A pipeline stage is therefore two
+// ([slice][16-byte K chunk][row][16 B]); for each BN-column block of B and K
+// block, the stacked tile is one contiguous S x BN x 32-byte run
+// ([chunk][slice * BN + column][16 B]). A pipeline stage is therefore two
 // bulk copies (cp.async.bulk, no tensor map, no multicast) issued by one
 // thread and completing on the stage's mbarrier by transaction count.
 //
@@ -42,11 +47,10 @@
 // which releases them as soon as they are in registers and stores while the
 // next tile's MMAs run. The accumulators fill most of the TMEM, so that no MMA
 // runs while they are drained, and the drain bounds the short-K products: the
-// levels are read and converted two at a time, and the accumulators released
-// before the last two are converted. (With eight warps
+// accumulators are released before the last level is converted. (With eight warps
 // that converted every level by the conversion instruction first, Z C^T of
-// 216 000 x 1600, K = 224 took 2.53 ms against 1.73, and the triangular products
-// of that size 4.69 against 4.26.) Every wait is bounded: a timeout sets a shared abort
+// 216 000 x 1600, K = 224 took 2.53 ms against 1.73 with sixteen, and the
+// triangular products of that size 4.69 against 4.26, all on 64 columns.) Every wait is bounded: a timeout sets a shared abort
 // flag and *err, the other waiters give up on seeing the flag, and before
 // the CTA exits the kernel still waits (bounded) for its issued copies and
 // MMAs, freeing its TMEM last.
@@ -64,7 +68,9 @@
 namespace isdf_b200 {
 namespace ozaki {
 
-constexpr int BM = 128, BN = 64, BKB = 32;  // tile rows, tile columns, K bytes per stage
+constexpr int BM = 128, BKB = 32;  // tile rows, K bytes per stage
+// Tile columns: as many as S accumulators leave in TMEM, in multiples of 16.
+constexpr int tile_columns(int S) { return S == 5 ? 96 : S == 6 ? 80 : 64; }
 constexpr int kTmemCols = 512;
 constexpr int kEpiWarps = 16;  // four per TMEM lane quarter, each draining a quarter of the columns
 constexpr int kThreads = (kEpiWarps + 2) * 32;
@@ -76,6 +82,7 @@ constexpr int kNoExponent = (int)0x80808080;  // byte-fill sentinel: below every
 
 template <int S>
 struct Cfg {
+  static constexpr int BN = tile_columns(S);
   static constexpr int A_PLANE = BM * BKB;  // bytes of one slice's A tile per stage
   static constexpr int A_STAGE = S * A_PLANE;
   static constexpr int B_ROWS = S * BN;     // stacked B slices
@@ -137,6 +144,19 @@ __host__ __device__ __forceinline__ long long tiled_offset(long long blk, int kb
         "=r"(v[13]), "=r"(v[14]), "=r"(v[15])                                                \
       : "r"(addr))
 
+#define ISDF_TMEM_LD4(v, addr)                                                       \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"        \
+               : "=r"((v)[0]), "=r"((v)[1]), "=r"((v)[2]), "=r"((v)[3])                \
+               : "r"(addr))
+
+// A warp's CW columns of one level.
+template <int CW>
+__device__ __forceinline__ void tmem_load(uint32_t (&v)[CW], uint32_t addr) {
+  ISDF_TMEM_LD16(v, addr);
+#pragma unroll
+  for (int j = 16; j < CW; j += 4) ISDF_TMEM_LD4(v + j, addr + (uint32_t)j);
+}
+
 // 2^e: the bit pattern of a normal power of two (e in [-1022, 1023]), else
 // ldexp; the same value either way. The epilogue scales every element by two
 // of them, and the library call would cost a large share of its time.
@@ -154,6 +174,7 @@ __device__ __forceinline__ double int_value(uint32_t v) {
 
 // Tile id -> (first row, first column), grouped raster: kGroupM row blocks
 // by all column blocks per group.
+template <int BN>
 __device__ __forceinline__ void tile_origin(long long id, int num_m, int num_n, long long* m0,
                                             int* n0) {
   const long long per_group = (long long)kGroupM * num_n;
@@ -167,7 +188,7 @@ __device__ __forceinline__ void tile_origin(long long id, int num_m, int num_n, 
 
 // K range of a tile in BKB blocks (triangular B: KMODE 1 keeps k < n0 + BN,
 // KMODE 2 keeps k >= n0).
-template <int KMODE>
+template <int KMODE, int BN>
 __device__ __forceinline__ void tile_k_range(int n0, int kp, int* kb, int* nk) {
   int b = 0, e = kp;
   if (KMODE == 1) e = min(kp, ((n0 + BN + BKB - 1) / BKB) * BKB);
@@ -178,8 +199,8 @@ __device__ __forceinline__ void tile_k_range(int n0, int kp, int* kb, int* nk) {
 
 // EPI 0: C = value; 1: C = value^2; 2: C = C * value.
 // KMODE 0: full K; 1: B(k, n) = 0 for k > n (upper); 2: B(k, n) = 0 for k < n (lower).
-// A, B: pre-tiled slices (tiled_offset<S, 128, false> and <S, 64, true>) over
-// ceil(M/128) row blocks and ceil(N/64) column blocks, kp / BKB K blocks, zero
+// A, B: pre-tiled slices (tiled_offset<S, 128, false> and <S, BN, true>) over
+// ceil(M/128) row blocks and ceil(N/BN) column blocks, kp / BKB K blocks, zero
 // slices past the true K and the true M, N.
 // rowmax (optional, initialised to kNoExponent): atomicMax of ilogb over each
 // output row's nonzero values, i.e. the row exponent the next slicing needs.
@@ -196,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                  double* __restrict__ C, long long ldc, int* __restrict__ rowmax,
                  int* __restrict__ err) {
   using Cf = Cfg<S>;
-  constexpr int NST = Cf::NSTAGE;
+  constexpr int NST = Cf::NSTAGE, BN = Cf::BN;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
@@ -244,8 +265,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (long long id = blockIdx.x; id < tiles && !stop; id += gridDim.x) {
         long long m0;
         int n0, kb, nk;
-        tile_origin(id, num_m, num_n, &m0, &n0);
-        tile_k_range<KMODE>(n0, kp, &kb, &nk);
+        tile_origin<BN>(id, num_m, num_n, &m0, &n0);
+        tile_k_range<KMODE, BN>(n0, kp, &kb, &nk);
         const int8_t* Ab = A + tiled_offset<S, BM, false>(m0 / BM, kb / BKB, nkb, 0, 0, 0);
         const int8_t* Bb = B + tiled_offset<S, BN, true>(n0 / BN, kb / BKB, nkb, 0, 0, 0);
         for (int t = 0; t < nk; ++t) {
@@ -277,8 +298,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (long long id = blockIdx.x; id < tiles; id += gridDim.x, ++it) {
         long long m0;
         int n0, kb, nk;
-        tile_origin(id, num_m, num_n, &m0, &n0);
-        tile_k_range<KMODE>(n0, kp, &kb, &nk);
+        tile_origin<BN>(id, num_m, num_n, &m0, &n0);
+        tile_k_range<KMODE, BN>(n0, kp, &kb, &nk);
         // the epilogue must have drained the previous tile's accumulators
         if (it > 0 && !mbar_wait(acc_empty, (uint32_t)(it - 1) & 1u, abortp)) stop = true;
         asm volatile("tcgen05.fence::after_thread_sync;\n");
@@ -320,7 +341,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // warp w reads TMEM lanes 32 (w % 4) .. + 31 (its rows) and columns
     // [ (w / 4) CW, + CW )
     constexpr int CW = BN / (kEpiWarps / 4);
-    static_assert(CW == 16, "one TMEM load per level");
+    static_assert(CW == 16 || CW == 20 || CW == 24, "the TMEM loads of a level");
     const int q = warp & 3, c_lo = (warp >> 2) * CW;
     double w[S];  // 254^{-(d+2)}
     w[0] = 1.0 / (kBase * kBase);
@@ -330,8 +351,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (long long id = blockIdx.x; id < tiles; id += gridDim.x, ++it) {
       long long m0;
       int n0, kb, nk;
-      tile_origin(id, num_m, num_n, &m0, &n0);
-      tile_k_range<KMODE>(n0, kp, &kb, &nk);
+      tile_origin<BN>(id, num_m, num_n, &m0, &n0);
+      tile_k_range<KMODE, BN>(n0, kp, &kb, &nk);
       bool ready = mbar_wait(acc_full, (uint32_t)it & 1u, abortp) && *abortp == 0;
       if (!__all_sync(0xffffffffu, ready)) break;  // warp-uniform: tcgen05.ld is collective
       asm volatile("tcgen05.fence::after_thread_sync;\n");
@@ -339,36 +360,26 @@ __global__ void __launch_bounds__(kThreads, 1)
       const long long m = m0 + row;
       const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
       // per column the levels accumulate in order d = 0, 1, ...
-      constexpr int H = S - 2;  // levels converted before the release, two at a time
       double out[CW];
 #pragma unroll
       for (int j = 0; j < CW; ++j) out[j] = 0.0;
-      uint32_t v[2][CW];
+      uint32_t v[CW];
       if (nk > 0) {
 #pragma unroll
-        for (int d0 = 0; d0 < H; d0 += 2) {
-#pragma unroll
-          for (int d = d0; d < d0 + 2 && d < H; ++d)
-            ISDF_TMEM_LD16(v[d - d0], lane_base + (uint32_t)(d * BN + c_lo));
+        for (int d = 0; d < S; ++d) {
+          tmem_load(v, lane_base + (uint32_t)(d * BN + c_lo));
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+          if (d == S - 1) break;
 #pragma unroll
-          for (int d = d0; d < d0 + 2 && d < H; ++d)
-#pragma unroll
-            for (int j = 0; j < CW; ++j) out[j] = __fma_rn(int_value(v[d - d0][j]), w[d], out[j]);
+          for (int j = 0; j < CW; ++j) out[j] = __fma_rn(int_value(v[j]), w[d], out[j]);
         }
-#pragma unroll
-        for (int d = H; d < S; ++d)
-          ISDF_TMEM_LD16(v[d - H], lane_base + (uint32_t)(d * BN + c_lo));
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
       }
       // accumulators drained: the MMA thread may start the next tile
       asm volatile("tcgen05.fence::before_thread_sync;\n");
       mbar_arrive(acc_empty);
       if (nk > 0) {
 #pragma unroll
-        for (int d = H; d < S; ++d)
-#pragma unroll
-          for (int j = 0; j < CW; ++j) out[j] = __fma_rn(int_value(v[d - H][j]), w[d], out[j]);
+        for (int j = 0; j < CW; ++j) out[j] = __fma_rn(int_value(v[j]), w[S - 1], out[j]);
       }
       if (m < M) {
         const double sa = pow2(ea[m]);
@@ -404,6 +415,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 #undef ISDF_TMEM_LD16
+#undef ISDF_TMEM_LD4
 
 }  // namespace ozaki
 }  // namespace isdf_b200

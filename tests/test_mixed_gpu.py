@@ -85,3 +85,28 @@ def test_mixed_tile_edges(torch_cuda, n, rk, slices):
     cond = np.linalg.cond(cct + 1e-10 * np.trace(cct) / len(p) * np.eye(len(p)))
     err = np.linalg.norm(th[0] - th[1]) / np.linalg.norm(th[0])
     assert err <= cond * max(rk, 24) * 254.0 ** -min(slices, 5 if slices < 7 else 6) + cond * 1e-14
+
+
+@pytest.mark.parametrize("slices", [5, 6])
+@pytest.mark.parametrize("rk", [79, 80, 81, 96, 97, 161, 193])
+def test_mixed_wide_tiles(torch_cuda, rk, slices):
+    """The tiles of 96 and 80 columns that five and six digits take, around their
+    edges; the bound as in test_mixed_tile_edges."""
+    torch = torch_cuda
+    n = (9, 8, 8)
+    ng = n[0] * n[1] * n[2]
+    psi = np.asfortranarray(np.random.default_rng(rk).standard_normal((ng, 24)))
+    piv = np.zeros(ng, dtype=np.int32)
+    d_psi = torch.from_numpy(np.ascontiguousarray(psi.T)).cuda()
+    dom = isdf.Domain(length=(3.0, 4.0, 5.0), num_grid=n)
+    th = []
+    for prec in (isdf.PRECISION_FP64, isdf.PRECISION_MIXED):
+        d_theta = torch.zeros((rk, ng), dtype=torch.float64, device="cuda")
+        r = isdf.ISDF(d_psi, dom, 12, 24, 12, 12, 12, 12, rk, d_theta, piv, 5,
+                      options=isdf.Options(precision=prec, mixed_slices=slices))
+        th.append(d_theta.cpu().numpy())
+    p = piv[:r.rk_eff]
+    cct = (psi[p] @ psi[p].T) ** 2
+    cond = np.linalg.cond(cct + 1e-10 * np.trace(cct) / len(p) * np.eye(len(p)))
+    err = np.linalg.norm(th[0] - th[1]) / np.linalg.norm(th[0])
+    assert err <= cond * max(rk, 24) * 254.0 ** -5 + cond * 1e-14
