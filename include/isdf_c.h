@@ -191,6 +191,7 @@ int isdf_check_sampled(const isdf_domain_t* dom, const double* d_psi, int nocc, 
  * check forms from theta (src/common/checkcode.cpp:249-288) and the operator a
  * GW / RPA / TDDFT code applies to interpolation-point quantities. d_theta:
  * device Ng x rk, ld = Ng (read only); d_A: device rk x rk, column-major.
+ * Synchronous: d_A is complete on return, whatever the stream.
  * Device memory: rk x 2 (nx/2+1) ny nz doubles of half spectra (Si216: 44 GB)
  * plus two 128-column transform buffers. */
 int isdf_coulomb_matrix(const isdf_domain_t* dom, const double* d_theta, int rk, double* d_A,

@@ -569,8 +569,8 @@ int coulomb_matrix_workspace_bytes(const int* num_grid, int rk, size_t* bytes) {
   return ISDF_OK;
 }
 
-int coulomb_matrix_run(const int* num_grid, const double* length, const double* d_theta, int rk,
-                       double* d_A, Arena& arena, cudaStream_t s) {
+static int queue_coulomb_matrix(const int* num_grid, const double* length, const double* d_theta,
+                                int rk, double* d_A, Arena& arena, cudaStream_t s) {
   const int nx = num_grid[0], ny = num_grid[1], nz = num_grid[2];
   const long long ng = (long long)nx * ny * nz;
   const long long nh = (long long)(nx / 2 + 1) * ny * nz;
@@ -610,6 +610,17 @@ int coulomb_matrix_run(const int* num_grid, const double* length, const double* 
   const long long K = 2 * nh;  // the GEMM's depth is an int
   if (K > (1LL << 30)) return record_error(ISDF_ERR_UNSUPPORTED, "Coulomb matrix: grid too large");
   return dsyrk_store(rk, (int)K, Yz, ldy, d_A, rk, buf, (size_t)ng * kBatch, s);
+}
+
+// Finished when it returns, with an error too: the caller gives up the workspace
+// mutex then, and may not be able to wait on s (the library's own stream).
+int coulomb_matrix_run(const int* num_grid, const double* length, const double* d_theta, int rk,
+                       double* d_A, Arena& arena, cudaStream_t s) {
+  const int rc = queue_coulomb_matrix(num_grid, length, d_theta, rk, d_A, arena, s);
+  const cudaError_t done = cudaStreamSynchronize(s);
+  ISDF_TRY(rc);
+  ISDF_CUDA(done);
+  return ISDF_OK;
 }
 
 }  // namespace isdf_b200

@@ -220,3 +220,48 @@ def test_coulomb_matrix_kept_plans(torch_cuda):
     for t in threads:
         t.join()
     assert not fail
+
+
+@pytest.mark.parametrize("own", [False, True])
+def test_coulomb_matrix_is_done_on_return(torch_cuda, own):
+    """Calls back to back, on the library's stream or on two of the caller's, and a
+    fit behind one, all in the same workspace: every result may be read at once, and
+    none is overwritten by the next call's scratch. The same bits as a call alone."""
+    torch = torch_cuda
+    grid, rk, ns = (40, 40, 40), 600, 40
+    n, dom = 64000, isdf.Domain(length=(7.0, 8.0, 9.0), num_grid=grid)
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    ths = [torch.randn((rk, n), dtype=torch.float64, device="cuda", generator=gen)
+           for _ in range(2)]
+    psi = torch.randn((ns, n), dtype=torch.float64, device="cuda", generator=gen)
+    piv = np.arange(64, dtype=np.int32) * 997
+    win = (ns // 2, ns // 2, ns // 2, ns // 2, ns // 2)
+    streams = [torch.cuda.Stream().cuda_stream if own else 0 for _ in range(2)]
+
+    def empty(*shape):
+        return torch.full(shape, float("nan"), dtype=torch.float64, device="cuda")
+
+    alone = []
+    for th in ths:
+        A = empty(rk, rk)
+        torch.cuda.synchronize()
+        isdf.coulomb_matrix(dom, th, rk, A, stream=streams[0])
+        torch.cuda.synchronize()
+        alone.append(A.cpu())
+    fit_alone = empty(64, n)
+    torch.cuda.synchronize()
+    isdf.fit(psi, n, ns, *win, 64, piv, fit_alone, stream=streams[1])
+    torch.cuda.synchronize()
+
+    got, theta = [empty(rk, rk) for _ in ths], empty(64, n)
+    torch.cuda.synchronize()
+    for A, th, st in zip(got, ths, streams):
+        isdf.coulomb_matrix(dom, th, rk, A, stream=st)
+    host = [A.cpu() for A in got]  # on the current stream, which waits for neither
+    assert all(torch.equal(h, w) for h, w in zip(host, alone))
+    last = empty(rk, rk)
+    torch.cuda.synchronize()
+    isdf.coulomb_matrix(dom, ths[0], rk, last, stream=streams[0])
+    isdf.fit(psi, n, ns, *win, 64, piv, theta, stream=streams[1])
+    assert torch.equal(last.cpu(), alone[0])
+    assert torch.equal(theta, fit_alone)
