@@ -216,6 +216,7 @@ struct CheckBuffers {
   cufftDoubleComplex* spec;
   int* piv;
   double2* part;
+  int* err;  // a pipeline wait of a symmetric product ran out
 };
 
 constexpr int kBatch = 128;
@@ -235,7 +236,16 @@ CheckBuffers carve(Arena& a, long long ng, long long nh, int npair, int rk, int 
   b.cac = a.take<double>((size_t)npair * npair);
   b.piv = a.take<int>((size_t)rk);
   b.part = a.take<double2>((size_t)(nfit_tiles > kDiffBlocks ? nfit_tiles : kDiffBlocks));
+  b.err = a.take<int>(1);
   return b;
+}
+
+// The status of the symmetric products queued so far (waits for s).
+int products_done(const int* d_err, cudaStream_t s) {
+  int err = 0;
+  ISDF_TRY(read_back(&err, d_err, sizeof(int), s));
+  if (err) return record_error(ISDF_ERR_TIMEOUT, "Y Y^T: a pipeline wait timed out");
+  return ISDF_OK;
 }
 
 int fit_tiles(long long ng, int npair) {
@@ -349,14 +359,18 @@ int check_run(const CheckArgs& args, Arena& arena, cudaStream_t s, double* fit_e
 
   // (ij|V|kl) = Y Y^T; A = Yz Yz^T; T^T = C^T A; ISDF form = C^T T
   const size_t nscratch = (size_t)ng * kBatch;  // the transforms are done with rho
-  ISDF_TRY(dsyrk_store(npair, (int)(2 * nh), b.Y, npair, b.ijkl, npair, b.rho, nscratch, s));
-  ISDF_TRY(dsyrk_store(rk, (int)(2 * nh), b.Yz, rk, b.aux, rk, b.rho, nscratch, s));
+  ISDF_CUDA(cudaMemsetAsync(b.err, 0, sizeof(int), s));
+  ISDF_TRY(dsyrk_store(npair, (int)(2 * nh), b.Y, npair, b.ijkl, npair, b.rho, nscratch,
+                       b.err, s));
+  ISDF_TRY(dsyrk_store(rk, (int)(2 * nh), b.Yz, rk, b.aux, rk, b.rho, nscratch,
+                       b.err, s));
   ISDF_TRY(dgemm_store(npair, rk, rk, b.C, npair, b.aux, rk, b.Tt, npair, s));
   ISDF_TRY(dgemm_store(npair, npair, rk, b.C, npair, b.Tt, npair, b.cac, npair, s));
   k_diff_norms<<<kDiffBlocks, 256, 0, s>>>(b.ijkl, b.cac, (long long)npair * npair, b.part);
   ISDF_CHECK_LAUNCH();
   std::vector<double2> h(kDiffBlocks);
   ISDF_TRY(read_back(h.data(), b.part, sizeof(double2) * kDiffBlocks, s));
+  ISDF_TRY(products_done(b.err, s));
   double e2 = 0, x2 = 0;
   for (auto& v : h) {
     e2 += v.x;
@@ -382,6 +396,7 @@ struct SampledBuffers {
   cufftDoubleComplex* spec;
   int *piv, *pairs;
   double2* part;
+  int* err;
 };
 
 SampledBuffers carve_sampled(Arena& a, long long ng, long long nh, int ns, int rk) {
@@ -398,6 +413,7 @@ SampledBuffers carve_sampled(Arena& a, long long ng, long long nh, int ns, int r
   b.piv = a.take<int>((size_t)rk);
   b.pairs = a.take<int>((size_t)ns);
   b.part = a.take<double2>((size_t)kDiffBlocks);
+  b.err = a.take<int>(1);
   return b;
 }
 
@@ -475,10 +491,14 @@ int check_sampled_run(const CheckArgs& args, const int* pairs, int ns, Arena& ar
   }
   *fit_err = std::sqrt(fe2) / std::sqrt(fr2);
   const size_t nscratch = (size_t)ng * kBatch;  // the transforms are done with rho
-  ISDF_TRY(dsyrk_store(ns, (int)(2 * nh), b.Y, ns, b.E, ns, b.rho, nscratch, s));
-  ISDF_TRY(dsyrk_store(ns, (int)(2 * nh), b.Yf, ns, b.Ef, ns, b.rho, nscratch, s));
+  ISDF_CUDA(cudaMemsetAsync(b.err, 0, sizeof(int), s));
+  ISDF_TRY(dsyrk_store(ns, (int)(2 * nh), b.Y, ns, b.E, ns, b.rho, nscratch,
+                       b.err, s));
+  ISDF_TRY(dsyrk_store(ns, (int)(2 * nh), b.Yf, ns, b.Ef, ns, b.rho, nscratch,
+                       b.err, s));
   double ce2 = 0, cx2 = 0;
   ISDF_TRY(diff_norms(b.E, b.Ef, (long long)ns * ns, b.part, s, &ce2, &cx2));
+  ISDF_TRY(products_done(b.err, s));
   *coul_err = std::sqrt(ce2) / std::sqrt(cx2);
   return ISDF_OK;
 }
@@ -565,6 +585,7 @@ int coulomb_matrix_workspace_bytes(const int* num_grid, int rk, size_t* bytes) {
   a.take<double>((size_t)nh);
   a.take<double>((size_t)(rk + (rk & 1)) * 2 * nh);
   a.take<char>(plan->work);
+  a.take<int>(1);
   *bytes = a.off;
   return ISDF_OK;
 }
@@ -582,6 +603,7 @@ static int queue_coulomb_matrix(const int* num_grid, const double* length, const
   KeptPlan* plan = nullptr;
   ISDF_TRY(kept_plan(num_grid, &plan));
   char* work = arena.take<char>(plan->work);
+  int* err = arena.take<int>(1);
   if (arena.overflowed()) return record_error(ISDF_ERR_NOMEM, "Coulomb matrix: workspace too small");
   const double vol = length[0] * length[1] * length[2];
   k_weights<<<grid_for(nh, 256), 256, 0, s>>>(nx, ny, nz, length[0], length[1], length[2],
@@ -609,7 +631,9 @@ static int queue_coulomb_matrix(const int* num_grid, const double* length, const
   ISDF_CHECK_LAUNCH();
   const long long K = 2 * nh;  // the GEMM's depth is an int
   if (K > (1LL << 30)) return record_error(ISDF_ERR_UNSUPPORTED, "Coulomb matrix: grid too large");
-  return dsyrk_store(rk, (int)K, Yz, ldy, d_A, rk, buf, (size_t)ng * kBatch, s);
+  ISDF_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+  ISDF_TRY(dsyrk_store(rk, (int)K, Yz, ldy, d_A, rk, buf, (size_t)ng * kBatch, err, s));
+  return products_done(err, s);
 }
 
 // Finished when it returns, with an error too: the caller gives up the workspace

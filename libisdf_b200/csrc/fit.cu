@@ -161,10 +161,7 @@ __global__ void __launch_bounds__(WsN::THREADS, 3)
 
 __global__ void __launch_bounds__(256) k_syrk_reduce(int n, int splits,
                                                      const double* __restrict__ part,
-                                                     double* __restrict__ C, long long ldc,
-                                                     const int* __restrict__ err) {
-  // a pipeline wait ran out: the result says so itself (nothing is read back)
-  const bool bad = *err != 0;
+                                                     double* __restrict__ C, long long ldc) {
   constexpr int kTileN = WsN::BM * WsN::BN;
   int bi, bj;
   syrk_tile(blockIdx.x, &bi, &bj);
@@ -174,7 +171,6 @@ __global__ void __launch_bounds__(256) k_syrk_reduce(int n, int splits,
 #pragma unroll 8
     for (int s = 0; s < splits; ++s) v += p[(size_t)s * gridDim.x * kTileN];
     const int r = bi * WsN::BM + e % WsN::BM, c = bj * WsN::BN + e / WsN::BM;
-    if (bad) v = __longlong_as_double(0x7ff8000000000000LL);
     if (r < n && c < n && r >= c) {
       C[r + c * ldc] = v;
       C[c + r * ldc] = v;
@@ -681,22 +677,18 @@ static int syrk_splits(int tiles, int K, size_t cap) {
 }
 
 int dsyrk_store(int n, int K, const double* Y, long long ldy, double* C, long long ldc,
-                double* scratch, size_t scratch_doubles, cudaStream_t s) {
+                double* scratch, size_t scratch_doubles, int* err, cudaStream_t s) {
   const int nb = (n + WsN::BM - 1) / WsN::BM, tiles = nb * (nb + 1) / 2;
-  // one double of the scratch holds the pipeline's error flag
-  const size_t cap = scratch_doubles > 0 ? scratch_doubles - 1 : 0;
-  int splits = syrk_splits(tiles, K, cap);
+  int splits = syrk_splits(tiles, K, scratch_doubles);
   if (!vec2_ok(Y, ldy, Y, ldy) || ldy < n + (n & 1) || splits < 1)
     return dgemm_store(n, n, K, Y, ldy, Y, ldy, C, ldc, s);
   ISDF_TRY(set_smem_attrs());
   // whole pipeline stages per split
   const int kper = ((K + splits - 1) / splits + WsN::BK - 1) / WsN::BK * WsN::BK;
   splits = (K + kper - 1) / kper;
-  int* err = reinterpret_cast<int*>(scratch + cap);
-  ISDF_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
   k_syrk_ws<<<dim3(tiles, splits), WsN::THREADS, WsN::SMEM_BYTES, s>>>(n, K, kper, Y, ldy, scratch,
                                                                        err);
-  k_syrk_reduce<<<dim3(tiles, 16), 256, 0, s>>>(n, splits, scratch, C, ldc, err);
+  k_syrk_reduce<<<dim3(tiles, 16), 256, 0, s>>>(n, splits, scratch, C, ldc);
   ISDF_CHECK_LAUNCH();
   return ISDF_OK;
 }

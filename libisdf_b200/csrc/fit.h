@@ -42,10 +42,11 @@ int fit_mixed(const FitArgs& args, Arena& arena, cudaStream_t stream, FitResult*
 int dgemm_store(int M, int N, int K, const double* A, long long lda, const double* B,
                 long long ldb, double* C, long long ldc, cudaStream_t s);
 // C = Y Y^T (n x n, both triangles) for Y column-major n x K (ldy), through
-// `scratch`. The call does not synchronise: a bounded wait of its pipeline
-// that runs out makes C NaN. An odd n takes the fast path with ldy > n, even.
+// `scratch`. The call does not synchronise: a bounded wait of its pipeline that
+// runs out sets *err (device, cleared by the caller, who reads it back). An odd n
+// takes the fast path with ldy > n, even.
 int dsyrk_store(int n, int K, const double* Y, long long ldy, double* C, long long ldc,
-                double* scratch, size_t scratch_doubles, cudaStream_t s);
+                double* scratch, size_t scratch_doubles, int* err, cudaStream_t s);
 // timed = false skips the stage timers (no CUDA events are created); the
 // launches are then only queued on `stream` after the Cholesky check.
 int fit_fp64(const FitArgs& args, Arena& arena, cudaStream_t stream, FitResult* res,
