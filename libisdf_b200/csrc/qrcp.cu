@@ -437,11 +437,13 @@ __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
   }
   after_previous();  // (A does not change from step to step)
   if (st->step < 0 || st->done) return;
-  if (!tile.run(smem, Bc + m0, ld, (m_rem + 1) & ~1, Qm, ldq, p, p, err)) return;
+  const bool ok = tile.run(smem, Bc + m0, ld, (m_rem + 1) & ~1, Qm, ldq, p, p, err);
   if (T::producer()) return;
   Best v{0.0, INT_MAX};
+  // a warp whose wait ran out has no product, but the others may have theirs and
+  // wait for it at the barrier below
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; ok && h < 2; ++h) {
     const int r = warp * 16 + g + 8 * h;
     double s = 0.0;
     if (r < m_rem) {

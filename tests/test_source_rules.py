@@ -22,3 +22,20 @@ def test_symmetric_products_report_a_wait_that_ran_out():
     assert len(users) == 3  # the check, the sampled check, the Coulomb matrix
     for f in users:
         assert "products_done(" in f[f.rindex("dsyrk_store("):], f
+
+
+def test_no_warp_of_a_tile_leaves_before_a_barrier():
+    """A tile's run() gives each warp its own answer where a wait runs out: one may
+    have its product while another has none. A kernel with a barrier behind run()
+    must not let the second one return before it, or the first waits for ever."""
+    early = re.compile(r"if \(!\w+\.run\((?:[^;{]|\n)*?\)\)\s*return")
+    seen = 0
+    for name in ("fit.cu", "qrcp.cu", "check.cu"):
+        for f in _functions(name):
+            if ".run(" not in f:
+                continue
+            seen += 1
+            behind = f[f.index(".run("):]
+            if "bar.sync" in behind or "__syncthreads" in behind:
+                assert not early.search(f), f
+    assert seen >= 4
