@@ -1048,9 +1048,8 @@ __device__ __forceinline__ double fold_serial(const double* comp, int cnt, doubl
 // an upper bound on the distance it moved (rounded upward); an empty cluster is
 // recorded, and the update compacts (its own entry is not used then).
 __device__ __forceinline__ void store_centroid(const double4& s, int c,
-                                               const double4* __restrict__ cen,
-                                               double4* __restrict__ sums,
-                                               double* __restrict__ shift, KmState* st) {
+                                               const double4* cen, double4* sums, double* shift,
+                                               KmState* st) {
   if (!(s.w != 0.0)) {
     sums[c] = s;
     st->any_empty = 1;
@@ -1141,8 +1140,8 @@ __global__ void __launch_bounds__(kFoldThreads) k_segsum(const __grid_constant__
 // k-th empty place (ascending) takes the k-th non-empty cluster from the end.
 // One block finds both lists by prefix counts (holes, fillers: scratch of rk
 // entries each; sums: the centroids beside their counts); the loop by one thread took 1.8 ms at 3000 centroids.
-__device__ int compact_empty(const double4* __restrict__ sums, int rk, double4* __restrict__ cen,
-                             int* __restrict__ holes, int* __restrict__ fillers, int* warp_tot) {
+__device__ int compact_empty(const double4* sums, int rk, double4* cen, int* holes, int* fillers,
+                             int* warp_tot) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int per = (rk + 1023) / 1024;
   const int b0 = min(rk, tid * per), b1 = min(rk, b0 + per);

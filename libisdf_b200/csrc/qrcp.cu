@@ -94,9 +94,8 @@ __device__ __forceinline__ double tol3z() { return sqrt(1.1102230246251565e-16);
 // The downdate of one active column's residual norm with t = q_k . x_c, as
 // dgeqpf does it. Returns false (and lists the column) where the cancellation
 // test fires: that column's norm is recomputed exactly after this kernel.
-__device__ __forceinline__ bool downdate_norm(int c, double t, double* __restrict__ nu,
-                                              const double* __restrict__ nu0, QrState* st,
-                                              int* __restrict__ rec_list) {
+__device__ __forceinline__ bool downdate_norm(int c, double t, double* nu, const double* nu0,
+                                              QrState* st, int* rec_list) {
   const double v = nu[c];
   if (v == 0.0) return true;
   const double ratio = fabs(t) / v;
@@ -243,18 +242,18 @@ __global__ void __launch_bounds__(64) k_first_best(const double* __restrict__ nu
 }
 
 // ------------------------------------------------------------- one pivot step
+// The kernels of a step are resident while the one before them still writes
+// (launch_early), so nothing that a step writes is read through a __restrict__
+// pointer: read-only loads want data that no one changes in a kernel's lifetime.
 // The pivot: the best of the blocks' candidates, its bookkeeping (one thread) and
 // its feature vector x[i + j*p] = B(c, i) * A(c, j). The step number comes from the
 // device, so that every step is the same launches and they loop in a graph; past
 // the last step, or where no norm is left, it ends the loop.
 __global__ void __launch_bounds__(1024) k_pick(int kmax, int p, int ld, int nbest,
-                                               const Best* __restrict__ best,
-                                               const double* __restrict__ Ac,
-                                               const double* __restrict__ Bc,
-                                               int* __restrict__ pos, int* __restrict__ perm,
-                                               unsigned char* __restrict__ active,
-                                               int* __restrict__ sel, QrState* st,
-                                               double* __restrict__ x, const LoopEnd le) {
+                                               const Best* best, const double* __restrict__ Ac,
+                                               const double* __restrict__ Bc, int* pos, int* perm,
+                                               unsigned char* active, int* sel, QrState* st,
+                                               double* x, const LoopEnd le) {
   after_previous();
   __shared__ int col;
   __shared__ Best warp_v[32];
@@ -303,9 +302,8 @@ __global__ void __launch_bounds__(1024) k_pick(int kmax, int p, int ld, int nbes
 
 // cdot[l] = Q[:, l] . x for l < k: one block per l (a strided partial per
 // thread, then a fixed-order tree), so the sums do not depend on scheduling.
-__global__ void __launch_bounds__(256) k_qt_x(const double* __restrict__ Q, int m,
-                                              const double* __restrict__ x, const QrState* st,
-                                              double* __restrict__ cdot) {
+__global__ void __launch_bounds__(256) k_qt_x(const double* Q, int m, const double* x,
+                                              const QrState* st, double* cdot) {
   after_previous();
   const int l = blockIdx.x;
   if (l >= st->step) return;
@@ -329,11 +327,9 @@ __global__ void __launch_bounds__(256) k_qt_x(const double* __restrict__ Q, int 
 // order. Q streams from L2 (4.9 MB at 961 features and 640 pivots); eight rows a
 // block spread it over 121 SMs (32 rows left 31 SMs to do it: 5.3 us a pass).
 constexpr int kMinusRows = 8;
-__global__ void __launch_bounds__(32 * kMinusRows) k_x_minus_qc(const double* __restrict__ Q,
-                                                                int m,
-                                                                const double* __restrict__ cdot,
-                                                                const QrState* st,
-                                                                double* __restrict__ x) {
+__global__ void __launch_bounds__(32 * kMinusRows) k_x_minus_qc(const double* Q, int m,
+                                                                const double* cdot,
+                                                                const QrState* st, double* x) {
   after_previous();
   const int k = st->step;
   if (k <= 0) return;
@@ -356,8 +352,8 @@ __global__ void __launch_bounds__(32 * kMinusRows) k_x_minus_qc(const double* __
 }
 
 // q_k = x / |x| into Q[:, k] and into Qm (depth-major: Qm[i*ldq + j] = q[i + j*p]).
-__global__ void __launch_bounds__(1024) k_normalise(int p, int ldq, const double* __restrict__ x,
-                                                    QrState* st, double* __restrict__ Q,
+__global__ void __launch_bounds__(1024) k_normalise(int p, int ldq, const double* x, QrState* st,
+                                                    double* __restrict__ Q,
                                                     double* __restrict__ Qm) {
   after_previous();
   const int k = st->step;
@@ -411,9 +407,8 @@ template <int BN, int MINB>
 __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
     k_update_ws(const double* __restrict__ Ac, const double* __restrict__ Bc, int ntot, int ld,
                 int p, int ldq,
-                const double* __restrict__ Qm, const unsigned char* __restrict__ active,
-                const int* __restrict__ pos, double* __restrict__ nu, double* __restrict__ nu0,
-                QrState* st, int* __restrict__ rec_list, Best* __restrict__ best, int* err) {
+                const double* Qm, const unsigned char* active, const int* pos, double* nu,
+                double* nu0, QrState* st, int* rec_list, Best* best, int* err) {
   using T = UpdTile<BN>;
   extern __shared__ __align__(128) double smem[];
   const int m0 = blockIdx.x * T::BM;
@@ -483,13 +478,10 @@ __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
 // block leaves its candidate for the next pivot.
 __global__ void __launch_bounds__(256) k_recompute(const double* __restrict__ Ac,
                                                    const double* __restrict__ Bc, int ld, int p,
-                                                   const double* __restrict__ Q, int m, int kmax,
-                                                   const int* __restrict__ rec_list,
-                                                   const int* __restrict__ pos,
-                                                   double* __restrict__ nu,
-                                                   double* __restrict__ nu0, QrState* st,
-                                                   double* __restrict__ cbuf,
-                                                   Best* __restrict__ best) {
+                                                   const double* Q, int m, int kmax,
+                                                   const int* rec_list, const int* pos, double* nu,
+                                                   double* nu0, QrState* st, double* cbuf,
+                                                   Best* best) {
   after_previous();
   extern __shared__ double x[];  // m features
   __shared__ double red[8];

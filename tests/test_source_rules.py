@@ -39,3 +39,24 @@ def test_no_warp_of_a_tile_leaves_before_a_barrier():
             if "bar.sync" in behind or "__syncthreads" in behind:
                 assert not early.search(f), f
     assert seen >= 4
+
+
+def test_early_kernels_read_no_loop_data_as_read_only():
+    """A kernel that begins with after_previous() is resident while the kernel before it
+    still writes. A __restrict__ pointer lets the compiler read through the read-only
+    path, which is valid for data that does not change in the kernel's lifetime: the
+    loops' constant operands, and outputs that the kernel does not read."""
+    constant = {"qrcp.cu": {"Ac", "Bc"}, "kmeans.cu": {"pidx"}}
+    written = {"k_normalise": {"Q", "Qm"}}
+    early = 0
+    for name, allowed in constant.items():
+        for f in _functions(name):
+            is_early = "after_previous();" in f
+            early += is_early
+            if not is_early and ("__global__" in f or "__device__" not in f):
+                continue  # a kernel launched in order, or host code
+            kernel = re.search(r"(\w+)\s*\((?:const|int|double|bool)", f)
+            ok = allowed | written.get(kernel.group(1) if kernel else "", set())
+            found = set(re.findall(r"__restrict__\s+(\w+)", f))
+            assert found <= ok, (name, found - ok)
+    assert early == 12
