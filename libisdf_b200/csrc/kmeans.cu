@@ -754,9 +754,14 @@ __global__ void __launch_bounds__(32 * kScanWarps)
   after_previous();
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
-  if (st->done) return;
+  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+  if (st->done) {
+    // it may have stopped before the graph began (the iterations ahead of it)
+    if (first && (!live || atomicAdd(live, 0) <= 0)) end_loop(le);
+    return;
+  }
   if (!goes_on(J)) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (first) {
       st->done = 1;
       if (!live || atomicSub(live, 1) == 1) end_loop(le);
     }

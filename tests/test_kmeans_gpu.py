@@ -296,6 +296,41 @@ def test_select_empty_clusters_match_oracle(torch_cuda, ng, mu):
         assert np.array_equal(piv, piv_o)
 
 
+def test_select_ends_when_it_has_converged(torch_cuda):
+    """Selections that converge within the first few iterations, under a cap far
+    beyond them: no rounds of the loop behind the last iteration (the launches
+    counted by the solve; for a batch, of which no count comes back, its time:
+    a million rounds of idle launches take seconds)."""
+    import time
+
+    torch = torch_cuda
+    g = load_golden("small_s1s2")
+    psi, ng = g["psi"], tuple(int(x) for x in g["ng"])
+    dom = isdf.Domain(length=tuple(float(x) for x in g["length"]), num_grid=ng)
+    a = (int(g["nocc"]), psi.shape[1]) + tuple(int(g[k]) for k in ("nv1", "nc1", "nv2", "nc2"))
+    d_psi = torch.from_numpy(np.ascontiguousarray(psi.T)).cuda()
+    d_theta = torch.zeros((1, psi.shape[0]), dtype=torch.float64, device="cuda")
+    few = None
+    for cap in (20, 100000):
+        piv = np.zeros(psi.shape[0], dtype=np.int32)
+        torch.cuda.synchronize()
+        rep = isdf.ISDF(d_psi, dom, *a, 1, d_theta, piv, cap)
+        assert rep.rk_eff == 1 and rep.kmeans_iters <= 3
+        few = few or rep.kernel_launches
+        assert rep.kernel_launches <= few + 24  # a body of the loop or two more
+    n = psi.shape[0]
+    w = torch.zeros((3, n), dtype=torch.float64, device="cuda")
+    w[:, 3:3 + 40 * 5:5] = 1.0  # as many kept points as centroids
+    for mu in (40, 1):
+        isdf.kmeans_select_batch([dom] * 3, list(w), [mu] * 3, [20] * 3, rand_seed=1)
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        got = isdf.kmeans_select_batch([dom] * 3, list(w), [mu] * 3, [10 ** 6, 20, 10 ** 6],
+                                       rand_seed=1)
+        assert time.perf_counter() - t0 < 1.0
+        assert all(it <= 3 for _, _, it, _ in got)
+
+
 def test_select_batch_groups_match_single(torch_cuda):
     """A batch of more than one launch's systems, of different grids, mu and
     iteration caps (one stops at once, one has fewer kept points than mu):
