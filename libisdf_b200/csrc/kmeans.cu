@@ -18,6 +18,7 @@
 // Centroids: double4 (x, y, z, 0) in cen[], rk on the device in st->rk.
 #include <mutex>
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -1802,12 +1803,13 @@ void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, cudaStream
 template <int N>
 void build_loop(LoopGraph& loop, const KmJobs<N>& J, const LoopDims& d, int max_iter, int* live,
                 cudaStream_t s) {
-  const LoopEnd no_graph{0, 0, 0x7fffffff};
+  const LoopEnd no_graph{0, 0, INT_MAX};
   for (int it = 0; it < kAheadIters; ++it) {
     launch_sums(J, d, no_graph, live, s);
     launch_assign(J, d, 1, s);
   }
-  loop.build(s, kAheadIters + max_iter + 4 * kBodyIters, [&](const LoopEnd& le) {
+  const long long rounds = (long long)max_iter + kAheadIters + 4 * kBodyIters;
+  loop.build(s, (int)std::min(rounds, (long long)INT_MAX), [&](const LoopEnd& le) {
     for (int it = 0; it < kBodyIters; ++it) {
       launch_sums(J, d, le, live, s);
       launch_assign(J, d, 1, s);
@@ -2071,7 +2073,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   const size_t rec_bytes = sizeof(double4) * ((size_t)mu + 1);
   std::vector<size_t> rcounts(ranks, rec_bytes), rdispls(ranks);
   for (int q = 0; q < ranks; ++q) rdispls[q] = (size_t)q * rec_bytes;
-  const LoopEnd no_graph{0, 0, 0x7fffffff};
+  const LoopEnd no_graph{0, 0, INT_MAX};
   auto launch_chunk = [&]() -> int {
     for (int it = 0; it < kIterChunk; ++it) {
       launch_sums(jobs, dims, no_graph, nullptr, stream);
@@ -2265,7 +2267,7 @@ int select_group(const KmeansArgs* args, int count, Arena& arena, cudaStream_t s
   if (loop.exec) {
     ISDF_CUDA(cudaGraphLaunch(loop.exec, stream));
   } else {
-    const LoopEnd no_graph{0, 0, 0x7fffffff};
+    const LoopEnd no_graph{0, 0, INT_MAX};
     for (int left = nj, chunks = 0; left > 0; ++chunks) {
       if (chunks > max_iter / kIterChunk + 2)
         return record_error(ISDF_ERR_CUDA, "kmeans batch: loop did not stop");

@@ -331,6 +331,25 @@ def test_select_ends_when_it_has_converged(torch_cuda):
         assert all(it <= 3 for _, _, it, _ in got)
 
 
+@pytest.mark.parametrize("cap", [2 ** 31 - 1, 2 ** 31 - 9])
+def test_select_until_converged(torch_cuda, cap):
+    """The largest iteration caps an int holds: 'until it converges', alone and as one
+    request of a batch."""
+    torch = torch_cuda
+    ng, length = (13, 12, 11), (4.0, 5.0, 6.0)
+    dom = isdf.Domain(length=length, num_grid=ng)
+    w = np.random.default_rng(2).uniform(0.1, 1.0, ng[0] * ng[1] * ng[2])
+    piv_o, rk_o, it_o = port.kmeans(w, ng, length, 37, 100000)
+    assert it_o < 1000
+    d_w = torch.from_numpy(w).cuda()
+    piv, rk, it, _ = isdf.kmeans_select(dom, d_w, 37, cap, rand_seed=1)
+    assert (rk, it) == (rk_o, it_o) and np.array_equal(piv, piv_o)
+    got = isdf.kmeans_select_batch([dom] * 2, [d_w] * 2, [37] * 2, [3, cap], rand_seed=1)
+    assert got[1][1:3] == (rk_o, it_o) and np.array_equal(got[1][0], piv_o)
+    piv_o, rk_o, it_o = port.kmeans(w, ng, length, 37, 3)
+    assert got[0][1:3] == (rk_o, it_o) and np.array_equal(got[0][0], piv_o)
+
+
 def test_select_batch_groups_match_single(torch_cuda):
     """A batch of more than one launch's systems, of different grids, mu and
     iteration caps (one stops at once, one has fewer kept points than mu):
