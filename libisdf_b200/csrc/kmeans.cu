@@ -1801,13 +1801,14 @@ void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, cudaStream
 // first kAheadIters iterations are launched directly: they run while the host
 // builds the graph (150 us, in which a small selection's GPU was idle).
 template <int N>
-void build_loop(LoopGraph& loop, const KmJobs<N>& J, const LoopDims& d, int max_iter, int* live,
+int build_loop(LoopGraph& loop, const KmJobs<N>& J, const LoopDims& d, int max_iter, int* live,
                 cudaStream_t s) {
   const LoopEnd no_graph{0, 0, INT_MAX};
   for (int it = 0; it < kAheadIters; ++it) {
     launch_sums(J, d, no_graph, live, s);
     launch_assign(J, d, 1, s);
   }
+  ISDF_CHECK_LAUNCH();
   const long long rounds = (long long)max_iter + kAheadIters + 4 * kBodyIters;
   loop.build(s, (int)std::min(rounds, (long long)INT_MAX), [&](const LoopEnd& le) {
     for (int it = 0; it < kBodyIters; ++it) {
@@ -1815,6 +1816,7 @@ void build_loop(LoopGraph& loop, const KmJobs<N>& J, const LoopDims& d, int max_
       launch_assign(J, d, 1, s);
     }
   });
+  return ISDF_OK;
 }
 
 }  // namespace
@@ -2063,7 +2065,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   launch_assign(jobs, dims, 0, stream);
   ISDF_CHECK_LAUNCH();
   LoopGraph loop;
-  if (!shard) build_loop(loop, jobs, dims, args.max_iter, nullptr, stream);
+  if (!shard) ISDF_TRY(build_loop(loop, jobs, dims, args.max_iter, nullptr, stream));
   // Sharded: the rank folds its own points [lo, lo + cnt) (utility.cpp:813-822),
   // the ranks exchange their partial sums and changed-label counts (one
   // all-gather per iteration, utility.cpp:825-826,908-917), and every rank
@@ -2263,7 +2265,7 @@ int select_group(const KmeansArgs* args, int count, Arena& arena, cudaStream_t s
   launch_assign(jobs, dims, 0, stream);
   ISDF_CHECK_LAUNCH();
   LoopGraph loop;
-  build_loop(loop, jobs, dims, max_iter, live, stream);
+  ISDF_TRY(build_loop(loop, jobs, dims, max_iter, live, stream));
   if (loop.exec) {
     ISDF_CUDA(cudaGraphLaunch(loop.exec, stream));
   } else {

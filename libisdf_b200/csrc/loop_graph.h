@@ -61,7 +61,8 @@ struct LoopGraph {
     if (graph) cudaGraphDestroy(graph);
   }
 
-  // body(le) launches one body of the loop on s.
+  // body(le) launches one body of the loop on s. Launches before it have to be checked
+  // before it: errors that it meets are its own, and cleared (exec is null then).
   template <class F>
   void build(cudaStream_t s, int max_rounds, F body_launches) {
     LoopEnd le{0, 1, max_rounds};
@@ -85,7 +86,9 @@ struct LoopGraph {
     }
     if (ok) {
       body_launches(le);
-      ok = cudaStreamEndCapture(s, &body) == cudaSuccess;
+      // (a body that lacks a launch is no loop)
+      const bool launched = cudaGetLastError() == cudaSuccess;
+      ok = cudaStreamEndCapture(s, &body) == cudaSuccess && launched;
     }
     if (!ok || cudaGraphInstantiate(&exec, graph, 0ull) != cudaSuccess) exec = nullptr;
     (void)cudaGetLastError();  // a refused capture leaves an error to clear

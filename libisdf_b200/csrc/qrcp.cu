@@ -782,6 +782,7 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
     constexpr int kBodySteps = 4, kAheadSteps = 8;
     const LoopEnd ahead{0, 0, 0x7fffffff};
     for (int i = 0; i < std::min(kmax, kAheadSteps); ++i) step(ahead);  // while it is built
+    ISDF_CHECK_LAUNCH();
     LoopGraph loop;
     loop.build(s, kAheadSteps + kmax + 2 * kBodySteps, [&](const LoopEnd& le) {
       for (int i = 0; i < kBodySteps; ++i) step(le);
@@ -806,6 +807,7 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
   int err = 0;
   ISDF_TRY(read_back(&err, b.err, sizeof(int), s));
   if (err) return record_error(ISDF_ERR_TIMEOUT, "QRCP: an update pipeline wait timed out");
+  if (hst.k != kmax && !hst.done) return record_error(ISDF_ERR_CUDA, "QRCP: steps are missing");
   ISDF_TRY(read_back(idx.data(), b.idx, sizeof(int) * ntot, s));
   ISDF_TRY(read_back(perm.data(), b.perm, sizeof(int) * ntot, s));
   if (kmax > 0) ISDF_TRY(read_back(sel.data(), b.sel, sizeof(int) * kmax, s));

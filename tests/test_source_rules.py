@@ -60,3 +60,18 @@ def test_early_kernels_read_no_loop_data_as_read_only():
             found = set(re.findall(r"__restrict__\s+(\w+)", f))
             assert found <= ok, (name, found - ok)
     assert early == 12
+
+
+def test_launches_ahead_of_a_loop_are_checked():
+    """Building a loop's graph clears the errors it meets itself, so the launches issued
+    ahead of it are checked before it."""
+    seen = 0
+    for name in ("kmeans.cu", "qrcp.cu"):
+        for f in _functions(name):
+            if "loop.build(" not in f:
+                continue
+            seen += 1
+            ahead = f[:f.index("loop.build(")]
+            last = max(ahead.rfind("launch_assign("), ahead.rfind("step(ahead)"))
+            assert last >= 0 and "ISDF_CHECK_LAUNCH();" in ahead[last:], f
+    assert seen == 2
