@@ -1779,20 +1779,20 @@ struct LoopDims {
 // labels. Every kernel returns at once where the loop has stopped.
 template <int N>
 void launch_sums(const KmJobs<N>& J, const LoopDims& d, const LoopEnd& le, int* live,
-                 cudaStream_t s) {
+                 LoopQueue& q) {
   const size_t hist_smem = sizeof(int) * (size_t)d.mu;
   const size_t scatter_smem = sizeof(short) * kScatterWarps * (size_t)d.mu;
-  launch_early(k_hist<N>, dim3(d.tiles, d.jobs), 256, hist_smem, s, J, le);
-  launch_early(k_hist_scan<N>, dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, hist_smem, s, J, le,
+  launch_early(k_hist<N>, dim3(d.tiles, d.jobs), 256, hist_smem, q, J, le);
+  launch_early(k_hist_scan<N>, dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, hist_smem, q, J, le,
                live);
-  launch_early(k_scatter<N>, dim3(d.tiles, d.jobs), 32 * kScatterWarps, scatter_smem, s, J);
-  launch_early(k_segsum<N>, dim3(d.mu, d.jobs), kFoldThreads, 0, s, J);
+  launch_early(k_scatter<N>, dim3(d.tiles, d.jobs), 32 * kScatterWarps, scatter_smem, q, J);
+  launch_early(k_segsum<N>, dim3(d.mu, d.jobs), kFoldThreads, 0, q, J);
 }
 
 template <int N>
-void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, cudaStream_t s) {
-  launch_early(k_centroids<N>, dim3(2, d.jobs), 1024, d.cells_smem, s, J, update);
-  launch_early(k_assign_warp<N>, dim3(d.assign, d.jobs), kAssignThreads, 0, s, J, update);
+void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, LoopQueue& q) {
+  launch_early(k_centroids<N>, dim3(2, d.jobs), 1024, d.cells_smem, q, J, update);
+  launch_early(k_assign_warp<N>, dim3(d.assign, d.jobs), kAssignThreads, 0, q, J, update);
 }
 
 // The Lloyd loop as a graph with kBodyIters iterations per body: no iteration
@@ -1802,18 +1802,18 @@ void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, cudaStream
 // builds the graph (150 us, in which a small selection's GPU was idle).
 template <int N>
 int build_loop(LoopGraph& loop, const KmJobs<N>& J, const LoopDims& d, int max_iter, int* live,
-                cudaStream_t s) {
+               LoopQueue& q) {
   const LoopEnd no_graph{0, 0, INT_MAX};
   for (int it = 0; it < kAheadIters; ++it) {
-    launch_sums(J, d, no_graph, live, s);
-    launch_assign(J, d, 1, s);
+    launch_sums(J, d, no_graph, live, q);
+    launch_assign(J, d, 1, q);
   }
   ISDF_CHECK_LAUNCH();
   const long long rounds = (long long)max_iter + kAheadIters + 4 * kBodyIters;
-  loop.build(s, (int)std::min(rounds, (long long)INT_MAX), [&](const LoopEnd& le) {
+  loop.build((int)std::min(rounds, (long long)INT_MAX), [&](const LoopEnd& le, LoopQueue& body) {
     for (int it = 0; it < kBodyIters; ++it) {
-      launch_sums(J, d, le, live, s);
-      launch_assign(J, d, 1, s);
+      launch_sums(J, d, le, live, body);
+      launch_assign(J, d, 1, body);
     }
   });
   return ISDF_OK;
@@ -2062,10 +2062,11 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   LoopDims dims;
   dims.add(job, mu, pgrid);
   ISDF_TRY(set_kmeans_smem_attrs());
-  launch_assign(jobs, dims, 0, stream);
+  LoopQueue queue(stream);
+  launch_assign(jobs, dims, 0, queue);
   ISDF_CHECK_LAUNCH();
   LoopGraph loop;
-  if (!shard) ISDF_TRY(build_loop(loop, jobs, dims, args.max_iter, nullptr, stream));
+  if (!shard) ISDF_TRY(build_loop(loop, jobs, dims, args.max_iter, nullptr, queue));
   // Sharded: the rank folds its own points [lo, lo + cnt) (utility.cpp:813-822),
   // the ranks exchange their partial sums and changed-label counts (one
   // all-gather per iteration, utility.cpp:825-826,908-917), and every rank
@@ -2078,7 +2079,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   const LoopEnd no_graph{0, 0, INT_MAX};
   auto launch_chunk = [&]() -> int {
     for (int it = 0; it < kIterChunk; ++it) {
-      launch_sums(jobs, dims, no_graph, nullptr, stream);
+      launch_sums(jobs, dims, no_graph, nullptr, queue);
       if (shard) {
         k_shard_header<<<1, 1, 0, stream>>>(b.st, sb.send);
         ISDF_CHECK_LAUNCH();
@@ -2089,7 +2090,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
         k_shard_sums<<<grid_for(mu, 128), 128, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, b.cen,
                                                             b.sums, b.shift);
       }
-      launch_assign(jobs, dims, 1, stream);
+      launch_assign(jobs, dims, 1, queue);
       ISDF_CHECK_LAUNCH();
     }
     return ISDF_OK;
@@ -2262,10 +2263,11 @@ int select_group(const KmeansArgs* args, int count, Arena& arena, cudaStream_t s
   ISDF_CUDA(cudaMemcpyAsync(records, host.data(), host.size(), cudaMemcpyHostToDevice, stream));
   ISDF_CUDA(cudaMemcpyAsync(live, &nj, sizeof(int), cudaMemcpyHostToDevice, stream));
   ISDF_TRY(set_kmeans_smem_attrs());
-  launch_assign(jobs, dims, 0, stream);
+  LoopQueue queue(stream);
+  launch_assign(jobs, dims, 0, queue);
   ISDF_CHECK_LAUNCH();
   LoopGraph loop;
-  ISDF_TRY(build_loop(loop, jobs, dims, max_iter, live, stream));
+  ISDF_TRY(build_loop(loop, jobs, dims, max_iter, live, queue));
   if (loop.exec) {
     ISDF_CUDA(cudaGraphLaunch(loop.exec, stream));
   } else {
@@ -2274,8 +2276,8 @@ int select_group(const KmeansArgs* args, int count, Arena& arena, cudaStream_t s
       if (chunks > max_iter / kIterChunk + 2)
         return record_error(ISDF_ERR_CUDA, "kmeans batch: loop did not stop");
       for (int it = 0; it < kIterChunk; ++it) {
-        launch_sums(jobs, dims, no_graph, live, stream);
-        launch_assign(jobs, dims, 1, stream);
+        launch_sums(jobs, dims, no_graph, live, queue);
+        launch_assign(jobs, dims, 1, queue);
       }
       ISDF_CHECK_LAUNCH();
       ISDF_TRY(read_back(&left, live, sizeof(int), stream));

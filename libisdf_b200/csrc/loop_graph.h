@@ -1,10 +1,12 @@
-// A device-ended loop as a CUDA graph: a WHILE node whose body is captured from
-// the caller's launches and which a kernel of the body ends, so that no round of
+// A device-ended loop as a CUDA graph: a WHILE node whose body is made of the
+// caller's launches and which a kernel of the body ends, so that no round of
 // the loop waits for the host; and launches whose start overlaps the kernel before
 // them, for loops of many short kernels.
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <tuple>
 
 namespace isdf_b200 {
 
@@ -33,13 +35,47 @@ __device__ __forceinline__ void after_previous() {
   cudaTriggerProgrammaticLaunchCompletion();
 }
 
+// Where a loop's launches go: onto a stream, or behind one another into a graph. (A
+// graph is put together node by node, not captured: a capture on the caller's stream
+// would take in what other threads launch there meanwhile.)
+struct LoopQueue {
+  cudaStream_t stream = nullptr;
+  cudaGraph_t graph = nullptr;
+  cudaGraphNode_t last = nullptr;
+  cudaError_t status = cudaSuccess;  // the first failure (of a graph; a stream's stay with the runtime)
+
+  explicit LoopQueue(cudaStream_t s) : stream(s) {}
+  explicit LoopQueue(cudaGraph_t g) : graph(g) {}
+};
+
 // Launches k, a kernel that begins with after_previous(), so that its blocks are
-// set up while the kernel before it on the stream drains (also as an edge of a
-// captured graph). An ordinary launch starts them only when that kernel has
-// finished: about a microsecond on each kernel of a loop.
+// set up while the kernel before it on the queue drains. An ordinary launch starts
+// them only when that kernel has finished: about a microsecond on each kernel of a
+// loop.
 template <class... P, class... A>
-void launch_early(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+void launch_early(void (*k)(P...), dim3 grid, dim3 block, size_t smem, LoopQueue& q,
                   const A&... args) {
+  if (q.graph) {
+    if (q.status != cudaSuccess) return;
+    std::tuple<P...> values(static_cast<P>(args)...);
+    void* params[sizeof...(P)];
+    std::apply([&](auto&... v) { int i = 0; ((params[i++] = &v), ...); }, values);
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeKernel;
+    np.kernel.func = reinterpret_cast<void*>(k);
+    np.kernel.gridDim = grid;
+    np.kernel.blockDim = block;
+    np.kernel.sharedMemBytes = (unsigned)smem;
+    np.kernel.kernelParams = params;
+    cudaGraphEdgeData edge = {};
+    edge.from_port = cudaGraphKernelNodePortProgrammatic;
+    edge.type = cudaGraphDependencyTypeProgrammatic;
+    cudaGraphNode_t node = nullptr;
+    q.status = cudaGraphAddNode_v2(&node, q.graph, q.last ? &q.last : nullptr,
+                                   q.last ? &edge : nullptr, q.last ? 1 : 0, &np);
+    q.last = node;
+    return;
+  }
   cudaLaunchAttribute attr = {};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -47,7 +83,7 @@ void launch_early(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStrea
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
+  cfg.stream = q.stream;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   (void)cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
@@ -55,20 +91,20 @@ void launch_early(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStrea
 
 struct LoopGraph {
   cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;  // null on a stream that cannot be captured
+  cudaGraphExec_t exec = nullptr;  // null where the graph could not be made
   ~LoopGraph() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
   }
 
-  // body(le) launches one body of the loop on s. Launches before it have to be checked
-  // before it: errors that it meets are its own, and cleared (exec is null then).
+  // body(le, queue) launches one body of the loop on queue. Launches before it have
+  // to be checked before it: errors that it meets are its own, and cleared (exec is
+  // null then).
   template <class F>
-  void build(cudaStream_t s, int max_rounds, F body_launches) {
+  void build(int max_rounds, F body_launches) {
     LoopEnd le{0, 1, max_rounds};
     cudaGraphNodeParams np = {};
     cudaGraphNode_t node;
-    cudaGraph_t body = nullptr;
     np.type = cudaGraphNodeTypeConditional;
     np.conditional.type = cudaGraphCondTypeWhile;
     np.conditional.size = 1;
@@ -80,18 +116,12 @@ struct LoopGraph {
       ok = cudaGraphAddNode(&node, graph, nullptr, 0, &np) == cudaSuccess;
     }
     if (ok) {
-      body = np.conditional.phGraph_out[0];
-      ok = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0,
-                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-    }
-    if (ok) {
-      body_launches(le);
-      // (a body that lacks a launch is no loop)
-      const bool launched = cudaGetLastError() == cudaSuccess;
-      ok = cudaStreamEndCapture(s, &body) == cudaSuccess && launched;
+      LoopQueue body(np.conditional.phGraph_out[0]);
+      body_launches(le, body);
+      ok = body.status == cudaSuccess;
     }
     if (!ok || cudaGraphInstantiate(&exec, graph, 0ull) != cudaSuccess) exec = nullptr;
-    (void)cudaGetLastError();  // a refused capture leaves an error to clear
+    (void)cudaGetLastError();  // a refused step leaves an error to clear
   }
 };
 

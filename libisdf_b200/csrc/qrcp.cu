@@ -659,33 +659,33 @@ int set_update_attrs() {
 }
 
 template <int BN>
-void launch_update_bn(const QrBuffers& b, int ntot, int ld, int p, cudaStream_t s) {
+void launch_update_bn(const QrBuffers& b, int ntot, int ld, int p, LoopQueue& q) {
   using T = UpdTile<BN>;
   const unsigned grid = (unsigned)((ntot + T::BM - 1) / T::BM);
-  launch_early(k_update_ws<BN, UpdMinBlocks<BN>::value>, grid, T::THREADS, T::SMEM_BYTES, s, b.Ac,
+  launch_early(k_update_ws<BN, UpdMinBlocks<BN>::value>, grid, T::THREADS, T::SMEM_BYTES, q, b.Ac,
                b.Bc, ntot, ld, p, p + (p & 1), b.Qm, b.active, b.pos, b.nu, b.nu0, b.st,
                b.rec_list, b.best, b.err);
 }
 
 // The downdate on the narrowest warp-specialised tile that holds p columns
 // (p rounded up to a multiple of 8).
-void launch_update_ws(const QrBuffers& b, int ntot, int ld, int p, cudaStream_t s) {
+void launch_update_ws(const QrBuffers& b, int ntot, int ld, int p, LoopQueue& q) {
   switch ((p + 7) / 8) {
-    case 0: case 1: case 2: launch_update_bn<16>(b, ntot, ld, p, s); break;
-    case 3: launch_update_bn<24>(b, ntot, ld, p, s); break;
-    case 4: launch_update_bn<32>(b, ntot, ld, p, s); break;
-    case 5: launch_update_bn<40>(b, ntot, ld, p, s); break;
-    case 6: launch_update_bn<48>(b, ntot, ld, p, s); break;
-    case 7: launch_update_bn<56>(b, ntot, ld, p, s); break;
-    case 8: launch_update_bn<64>(b, ntot, ld, p, s); break;
-    case 9: launch_update_bn<72>(b, ntot, ld, p, s); break;
-    case 10: launch_update_bn<80>(b, ntot, ld, p, s); break;
-    case 11: launch_update_bn<88>(b, ntot, ld, p, s); break;
-    case 12: launch_update_bn<96>(b, ntot, ld, p, s); break;
-    case 13: launch_update_bn<104>(b, ntot, ld, p, s); break;
-    case 14: launch_update_bn<112>(b, ntot, ld, p, s); break;
-    case 15: launch_update_bn<120>(b, ntot, ld, p, s); break;
-    default: launch_update_bn<128>(b, ntot, ld, p, s); break;
+    case 0: case 1: case 2: launch_update_bn<16>(b, ntot, ld, p, q); break;
+    case 3: launch_update_bn<24>(b, ntot, ld, p, q); break;
+    case 4: launch_update_bn<32>(b, ntot, ld, p, q); break;
+    case 5: launch_update_bn<40>(b, ntot, ld, p, q); break;
+    case 6: launch_update_bn<48>(b, ntot, ld, p, q); break;
+    case 7: launch_update_bn<56>(b, ntot, ld, p, q); break;
+    case 8: launch_update_bn<64>(b, ntot, ld, p, q); break;
+    case 9: launch_update_bn<72>(b, ntot, ld, p, q); break;
+    case 10: launch_update_bn<80>(b, ntot, ld, p, q); break;
+    case 11: launch_update_bn<88>(b, ntot, ld, p, q); break;
+    case 12: launch_update_bn<96>(b, ntot, ld, p, q); break;
+    case 13: launch_update_bn<104>(b, ntot, ld, p, q); break;
+    case 14: launch_update_bn<112>(b, ntot, ld, p, q); break;
+    case 15: launch_update_bn<120>(b, ntot, ld, p, q); break;
+    default: launch_update_bn<128>(b, ntot, ld, p, q); break;
   }
 }
 
@@ -763,29 +763,30 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
   ISDF_CUDA(cudaMemsetAsync(b.best, 0, sizeof(Best) * (size_t)nbest, s));
   if (ublocks > 0) k_first_best<<<ublocks, 64, 0, s>>>(b.nu, ntot, ublocks, b.best);
   // One pivot step; the step number lives on the device.
-  auto step = [&](const LoopEnd& le) {
-    launch_early(k_pick, 1, 1024, 0, s, kmax, p, ld, nbest, b.best, b.Ac, b.Bc, b.pos, b.perm,
+  auto step = [&](const LoopEnd& le, LoopQueue& q) {
+    launch_early(k_pick, 1, 1024, 0, q, kmax, p, ld, nbest, b.best, b.Ac, b.Bc, b.pos, b.perm,
                  b.active, b.sel, b.st, b.x, le);
     for (int pass = 0; pass < 2; ++pass) {
-      launch_early(k_qt_x, kmax, 256, 0, s, b.Q, m, b.x, b.st, b.cdot);
-      launch_early(k_x_minus_qc, (m + kMinusRows - 1) / kMinusRows, 32 * kMinusRows, 0, s, b.Q, m,
+      launch_early(k_qt_x, kmax, 256, 0, q, b.Q, m, b.x, b.st, b.cdot);
+      launch_early(k_x_minus_qc, (m + kMinusRows - 1) / kMinusRows, 32 * kMinusRows, 0, q, b.Q, m,
                    b.cdot, b.st, b.x);
     }
-    launch_early(k_normalise, 1, 1024, 0, s, p, ldq, b.x, b.st, b.Q, b.Qm);
-    launch_update_ws(b, ntot, ld, p, s);
-    launch_early(k_recompute, kRecomputeGrid, 256, sizeof(double) * m, s, b.Ac, b.Bc, ld, p, b.Q,
+    launch_early(k_normalise, 1, 1024, 0, q, p, ldq, b.x, b.st, b.Q, b.Qm);
+    launch_update_ws(b, ntot, ld, p, q);
+    launch_early(k_recompute, kRecomputeGrid, 256, sizeof(double) * m, q, b.Ac, b.Bc, ld, p, b.Q,
                  m, kmax_cap, b.rec_list, b.pos, b.nu, b.nu0, b.st, b.rec_dots, b.best + ublocks);
   };
   if (kmax > 0) {
     // a graph that loops on the device: launched step by step, the nine launches
     // of a step took the host longer than the GPU at numPre = 31
     constexpr int kBodySteps = 4, kAheadSteps = 8;
-    const LoopEnd ahead{0, 0, 0x7fffffff};
-    for (int i = 0; i < std::min(kmax, kAheadSteps); ++i) step(ahead);  // while it is built
+    const LoopEnd ahead{0, 0, INT_MAX};
+    LoopQueue queue(s);
+    for (int i = 0; i < std::min(kmax, kAheadSteps); ++i) step(ahead, queue);  // while it is built
     ISDF_CHECK_LAUNCH();
     LoopGraph loop;
-    loop.build(s, kAheadSteps + kmax + 2 * kBodySteps, [&](const LoopEnd& le) {
-      for (int i = 0; i < kBodySteps; ++i) step(le);
+    loop.build(kAheadSteps + kmax + 2 * kBodySteps, [&](const LoopEnd& le, LoopQueue& body) {
+      for (int i = 0; i < kBodySteps; ++i) step(le, body);
     });
     if (loop.exec) {
       ISDF_CUDA(cudaGraphLaunch(loop.exec, s));
@@ -793,7 +794,7 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
       ISDF_TRY(read_back(&hst, b.st, sizeof(QrState), s));
     } else {
       for (int k = kAheadSteps; k < kmax; ++k) {
-        step(ahead);
+        step(ahead, queue);
         if ((k & 255) == 255) ISDF_CHECK_LAUNCH();
       }
     }

@@ -375,3 +375,56 @@ def test_select_batch_groups_match_single(torch_cuda):
         one = isdf.kmeans_select(d, w, mu, it, rand_seed=1)
         assert g[1:] == one[1:]
         assert np.array_equal(g[0], one[0])
+
+
+def test_loops_leave_the_callers_stream_to_others(torch_cuda):
+    """Another thread launches on the stream that a selection runs on (alone, batched, by
+    QRCP): what it launches runs once, and the selections stay what they are."""
+    import threading
+
+    torch = torch_cuda
+    ng = (24, 23, 22)
+    n = ng[0] * ng[1] * ng[2]
+    dom = isdf.Domain(length=(5.0, 6.0, 7.0), num_grid=ng)
+    w = np.random.default_rng(4).uniform(0.1, 1.0, n)
+    d_w = torch.from_numpy(w).cuda()
+    piv_o, rk_o, it_o = port.kmeans(w, ng, (5.0, 6.0, 7.0), 90, 40)
+    psi = torch.from_numpy(np.random.default_rng(5).standard_normal((16, n))).cuda()
+    theta = torch.empty((60, n), dtype=torch.float64, device="cuda")
+    st = torch.cuda.Stream()
+    opt = isdf.Options(stream=st.cuda_stream)
+    piv_q = np.zeros(n, dtype=np.int32)
+    torch.cuda.synchronize()
+    isdf.ISDF(psi, dom, 8, 16, 8, 8, 8, 8, 60, theta, piv_q, 1, "QRCP", options=opt)
+    added = torch.zeros(1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    stop, count, fail = threading.Event(), [0], []
+
+    def others():
+        try:
+            with torch.cuda.stream(st):
+                while not stop.wait(2e-5):
+                    added.add_(1)
+                    count[0] += 1
+        except Exception as e:  # noqa: BLE001 - reported by the assertion below
+            fail.append(repr(e))
+
+    t = threading.Thread(target=others)
+    t.start()
+    try:
+        for _ in range(30):
+            piv, rk, it, _ = isdf.kmeans_select(dom, d_w, 90, 40, rand_seed=1,
+                                                stream=st.cuda_stream)
+            assert (rk, it) == (rk_o, it_o) and np.array_equal(piv, piv_o)
+            got = isdf.kmeans_select_batch([dom] * 2, [d_w] * 2, [90] * 2, [40] * 2, rand_seed=1,
+                                           stream=st.cuda_stream)
+            assert all(g[1:3] == (rk_o, it_o) and np.array_equal(g[0], piv_o) for g in got)
+            piv = np.zeros(n, dtype=np.int32)
+            isdf.ISDF(psi, dom, 8, 16, 8, 8, 8, 8, 60, theta, piv, 1, "QRCP", options=opt)
+            assert np.array_equal(piv, piv_q)
+    finally:
+        stop.set()
+        t.join()
+    torch.cuda.synchronize()
+    assert not fail and count[0] > 0
+    assert int(added) == count[0]

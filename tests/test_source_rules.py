@@ -72,6 +72,6 @@ def test_launches_ahead_of_a_loop_are_checked():
                 continue
             seen += 1
             ahead = f[:f.index("loop.build(")]
-            last = max(ahead.rfind("launch_assign("), ahead.rfind("step(ahead)"))
+            last = max(ahead.rfind("launch_assign("), ahead.rfind("step(ahead"))
             assert last >= 0 and "ISDF_CHECK_LAUNCH();" in ahead[last:], f
     assert seen == 2
