@@ -18,10 +18,10 @@
 // Centroids: double4 (x, y, z, 0) in cen[], rk on the device in st->rk.
 #include <mutex>
 #include <algorithm>
-#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <optional>
 #include <type_traits>
 #include <vector>
 
@@ -39,9 +39,10 @@ namespace {
 
 constexpr int kTile = 2048;      // points per counting-sort tile (one walking warp each)
 constexpr int kFinalChunk = 4096;  // points per partial argmin chunk
-constexpr int kIterChunk = 8;    // Lloyd iterations launched between host checks (no graph)
-constexpr int kBodyIters = 2;    // Lloyd iterations per body of the loop's graph
-constexpr int kAheadIters = 4;   // Lloyd iterations launched before the graph is built
+constexpr int kIterChunk = 8;    // Lloyd iterations launched between host checks (sharded)
+constexpr int kBodyIters = 2;    // Lloyd iterations per graph of the loop
+constexpr int kSlackIters = 1;   // ... behind the running one when the next graph is launched
+constexpr int kAheadIters = 4;   // Lloyd iterations launched before the graph is made
 constexpr int kMaxCellsPerDim = 20;  // centroid cell grid of the pruned assignment
 constexpr int kMaxCells = kMaxCellsPerDim * kMaxCellsPerDim * kMaxCellsPerDim;
 
@@ -720,11 +721,14 @@ __device__ __forceinline__ bool goes_on(const KmJob& J) {
 // in increasing point index: the exact sequence of additions of
 // utility.cpp:816-822.
 template <int N>
-__global__ void __launch_bounds__(256) k_hist(const __grid_constant__ KmJobs<N> JS, const LoopEnd le) {
+__global__ void __launch_bounds__(256) k_hist(const __grid_constant__ KmJobs<N> JS, const LoopSignal sig) {
   after_previous();
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && ++st->rounds > le.max_rounds) end_loop(le);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const int rounds = ++st->rounds;
+    if (blockIdx.y == 0) loop_round(sig, rounds);
+  }
   if (st->done || !goes_on(J) || blockIdx.x * kTile >= J.f_n) return;
   extern __shared__ int sh[];
   const int rk = st->rk;
@@ -751,20 +755,15 @@ constexpr int kScanWarps = 16;
 
 template <int N>
 __global__ void __launch_bounds__(32 * kScanWarps)
-    k_hist_scan(const __grid_constant__ KmJobs<N> JS, const LoopEnd le, int* live) {
+    k_hist_scan(const __grid_constant__ KmJobs<N> JS, const LoopSignal sig, int* live) {
   after_previous();
   const KmJob& J = JS.j[N == 1 ? 0 : blockIdx.y];
   KmState* st = J.st;
-  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
-  if (st->done) {
-    // it may have stopped before the graph began (the iterations ahead of it)
-    if (first && (!live || atomicAdd(live, 0) <= 0)) end_loop(le);
-    return;
-  }
+  if (st->done) return;
   if (!goes_on(J)) {
-    if (first) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
       st->done = 1;
-      if (!live || atomicSub(live, 1) == 1) end_loop(le);
+      if (!live || atomicSub(live, 1) == 1) loop_over(sig);
     }
     return;
   }
@@ -1778,12 +1777,12 @@ struct LoopDims {
 // One Lloyd iteration is six launches: the sums, then the centroids and the
 // labels. Every kernel returns at once where the loop has stopped.
 template <int N>
-void launch_sums(const KmJobs<N>& J, const LoopDims& d, const LoopEnd& le, int* live,
+void launch_sums(const KmJobs<N>& J, const LoopDims& d, const LoopSignal& sig, int* live,
                  LoopQueue& q) {
   const size_t hist_smem = sizeof(int) * (size_t)d.mu;
   const size_t scatter_smem = sizeof(short) * kScatterWarps * (size_t)d.mu;
-  launch_early(k_hist<N>, dim3(d.tiles, d.jobs), 256, hist_smem, q, J, le);
-  launch_early(k_hist_scan<N>, dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, hist_smem, q, J, le,
+  launch_early(k_hist<N>, dim3(d.tiles, d.jobs), 256, hist_smem, q, J, sig);
+  launch_early(k_hist_scan<N>, dim3((d.mu + 31) / 32, d.jobs), 32 * kScanWarps, hist_smem, q, J, sig,
                live);
   launch_early(k_scatter<N>, dim3(d.tiles, d.jobs), 32 * kScatterWarps, scatter_smem, q, J);
   launch_early(k_segsum<N>, dim3(d.mu, d.jobs), kFoldThreads, 0, q, J);
@@ -1795,28 +1794,13 @@ void launch_assign(const KmJobs<N>& J, const LoopDims& d, int update, LoopQueue&
   launch_early(k_assign_warp<N>, dim3(d.assign, d.jobs), kAssignThreads, 0, q, J, update);
 }
 
-// The Lloyd loop as a graph with kBodyIters iterations per body: no iteration
-// waits for the host (reading the state back after every 8 iterations left the GPU
-// idle for 75 us each time, and the graph of 8 took twice as long to build). The
-// first kAheadIters iterations are launched directly: they run while the host
-// builds the graph (150 us, in which a small selection's GPU was idle).
+// One Lloyd iteration on a queue: a round of the selection's loop.
 template <int N>
-int build_loop(LoopGraph& loop, const KmJobs<N>& J, const LoopDims& d, int max_iter, int* live,
-               LoopQueue& q) {
-  const LoopEnd no_graph{0, 0, INT_MAX};
-  for (int it = 0; it < kAheadIters; ++it) {
-    launch_sums(J, d, no_graph, live, q);
+auto lloyd_round(const KmJobs<N>& J, const LoopDims& d, int* live) {
+  return [&J, &d, live](LoopQueue& q, const LoopSignal& sig) {
+    launch_sums(J, d, sig, live, q);
     launch_assign(J, d, 1, q);
-  }
-  ISDF_CHECK_LAUNCH();
-  const long long rounds = (long long)max_iter + kAheadIters + 4 * kBodyIters;
-  loop.build((int)std::min(rounds, (long long)INT_MAX), [&](const LoopEnd& le, LoopQueue& body) {
-    for (int it = 0; it < kBodyIters; ++it) {
-      launch_sums(J, d, le, live, body);
-      launch_assign(J, d, 1, body);
-    }
-  });
-  return ISDF_OK;
+  };
 }
 
 }  // namespace
@@ -2065,8 +2049,6 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   LoopQueue queue(stream);
   launch_assign(jobs, dims, 0, queue);
   ISDF_CHECK_LAUNCH();
-  LoopGraph loop;
-  if (!shard) ISDF_TRY(build_loop(loop, jobs, dims, args.max_iter, nullptr, queue));
   // Sharded: the rank folds its own points [lo, lo + cnt) (utility.cpp:813-822),
   // the ranks exchange their partial sums and changed-label counts (one
   // all-gather per iteration, utility.cpp:825-826,908-917), and every rank
@@ -2076,20 +2058,18 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   const size_t rec_bytes = sizeof(double4) * ((size_t)mu + 1);
   std::vector<size_t> rcounts(ranks, rec_bytes), rdispls(ranks);
   for (int q = 0; q < ranks; ++q) rdispls[q] = (size_t)q * rec_bytes;
-  const LoopEnd no_graph{0, 0, INT_MAX};
+  const LoopSignal no_signal{nullptr};
   auto launch_chunk = [&]() -> int {
     for (int it = 0; it < kIterChunk; ++it) {
-      launch_sums(jobs, dims, no_graph, nullptr, queue);
-      if (shard) {
-        k_shard_header<<<1, 1, 0, stream>>>(b.st, sb.send);
-        ISDF_CHECK_LAUNCH();
-        ISDF_TRY(shard->allgatherv(sb.send, rec_bytes, sb.recv, rcounts.data(), rdispls.data(),
-                                   stream));
-        k_shard_begin<<<1, 1, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, job.max_f,
-                                           args.max_iter);
-        k_shard_sums<<<grid_for(mu, 128), 128, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, b.cen,
-                                                            b.sums, b.shift);
-      }
+      launch_sums(jobs, dims, no_signal, nullptr, queue);
+      k_shard_header<<<1, 1, 0, stream>>>(b.st, sb.send);
+      ISDF_CHECK_LAUNCH();
+      ISDF_TRY(shard->allgatherv(sb.send, rec_bytes, sb.recv, rcounts.data(), rdispls.data(),
+                                 stream));
+      k_shard_begin<<<1, 1, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, job.max_f,
+                                         args.max_iter);
+      k_shard_sums<<<grid_for(mu, 128), 128, 0, stream>>>(b.st, sb.recv, ranks, mu + 1, b.cen,
+                                                          b.sums, b.shift);
       launch_assign(jobs, dims, 1, queue);
       ISDF_CHECK_LAUNCH();
     }
@@ -2097,9 +2077,21 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   };
   int chunks = 0;
   const int max_chunks = args.max_iter / kIterChunk + 2;
-  if (loop.exec) {
-    ISDF_CUDA(cudaGraphLaunch(loop.exec, stream));
+  std::optional<Loop> loop;  // (taken apart once the selection has been read back)
+  if (!shard) {
+    loop.emplace(stream);
+    const auto round = lloyd_round(jobs, dims, nullptr);
+    ISDF_TRY(loop->start(kAheadIters, round));
+    // the caller's piv is paged in while the loop runs
+    std::memset(args.piv, 0, sizeof(int) * (size_t)n);
+    ISDF_TRY(loop->finish((long long)args.max_iter + 1, kBodyIters, kSlackIters, round,
+                          [&](bool* over) -> int {
+                            ISDF_TRY(read_back(&hst, b.st, sizeof(KmState), stream));
+                            *over = hst.done != 0;
+                            return ISDF_OK;
+                          }));
   } else {
+    std::memset(args.piv, 0, sizeof(int) * (size_t)n);
     for (;;) {
       ISDF_TRY(launch_chunk());
       ISDF_TRY(read_back(&hst, b.st, sizeof(KmState), stream));
@@ -2134,8 +2126,6 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
     k_minloc<<<grid_for(rk, 128), 128, 0, stream>>>(sb.frecv, ranks, mu, b.st, b.sel);
   }
   ISDF_CHECK_LAUNCH();
-  // the caller's piv is paged in while the loop runs
-  std::memset(args.piv, 0, sizeof(int) * (size_t)n);
   std::vector<char> out(sizeof(KmState) + sizeof(int) * (size_t)mu);
   ISDF_TRY(read_back(out.data(), b.st, out.size(), stream));
   std::memcpy(&hst, out.data(), sizeof(KmState));
@@ -2266,23 +2256,16 @@ int select_group(const KmeansArgs* args, int count, Arena& arena, cudaStream_t s
   LoopQueue queue(stream);
   launch_assign(jobs, dims, 0, queue);
   ISDF_CHECK_LAUNCH();
-  LoopGraph loop;
-  ISDF_TRY(build_loop(loop, jobs, dims, max_iter, live, queue));
-  if (loop.exec) {
-    ISDF_CUDA(cudaGraphLaunch(loop.exec, stream));
-  } else {
-    const LoopEnd no_graph{0, 0, INT_MAX};
-    for (int left = nj, chunks = 0; left > 0; ++chunks) {
-      if (chunks > max_iter / kIterChunk + 2)
-        return record_error(ISDF_ERR_CUDA, "kmeans batch: loop did not stop");
-      for (int it = 0; it < kIterChunk; ++it) {
-        launch_sums(jobs, dims, no_graph, live, queue);
-        launch_assign(jobs, dims, 1, queue);
-      }
-      ISDF_CHECK_LAUNCH();
-      ISDF_TRY(read_back(&left, live, sizeof(int), stream));
-    }
-  }
+  Loop loop(stream);
+  const auto round = lloyd_round(jobs, dims, live);
+  ISDF_TRY(loop.start(kAheadIters, round));
+  ISDF_TRY(loop.finish((long long)max_iter + 1, kBodyIters, kSlackIters, round,
+                       [&](bool* over) -> int {
+                         int left = 0;
+                         ISDF_TRY(read_back(&left, live, sizeof(int), stream));
+                         *over = left <= 0;
+                         return ISDF_OK;
+                       }));
   k_final_near<kBatchJobs><<<dim3(grid_for(dims.mu, 4), dims.jobs), 128, 0, stream>>>(jobs);
   ISDF_CHECK_LAUNCH();
   ISDF_TRY(read_back(host.data(), records, host.size(), stream));

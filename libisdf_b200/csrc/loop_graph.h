@@ -1,26 +1,31 @@
-// A device-ended loop as a CUDA graph: a WHILE node whose body is made of the
-// caller's launches and which a kernel of the body ends, so that no round of
-// the loop waits for the host; and launches whose start overlaps the kernel before
-// them, for loops of many short kernels.
+// Loops of many short kernels that a kernel of the loop ends: rounds go to the device
+// a body's graph at a time, a little ahead of it, and the host watches their number
+// and the end in mapped memory, so that neither waits for the other; and launches
+// whose start overlaps the kernel before them.
 #pragma once
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <thread>
 #include <tuple>
+
+#include "errors.h"
+#include "readback.h"
 
 namespace isdf_b200 {
 
-// What the body's kernels get: with in_graph, end_loop() lets the running body be
-// the last. max_rounds bounds the loop whatever else happens: the kernel that
-// counts the rounds ends the loop beyond it.
-struct LoopEnd {
-  cudaGraphConditionalHandle handle;
-  int in_graph;
-  int max_rounds;
+// What a loop's kernels tell the host, in mapped host memory: words[0] the rounds
+// begun, words[1] whether the loop is over. nullptr: no one looks.
+struct LoopSignal {
+  int* words;
 };
 
-__device__ __forceinline__ void end_loop(const LoopEnd& le) {
-  if (le.in_graph) cudaGraphSetConditional(le.handle, 0);
+__device__ __forceinline__ void loop_round(const LoopSignal& sig, int rounds) {
+  if (sig.words) *static_cast<volatile int*>(sig.words) = rounds;
+}
+__device__ __forceinline__ void loop_over(const LoopSignal& sig) {
+  if (sig.words) *static_cast<volatile int*>(sig.words + 1) = 1;
 }
 
 // Begins a kernel launched by launch_early (what no kernel of the loop writes may
@@ -89,40 +94,96 @@ void launch_early(void (*k)(P...), dim3 grid, dim3 block, size_t smem, LoopQueue
   (void)cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
 }
 
-struct LoopGraph {
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;  // null where the graph could not be made
-  ~LoopGraph() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
+// Runs a loop's rounds on a stream. A round in which the loop is over returns at once
+// from each of its kernels, so a few too many do no harm.
+//
+// The rounds are launched as graphs of a body of them (a launch each would take the
+// host longer than the GPU where the kernels are small), the first few directly, while
+// the graph is made. A loop inside one graph, a WHILE node that a kernel ends, needs no
+// host and runs as fast; but destroying such a graph waits for the whole device, so that
+// a selection waited for every copy and every solve on other streams (75 ms behind a
+// 4 GB copy; an ordinary graph's 0.2 ms does not), and with it the copy of the previous
+// result to the host, which a pipeline of solves overlaps with the next one.
+class Loop {
+ public:
+  explicit Loop(cudaStream_t s) : queue_(s) {
+    progress_words(&host_, &sig_.words);
+    if (host_) host_[0] = host_[1] = 0;
+  }
+  ~Loop() {
+    // (no round may report once the words serve the next loop)
+    (void)cudaStreamSynchronize(queue_.stream);
+    if (exec_) cudaGraphExecDestroy(exec_);
+    if (graph_) cudaGraphDestroy(graph_);
+  }
+  Loop(const Loop&) = delete;
+  Loop& operator=(const Loop&) = delete;
+
+  // Launches the first `rounds` rounds; round(queue, signal) launches one.
+  template <class Round>
+  int start(int rounds, Round round) {
+    for (; launched_ < rounds; ++launched_) round(queue_, sig_);
+    ISDF_CHECK_LAUNCH();
+    return ISDF_OK;
   }
 
-  // body(le, queue) launches one body of the loop on queue. Launches before it have
-  // to be checked before it: errors that it meets are its own, and cleared (exec is
-  // null then).
-  template <class F>
-  void build(int max_rounds, F body_launches) {
-    LoopEnd le{0, 1, max_rounds};
-    cudaGraphNodeParams np = {};
-    cudaGraphNode_t node;
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    bool ok = cudaGraphCreate(&graph, 0) == cudaSuccess &&
-              cudaGraphConditionalHandleCreate(&le.handle, graph, 1,
-                                               cudaGraphCondAssignDefault) == cudaSuccess;
-    if (ok) {
-      np.conditional.handle = le.handle;
-      ok = cudaGraphAddNode(&node, graph, nullptr, 0, &np) == cudaSuccess;
+  // Launches the others, `per_body` at a time, until the loop is over or max_rounds
+  // have been launched: the next body when no more than `slack` rounds are behind the
+  // running one. stopped(&over) asks the device where no memory could be mapped.
+  template <class Round, class Stopped>
+  int finish(long long max_rounds, int per_body, int slack, Round round, Stopped stopped) {
+    if (launched_ >= max_rounds || over()) return ISDF_OK;
+    build(per_body, round);
+    constexpr int kAskRounds = 8;
+    long long idle = 0, ask = launched_ + kAskRounds;  // rounds known to have run; to ask at
+    unsigned polls = 0;
+    while (launched_ < max_rounds && !over()) {
+      if (host_) {
+        if (launched_ - std::max<long long>(idle, host_[0]) > slack) {
+          // every so often, what the stream says: an error, or that nothing runs
+          if ((++polls & 4095) == 0) {
+            const cudaError_t e = cudaStreamQuery(queue_.stream);
+            if (e == cudaSuccess) idle = launched_;
+            else if (e != cudaErrorNotReady) ISDF_CUDA(e);
+          }
+          if ((polls & 63) == 0) std::this_thread::yield();
+          continue;
+        }
+      } else if (launched_ >= ask) {
+        bool done = false;
+        ISDF_TRY(stopped(&done));
+        if (done) break;
+        ask = launched_ + kAskRounds;
+      }
+      if (exec_) ISDF_CUDA(cudaGraphLaunch(exec_, queue_.stream));
+      else for (int i = 0; i < per_body; ++i) round(queue_, sig_);
+      launched_ += per_body;
+      ISDF_CHECK_LAUNCH();
     }
+    return ISDF_OK;
+  }
+
+ private:
+  bool over() const { return host_ && host_[1] != 0; }
+
+  template <class Round>
+  void build(int rounds, Round round) {
+    bool ok = cudaGraphCreate(&graph_, 0) == cudaSuccess;
     if (ok) {
-      LoopQueue body(np.conditional.phGraph_out[0]);
-      body_launches(le, body);
+      LoopQueue body(graph_);
+      for (int i = 0; i < rounds; ++i) round(body, sig_);
       ok = body.status == cudaSuccess;
     }
-    if (!ok || cudaGraphInstantiate(&exec, graph, 0ull) != cudaSuccess) exec = nullptr;
+    if (!ok || cudaGraphInstantiate(&exec_, graph_, 0ull) != cudaSuccess) exec_ = nullptr;
     (void)cudaGetLastError();  // a refused step leaves an error to clear
   }
+
+  LoopQueue queue_;
+  LoopSignal sig_{nullptr};
+  volatile int* host_ = nullptr;
+  cudaGraph_t graph_ = nullptr;
+  cudaGraphExec_t exec_ = nullptr;  // null where the graph could not be made
+  long long launched_ = 0;          // rounds
 };
 
 }  // namespace isdf_b200

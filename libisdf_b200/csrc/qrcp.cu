@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(1024) k_pick(int kmax, int p, int ld, int nbes
                                                const Best* best, const double* __restrict__ Ac,
                                                const double* __restrict__ Bc, int* pos, int* perm,
                                                unsigned char* active, int* sel, QrState* st,
-                                               double* x, const LoopEnd le) {
+                                               double* x, const LoopSignal sig) {
   after_previous();
   __shared__ int col;
   __shared__ Best warp_v[32];
@@ -285,10 +285,10 @@ __global__ void __launch_bounds__(1024) k_pick(int kmax, int p, int ld, int nbes
       } else {
         if (run) st->done = 1;
         st->step = -1;
-        end_loop(le);
+        loop_over(sig);
       }
       st->nrec = 0;
-      if (++st->rounds > le.max_rounds) end_loop(le);
+      loop_round(sig, ++st->rounds);
     }
   }
   __syncthreads();
@@ -763,9 +763,9 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
   ISDF_CUDA(cudaMemsetAsync(b.best, 0, sizeof(Best) * (size_t)nbest, s));
   if (ublocks > 0) k_first_best<<<ublocks, 64, 0, s>>>(b.nu, ntot, ublocks, b.best);
   // One pivot step; the step number lives on the device.
-  auto step = [&](const LoopEnd& le, LoopQueue& q) {
+  auto step = [&](LoopQueue& q, const LoopSignal& sig) {
     launch_early(k_pick, 1, 1024, 0, q, kmax, p, ld, nbest, b.best, b.Ac, b.Bc, b.pos, b.perm,
-                 b.active, b.sel, b.st, b.x, le);
+                 b.active, b.sel, b.st, b.x, sig);
     for (int pass = 0; pass < 2; ++pass) {
       launch_early(k_qt_x, kmax, 256, 0, q, b.Q, m, b.x, b.st, b.cdot);
       launch_early(k_x_minus_qc, (m + kMinusRows - 1) / kMinusRows, 32 * kMinusRows, 0, q, b.Q, m,
@@ -776,28 +776,17 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
     launch_early(k_recompute, kRecomputeGrid, 256, sizeof(double) * m, q, b.Ac, b.Bc, ld, p, b.Q,
                  m, kmax_cap, b.rec_list, b.pos, b.nu, b.nu0, b.st, b.rec_dots, b.best + ublocks);
   };
+  Loop loop(s);
   if (kmax > 0) {
-    // a graph that loops on the device: launched step by step, the nine launches
-    // of a step took the host longer than the GPU at numPre = 31
-    constexpr int kBodySteps = 4, kAheadSteps = 8;
-    const LoopEnd ahead{0, 0, INT_MAX};
-    LoopQueue queue(s);
-    for (int i = 0; i < std::min(kmax, kAheadSteps); ++i) step(ahead, queue);  // while it is built
-    ISDF_CHECK_LAUNCH();
-    LoopGraph loop;
-    loop.build(kAheadSteps + kmax + 2 * kBodySteps, [&](const LoopEnd& le, LoopQueue& body) {
-      for (int i = 0; i < kBodySteps; ++i) step(le, body);
-    });
-    if (loop.exec) {
-      ISDF_CUDA(cudaGraphLaunch(loop.exec, s));
-      // (the graph must outlive its launch)
+    // launched step by step, the nine launches of a step took the host longer than the
+    // GPU at numPre = 31
+    constexpr int kBodySteps = 4, kSlackSteps = 2, kAheadSteps = 8;
+    ISDF_TRY(loop.start(std::min(kmax, kAheadSteps), step));
+    ISDF_TRY(loop.finish(kmax, kBodySteps, kSlackSteps, step, [&](bool* over) -> int {
       ISDF_TRY(read_back(&hst, b.st, sizeof(QrState), s));
-    } else {
-      for (int k = kAheadSteps; k < kmax; ++k) {
-        step(ahead, queue);
-        if ((k & 255) == 255) ISDF_CHECK_LAUNCH();
-      }
-    }
+      *over = hst.done != 0;
+      return ISDF_OK;
+    }));
     launches += 8 * kmax + 1;
   }
   ISDF_CHECK_LAUNCH();

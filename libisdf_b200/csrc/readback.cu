@@ -20,8 +20,11 @@ struct Mailbox {
   void* dev = nullptr;
   size_t cap = 0;
   bool enabled = true;
+  int* words = nullptr;  // progress_words()
+  int* words_dev = nullptr;
   ~Mailbox() {
     if (host) cudaFreeHost(host);
+    if (words) cudaFreeHost(words);
   }
 };
 
@@ -33,6 +36,28 @@ constexpr size_t kMinMailbox = 64 << 10;
 
 void set_readback_mailbox(bool on) { tl_mailbox.enabled = on; }
 bool readback_mailbox() { return tl_mailbox.enabled; }
+
+void progress_words(volatile int** host, int** dev) {
+  Mailbox& m = tl_mailbox;
+  *host = nullptr;
+  *dev = nullptr;
+  if (!m.enabled) return;
+  if (!m.words) {
+    void *h = nullptr, *d = nullptr;
+    if (cudaHostAlloc(&h, 2 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) ==
+        cudaSuccess) {
+      if (cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess) {
+        m.words = static_cast<int*>(h);
+        m.words_dev = static_cast<int*>(d);
+      } else {
+        cudaFreeHost(h);
+      }
+    }
+    (void)cudaGetLastError();  // a refused mapping: the caller asks the device
+  }
+  *host = m.words;
+  *dev = m.words_dev;
+}
 
 int read_back(void* dst, const void* dsrc, size_t bytes, cudaStream_t s) {
   if (bytes == 0) return ISDF_OK;

@@ -21,6 +21,11 @@ namespace isdf_b200 {
 // Synchronises s.
 int read_back(void* dst, const void* dsrc, size_t bytes, cudaStream_t s);
 
+// Two words of mapped host memory, the calling thread's own, that running kernels
+// write and the host looks at: their host and device addresses, or null where none
+// can be mapped (or the mailbox is off).
+void progress_words(volatile int** host, int** dev);
+
 // Thread-local: false makes read_back use cudaMemcpyAsync (no host allocation).
 void set_readback_mailbox(bool on);
 bool readback_mailbox();

@@ -428,3 +428,38 @@ def test_loops_leave_the_callers_stream_to_others(torch_cuda):
     torch.cuda.synchronize()
     assert not fail and count[0] > 0
     assert int(added) == count[0]
+
+
+def test_loops_do_not_wait_for_other_streams(torch_cuda):
+    """A selection (alone, batched, by QRCP) returns while a long copy to the host runs on
+    another stream: a pipeline of solves overlaps the previous result's copy with the next
+    solve. The copy takes tens of milliseconds, the calls a few."""
+    torch = torch_cuda
+    ng = (24, 23, 22)
+    n = ng[0] * ng[1] * ng[2]
+    dom = isdf.Domain(length=(5.0, 6.0, 7.0), num_grid=ng)
+    d_w = torch.from_numpy(np.random.default_rng(4).uniform(0.1, 1.0, n)).cuda()
+    psi = torch.from_numpy(np.random.default_rng(5).standard_normal((16, n))).cuda()
+    theta = torch.empty((60, n), dtype=torch.float64, device="cuda")
+    src = torch.zeros(3 << 30, dtype=torch.uint8, device="cuda")
+    dst = torch.empty(3 << 30, dtype=torch.uint8, pin_memory=True)
+    copies = torch.cuda.Stream()
+    calls = {
+        "single": lambda: isdf.kmeans_select(dom, d_w, 90, 40, rand_seed=1),
+        "batch": lambda: isdf.kmeans_select_batch([dom] * 2, [d_w] * 2, [90] * 2, [40] * 2,
+                                                  rand_seed=1),
+        "qrcp": lambda: isdf.ISDF(psi, dom, 8, 16, 8, 8, 8, 8, 60, theta,
+                                  np.zeros(n, dtype=np.int32), 1, "QRCP"),
+    }
+    for call in calls.values():
+        call()  # the workspace, the kernels
+    torch.cuda.synchronize()
+    for name, call in calls.items():
+        done = torch.cuda.Event()
+        with torch.cuda.stream(copies):
+            dst.copy_(src, non_blocking=True)
+            done.record()
+        call()
+        running = not done.query()
+        torch.cuda.synchronize()
+        assert running, name
