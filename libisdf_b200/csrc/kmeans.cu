@@ -938,7 +938,8 @@ __device__ __forceinline__ double pow2_bits(int e) {
 // (c rounded to the ulp grid), unless c's remainder is exactly half an ulp
 // (a tie, which depends on acc's parity): those steps, binade crossings and
 // accumulators outside [2^-900, 2^900] (where the scaling by the ulp would
-// not be exact) are taken one at a time; the rest are jumped. One thread runs
+// not be exact) are taken one at a time, as is a c that is not >= 0; the rest
+// are jumped. One thread runs
 // it on the critical path of its cluster, so the scaling is by powers of two
 // built from the exponent bits: the library's ilogb and ldexp and two
 // divisions per binade took most of the 52 us of a fold with a 5551-point
@@ -948,7 +949,8 @@ __device__ double repeat_add(double acc, double c, long long m) {
   while (m > 0) {
     if (c == 0.0) return radd(acc, 0.0);
     const int e = (int)((__double_as_longlong(acc) >> 52) & 0x7ff) - 1023;
-    if (e < -900 || e > 900 || c >= pow2_bits(e)) {
+    // (a negative c is no weight, but the caller's to give: it must not jump back)
+    if (e < -900 || e > 900 || !(c >= 0.0 && c < pow2_bits(e))) {
       acc = radd(acc, c);
       --m;
       continue;

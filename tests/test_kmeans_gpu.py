@@ -463,3 +463,20 @@ def test_loops_do_not_wait_for_other_streams(torch_cuda):
         running = not done.query()
         torch.cuda.synchronize()
         assert running, name
+
+
+def test_select_ends_with_a_negative_tail(torch_cuda):
+    """Weights are products of squares, but the caller's: a negative one at grid point 0,
+    which the zero tail repeats in its cluster's sum, must not keep the sum from ending.
+    One centroid, so that the sums decide nothing else."""
+    torch = torch_cuda
+    ng, length = (9, 8, 7), (4.0, 5.0, 6.0)
+    n = ng[0] * ng[1] * ng[2]
+    w = np.random.default_rng(1).uniform(0.1, 1.0, n)
+    w[n // 2:] = 0.0
+    w[0] = -2.0 ** -12
+    piv_o, rk_o, it_o = port.kmeans(w, ng, length, 1, 10)
+    piv, rk, it, _ = isdf.kmeans_select(isdf.Domain(length=length, num_grid=ng),
+                                        torch.from_numpy(w).cuda(), 1, 10, rand_seed=1)
+    assert (rk, it) == (rk_o, it_o)
+    assert np.array_equal(piv, piv_o)
