@@ -515,8 +515,8 @@ int check_sampled_run(const CheckArgs& args, const int* pairs, int ns, Arena& ar
 // 2.2 ms at 40^3 and 320 columns), so the plans of the last kPlans grids are kept
 // per device. Their work areas are not: each call gives the plan one from its own
 // workspace, so that a kept plan holds no device buffer and two calls share no more
-// than they share of the workspace. Callers hold the device's workspace mutex;
-// isdf_release_workspace() gives the plans back.
+// than they share of the workspace. Callers hold the device's workspace mutex, under
+// which every call finishes; isdf_release_workspace() gives the plans back.
 namespace {
 constexpr int kPlans = 4;
 struct KeptPlan {
@@ -542,9 +542,8 @@ int kept_plan(const int* num_grid, KeptPlan** out) {
     if (p.used < oldest->used) oldest = &p;
   }
   KeptPlan& p = *oldest;
-  if (p.used) {
+  if (p.used) {  // (its last call has finished)
     p.used = 0;
-    (void)cudaDeviceSynchronize();  // a transform may still be running
     cufftDestroy(p.h);
   }
   int dims[3] = {num_grid[2], num_grid[1], num_grid[0]};
@@ -565,7 +564,6 @@ int kept_plan(const int* num_grid, KeptPlan** out) {
 
 void release_coulomb_plans(int dev) {
   if (dev < 0 || dev >= 64) return;
-  (void)cudaDeviceSynchronize();
   for (KeptPlan& p : g_plans[dev])
     if (p.used) {
       p.used = 0;

@@ -902,8 +902,8 @@ constexpr int kSliceK = 32;     // K bytes per slicing tile
 // Row-scaled slicing of an M x K FP64 operand, element (m, k) at
 // X[m*rs + k*ks], into S int8 slices written in the pre-tiled layout of the
 // Ozaki GEMM (ozaki::tiled_offset: blocks of R rows, 32-byte K blocks; the A
-// side unstacked with R = 128, the B side stacked with R = 64), rows padded to
-// mp and K to kp with zeros, and exponents e[m] (|x| 2^-e < 1/2).
+// side unstacked with R = 128, the B side stacked with R = tile_columns(S)),
+// rows padded to mp and K to kp with zeros, and exponents e[m] (|x| 2^-e < 1/2).
 __device__ __forceinline__ int exponent_of(double mx) { return mx > 0.0 ? ilogb(mx) + 2 : 0; }
 
 // Contiguous rows (rs = 1, the A side's ng of them): a thread per row.

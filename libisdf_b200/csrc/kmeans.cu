@@ -59,7 +59,7 @@ struct KmState {
   unsigned long long maxshift_bits;  // largest centroid move of this iteration (bit pattern)
   unsigned long long searches;       // assignments that ran the cell search (all iterations)
   unsigned ticket;  // blocks of k_hist_scan that have finished
-  int rounds;       // loop bodies run
+  int rounds;       // iterations launched and begun, with those after the end
 };
 
 // ---------------------------------------------------------------- weight
@@ -2055,8 +2055,8 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   // the ranks exchange their partial sums and changed-label counts (one
   // all-gather per iteration, utility.cpp:825-826,908-917), and every rank
   // combines them in the same order, so that all ranks hold the same
-  // centroids without a broadcast. Its collectives keep the loop out of a
-  // CUDA graph.
+  // centroids without a broadcast. Its collectives keep its iterations out of
+  // the loop's graphs.
   const size_t rec_bytes = sizeof(double4) * ((size_t)mu + 1);
   std::vector<size_t> rcounts(ranks, rec_bytes), rdispls(ranks);
   for (int q = 0; q < ranks; ++q) rdispls[q] = (size_t)q * rec_bytes;
@@ -2137,7 +2137,7 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
   res->rk_eff = piv_from_selection(sel, n, args.piv);
   res->iters = hst.s;
   res->search_frac = (double)hst.searches / ((double)cnt * (hst.s + 1));
-  // filter, points, cells, first assignment, the loop's bodies, the final
+  // filter, points, cells, first assignment, the loop's rounds, the final
   // search, and the reads through the mapped mailbox
   res->launches = 4 + 4 + (am.g2p ? 1 : 0) + hst.rounds * (shard ? 9 : 6) + (am.brick && !shard ? 1 : 2) +
                   (readback_mailbox() ? chunks + 2 : 0);
@@ -2147,12 +2147,12 @@ int kmeans_select(const KmeansArgs& args, Arena& arena, cudaStream_t stream, Kme
 // ===================================================================== batched small selections
 // Several small K-means selections at once (the serving loop's batches of small
 // requests): the kernels of kmeans_select with a job per blockIdx.y, up to
-// kBatchJobs of them, in one loop graph that ends when the last job has. A
+// kBatchJobs of them, in one loop that ends when the last job has. A
 // small selection alone is bound by the latency of its launches, so a batch
 // costs little more than one; piv is the single selection's bit for bit, the
 // kernels being the same. Eight 36^3 systems with 256 centroids: 28.0 ms in one
 // cooperative launch of a group of CTAs per system (brute-force assignment,
-// group barriers between the phases), 7.1 ms here.
+// group barriers between the phases), 6.9 ms here.
 namespace {
 
 // The states and selections of a batch lie in one block, so that one copy

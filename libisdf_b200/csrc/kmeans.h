@@ -8,7 +8,9 @@
 
 namespace isdf_b200 {
 
-constexpr int kKmeansMaxMu = 12288;  // per-tile label histograms live in 48 KB of shared memory
+// A tile's counts by label live in shared memory: 48 KB for the histogram, 192 KB for
+// the scatter's eight warps of 16-bit counts.
+constexpr int kKmeansMaxMu = 12288;
 
 struct KmeansArgs {
   const double* d_w;  // device weight[ng]

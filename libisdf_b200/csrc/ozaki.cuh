@@ -24,7 +24,8 @@
 // products, and the operand reads fill 0.9 of the shared memory's pipe. With 64
 // columns everywhere (13 % and 22 % more reads per product, and a tenth more
 // reads of A by the MMAs) a fit of 373 248 rows, 4314 points and 864 states took
-// 155.5 ms against 150.0, its triangular products 47.8 + 54.4 against 44.1 + 51.2. That is 2S - 1 or fewer MMAs per K step instead of S(S+1)/2 narrow
+// 155.5 ms against 150.0, its triangular products 47.8 + 54.4 against 44.1 + 51.2.
+// The stacked B takes 2S - 1 or fewer MMAs per K step instead of S(S+1)/2 narrow
 // ones, and the shared-memory reads per MMA fall accordingly.
 //
 // Operands arrive pre-tiled (the slicing kernel writes them so): for each

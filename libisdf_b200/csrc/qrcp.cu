@@ -247,13 +247,13 @@ __global__ void __launch_bounds__(64) k_first_best(const double* __restrict__ nu
 // pointer: read-only loads want data that no one changes in a kernel's lifetime.
 // The pivot: the best of the blocks' candidates, its bookkeeping (one thread) and
 // its feature vector x[i + j*p] = B(c, i) * A(c, j). The step number comes from the
-// device, so that every step is the same launches and they loop in a graph; past
+// device, so that every step is the same launches and one graph serves them all; past
 // the last step, or where no norm is left, it ends the loop.
 __global__ void __launch_bounds__(1024) k_pick(int kmax, int p, int ld, int nbest,
                                                const Best* best, const double* __restrict__ Ac,
                                                const double* __restrict__ Bc, int* pos, int* perm,
-                                               unsigned char* active, int* sel, QrState* st,
-                                               double* x, const LoopSignal sig) {
+                                               unsigned char* active, QrState* st, double* x,
+                                               const LoopSignal sig) {
   after_previous();
   __shared__ int col;
   __shared__ Best warp_v[32];
@@ -278,7 +278,6 @@ __global__ void __launch_bounds__(1024) k_pick(int kmax, int p, int ld, int nbes
         pos[ck] = q;
         pos[c] = k;
         active[c] = 0;
-        sel[k] = c;
         col = c;
         st->k = k + 1;
         st->step = k;
@@ -588,7 +587,7 @@ std::vector<double> gaussian_draws(int m, int n) {
 
 struct QrBuffers {
   double *A, *B, *norm2, *Ac, *Bc, *nu, *nu0, *Q, *Qm, *x, *cdot, *G1, *G2, *rec_dots;
-  int *idx, *pos, *perm, *sel, *tile_cnt, *rec_list;
+  int *idx, *pos, *perm, *tile_cnt, *rec_list;
   Best* best;  // candidates: one per 64 columns, then one per recompute block
   unsigned char* active;
   QrState* st;
@@ -615,7 +614,6 @@ QrBuffers carve(Arena& a, long long n, int p, int k1, int k2, int kmax) {
   b.idx = a.take<int>((size_t)n);
   b.pos = a.take<int>((size_t)n);
   b.perm = a.take<int>((size_t)n);
-  b.sel = a.take<int>((size_t)kmax);
   b.tile_cnt = a.take<int>((size_t)ntiles);
   b.rec_list = a.take<int>((size_t)n);
   b.rec_dots = a.take<double>((size_t)kRecomputeGrid * kmax);
@@ -765,7 +763,7 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
   // One pivot step; the step number lives on the device.
   auto step = [&](LoopQueue& q, const LoopSignal& sig) {
     launch_early(k_pick, 1, 1024, 0, q, kmax, p, ld, nbest, b.best, b.Ac, b.Bc, b.pos, b.perm,
-                 b.active, b.sel, b.st, b.x, sig);
+                 b.active, b.st, b.x, sig);
     for (int pass = 0; pass < 2; ++pass) {
       launch_early(k_qt_x, kmax, 256, 0, q, b.Q, m, b.x, b.st, b.cdot);
       launch_early(k_x_minus_qc, (m + kMinusRows - 1) / kMinusRows, 32 * kMinusRows, 0, q, b.Q, m,
@@ -792,7 +790,7 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
   ISDF_CHECK_LAUNCH();
 
   // piv = MGIdx[pivots], then the remaining kept columns in pivoted order, then 0
-  std::vector<int> idx(ntot), perm(ntot), sel(kmax);
+  std::vector<int> idx(ntot), perm(ntot);
   ISDF_TRY(read_back(&hst, b.st, sizeof(QrState), s));
   int err = 0;
   ISDF_TRY(read_back(&err, b.err, sizeof(int), s));
@@ -800,14 +798,13 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
   if (hst.k != kmax && !hst.done) return record_error(ISDF_ERR_CUDA, "QRCP: steps are missing");
   ISDF_TRY(read_back(idx.data(), b.idx, sizeof(int) * ntot, s));
   ISDF_TRY(read_back(perm.data(), b.perm, sizeof(int) * ntot, s));
-  if (kmax > 0) ISDF_TRY(read_back(sel.data(), b.sel, sizeof(int) * kmax, s));
   std::memset(args.piv, 0, sizeof(int) * (size_t)n);
   for (int j = 0; j < ntot; ++j) args.piv[j] = idx[perm[j]];
   res->steps = kmax;
   res->num_pre = p;
   res->recomputes = hst.total_rec;
   res->done_early = hst.done;
-  res->launches = launches + (readback_mailbox() ? (kmax > 0 ? 6 : 5) : 0);
+  res->launches = launches + (readback_mailbox() ? (ntot > 0 ? 5 : 3) : 0);
   return ISDF_OK;
 }
 

@@ -4,8 +4,7 @@
 // A caller that consumes theta on the host streams the previous solve's theta
 // out while the next one runs; a cudaMemcpyAsync device-to-host of a few bytes
 // queues on the same copy engine behind those large copies, and the solve
-// waits for them at every one of its host synchronisation points (one per
-// K-means iteration chunk). read_back() instead launches a one-block kernel
+// waits for them at every one of its host synchronisation points. read_back() instead launches a one-block kernel
 // that stores the bytes into mapped pinned host memory (over the bus, no copy
 // engine), synchronises the stream and copies them out. The mapped buffer is
 // per host thread and grows on demand; a thread that must not allocate (the

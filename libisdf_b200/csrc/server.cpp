@@ -20,8 +20,8 @@
 // Small K-means requests (Ng <= 2^20, mu <= 512, cold start) queue apart: a
 // batcher thread takes up to batch_small of them at once, computes their
 // weights and runs all their selections together (kmeans_select_batch: the
-// kernels of one selection with a system per block row, up to kBatchJobs of
-// them in one loop graph), then puts them back at the head of the main queue,
+// kernels of one selection with a system per block row, up to kKmeansBatchGroup
+// of them in one loop), then puts them back at the head of the main queue,
 // where the slots run their fits. A small solve is latency bound (about a
 // hundred Lloyd iterations of six small kernels each), so running many of them
 // in the same launches raises the rate at which they are served.
