@@ -39,7 +39,9 @@ size_t kmeans_workspace_bytes(long long ng, int mu);
 // serving loop's batches): cold start only, ng <= kKmeansBatchMaxNg,
 // mu <= kKmeansBatchMaxMu. piv and the results equal kmeans_select()'s for each
 // request. The groups run one after the other in the same workspace, which
-// holds the largest group's requests.
+// holds the largest group's requests. Groups of 8 / 16 / 32 take 13.4 / 10.4 / 10.4 ms
+// for 16 systems of 36^3 points with 256 centroids and 27.0 / 21.7 / 19.9 ms for 32; 32
+// wants twice the workspace.
 constexpr int kKmeansBatchGroup = 16;
 constexpr int kKmeansBatchMaxMu = 512;
 constexpr long long kKmeansBatchMaxNg = 1 << 20;

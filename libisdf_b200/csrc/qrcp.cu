@@ -395,12 +395,16 @@ template <int BN>
 using UpdTile = dmma::WsTile<64, BN, 4, 1, 16, 3>;
 // CTAs per SM while the accumulators (and, for the narrow tiles, the columns of A
 // read ahead of the dot) leave registers: a narrow tile's CTA is short, and its
-// loads' latency is what it waits for
+// loads' latency is what it waits for. 200 pivots on 48^3 points with four CTAs against
+// three: 10.2 and 11.2 ms at p = 31, 13.4 and 14.4 at 38, 13.8 and 14.0 at 46; with three
+// against two: 35.3 and 39.2 at 94, 48.3 and 48.6 at 110, 76.0 and 59.0 at 126.
 template <int BN>
 struct UpdMinBlocks {
   static constexpr int value = BN <= 40 ? 4 : BN <= 96 ? 3 : 2;
 };
-constexpr int kUpdAhead = 40;  // widest tile whose columns of A are read ahead
+// Widest tile whose columns of A are read ahead: with and without 10.1 and 10.4 ms at
+// p = 31, 13.4 and 13.7 at 38, 14.4 and 14.0 at 46, 22.8 and 21.6 at 62.
+constexpr int kUpdAhead = 40;
 
 template <int BN, int MINB>
 __global__ void __launch_bounds__(UpdTile<BN>::THREADS, MINB)
