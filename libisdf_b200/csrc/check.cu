@@ -216,7 +216,7 @@ struct CheckBuffers {
   cufftDoubleComplex* spec;
   int* piv;
   double2* part;
-  int* err;  // a pipeline wait of a symmetric product ran out
+  int* err;  // WaitFlag's device word
 };
 
 constexpr int kBatch = 128;
@@ -240,10 +240,34 @@ CheckBuffers carve(Arena& a, long long ng, long long nh, int npair, int rk, int 
   return b;
 }
 
+// Where the symmetric products say that a pipeline wait ran out: a word of mapped host
+// memory, which costs nothing unless one does (a device word, cleared and read back,
+// took 9 us of a 700 us call), or the caller's device word where none can be mapped.
+struct WaitFlag {
+  volatile int* host = nullptr;
+  int* dev = nullptr;
+
+  int clear(int* device_word, cudaStream_t s) {
+    progress_words(&host, &dev);
+    if (host) {
+      *host = 0;
+    } else {
+      dev = device_word;
+      ISDF_CUDA(cudaMemsetAsync(dev, 0, sizeof(int), s));
+    }
+    return ISDF_OK;
+  }
+};
+
 // The status of the symmetric products queued so far (waits for s).
-int products_done(const int* d_err, cudaStream_t s) {
+int products_done(const WaitFlag& flag, cudaStream_t s) {
   int err = 0;
-  ISDF_TRY(read_back(&err, d_err, sizeof(int), s));
+  if (flag.host) {
+    ISDF_CUDA(cudaStreamSynchronize(s));
+    err = *flag.host;
+  } else {
+    ISDF_TRY(read_back(&err, flag.dev, sizeof(int), s));
+  }
   if (err) return record_error(ISDF_ERR_TIMEOUT, "Y Y^T: a pipeline wait timed out");
   return ISDF_OK;
 }
@@ -359,18 +383,19 @@ int check_run(const CheckArgs& args, Arena& arena, cudaStream_t s, double* fit_e
 
   // (ij|V|kl) = Y Y^T; A = Yz Yz^T; T^T = C^T A; ISDF form = C^T T
   const size_t nscratch = (size_t)ng * kBatch;  // the transforms are done with rho
-  ISDF_CUDA(cudaMemsetAsync(b.err, 0, sizeof(int), s));
+  WaitFlag flag;
+  ISDF_TRY(flag.clear(b.err, s));
   ISDF_TRY(dsyrk_store(npair, (int)(2 * nh), b.Y, npair, b.ijkl, npair, b.rho, nscratch,
-                       b.err, s));
+                       flag.dev, s));
   ISDF_TRY(dsyrk_store(rk, (int)(2 * nh), b.Yz, rk, b.aux, rk, b.rho, nscratch,
-                       b.err, s));
+                       flag.dev, s));
   ISDF_TRY(dgemm_store(npair, rk, rk, b.C, npair, b.aux, rk, b.Tt, npair, s));
   ISDF_TRY(dgemm_store(npair, npair, rk, b.C, npair, b.Tt, npair, b.cac, npair, s));
   k_diff_norms<<<kDiffBlocks, 256, 0, s>>>(b.ijkl, b.cac, (long long)npair * npair, b.part);
   ISDF_CHECK_LAUNCH();
   std::vector<double2> h(kDiffBlocks);
   ISDF_TRY(read_back(h.data(), b.part, sizeof(double2) * kDiffBlocks, s));
-  ISDF_TRY(products_done(b.err, s));
+  ISDF_TRY(products_done(flag, s));
   double e2 = 0, x2 = 0;
   for (auto& v : h) {
     e2 += v.x;
@@ -491,14 +516,15 @@ int check_sampled_run(const CheckArgs& args, const int* pairs, int ns, Arena& ar
   }
   *fit_err = std::sqrt(fe2) / std::sqrt(fr2);
   const size_t nscratch = (size_t)ng * kBatch;  // the transforms are done with rho
-  ISDF_CUDA(cudaMemsetAsync(b.err, 0, sizeof(int), s));
+  WaitFlag flag;
+  ISDF_TRY(flag.clear(b.err, s));
   ISDF_TRY(dsyrk_store(ns, (int)(2 * nh), b.Y, ns, b.E, ns, b.rho, nscratch,
-                       b.err, s));
+                       flag.dev, s));
   ISDF_TRY(dsyrk_store(ns, (int)(2 * nh), b.Yf, ns, b.Ef, ns, b.rho, nscratch,
-                       b.err, s));
+                       flag.dev, s));
   double ce2 = 0, cx2 = 0;
   ISDF_TRY(diff_norms(b.E, b.Ef, (long long)ns * ns, b.part, s, &ce2, &cx2));
-  ISDF_TRY(products_done(b.err, s));
+  ISDF_TRY(products_done(flag, s));
   *coul_err = std::sqrt(ce2) / std::sqrt(cx2);
   return ISDF_OK;
 }
@@ -588,8 +614,8 @@ int coulomb_matrix_workspace_bytes(const int* num_grid, int rk, size_t* bytes) {
   return ISDF_OK;
 }
 
-static int queue_coulomb_matrix(const int* num_grid, const double* length, const double* d_theta,
-                                int rk, double* d_A, Arena& arena, cudaStream_t s) {
+static int coulomb_matrix(const int* num_grid, const double* length, const double* d_theta, int rk,
+                          double* d_A, Arena& arena, cudaStream_t s) {
   const int nx = num_grid[0], ny = num_grid[1], nz = num_grid[2];
   const long long ng = (long long)nx * ny * nz;
   const long long nh = (long long)(nx / 2 + 1) * ny * nz;
@@ -629,20 +655,19 @@ static int queue_coulomb_matrix(const int* num_grid, const double* length, const
   ISDF_CHECK_LAUNCH();
   const long long K = 2 * nh;  // the GEMM's depth is an int
   if (K > (1LL << 30)) return record_error(ISDF_ERR_UNSUPPORTED, "Coulomb matrix: grid too large");
-  ISDF_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-  ISDF_TRY(dsyrk_store(rk, (int)K, Yz, ldy, d_A, rk, buf, (size_t)ng * kBatch, err, s));
-  return products_done(err, s);
+  WaitFlag flag;
+  ISDF_TRY(flag.clear(err, s));
+  ISDF_TRY(dsyrk_store(rk, (int)K, Yz, ldy, d_A, rk, buf, (size_t)ng * kBatch, flag.dev, s));
+  return products_done(flag, s);
 }
 
 // Finished when it returns, with an error too: the caller gives up the workspace
 // mutex then, and may not be able to wait on s (the library's own stream).
 int coulomb_matrix_run(const int* num_grid, const double* length, const double* d_theta, int rk,
                        double* d_A, Arena& arena, cudaStream_t s) {
-  const int rc = queue_coulomb_matrix(num_grid, length, d_theta, rk, d_A, arena, s);
-  const cudaError_t done = cudaStreamSynchronize(s);
-  ISDF_TRY(rc);
-  ISDF_CUDA(done);
-  return ISDF_OK;
+  const int rc = coulomb_matrix(num_grid, length, d_theta, rk, d_A, arena, s);
+  if (rc != ISDF_OK) (void)cudaStreamSynchronize(s);
+  return rc;
 }
 
 }  // namespace isdf_b200

@@ -43,8 +43,8 @@ int dgemm_store(int M, int N, int K, const double* A, long long lda, const doubl
                 long long ldb, double* C, long long ldc, cudaStream_t s);
 // C = Y Y^T (n x n, both triangles) for Y column-major n x K (ldy), through
 // `scratch`. The call does not synchronise: a bounded wait of its pipeline that
-// runs out sets *err (device, cleared by the caller, who reads it back). An odd n
-// takes the fast path with ldy > n, even.
+// runs out sets *err (writable by the device; cleared and looked at by the caller). An
+// odd n takes the fast path with ldy > n, even.
 int dsyrk_store(int n, int K, const double* Y, long long ldy, double* C, long long ldc,
                 double* scratch, size_t scratch_doubles, int* err, cudaStream_t s);
 // timed = false skips the stage timers (no CUDA events are created); the
