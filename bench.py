@@ -545,9 +545,9 @@ def run_ours(args, shape):
     if plain is not None or not mixed:
         # k_trsm_ws, the two triangular sweeps of the FP64 form as in-place FP64
         # tensor-core GEMMs: 2*Ng*rk^2 flops per solve over the stage's
-        # CUDA-event time (the k_trsm_ws launches plus the small k_build_w
-        # launches between them, so a slight underestimate of the kernel's
-        # own rate). DRAM traffic per launch: 8.40 B per grid row and solved
+        # CUDA-event time (the k_trsm_ws launches plus the four small launches
+        # that build the sweeps' panels, so a slight underestimate of the
+        # kernel's own rate). DRAM traffic per launch: 8.40 B per grid row and solved
         # column (ncu on the 40^3-grid case) x the mean solved width (rk/2 + 32).
         ach = 2.0 * ng * rk * rk / (solve_ms * 1e-3) / 1e12 if solve_ms > 0 else None
         roof64 = {"kernel": "k_trsm_ws (both sweeps of the FP64 triangular solve)",
@@ -568,13 +568,13 @@ def run_ours(args, shape):
         ops = 2 * 2.0 * ng * rk * (rk / 2 + 32) * S * (S + 1) / 2
         ach = ops / (gemm_ms * 1e-3) / 1e12 if gemm_ms > 0 else None
         # DRAM traffic per launch from ncu on the 40^3-grid case (Ng = 64000,
-        # rk = 4312, S = 6; mean of the two products): 8.855 GB read (the
+        # rk = 4312, S = 6; mean of the two products): 9.208 GB read (the
         # digits of both operands, B's re-read once per raster group, so
-        # ~ rows x rk^2) and 2.195 GB written (the FP64 output, rows x rk).
+        # ~ rows x rk^2) and 2.190 GB written (the FP64 output, rows x rk).
         # Reported only near that shape, where the scaling holds.
         if S == 6 and 0.8 <= rk / 4312 <= 1.25:
-            traffic = (8.855e9 * (ng / 64000) * (rk / 4312) ** 2 +
-                       2.195e9 * (ng / 64000) * (rk / 4312))
+            traffic = (9.208e9 * (ng / 64000) * (rk / 4312) ** 2 +
+                       2.190e9 * (ng / 64000) * (rk / 4312))
             traffic_note = ("bytes per launch (mean of the two products), scaled from the ncu "
                             "capture at Ng = 64000, rk = 4312: reads by rows x rk^2, writes "
                             f"by rows x rk; algorithmic {(ng * rk * (S + 8)) / 1e9:.1f} GB")
