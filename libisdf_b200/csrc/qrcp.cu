@@ -778,6 +778,7 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
     launch_early(k_recompute, kRecomputeGrid, 256, sizeof(double) * m, q, b.Ac, b.Bc, ld, p, b.Q,
                  m, kmax_cap, b.rec_list, b.pos, b.nu, b.nu0, b.st, b.rec_dots, b.best + ublocks);
   };
+  ISDF_CHECK_LAUNCH();
   Loop loop(s);
   if (kmax > 0) {
     // launched step by step, the nine launches of a step took the host longer than the

@@ -32,6 +32,17 @@ thread_local Mailbox tl_mailbox;
 
 constexpr size_t kMinMailbox = 64 << 10;
 
+// Mapped host memory and its device address, or false. A refusal's own error is
+// cleared, and no other: one of an earlier launch may be waiting to be seen.
+bool map_host(size_t bytes, void** host, void** dev) {
+  if (cudaHostAlloc(host, bytes, cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
+    if (cudaHostGetDevicePointer(dev, *host, 0) == cudaSuccess) return true;
+    cudaFreeHost(*host);
+  }
+  (void)cudaGetLastError();
+  return false;
+}
+
 }  // namespace
 
 void set_readback_mailbox(bool on) { tl_mailbox.enabled = on; }
@@ -44,16 +55,10 @@ void progress_words(volatile int** host, int** dev) {
   if (!m.enabled) return;
   if (!m.words) {
     void *h = nullptr, *d = nullptr;
-    if (cudaHostAlloc(&h, 2 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) ==
-        cudaSuccess) {
-      if (cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess) {
-        m.words = static_cast<int*>(h);
-        m.words_dev = static_cast<int*>(d);
-      } else {
-        cudaFreeHost(h);
-      }
+    if (map_host(2 * sizeof(int), &h, &d)) {  // else the caller asks the device
+      m.words = static_cast<int*>(h);
+      m.words_dev = static_cast<int*>(d);
     }
-    (void)cudaGetLastError();  // a refused mapping: the caller asks the device
   }
   *host = m.words;
   *dev = m.words_dev;
@@ -71,18 +76,12 @@ int read_back(void* dst, const void* dsrc, size_t bytes, cudaStream_t s) {
     }
     size_t cap = kMinMailbox;
     while (cap < bytes) cap *= 2;
-    void* h = nullptr;
-    if (cudaHostAlloc(&h, cap, cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
-      void* d = nullptr;
-      if (cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess) {
-        m.host = h;
-        m.dev = d;
-        m.cap = cap;
-      } else {
-        cudaFreeHost(h);
-      }
+    void *h = nullptr, *d = nullptr;
+    if (map_host(cap, &h, &d)) {  // else by copies
+      m.host = h;
+      m.dev = d;
+      m.cap = cap;
     }
-    (void)cudaGetLastError();  // a refused mapping falls back to copies
   }
   if (m.enabled && m.cap >= bytes) {
     const size_t n = bytes / 4;

@@ -72,3 +72,14 @@ def test_launches_ahead_of_a_loop_are_checked():
         text = open(os.path.join(CSRC, name)).read()
         assert len(re.findall(r"loop(?:\.|->)finish\(", text)) == \
             len(re.findall(r"loop(?:\.|->)start\(", text)) > 0
+
+
+def test_mapping_host_memory_clears_only_its_own_error():
+    """An earlier launch's error may be waiting to be seen when a host buffer is mapped:
+    only the branch of a refused mapping clears the last error."""
+    text = open(os.path.join(CSRC, "readback.cu")).read()
+    assert text.count("cudaGetLastError()") == 1
+    helper = text[text.index("bool map_host("):]
+    helper = helper[:helper.index("\n}\n")]
+    assert "return true;" in helper[:helper.index("cudaGetLastError()")]
+    assert text.count("cudaHostAlloc(") == 1
