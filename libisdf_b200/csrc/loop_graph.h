@@ -29,12 +29,12 @@ __device__ __forceinline__ void loop_over(const LoopSignal& sig) {
 }
 
 // Begins a kernel launched by launch_early (what no kernel of the loop writes may
-// be read before): waits for the whole of
-// the kernel before it and its writes, then lets the next kernel's blocks become
-// resident (they wait here in turn). Every block passes here before it reads,
-// writes or returns: a kernel that completed without waiting would let the next one
-// run ahead of the one before it. What follows reads its state through plain
-// pointers first, so that no read-only load moves above the wait.
+// be read before): waits for the whole of the kernel before it and its writes, then
+// lets the next kernel's blocks become resident (they wait here in turn). Every block
+// passes here before it reads, writes or returns: a kernel that completed without
+// waiting would let the next one run ahead of the one before it. What a kernel of the
+// loop writes is read through plain pointers: the block was resident while it was
+// written, so that it is no read-only data.
 __device__ __forceinline__ void after_previous() {
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();

@@ -781,8 +781,8 @@ int qrcp_select(const QrcpArgs& args, Arena& arena, cudaStream_t s, QrcpResult* 
   ISDF_CHECK_LAUNCH();
   Loop loop(s);
   if (kmax > 0) {
-    // launched step by step, the nine launches of a step took the host longer than the
-    // GPU at numPre = 31
+    // (launched one by one, the eight kernels of a step took the host longer than the
+    // GPU at numPre = 31)
     constexpr int kBodySteps = 4, kSlackSteps = 2, kAheadSteps = 8;
     ISDF_TRY(loop.start(std::min(kmax, kAheadSteps), step));
     ISDF_TRY(loop.finish(kmax, kBodySteps, kSlackSteps, step, [&](bool* over) -> int {
